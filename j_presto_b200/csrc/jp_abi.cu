@@ -170,7 +170,8 @@ void pack_ge(const jp_ge &g, double *dst) {
 }
 
 // ---- rebuild: cells + tiles -------------------------------------------------------------
-void enqueue_rebuild(jp_ctx *c) {
+// count_only: as far as the records per unit (the tuner needs no more)
+void enqueue_rebuild(jp_ctx *c, bool count_only = false) {
   DevPtrs &P = c->P;
   cudaStream_t st = c->st;
   const int nt = 256;
@@ -198,7 +199,6 @@ void enqueue_rebuild(jp_ctx *c) {
   k_fill_slots<<<(c->natom + nt - 1) / nt, nt, 0, st>>>(P, c->natom);
   k_excl_slots<<<(c->natom + nt - 1) / nt, nt, 0, st>>>(P, c->natom);
   k_block_setup<<<(c->nblk * 32 + nt - 1) / nt, nt, 0, st>>>(P, c->nblk, c->qscale);
-  if (c->fp64) k_fill_pos_d<<<(c->nslot + nt - 1) / nt, nt, 0, st>>>(P, c->nslot, c->qscale);
   const double rlim = c->zc.rlim;   // rc + 1.5; CMM: the farthest near-field pair
   const double rc = c->prm.cutoff;
   const int nwb = (c->nchunk * 32 + 127) / 128;
@@ -208,9 +208,10 @@ void enqueue_rebuild(jp_ctx *c) {
     nl += scan_exclusive(P.chunk_ent + h * (c->nchunk + 1), P.chunk_eoff + h * (c->nchunk + 1), c->nchunk + 1,
                          c->scan_scratch, nullptr, st);
   k_tile_emit<<<nwb, 128, 0, st>>>(P, c->nchunk, c->cmm ? 1 : 0);
-  nl += launch_compact_tiles(P, c->nblk, c->nchunk, c->nsm, c->cmm, c->scan_scratch, st);
+  nl += launch_compact_tiles(P, c->nblk, c->nchunk, c->nsm, c->cmm, c->zc.nt1 - 1, c->scan_scratch, count_only, st);
+  if (count_only) return;
   if (c->hbond) launch_hb_list(P, c->hb_cap, c->zc.nt1, c->nblk, st);
-  c->launches_rebuild = nl + (c->fp64 ? 1 : 0) + ncmm + (c->hbond ? 1 : 0);
+  c->launches_rebuild = nl + ncmm + (c->hbond ? 1 : 0);
 }
 
 // ---- one MD step ------------------------------------------------------------------------
@@ -384,7 +385,7 @@ int snap_copy(jp_ctx *c, Snap &S, bool to, int row) {
     CK(cp(S.acnt2, P.alsd_cnt2, n2 * sizeof(unsigned long long)));
     CK(cp(S.af2, P.alsd_f2, n2 * sizeof(double)));
   }
-  if (!to) launch_update_pos(P, c->nslot, c->fp64, c->qscale, c->st);
+  if (!to) launch_update_pos(P, c->natom, c->fp64, c->qscale, c->st);
   return 0;
 }
 
@@ -416,7 +417,7 @@ int snap_copy_rep(jp_ctx *c, Snap &S, bool to, int r) {
     CK(cp(S.acnt2 + r * n2, P.alsd_cnt2 + r * n2, n2 * sizeof(unsigned long long)));
     CK(cp(S.af2 + r * n2, P.alsd_f2 + r * n2, n2 * sizeof(double)));
   }
-  if (!to) launch_update_pos(P, c->nslot, c->fp64, c->qscale, c->st);
+  if (!to) launch_update_pos(P, c->natom, c->fp64, c->qscale, c->st);
   return 0;
 }
 
@@ -848,7 +849,7 @@ int tune_blocks(jp_ctx *c, bool tune) {
   for (int q = 0; q < (tune ? nq : 0); ++q) {
     for (int r = 0; r < c->nrep; ++r) set_grid(c->reps[r], c->tune_grid.data() + ((size_t)r * nq + q) * 2);
     CK(cudaMemcpy(c->P.reps, c->reps.data(), sizeof(Rep) * c->nrep, cudaMemcpyHostToDevice));
-    enqueue_rebuild(c);
+    enqueue_rebuild(c, true);
     CK(cudaMemcpyAsync(cnt.data(), c->P.ct_cnt, sizeof(int) * 2 * c->nblk, cudaMemcpyDeviceToHost, c->st));
     CK(cudaStreamSynchronize(c->st));
     int rs = check_status(c);
@@ -1560,9 +1561,9 @@ int jp_create(const jp_system *sys, int32_t nrep, const jp_params *prm, jp_ctx *
   e |= dput(c, &P.excl_ptr, hexp);
   e |= dput(c, &P.excl_idx, hexi);
   e |= dalloc(c, &P.excl_slot, hexi.size());
-  e |= dalloc(c, &P.pos_f, (size_t)c->nslot);
-  e |= dalloc(c, &P.pos_d, (size_t)c->nslot);
-  e |= dalloc(c, &P.off, 3 * (size_t)c->nslot);
+  e |= dalloc(c, &P.pos_f, (size_t)N);
+  e |= dalloc(c, &P.pos_d, (size_t)N);
+  e |= dalloc(c, &P.off, 3 * (size_t)N);
   e |= dalloc(c, &P.styp, (size_t)c->nslot);
   e |= dalloc(c, &P.satom, (size_t)c->nslot);
   e |= dput(c, &P.blk_rep, hblk_rep);
@@ -1576,23 +1577,21 @@ int jp_create(const jp_system *sys, int32_t nrep, const jp_params *prm, jp_ctx *
   e |= dalloc(c, &P.chunk_off, (size_t)c->nchunk + 1);
   e |= dalloc(c, &P.tmp_masks, (size_t)c->tile_cap_total * 32);
   e |= dalloc(c, &P.tiles, (size_t)c->tile_cap_total);
-  e |= dalloc(c, &P.tile_shift, (size_t)c->tile_cap_total);
   e |= dalloc(c, &P.tile_src, (size_t)c->tile_cap_total);
   // compact tiles: at most one per tile (an i-block's j entries never outnumber 32 per tile)
   e |= dput(c, &P.blk_chunk0, blk_chunk0);
   // pair records: at most one per tile and half (a unit's records never outnumber the tiles
-  // of its block), plus one so that the kernels' record pairs stay inside the arrays
-  const size_t rec_cap = 2 * (size_t)c->tile_cap_total + 2;
+  // of its block), plus padding so that the kernels' record groups (up to four) stay inside
+  const size_t rec_cap = 2 * (size_t)c->tile_cap_total + 4;
   e |= dalloc(c, &P.ct_cnt, 2 * (size_t)c->nblk + 1);
   e |= dalloc(c, &P.ct_off, 2 * (size_t)c->nblk + 1);
   e |= dalloc(c, &P.ct_blk, rec_cap);
-  e |= dalloc(c, &P.ct_info, rec_cap);
   e |= dalloc(c, &P.tmp_occ, (size_t)c->nchunk * 32 * 2);
   e |= dalloc(c, &P.chunk_ent, 2 * ((size_t)c->nchunk + 1));
   e |= dalloc(c, &P.chunk_eoff, 2 * ((size_t)c->nchunk + 1));
-  e |= dalloc(c, &P.tile_occ, 2 * (size_t)c->tile_cap_total);
   e |= dalloc(c, &P.tile_eoff, 2 * (size_t)c->tile_cap_total);
   e |= dalloc(c, &P.ct_j, rec_cap * 32);
+  e |= dalloc(c, &P.ct_ty, rec_cap * 32);
   e |= dalloc(c, &P.ct_mask, rec_cap * kHalf);
   e |= dalloc(c, &P.nctiles, 1);
   if (c->cmm) e |= dalloc(c, &P.ct_mask_el, rec_cap * kHalf);
@@ -1671,6 +1670,9 @@ int jp_create(const jp_system *sys, int32_t nrep, const jp_params *prm, jp_ctx *
   e |= dalloc(c, &P.temp_hist, (size_t)c->hist_cap * nrep);
   e |= dalloc(c, &P.step_ctr, 2);
   e |= dput(c, &P.lj_f, ljf);
+  std::vector<float> ljtab;
+  pack_lj_table(ljf.data(), nt1, ljtab);
+  e |= dput(c, &P.lj_tab, ljtab);
   e |= dput(c, &P.lj_d, ljd);
   e |= dput(c, &P.lj14, lj14);
   c->nres = (int)hres.size();
@@ -1751,7 +1753,7 @@ int jp_create(const jp_system *sys, int32_t nrep, const jp_params *prm, jp_ctx *
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, c->device);
   c->nsm = std::max(1, nsm);
   // one wave: every warp resident at once, each with an equal share of the tiles
-  c->pair_warps = std::max(1, nsm) * (256 / 32) * pair_blocks_per_sm(c->fp64, c->zc.nt1);
+  c->pair_warps = std::max(1, nsm) * (256 / 32) * pair_blocks_per_sm(c->fp64, !c->split && !c->cmm, c->zc.nt1);
   c->cano_grid = cano_grid(c->fp64, c->device);
   CK(cudaStreamCreateWithFlags(&c->st, cudaStreamNonBlocking));
   CK(cudaStreamCreateWithFlags(&c->st2, cudaStreamNonBlocking));
@@ -1759,6 +1761,7 @@ int jp_create(const jp_system *sys, int32_t nrep, const jp_params *prm, jp_ctx *
   CK(cudaEventCreateWithFlags(&c->ev_join, cudaEventDisableTiming));
   CK(cudaEventCreate(&c->ev_a));
   CK(cudaEventCreate(&c->ev_b));
+  if (c->fp64) launch_update_pos(P, N, true, c->qscale, c->st);   // the mixed path's: at each list build
   int rs = tune_blocks(c, prm->tune_blocks != 0);
   if (rs < 0) { jp_destroy(c); return rs; }
   *out = c;
@@ -1800,7 +1803,7 @@ int jp_set_state(jp_ctx *c, int32_t r, const double *cord, const double *vel) {
                                cudaMemcpyHostToDevice, c->st));
   if (vel) CK(cudaMemcpyAsync(c->P.v + 3 * (size_t)R.atom0, vel, sizeof(double) * 3 * R.natom,
                               cudaMemcpyHostToDevice, c->st));
-  if (cord) launch_update_pos(c->P, c->nslot, c->fp64, c->qscale, c->st);
+  if (cord) launch_update_pos(c->P, c->natom, c->fp64, c->qscale, c->st);
   CK(cudaStreamSynchronize(c->st));
   return JP_OK;
 }
@@ -1825,7 +1828,7 @@ int eval_forces(jp_ctx *c, int32_t r, const double *cord) {
   if (cord) {
     CK(cudaMemcpyAsync(c->P.x + 3 * (size_t)R.atom0, cord, sizeof(double) * 3 * R.natom,
                        cudaMemcpyHostToDevice, c->st));
-    launch_update_pos(c->P, c->nslot, c->fp64, c->qscale, c->st);
+    launch_update_pos(c->P, c->natom, c->fp64, c->qscale, c->st);
   }
   enqueue_forces(c, true, true);
   enqueue_bonded(c);
@@ -2219,7 +2222,7 @@ int jp_minimize(jp_ctx *c, const jp_min_params *mp, int32_t *iters, double *enev
     launch_shake_only(P, c->ic, 0, c->nunit, st);
     launch_min_commit(P, c->natom, nmax, st);
   }
-  launch_update_pos(P, c->nslot, c->fp64, c->qscale, st);
+  launch_update_pos(P, c->natom, c->fp64, c->qscale, st);
   enqueue_zero(c, false);
   enqueue_pair(c, false, true);   // CMM: the far field at every evaluation
   enqueue_bonded(c);
@@ -2509,7 +2512,7 @@ int jp_step_io(jp_ctx *c, int32_t nsteps, const double *cord_in, const double *v
   const size_t n3 = sizeof(double) * 3 * (size_t)c->natom;
   if (cord_in) CK(cudaMemcpyAsync(c->P.x, cord_in, n3, cudaMemcpyHostToDevice, c->st));
   if (vel_in) CK(cudaMemcpyAsync(c->P.v, vel_in, n3, cudaMemcpyHostToDevice, c->st));
-  if (cord_in) launch_update_pos(c->P, c->nslot, c->fp64, c->qscale, c->st);
+  if (cord_in) launch_update_pos(c->P, c->natom, c->fp64, c->qscale, c->st);
   if (nsteps == 0) {
     if (cord_out) CK(cudaMemcpyAsync(cord_out, c->P.x, n3, cudaMemcpyDeviceToHost, c->st));
     if (vel_out) CK(cudaMemcpyAsync(vel_out, c->P.v, n3, cudaMemcpyDeviceToHost, c->st));

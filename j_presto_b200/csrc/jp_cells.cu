@@ -146,27 +146,14 @@ __global__ void k_block_setup(DevPtrs P, int nblk, double qscale) {
     }
   }
   double o[3];
+  if (a < 0) return;
   for (int k = 0; k < 3; ++k) o[k] = ref[k] + R.box[k] * img[k];
-  P.off[3 * slot + 0] = o[0];
-  P.off[3 * slot + 1] = o[1];
-  P.off[3 * slot + 2] = o[2];
-  if (a >= 0) {
-    float q = (float)((double)qscale * P.chg[a]);
-    P.pos_f[slot] = make_float4((float)(P.x[3 * a] - o[0]), (float)(P.x[3 * a + 1] - o[1]),
-                                (float)(P.x[3 * a + 2] - o[2]), q);
-  } else {
-    P.pos_f[slot] = make_float4(0.f, 0.f, 0.f, 0.f);
-  }
-}
-
-// FP64 slot positions (absolute master coordinates) + charges; used every step by the FP64
-// path and after a rebuild by both paths.
-__global__ void k_fill_pos_d(DevPtrs P, int nslot, double qscale) {
-  int s = blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= nslot) return;
-  int a = P.satom[s];
-  if (a >= 0) P.pos_d[s] = make_double4(P.x[3 * a], P.x[3 * a + 1], P.x[3 * a + 2], qscale * P.chg[a]);
-  else P.pos_d[s] = make_double4(0.0, 0.0, 0.0, 0.0);
+  P.off[3 * a + 0] = o[0];
+  P.off[3 * a + 1] = o[1];
+  P.off[3 * a + 2] = o[2];
+  const float q = (float)((double)qscale * P.chg[a]);
+  P.pos_f[a] = make_float4((float)(P.x[3 * a] - o[0]), (float)(P.x[3 * a + 1] - o[1]),
+                           (float)(P.x[3 * a + 2] - o[2]), q);
 }
 
 // slot of every exclusion partner, refreshed after each sort: lets the tile build clear
@@ -278,7 +265,7 @@ __device__ __forceinline__ unsigned tile_row_f32(const DevPtrs& P, const Rep& R,
     const double d = P.blk_ref[3 * bi + k] - P.blk_ref[3 * bj + k];
     cj[k] = (float)(R.box[k] * anint(d * R.invbox[k]) - d);
   }
-  const float4 pj = P.pos_f[bj * kTile + lane];
+  const float4 pj = aj >= 0 ? P.pos_f[aj] : make_float4(0.f, 0.f, 0.f, 0.f);
   const float r[3] = {pj.x + cj[0], pj.y + cj[1], pj.z + cj[2]};
   unsigned live;
   if (PIMG) {   // every real i atom (padding slots sit at 1e18)
@@ -512,21 +499,13 @@ __global__ void k_tile_emit(DevPtrs P, int nchunk, int cmm) {
       if (lane >= o) e += y;
     }
     if (lane < cnt) {
-      P.tile_occ[2 * (size_t)(t0 + lane) + h] = occ;
       P.tile_eoff[2 * (size_t)(t0 + lane) + h] = P.chunk_eoff[h * (nchunk + 1) + w] + e - __popc(occ);
     }
   }
-  if (lane < cnt) {   // lane q: the chunk's q-th tile, its block pair and image shift
-    const Rep& R = P.reps[P.blk_rep[bi]];
+  if (lane < cnt) {   // lane q: the chunk's q-th tile and its block pair
     const int bj = j0 + (int)__fns(nz, 0, lane + 1);
     P.tiles[t0 + lane] = make_int2(bi, bj);
     P.tile_src[t0 + lane] = w * 32 + (bj - j0);   // its mask rows stay where the scan wrote them
-    float sh[3];
-    for (int k = 0; k < 3; ++k) {
-      const double d = P.blk_ref[3 * bi + k] - P.blk_ref[3 * bj + k];
-      sh[k] = (float)(d - R.box[k] * anint(d * R.invbox[k]));
-    }
-    P.tile_shift[t0 + lane] = make_float4(sh[0], sh[1], sh[2], 0.f);
   }
 }
 
@@ -539,7 +518,7 @@ __global__ void k_tile_emit(DevPtrs P, int nchunk, int cmm) {
 // span a smaller volume than 32 (within the cut-off: 32 % of the slots with whole blocks,
 // 39 % with half blocks), and the pair kernels' work per pair falls in proportion.  The
 // listed pair set is unchanged.  Each entry carries its tile's image shift (into the i
-// block's frame) and its slot; the mask of i atom l (0..15) has bit k = entry (l + k) & 15
+// block's frame) and its atom, with the atom's type beside it; the mask of i atom l (0..15) has bit k = entry (l + k) & 15
 // and bit 16 + k = entry 16 + ((l + k) & 15), the order in which the kernels meet them.
 
 // tiles of i-block bi: [chunk_off[blk_chunk0[bi]], chunk_off[blk_chunk0[bi + 1]]); the
@@ -576,7 +555,9 @@ __global__ void k_ct_index(DevPtrs P, int nchunk) {
       const int u = 2 * b + h;
       for (int k = (lo + 31) >> 5; 32 * k < hi; ++k) {
         P.ct_blk[P.ct_off[u] + k] = u;
-        P.ct_info[P.ct_off[u] + k] = make_int4(t, e0 + 32 * k, eoff[c1], ((tl + 1) << 1) | h);
+        // kept in the record's own entry space until the emit, which fills that
+        reinterpret_cast<int4*>(P.ct_j)[(size_t)(P.ct_off[u] + k) * 32] =
+            make_int4(t, e0 + 32 * k, eoff[c1], ((tl + 1) << 1) | h);
       }
     }
   }
@@ -592,19 +573,20 @@ __device__ __forceinline__ unsigned record_row(unsigned row, int l) {
 }
 
 // One warp per record, lane p for slot p.  The record's source tiles are consecutive from
-// ct_info's first tile and at most 32 (each holds at least one entry and the first covers
+// k_ct_index's first tile and at most 32 (each holds at least one entry and the first covers
 // slot 0), so lane q reads source tile q's entry offset, occupancy, j block, image shift and
 // mask rows' place in one coalesced pass; each slot finds its tile and its rank among the
 // tile's entries by shuffles, and writes its entry.  Record row r (i atom 16 h + r) is then
 // one ballot: every slot contributes the bit of its j lane in row 16 h + r of its tile, so no
 // lane packs bits and lane r keeps row r.
-__global__ void k_ct_emit(DevPtrs P, int nchunk, int cmm) {
+__global__ void k_ct_emit(DevPtrs P, int nchunk, int cmm, int dummy_type) {
   const unsigned full = 0xffffffffu;
   const int lane = threadIdx.x & 31;
   const int nw = (gridDim.x * blockDim.x) >> 5;
   const int T = *P.nctiles;
   for (int ct = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; ct < T; ct += nw) {
-    const int4 info = P.ct_info[ct];
+    const int4 info = reinterpret_cast<const int4*>(P.ct_j)[(size_t)ct * 32];   // k_ct_index's
+    __syncwarp();   // read by every lane before the entries overwrite it
     const int ts = info.x, s0 = info.y, e1 = info.z, t1 = info.w >> 1, h = info.w & 1;
     const int tq = ts + lane;   // lane q: source tile q
     int qb = 32, qy = 0, qs = 0;
@@ -613,10 +595,17 @@ __global__ void k_ct_emit(DevPtrs P, int nchunk, int cmm) {
     if (tq < t1) {
       qb = P.tile_eoff[2 * (size_t)tq + h] - s0;   // slot of the tile's first entry (may be < 0)
       if (qb < 32) {
-        qocc = P.tile_occ[2 * (size_t)tq + h];
-        qy = P.tiles[tq].y;
-        qsh = P.tile_shift[tq];
         qs = P.tile_src[tq];
+        qocc = P.tmp_occ[2 * (size_t)qs + h];
+        const int2 ij = P.tiles[tq];
+        qy = ij.y;
+        const Rep& R = P.reps[P.blk_rep[ij.x]];   // image shift of block j into the i block's frame
+        float sh[3];
+        for (int k = 0; k < 3; ++k) {
+          const double d = P.blk_ref[3 * ij.x + k] - P.blk_ref[3 * ij.y + k];
+          sh[k] = (float)(d - R.box[k] * anint(d * R.invbox[k]));
+        }
+        qsh = make_float4(sh[0], sh[1], sh[2], 0.f);
       }
     }
     const int nt = __popc(__ballot_sync(full, tq < t1 && qb < 32));   // lanes 0 .. nt-1
@@ -640,8 +629,14 @@ __global__ void k_ct_emit(DevPtrs P, int nchunk, int cmm) {
     const bool live = src >= 0 && s0 + lane < e1;
     const int jl = live ? (int)__fns(socc, 0, kk + 1) : 0;   // the slot's j lane in its tile
     float4 ent = make_float4(0.f, 0.f, 0.f, __int_as_float(-1));
-    if (live) ent = make_float4(shx, shy, shz, __int_as_float(sy * kTile + jl));
+    int ty = dummy_type;
+    if (live) {
+      const int slot = sy * kTile + jl;
+      ent = make_float4(shx, shy, shz, __int_as_float(P.satom[slot]));
+      ty = P.styp[slot];
+    }
     P.ct_j[(size_t)ct * 32 + lane] = ent;
+    P.ct_ty[(size_t)ct * 32 + lane] = type_half(ty);
     // record row r (bit p: slot p) is one ballot: slot p's bit is bit jl of row 16 h + r of its
     // source tile (stored rotated: bit k is j lane (row + k) & 31); lane r keeps row r
     {
@@ -672,13 +667,14 @@ __global__ void k_ct_emit(DevPtrs P, int nchunk, int cmm) {
   }
 }
 
-int launch_compact_tiles(const DevPtrs& P, int nblk, int nchunk, int nsm, bool cmm, int* scan_scratch,
-                         cudaStream_t st) {
+int launch_compact_tiles(const DevPtrs& P, int nblk, int nchunk, int nsm, bool cmm, int dummy_type,
+                         int* scan_scratch, bool count_only, cudaStream_t st) {
   const int nb = (2 * nblk + 127) / 128;
   k_ct_count<<<nb, 128, 0, st>>>(P, nblk, nchunk);
+  if (count_only) return 1;
   const int ns = scan_exclusive(P.ct_cnt, P.ct_off, 2 * nblk + 1, scan_scratch, P.nctiles, st);
   k_ct_index<<<nsm * 4, 256, 0, st>>>(P, nchunk);
-  k_ct_emit<<<nsm * 8, 256, 0, st>>>(P, nchunk, cmm ? 1 : 0);
+  k_ct_emit<<<nsm * 8, 256, 0, st>>>(P, nchunk, cmm ? 1 : 0, dummy_type);
   return 3 + ns;
 }
 

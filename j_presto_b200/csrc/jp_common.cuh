@@ -5,10 +5,10 @@
 //   atoms : x, v      double[N][3]   master FP64 state (cord, vel of md_run)
 //           frc       long long[N][3] 64-bit fixed-point gradient (mixed path)
 //           grd       double[N][3]   FP64 gradient (FP64 path)
-//   slots : pos_f     float4[S]      (x-off, y-off, z-off, q*sqrt(332/eps)) block-local
-//           pos_d     double4[S]     (x, y, z, q*sqrt(332/eps)) absolute (FP64 path)
-//           off       double[S][3]   block frame origin of the slot (ref + L*image)
-//           styp      int[S]         LJ type (padding -> dummy zero type)
+//           pos_f     float4[N]      (x-off, y-off, z-off, q*sqrt(332/eps)) block-local
+//           pos_d     double4[N]     (x, y, z, q*sqrt(332/eps)) absolute (FP64 path)
+//           off       double[N][3]   frame origin of the atom's block (ref + L*image)
+//   slots : styp      int[S]         LJ type (padding -> dummy zero type)
 //           satom     int[S]         atom of the slot, -1 for padding
 //   blocks: 32 slots each; tiles = (i-block, j-block) pairs with a 32x32 interaction mask.
 #pragma once
@@ -113,6 +113,13 @@ __host__ __device__ __forceinline__ double cls_weight(const Rep& R, double lam, 
 constexpr int kTypeMask = 0xffff;
 constexpr int kRegionShift = 28;
 
+// a type word in 16 bits, as the pair records carry it: type (below 4,096, far above the types
+// whose pair table fits shared memory), region code in bits 12-13, cluster in bit 14
+__device__ __forceinline__ unsigned short type_half(int t) {
+  return (unsigned short)((t & 0xfff) | ((t >> 16) & 0x7000));
+}
+__device__ __forceinline__ int type_word(unsigned short h) { return (h & 0xfff) | ((h & 0x7000) << 16); }
+
 // integration unit: a SHAKE group (2-4 atoms) or a lone atom (n = 1)
 struct Unit {
   int n;
@@ -172,10 +179,10 @@ struct DevPtrs {
   // exclusions (global atom ids)
   int *excl_ptr, *excl_idx;
   int *excl_slot;                 // slot of each partner after the last sort
-  // slots / blocks
-  float4 *pos_f;
-  double4 *pos_d;
+  float4 *pos_f;                  // kernel positions, by atom: the integration writes them in
+  double4 *pos_d;                 // atom order and the pair kernels gather them by atom
   double *off;
+  // slots / blocks
   int *styp, *satom;
   int *blk_rep;
   float4 *blk_ctr, *blk_half;     // bbox (wrapped frame) centre / half extent
@@ -187,21 +194,21 @@ struct DevPtrs {
   unsigned *tmp_masks;            // [nchunk*32][32] masks of the chunk candidates
   // tiles
   int2 *tiles;                    // dense (i-block, j-block)
-  float4 *tile_shift;             // dense min-image shift of block refs (mixed path)
   int *tile_src;                  // [T] where each tile's mask rows are in tmp_masks: chunk * 32 + candidate
   int *ntiles;                    // device scalar
   // compact tiles (what the pair kernels run on): an i-block and 32 j entries
   int *blk_chunk0;                // [nblk+1] first chunk of each i-block (static)
   int *ct_cnt, *ct_off;           // pair records per unit (2 i-block + half) and their scan [2 nblk+1]
   int *ct_blk;                    // [CT] unit of each pair record
-  int4 *ct_info;                  // [CT] what the emit needs of each record: its first source tile,
-                                  // the global entry of its slot 0, the end of its unit's entries,
-                                  // and (end of its block's tiles) << 1 | half
   unsigned *tmp_occ;              // [nchunk*32][2] occupied j lanes of each chunk candidate, per half
   int *chunk_ent, *chunk_eoff;    // per half [2][nchunk+1]: entries per chunk, their exclusive scan
-  unsigned *tile_occ;             // [T][2] occupied j lanes of each tile, per half
   int *tile_eoff;                 // [T][2] first entry of each tile in its half's order (global)
-  float4 *ct_j;                   // [CT][32] (image shift into the i frame, slot bits; -1 = empty)
+  float4 *ct_j;                   // [CT][32] (image shift into the i frame, atom bits; -1 = empty).
+                                  // Between k_ct_index and the emit, entry 0 holds what the emit
+                                  // needs: the record's first source tile, the global entry of its
+                                  // slot 0, the end of its unit's entries, and (end of its block's
+                                  // tiles) << 1 | half
+  unsigned short *ct_ty;          // [CT][32] type word of each entry (type_half; empty: dummy type)
   unsigned *ct_mask, *ct_mask_el; // [CT][32] rotated masks (listed pairs; CMM Coulomb pairs)
   int *nctiles;                   // device scalar
   // cell sort
@@ -260,6 +267,7 @@ struct DevPtrs {
   // LJ tables [(nt+1)^2]: the pair kernels' (C6, C12), zero for H-bond type pairs; the
   // 1-4 terms' (C6, C12) of every type pair
   float2 *lj_f;
+  float *lj_tab;                  // the packed pair kernel's LJ table (pack_lj_table)
   double2 *lj_d;
   double2 *lj14;
   // H-bond 10-12 term: (C10, C12h) and flag per type pair, flag per type; the listed

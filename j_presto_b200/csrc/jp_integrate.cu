@@ -318,18 +318,18 @@ __device__ __forceinline__ void add_kin(const DevPtrs& P, int nsub_total, int ks
   }
 }
 
+// an atom's new position in the pair kernels' arrays
 __device__ __forceinline__ void write_slot(const DevPtrs& P, int a, const double* x, bool fp64) {
-  const int s = P.slot_of[a];
   if (fp64) {
-    double4 p = P.pos_d[s];
+    double4 p = P.pos_d[a];
     p.x = x[0]; p.y = x[1]; p.z = x[2];
-    P.pos_d[s] = p;
+    P.pos_d[a] = p;
   } else {
-    float4 p = P.pos_f[s];
-    p.x = (float)(x[0] - P.off[3 * s]);
-    p.y = (float)(x[1] - P.off[3 * s + 1]);
-    p.z = (float)(x[2] - P.off[3 * s + 2]);
-    P.pos_f[s] = p;
+    float4 p = P.pos_f[a];
+    p.x = (float)(x[0] - P.off[3 * a]);
+    p.y = (float)(x[1] - P.off[3 * a + 1]);
+    p.z = (float)(x[2] - P.off[3 * a + 2]);
+    P.pos_f[a] = p;
   }
 }
 
@@ -1011,17 +1011,17 @@ __global__ void __launch_bounds__(64) k_micr_fused(DevPtrs P, IntConst c, int nu
 // between two loads holds the later load back until the store's own inputs have arrived, and
 // a unit would wait for memory once per atom component instead of once.
 
-// an atom's slot record, read ahead of the position update that rewrites it (write_slot)
+// an atom's kernel-position record, read ahead of the update that rewrites it (write_slot)
 struct SlotRef {
-  int s;
+  int s;            // the atom
   float w;          // the mixed path's scaled charge (pos_f.w)
-  double o[3];      // the mixed path's block frame origin of the slot
+  double o[3];      // the mixed path's block frame origin
   double w64;       // the FP64 path's scaled charge (pos_d.w)
 };
 
 template <bool FP64>
 __device__ __forceinline__ void slot_load(const DevPtrs& P, int a, SlotRef& r) {
-  r.s = P.slot_of[a];
+  r.s = a;
   if (FP64) {
     r.w64 = P.pos_d[r.s].w;
   } else {

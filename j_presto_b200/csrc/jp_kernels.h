@@ -1,5 +1,7 @@
 // jp_kernels.h -- kernel entry points shared between the engine's translation units.
 #pragma once
+#include <vector>
+
 #include "jp_common.cuh"
 
 namespace jp {
@@ -13,15 +15,15 @@ __global__ void k_clear_slots(DevPtrs P, int nslot, int dummy_type);
 __global__ void k_fill_slots(DevPtrs P, int natom);
 __global__ void k_excl_slots(DevPtrs P, int natom);
 __global__ void k_block_setup(DevPtrs P, int nblk, double qscale);
-__global__ void k_fill_pos_d(DevPtrs P, int nslot, double qscale);
 // CMM: masks from the level-1 cells (neighbours: Coulomb + LJ into masks and masks_el;
 // cells up to idelay apart and r^2 < rc2: LJ only) instead of the list radius
 void launch_tile_scan(const DevPtrs& P, int nchunk, double rlim2, float rlimf, double rc2, bool cmm,
                       cudaStream_t st);
 __global__ void k_tile_emit(DevPtrs P, int nchunk, int cmm);
-// compact tiles of every i-block from the tile list (count, scan, emit); returns the launches
-int launch_compact_tiles(const DevPtrs& P, int nblk, int nchunk, int nsm, bool cmm, int* scan_scratch,
-                         cudaStream_t st);
+// pair records of every i-block from the tile list (count, scan, emit; with count_only the
+// records per unit alone); returns the launches
+int launch_compact_tiles(const DevPtrs& P, int nblk, int nchunk, int nsm, bool cmm, int dummy_type,
+                         int* scan_scratch, bool count_only, cudaStream_t st);
 // deterministic exclusive scan of n ints (total: the sum, or null); returns the launches
 int scan_exclusive(const int* in, int* out, int n, int* scratch, int* total, cudaStream_t st);
 
@@ -48,8 +50,11 @@ void launch_pair_mixed(const DevPtrs& P, const ZdConst& z, int nwarps, bool coun
 void launch_pair_fp64(const DevPtrs& P, const ZdConst& z, int nwarps, bool count, bool alsd, bool split,
                       cudaStream_t st);
 // co-resident blocks per SM of the (non-counting) pair kernel: the grid is one full wave
-int pair_blocks_per_sm(bool fp64, int nt1);
-void launch_update_pos(const DevPtrs& P, int nslot, bool fp64, double qscale, cudaStream_t st);
+// (packed: the mixed path without CMM and partial McMD)
+int pair_blocks_per_sm(bool fp64, bool packed, int nt1);
+// LJ table of the packed kernel (DevPtrs::lj_tab) from the type-pair (C6, C12)
+void pack_lj_table(const float2* lj, int nt1, std::vector<float>& out);
+void launch_update_pos(const DevPtrs& P, int natom, bool fp64, double qscale, cudaStream_t st);
 
 // H-bond 10-12 pairs (jp_hbond.cu): their list at a rebuild (after the tile list), their
 // term at every force evaluation

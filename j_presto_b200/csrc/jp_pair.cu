@@ -10,25 +10,27 @@
 //
 // Work unit: a pair record (jp_cells.cu) = half an i-block (16 cell-sorted atoms) and 32 j
 // entries (j atoms with at least one listed pair in the half block, each with the image
-// shift of its block) with an interaction mask fixed at list-build time.  One warp takes two
-// consecutive records, a half-warp each: lane l (l < 16 of its half) holds i atom l and at
-// step k (k < 16) meets entries a = (l + k) & 15 and b = 16 + a; the j-force accumulators of
-// a and b rotate one lane per step inside the half-warp (warp shuffles), so after 16 steps
-// lane l holds those of entries l and 16 + l, the ones it gathered.  Newton's third law:
-// each unordered pair is evaluated once.
+// shift of its block) with an interaction mask fixed at list-build time.  Newton's third
+// law: each unordered pair is evaluated once.
 //
-// Warps take short runs of consecutive record pairs from a global counter, so all finish
-// together whatever their records hold.
-// Mixed path: FP32 pair arithmetic on block-local coordinates (|x| < ~30 A), every step of a
+// Mixed path, k_pair_packed (plain and ALSD contexts): a warp takes four consecutive records,
+// eight lanes each; a lane holds two i atoms (l and l + 8 of its record) and meets one j entry
+// per step, two pairs in packed FP32x2 arithmetic.  k_pair_mixed (CMM and partial McMD): two
+// records, a half-warp each, one i atom a lane, the two entries of a step in scalar
+// arithmetic.  FP32 pair arithmetic on block-local coordinates (|x| < ~30 A), every step of a
 // record branch-free (a pair outside the mask or the cut-off contributes an exact zero);
 // forces summed per record in FP32, energies in FP32 over 4 steps then in FP64, both added
 // as 64-bit fixed point (2^-32 kcal/mol/A) with integer atomics -- order independent, so
-// results are bit-identical run to run.  A warp keeps two record pairs in flight ahead of
-// the one it computes: the bulk-copy engine (cp.async.bulk, completion on an mbarrier)
-// brings the entries and masks of the pair after next into shared memory, and the gathers
-// of the next pair's j atoms are issued before the current pair's arithmetic.
+// results are bit-identical run to run.  Warps take short runs of consecutive record groups,
+// the first by their own index and the next from a global counter, so all finish together
+// whatever their records hold.  A warp keeps two groups in flight ahead of the one it
+// computes: the bulk-copy engine (cp.async.bulk, completion on an mbarrier) brings the
+// entries and masks of the group after next into shared memory, and the gathers of the next
+// group's j atoms are issued before the current group's arithmetic.
 // FP64 path: the same records in FP64 with absolute coordinates, per-pair minimum image and
 // FP64 force atomics.
+#include <vector>
+
 #include "jp_kernels.h"
 
 namespace jp {
@@ -83,14 +85,15 @@ __device__ __forceinline__ bool mbar_wait(unsigned long long* bar, unsigned pari
   }
 }
 
-// each half-warp's energies (ELE15, VDW15; ALSD class AA / AB, BB the rest) and pair count
+// each lane group's energies (ELE15, VDW15; ALSD class AA / AB, BB the rest) and pair count
 // into the slots of its replica: 64-bit fixed point, summed per record, so the totals do not
 // depend on which warp took which record (the kernels claim their records dynamically).  The
-// two halves of a warp may work for different replicas: the sums stay inside each half.
+// W-lane groups of a warp may work for different replicas: the sums stay inside each group.
+template <int W>
 __device__ __forceinline__ void flush_fix(const DevPtrs& P, int rep, long long eel, long long elj,
                                           long long eaa, long long eab, long long npair, bool count,
                                           bool alsd) {
-  for (int o = 8; o > 0; o >>= 1) {
+  for (int o = W / 2; o > 0; o >>= 1) {
     eel += __shfl_xor_sync(0xffffffffu, eel, o);
     elj += __shfl_xor_sync(0xffffffffu, elj, o);
     if (alsd) {
@@ -99,7 +102,7 @@ __device__ __forceinline__ void flush_fix(const DevPtrs& P, int rep, long long e
     }
     if (count) npair += __shfl_xor_sync(0xffffffffu, npair, o);
   }
-  if ((threadIdx.x & 15) == 0 && rep >= 0) {
+  if ((threadIdx.x & (W - 1)) == 0 && rep >= 0) {
     atomic_add_ll(&P.ene_fix[rep * 16 + JP_E_ELE15], eel);
     atomic_add_ll(&P.ene_fix[rep * 16 + JP_E_VDW15], elj);
     if (alsd) {
@@ -112,7 +115,7 @@ __device__ __forceinline__ void flush_fix(const DevPtrs& P, int rep, long long e
   }
 }
 
-// Per-warp shared memory of the mixed kernel: two bulk-copy buffers (entries and masks of a
+// Per-warp shared memory of k_pair_mixed: two bulk-copy buffers (entries and masks of a
 // record pair: record 0 in entries 0-31 and masks 0-15, record 1 in 32-63 and 16-31) and the
 // staged j atoms of the pair being computed.  Half-warp h stages its record at [32 h, 32 h +
 // 32): lane l's entries a = l and b = 16 + l side by side, stored twice (at 32 h + l and
@@ -123,7 +126,7 @@ struct __align__(16) MixStage {
   unsigned msk_el[2][32];
   float4 p2[64];      // x_a, x_b, y_a, y_b
   float4 q2[64];      // z_a, z_b, q_a, q_b
-  int2 t2[64];        // their LJ type words (with TRI: x = the type-triple index a * nt1 + b)
+  int2 t2[64];        // their LJ type words
   unsigned long long bar[2];
 };
 
@@ -148,97 +151,484 @@ __device__ __forceinline__ float rint1(float v) {
   return __fadd_rn(__fadd_rn(v, 12582912.f), -12582912.f);
 }
 
-// One record, two pairs per step in packed FP32x2 arithmetic (Blackwell's FFMA2 / FADD2 /
-// FMUL2): at step k (k < 16) lane l of the half-warp meets entries a = (l + k) & 15 and
-// b = 16 + a, staged at sidx + k (sidx = 32 h + l).  A slot outside the mask or the cut-off
-// takes r^2 = 1e30 (its r^-6 = 1e-90 is zero in FP32) and a zero charge product, so it
-// contributes an exact zero without a branch.  The j-force accumulators of a and b move one
-// lane per step (from lane src = l + 1 of the same half); after 16 steps lane l holds those
-// of entries l and 16 + l, returned in (gja, gjb).  Energies in FP32 over 4 steps, then FP64.
-// TRI: the LJ parameters of both pairs come from one 16-byte record of the type-triple
-// table (i type, a type, b type) -> (C6_a, C6_b, C12_a, C12_b), indexed by row3 (the i type)
-// plus the staged a * nt1 + b; else from two type-pair records.
-template <bool MINIMG, bool COUNT, bool TRI>
-__device__ __forceinline__ void tile_mixed2(const MixStage& S, const float2* __restrict__ s_lj,
-                                            const float4* __restrict__ s_lj3, int row,
-                                            float4 pi, unsigned m, int sidx, int src, float bx, float by,
-                                            float bz, float ibx, float iby, float ibz, float rc2, float zb,
-                                            float zf, float zc, float& fix, float& fiy, float& fiz,
-                                            float3& gja, float3& gjb, double& te, double& tl, int& tn) {
+// The last flush of a block's warps: their sums are added in shared memory first and reach the
+// slots as one atomic per block and slot.  Every warp of a single-system launch adds to the
+// same two addresses, and L2 takes atomics on one address one after the other: with one pair
+// of them per lane group (19,000 atomics) a launch on 24,000 atoms took 59.1 us, so 52.0.
+// Called by all threads of the block.
+template <int W>
+__device__ __forceinline__ void flush_block(const DevPtrs& P, int rep, long long eel, long long elj, long long npair,
+                                            bool count, bool cls) {
+  __shared__ long long s_sum[kPairWarps][3];
+  __shared__ int s_rep[kPairWarps];
   const unsigned full = 0xffffffffu;
-  const float2 m1 = make_float2(-1.f, -1.f);
-  const float2 px = make_float2(pi.x, pi.x), py = make_float2(pi.y, pi.y), pz = make_float2(pi.z, pi.z);
-  const float2 pw = make_float2(pi.w, pi.w);
-  const float2 zb2 = make_float2(zb, zb), mzc = make_float2(-zc, -zc), mzf = make_float2(-zf, -zf);
-  const float2 c12 = make_float2(12.f, 12.f), cm6 = make_float2(-6.f, -6.f);
-  float2 fx = make_float2(0.f, 0.f), fy = fx, fz = fx;   // i force, a and b halves (sign: -sum)
-  float2 gx = fx, gy = fx, gz = fx;                      // j forces of the a and b entries
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  int r = __reduce_max_sync(full, rep);
+  if (!__all_sync(full, rep < 0 || rep == r)) {   // lane groups of several replicas
+    flush_fix<W>(P, rep, eel, elj, 0, 0, npair, count, cls);
+    r = -1;
+  }
+  for (int o = 16; o > 0; o >>= 1) {
+    eel += __shfl_xor_sync(full, eel, o);
+    elj += __shfl_xor_sync(full, elj, o);
+    if (count) npair += __shfl_xor_sync(full, npair, o);
+  }
+  if (lane == 0) {
+    s_rep[warp] = r;
+    s_sum[warp][0] = eel;
+    s_sum[warp][1] = elj;
+    s_sum[warp][2] = count ? npair : 0;
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int w = 0; w < kPairWarps; ++w) {
+      const int rw = s_rep[w];
+      if (rw < 0) continue;
+      long long a = 0, b = 0, n = 0;   // the warps of this replica, taken together
+      for (int v = w; v < kPairWarps; ++v)
+        if (s_rep[v] == rw) {
+          a += s_sum[v][0];
+          b += s_sum[v][1];
+          n += s_sum[v][2];
+          s_rep[v] = -1;
+        }
+      atomic_add_ll(&P.ene_fix[rw * 16 + JP_E_ELE15], a);
+      atomic_add_ll(&P.ene_fix[rw * 16 + JP_E_VDW15], b);
+      if (cls) atomic_add_ll(&P.ene_cls[rw * 4 + 2], a + b);
+      if (count) atomic_add_ll(&P.pair_cnt[rw], n);
+    }
+  }
+}
+
+// ---- packed kernel: four records a warp, eight lanes and two i atoms a lane -----------------
+// In ALSD contexts (CLS) a group whose records hold no cluster atom takes the plain loop; the
+// others add class weights and class energies to it (32 replicas of 9,100 atoms with four
+// cluster residues each: 897 us with the classes in every record, 686 so).
+// Per-warp shared memory: two bulk-copy buffers (entries, their atoms and types, and masks of a
+// record group: record q in entries 32 q and masks 16 q), and the staged j atoms of the group
+// being computed.  The position of entry 8 g + e of record q is staged twice, at 64 q + 16 g + e
+// and 8 further on, so that step k of group g reads slot 64 q + 16 g + l + k at a constant
+// offset (l: lane in the record); its type moves from lane to lane instead (a shuffle costs
+// the pipe what a 4-byte read does).
+struct __align__(16) QuadStage {
+  float4 ent[2][128];
+  unsigned short ty[2][128];
+  unsigned msk[2][64];
+  float4 p[256];            // x, y, z in the i block's frame, scaled charge
+  int2 at[4 * 36];          // (atom, type word) of entry 8 g + e at 36 q + 8 g + e
+  // of each record's replica: box edges and their inverses (per-pair images), class weights
+  // BB, AB, AA (ALSD); read where a group needs them, which spares registers in the others
+  float rep[4][12];
+  unsigned long long bar[2];
+};
+
+// a record's mask word of i atom r (entry halves rotated right by r, jp_cells.cu) in this
+// kernel's order: bit 8 g + k is entry 8 g + ((l + k) & 7), l = r & 7
+__device__ __forceinline__ unsigned byte_rotr(unsigned row, int l) {
+  const unsigned m = (0xffu >> l) * 0x01010101u;
+  return ((row >> l) & m) | ((row << (8 - l)) & ~m);
+}
+
+__device__ __forceinline__ unsigned step_mask(unsigned w, int r) {
+  const unsigned lo = __byte_perm(w, 0, 0x1010), hi = __byte_perm(w, 0, 0x3232);
+  return byte_rotr(((lo << r) >> 16) | ((hi << r) & 0xffff0000u), r & 7);
+}
+
+// what the inner loop reads of a lane's replica and classes
+struct PackedArgs {
+  float2 nx, ny, nz, qi;                 // minus the two i positions, their charges
+  unsigned ma, mb;                       // their mask words (step_mask order)
+  float rc2, zb, zf, zc;
+  // ALSD classes (CLS): cluster bits of the entries (step order) and of the i atoms, class
+  // weights of a pair with a plain (0) or a cluster (1) entry
+  unsigned jc;
+  bool ca, cb;
+  float2 w0, w1;
+};
+
+// One record: four groups of eight entries; at step k of group g lane l meets entry
+// 8 g + ((l + k) & 7) with its two i atoms, the pairs side by side in packed FP32x2 arithmetic
+// (Blackwell's FFMA2 / FADD2 / FMUL2).  A pair outside the mask or the cut-off takes r^2 = 1e30
+// (its r^-6 = 1e-90 is zero in FP32) and a zero charge product, so it contributes an exact
+// zero without a branch.  The j-force accumulator moves one lane a step (from lane src = l + 1
+// of the record) and after a group's eight steps lane l holds entry (l + 7) & 7, whose atom it
+// adds to.  LJ from (-6 C6, 12 C12): with p = 12 C12 r^-6 the force factor is (p - 6 C6) r^-8
+// and six times the energy (p / 2 - 6 C6) r^-6.
+// Why two i atoms a lane: the shared-memory and shuffle pipe (one 128-byte wavefront a cycle
+// per SM) bounds the loop.  A step of 64 pairs reads one j position (4 wavefronts), one type
+// (1), one LJ record (4) and shuffles one force (3): 12, where one i atom and two entries a
+// lane took 20 (two positions, two forces).  Measured on 64 replicas (883,000 atoms): 1,612 us with
+// one i atom a lane, 1,494 so; 190 and 179 us on 99,200 atoms, 59 and 52 us on 22,700.  Now 59 % of the issue slots and
+// 70 % of that pipe are busy (24 % of it staging, 17 % the force atomics), the FMA pipe 45 %.
+// Half or quarter groups as work units of small lists measured slower (the per-record work).
+template <bool MINIMG, bool COUNT, bool TRI, bool CLS>
+__device__ __forceinline__ void record_packed(const DevPtrs& P, const QuadStage& S, const float2* __restrict__ s_lj,
+                                              const float4* __restrict__ s_lj3, int rowa, int rowb,
+                                              const PackedArgs& A, int sp, int st, int sat, int src,
+                                              float2& fx, float2& fy, float2& fz, double& te, double& tl,
+                                              int& tn, double& ea, double& eb) {
+  const unsigned full = 0xffffffffu;
+  const float2 zb2 = make_float2(A.zb, A.zb), mzc = make_float2(-A.zc, -A.zc), mzf = make_float2(-A.zf, -A.zf);
+  const float2 half2 = make_float2(0.5f, 0.5f);
+  float bx = 0.f, by = 0.f, bz = 0.f, ibx = 0.f, iby = 0.f, ibz = 0.f;
+  if (MINIMG) {
+    const float* rp = S.rep[(threadIdx.x & 31) >> 3];
+    bx = rp[0]; by = rp[1]; bz = rp[2];
+    ibx = rp[3]; iby = rp[4]; ibz = rp[5];
+  }
 #pragma unroll 1
-  for (int k0 = 0; k0 < 16; k0 += 4) {
-    const float4* __restrict__ sp = S.p2 + sidx + k0;
-    const float4* __restrict__ sq = S.q2 + sidx + k0;
-    const int2* __restrict__ st = S.t2 + sidx + k0;
-    const unsigned ma = m >> k0, mb = m >> (k0 + 16);
+  for (int g = 0; g < 4; ++g) {
+    const float4* __restrict__ pp = S.p + sp + 16 * g;
+    int tj = S.at[st + 8 * g].y;
+    if (CLS) tj &= kTypeMask;
+    const unsigned ma = A.ma >> (8 * g), mb = A.mb >> (8 * g);
+    const unsigned jc = CLS ? A.jc >> (8 * g) : 0u;
+    float gx = 0.f, gy = 0.f, gz = 0.f;   // minus the j force of the entry this lane meets
     float2 te4 = make_float2(0.f, 0.f), tl4 = te4;
+    float ea4 = 0.f, eb4 = 0.f;
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      const float4 a = sp[k];
-      const float4 b = sq[k];
-      float2 dx = __ffma2_rn(make_float2(a.x, a.y), m1, px);
-      float2 dy = __ffma2_rn(make_float2(a.z, a.w), m1, py);
-      float2 dz = __ffma2_rn(make_float2(b.x, b.y), m1, pz);
+    for (int k = 0; k < 8; ++k) {
+      const float4 j = pp[k];
+      float2 dx = __fadd2_rn(make_float2(j.x, j.x), A.nx);   // x_j - x_i
+      float2 dy = __fadd2_rn(make_float2(j.y, j.y), A.ny);
+      float2 dz = __fadd2_rn(make_float2(j.z, j.z), A.nz);
       if (MINIMG) {
         dx = __ffma2_rn(make_float2(-bx, -bx), rint2(__fmul2_rn(dx, make_float2(ibx, ibx))), dx);
         dy = __ffma2_rn(make_float2(-by, -by), rint2(__fmul2_rn(dy, make_float2(iby, iby))), dy);
         dz = __ffma2_rn(make_float2(-bz, -bz), rint2(__fmul2_rn(dz, make_float2(ibz, ibz))), dz);
       }
       const float2 r2 = __ffma2_rn(dx, dx, __ffma2_rn(dy, dy, __fmul2_rn(dz, dz)));
-      const bool ia = ((ma >> k) & 1u) && r2.x <= rc2;
-      const bool ib = ((mb >> k) & 1u) && r2.y <= rc2;
+      const bool ia = ((ma >> k) & 1u) && r2.x <= A.rc2;
+      const bool ib = ((mb >> k) & 1u) && r2.y <= A.rc2;
       const float2 rinv = make_float2(rsqrt_ftz(ia ? r2.x : 1e30f), rsqrt_ftz(ib ? r2.y : 1e30f));
       const float2 r2i = __fmul2_rn(rinv, rinv);
       const float2 r6 = __fmul2_rn(__fmul2_rn(r2i, r2i), r2i);
-      float2 c6, c12v;
+      float2 m6, p12;   // -6 C6, 12 C12
       if (TRI) {
-        const float4 lj = s_lj3[row + st[k].x];
-        c6 = make_float2(lj.x, lj.y);
-        c12v = make_float2(lj.z, lj.w);
+        const float4 lj = s_lj3[rowa + tj];
+        m6 = make_float2(lj.x, lj.y);
+        p12 = make_float2(lj.z, lj.w);
       } else {
-        const int2 t = st[k];
-        const float2 lja = s_lj[row + t.x], ljb = s_lj[row + t.y];
-        c6 = make_float2(lja.x, ljb.x);
-        c12v = make_float2(lja.y, ljb.y);
+        const float2 lja = s_lj[rowa + tj], ljb = s_lj[rowb + tj];
+        m6 = make_float2(lja.x, ljb.x);
+        p12 = make_float2(lja.y, ljb.y);
       }
-      const float2 qf = __fmul2_rn(pw, make_float2(b.z, b.w));
+      const float2 qf = __fmul2_rn(A.qi, make_float2(j.w, j.w));
       const float2 qq = make_float2(ia ? qf.x : 0.f, ib ? qf.y : 0.f);
-      const float2 v1 = __fmul2_rn(c6, r6);
-      const float2 v2 = __fmul2_rn(__fmul2_rn(c12v, r6), r6);
-      const float2 eel = __fmul2_rn(qq, __fadd2_rn(rinv, __ffma2_rn(zb2, r2, mzc)));
-      const float2 elj = __ffma2_rn(v1, m1, v2);
-      const float2 fs = __ffma2_rn(qq, __ffma2_rn(rinv, r2i, mzf),
-                                   __fmul2_rn(__ffma2_rn(c12, v2, __fmul2_rn(cm6, v1)), r2i));
-      te4 = __fadd2_rn(te4, eel);
-      tl4 = __fadd2_rn(tl4, elj);
-      const float2 ffx = __fmul2_rn(dx, fs), ffy = __fmul2_rn(dy, fs), ffz = __fmul2_rn(dz, fs);
-      fx = __ffma2_rn(ffx, m1, fx);
-      fy = __ffma2_rn(ffy, m1, fy);
-      fz = __ffma2_rn(ffz, m1, fz);
-      gx = __fadd2_rn(gx, ffx);
-      gy = __fadd2_rn(gy, ffy);
-      gz = __fadd2_rn(gz, ffz);
+      const float2 p = __fmul2_rn(p12, r6);
+      const float2 h = __ffma2_rn(p, half2, m6);
+      const float2 c = __fadd2_rn(rinv, __ffma2_rn(zb2, r2, mzc));
+      const float2 el = __fmul2_rn(qq, __ffma2_rn(rinv, r2i, mzf));
+      float2 fs = __ffma2_rn(__fadd2_rn(p, m6), __fmul2_rn(r6, r2i), el);
+      if (CLS) {   // the pair's class from the number of cluster atoms in it
+        const float2 eel = __fmul2_rn(qq, c), elj = __fmul2_rn(h, r6);
+        te4 = __fadd2_rn(te4, eel);
+        tl4 = __fadd2_rn(tl4, elj);
+        const bool cj = ((jc >> k) & 1u) != 0u;
+        const float2 e2 = __ffma2_rn(elj, make_float2(1.f / 6.f, 1.f / 6.f), eel);
+        ea4 += (cj && A.ca ? e2.x : 0.f) + (cj && A.cb ? e2.y : 0.f);
+        eb4 += (cj != A.ca ? e2.x : 0.f) + (cj != A.cb ? e2.y : 0.f);
+        fs = __fmul2_rn(fs, cj ? A.w1 : A.w0);
+      } else {
+        te4 = __ffma2_rn(qq, c, te4);
+        tl4 = __ffma2_rn(h, r6, tl4);
+      }
+      fx = __ffma2_rn(dx, fs, fx);
+      fy = __ffma2_rn(dy, fs, fy);
+      fz = __ffma2_rn(dz, fs, fz);
+      gx = fmaf(dx.y, fs.y, fmaf(dx.x, fs.x, gx));
+      gy = fmaf(dy.y, fs.y, fmaf(dy.x, fs.x, gy));
+      gz = fmaf(dz.y, fs.y, fmaf(dz.x, fs.x, gz));
       if (COUNT) tn += (ia ? 1 : 0) + (ib ? 1 : 0);
-      gx.x = __shfl_sync(full, gx.x, src); gx.y = __shfl_sync(full, gx.y, src);
-      gy.x = __shfl_sync(full, gy.x, src); gy.y = __shfl_sync(full, gy.y, src);
-      gz.x = __shfl_sync(full, gz.x, src); gz.y = __shfl_sync(full, gz.y, src);
+      if (k < 7) {
+        gx = __shfl_sync(full, gx, src);
+        gy = __shfl_sync(full, gy, src);
+        gz = __shfl_sync(full, gz, src);
+        tj = __shfl_sync(full, tj, src);
+      }
+      if (k == 3 || k == 7) {   // energies: FP32 over 4 steps, then FP64
+        te += (double)te4.x + (double)te4.y;
+        tl += (double)tl4.x + (double)tl4.y;
+        te4 = tl4 = make_float2(0.f, 0.f);
+        if (CLS) {
+          ea += (double)ea4;
+          eb += (double)eb4;
+          ea4 = eb4 = 0.f;
+        }
+      }
     }
-    te += (double)te4.x + (double)te4.y;
-    tl += (double)tl4.x + (double)tl4.y;
+    const int aj = S.at[sat + 8 * g].x;
+    if (aj >= 0 && (gx != 0.f || gy != 0.f || gz != 0.f)) {
+      atomic_add_ll(&P.frc[3 * aj + 0], to_fix_f(-gx, P.status));
+      atomic_add_ll(&P.frc[3 * aj + 1], to_fix_f(-gy, P.status));
+      atomic_add_ll(&P.frc[3 * aj + 2], to_fix_f(-gz, P.status));
+    }
   }
-  fix += fx.x + fx.y;
-  fiy += fy.x + fy.y;
-  fiz += fz.x + fz.y;
-  gja = make_float3(gx.x, gy.x, gz.x);
-  gjb = make_float3(gx.y, gy.y, gz.y);
+}
+
+// what a lane gathers for a record group before computing it: the positions (in their own
+// blocks' frames, with the charge) of entries 8 g + l of its record, and its record's unit
+// (-1: none)
+struct Gather4 {
+  float4 p[4];
+  int unit;
+};
+
+// dynamic shared memory of the packed kernel: the stages, then the LJ table -- type triples
+// (i type, i type, j type) up to kTriMaxTypes types, where two blocks still fit an SM
+// (85 KB of stages + 28 KB of table each), type pairs above (two 8-byte reads a step)
+constexpr int kTriMaxTypes = 12;
+__host__ __device__ constexpr bool lj_tri(int nt1) { return nt1 <= kTriMaxTypes; }
+__host__ __device__ constexpr size_t lj_bytes(int nt1) {
+  return lj_tri(nt1) ? (size_t)nt1 * nt1 * nt1 * 16 : ((size_t)nt1 * nt1 * 8 + 15) / 16 * 16;
+}
+constexpr size_t kPackedStageBytes = sizeof(QuadStage) * kPairWarps;
+
+template <bool COUNT, bool CLS, bool TRI>
+__global__ void __launch_bounds__(kPairThreads, 2) k_pair_packed(DevPtrs P, ZdConst z) {
+  extern __shared__ __align__(16) unsigned char s_dyn[];
+  __shared__ unsigned long long s_tab_bar;
+  const unsigned full = 0xffffffffu;
+  QuadStage& S = reinterpret_cast<QuadStage*>(s_dyn)[threadIdx.x >> 5];
+  const float2* s_lj = reinterpret_cast<const float2*>(s_dyn + kPackedStageBytes);
+  const float4* s_lj3 = reinterpret_cast<const float4*>(s_dyn + kPackedStageBytes);
+  const int lane = threadIdx.x & 31;
+  const int qd = lane >> 3, lp = lane & 7;              // record of the group, lane inside it
+  const int sp = 64 * qd + lp, sta = 36 * qd + lp;      // this lane's staging slots
+  const int sat = 36 * qd + ((lp + 7) & 7);
+  const int src = (lane & 24) | ((lp + 1) & 7);         // rotation: from the next lane of the record
+  for (int k = lp; k < 12; k += 8) S.rep[qd][k] = k < 6 ? 0.f : 1.f;   // a record group past the list
+  if (lane == 0) {
+    mbar_init(&S.bar[0]);
+    mbar_init(&S.bar[1]);
+  }
+  if (threadIdx.x == 0) {
+    mbar_init(&s_tab_bar);
+    mbar_expect(&s_tab_bar, (unsigned)lj_bytes(z.nt1));
+    bulk_load(s_dyn + kPackedStageBytes, P.lj_tab, (unsigned)lj_bytes(z.nt1), &s_tab_bar);
+  }
+  __syncthreads();
+  const int T = *P.nctiles;         // records
+  const int TU = (T + 3) >> 2;      // record groups: a warp's work units
+  // a 2.5-KiB copy lands in microseconds; the bound (about a second of SM clock) only ends
+  // the wait on a broken device, and it is not the integrator's adjustable barrier bound:
+  // a block must never leave with one of its copies still in flight
+  const long long wlim = kCopyWaitCycles;
+  unsigned phase = 0u, pend = 0u;   // per buffer: barrier parity to wait for; copy in flight
+  bool ok = true;
+
+  // record groups are claimed in runs of `run` consecutive ones: the records of a unit are
+  // consecutive, so a run mostly keeps its i atoms; the run is short enough that every warp
+  // still gets several.  A warp's first run goes by its index, without the counter's latency;
+  // a list that these runs cover makes no claim at all.
+  const int gw = blockIdx.x * kPairWarps + (threadIdx.x >> 5), nw = gridDim.x * kPairWarps;
+  const int run = max(1, min(8, TU / (nw * 8)));
+  int run_next = min(gw * run, TU), run_end = min(run_next + run, TU);
+  auto claim = [&]() {
+    if (run_next >= run_end) {
+      if (nw * run >= TU) return TU;
+      int t = 0;
+      if (lane == 0) t = atomicAdd(P.tile_ctr, run);
+      t = __shfl_sync(full, t, 0) + nw * run;
+      run_next = t;
+      run_end = min(t + run, TU);
+    }
+    return run_next < run_end ? run_next++ : TU;
+  };
+  // the entries, types and masks of records 4t .. 4t + 3 into buffer b (up to three past
+  // the last record are padding inside the arrays: read, never used)
+  auto issue = [&](int t, int b) {
+    if (lane == 0) {
+      fence_proxy_async();
+      mbar_expect(&S.bar[b], 2560u);
+      bulk_load(S.ent[b], P.ct_j + (size_t)t * 128, 2048u, &S.bar[b]);
+      bulk_load(S.ty[b], P.ct_ty + (size_t)t * 128, 256u, &S.bar[b]);
+      bulk_load(S.msk[b], P.ct_mask + (size_t)t * 64, 256u, &S.bar[b]);
+    }
+    pend |= 1u << b;
+  };
+  // group t's copy has landed in buffer b: start the gathers of this lane's four entries
+  auto fetch = [&](int t, int b, Gather4& G) {
+    if (!mbar_wait(&S.bar[b], (phase >> b) & 1u, wlim)) {
+      ok = false;
+      atomicOr(P.status, ERR_TIMEOUT);
+      return;
+    }
+    phase ^= 1u << b;
+    pend &= ~(1u << b);
+    const int rec = 4 * t + qd;
+    const bool valid = rec < T;
+    G.unit = valid ? P.ct_blk[rec] : -1;
+#pragma unroll
+    for (int g = 0; g < 4; ++g) {
+      const int aj = valid ? __float_as_int(S.ent[b][32 * qd + 8 * g + lp].w) : -1;
+      G.p[g] = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (aj >= 0) G.p[g] = P.pos_f[aj];
+    }
+  };
+
+  PackedArgs A;
+  A.rc2 = (float)z.rc2; A.zb = (float)z.bcoeff; A.zf = (float)z.fcoeff; A.zc = (float)z.zcore;
+  A.nx = A.ny = A.nz = A.qi = make_float2(0.f, 0.f);
+  A.jc = 0u;
+  A.ca = A.cb = false;
+  A.w0 = A.w1 = make_float2(1.f, 1.f);   // set where a record holds classes
+  int cur_unit = -2, cur_rep = -1, rep = -1, aia = -1, aib = -1, tia = z.nt1 - 1, tib = tia;
+  long long gia[3] = {0, 0, 0}, gib[3] = {0, 0, 0};
+  long long eel = 0, elj = 0;
+  long long npair = 0;
+  bool mi = false;
+  auto flush_i = [&]() {
+    if (aia >= 0 && (gia[0] | gia[1] | gia[2]))
+      for (int k = 0; k < 3; ++k) atomic_add_ll(&P.frc[3 * aia + k], gia[k]);
+    if (aib >= 0 && (gib[0] | gib[1] | gib[2]))
+      for (int k = 0; k < 3; ++k) atomic_add_ll(&P.frc[3 * aib + k], gib[k]);
+    for (int k = 0; k < 3; ++k) gia[k] = gib[k] = 0;
+  };
+
+  int t = claim(), tn = TU;
+  Gather4 G;
+  if (t < TU) {
+    issue(t, 0);
+    tn = claim();
+    if (tn < TU) issue(tn, 1);
+    fetch(t, 0, G);
+  }
+  if (!mbar_wait(&s_tab_bar, 0u, wlim)) {
+    ok = false;
+    atomicOr(P.status, ERR_TIMEOUT);
+  }
+  int b = 0;
+  while (t < TU && ok) {
+    // this lane's four entries into the stage, twice
+    __syncwarp();
+    unsigned jc = 0u;
+#pragma unroll
+    for (int g = 0; g < 4; ++g) {
+      // buffer b still holds this group's entries, types and masks (a record past the last one:
+      // no atom, the zero dummy type).  The shift into the i block's frame waits
+      // until here, as nothing may use a gather's result before the last group's arithmetic
+      const float4 e = S.ent[b][32 * qd + 8 * g + lp];
+      const float4 q = make_float4(G.p[g].x - e.x, G.p[g].y - e.y, G.p[g].z - e.z, G.p[g].w);
+      S.p[sp + 16 * g] = q;
+      S.p[sp + 16 * g + 8] = q;
+      const int2 ta = G.unit >= 0 ? make_int2(__float_as_int(e.w), type_word(S.ty[b][32 * qd + 8 * g + lp]))
+                                  : make_int2(-1, z.nt1 - 1);
+      S.at[sta + 8 * g] = ta;
+      if (CLS) jc |= ((__ballot_sync(full, (ta.y >> 30) & 1) >> (8 * qd)) & 0xffu) << (8 * g);
+    }
+    const int unit = G.unit;
+    A.ma = unit >= 0 ? step_mask(S.msk[b][16 * qd + lp], lp) : 0u;
+    A.mb = unit >= 0 ? step_mask(S.msk[b][16 * qd + 8 + lp], lp + 8) : 0u;
+    // the lane's i atoms: a new unit flushes the last one's forces and loads the new atoms
+    if (unit != cur_unit) {
+      flush_i();
+      cur_unit = unit;
+      if (unit >= 0) {
+        const int si = unit * kHalf + lp;
+        aia = P.satom[si];
+        aib = P.satom[si + 8];
+        const float4 pa = aia >= 0 ? P.pos_f[aia] : make_float4(0.f, 0.f, 0.f, 0.f);
+        const float4 pb = aib >= 0 ? P.pos_f[aib] : make_float4(0.f, 0.f, 0.f, 0.f);
+        A.nx = make_float2(-pa.x, -pb.x);
+        A.ny = make_float2(-pa.y, -pb.y);
+        A.nz = make_float2(-pa.z, -pb.z);
+        A.qi = make_float2(pa.w, pb.w);
+        tia = P.styp[si];
+        tib = P.styp[si + 8];
+        rep = P.blk_rep[unit >> 1];
+      } else {
+        A.nx = A.ny = A.nz = A.qi = make_float2(0.f, 0.f);
+        tia = tib = z.nt1 - 1;
+        aia = aib = -1;
+      }
+    }
+    // a new replica in any record: every record's energies go to its replica so far
+    if (__any_sync(full, rep != cur_rep)) {
+      flush_fix<8>(P, cur_rep, eel, elj, 0, 0, npair, COUNT, CLS);
+      eel = elj = 0;
+      npair = 0;
+      if (rep != cur_rep) {
+        cur_rep = rep;
+        const Rep& R = P.reps[rep];
+        if (lp < 6) S.rep[qd][lp] = (float)(lp < 3 ? R.box[lp] : R.invbox[lp - 3]);
+        if (CLS && lp < 3) S.rep[qd][6 + lp] = (float)cls_weight(R, P.lam[2 * rep], 2 - lp);
+        // Per-pair minimum image is needed only where a pair within the cut-off can have
+        // another image than its tile's.  Per axis the tile's image puts the two block
+        // references at most box/2 apart, and a pair's separation differs from theirs by at
+        // most h_i + h_j <= 2 h_max plus the atoms' motion since the build (2 A margin), so
+        // in the tile's image |d| <= box/2 + 2 h_max + 2; in any other image |d| >= box - rc.
+        // Both hold at once only if box/2 <= rc + 2 h_max + 2.
+        mi = false;
+        for (int k = 0; k < 3; ++k)
+          if (0.5 * R.box[k] < sqrt(z.rc2) + 2.0 * (double)P.rep_hmax[3 * rep + k] + 2.0) mi = true;
+      }
+    }
+    const bool wmi = __any_sync(full, mi);   // one image form for the whole warp
+    bool wcls = false;                       // does any record of the group hold a class but BB?
+    __syncwarp();
+    if (CLS)   // BB records keep the plain form unless BB itself is weighted (per-class evaluation)
+      wcls = __any_sync(full, jc != 0u || (((tia | tib) >> 30) & 1) || S.rep[qd][6] != 1.f);
+    // buffer b is free again: the group after next goes into it; the next group's gathers
+    // are issued before this group's arithmetic
+    int t2 = TU;
+    if (tn < TU) {
+      t2 = claim();
+      if (t2 < TU) issue(t2, b);
+    }
+    if (tn < TU) fetch(tn, b ^ 1, G);
+    float2 fx = make_float2(0.f, 0.f), fy = fx, fz = fx;
+    double te = 0.0, tl = 0.0;
+    int tn_pairs = 0;
+    const int ka = CLS ? (tia & kTypeMask) : tia, kb = CLS ? (tib & kTypeMask) : tib;
+    const int rowa = TRI ? (ka * z.nt1 + kb) * z.nt1 : ka * z.nt1, rowb = kb * z.nt1;
+    double ea = 0.0, eb = 0.0;
+    if (CLS && wcls) {
+      const float f0 = S.rep[qd][6], f1 = S.rep[qd][7], f2 = S.rep[qd][8];
+      A.ca = ((tia >> 30) & 1) != 0;
+      A.cb = ((tib >> 30) & 1) != 0;
+      A.jc = byte_rotr(jc, lp);
+      A.w0 = make_float2(A.ca ? f1 : f0, A.cb ? f1 : f0);
+      A.w1 = make_float2(A.ca ? f2 : f1, A.cb ? f2 : f1);
+      if (wmi)
+        record_packed<true, COUNT, TRI, CLS>(P, S, s_lj, s_lj3, rowa, rowb, A, sp, sta, sat, src, fx, fy, fz, te,
+                                             tl, tn_pairs, ea, eb);
+      else
+        record_packed<false, COUNT, TRI, CLS>(P, S, s_lj, s_lj3, rowa, rowb, A, sp, sta, sat, src, fx, fy, fz, te,
+                                              tl, tn_pairs, ea, eb);
+      // classes AA and AB of these few records go to their slots at once; BB, which the flush
+      // credits with everything, gives them back
+      const long long xa = to_fix(ea, kEneScale, P.status), xb = to_fix(eb, kEneScale, P.status);
+      if (cur_rep >= 0 && (xa | xb)) {
+        atomic_add_ll(&P.ene_cls[cur_rep * 4 + 0], xa);
+        atomic_add_ll(&P.ene_cls[cur_rep * 4 + 1], xb);
+        atomic_add_ll(&P.ene_cls[cur_rep * 4 + 2], -(xa + xb));
+      }
+    } else if (wmi) {
+      record_packed<true, COUNT, TRI, false>(P, S, s_lj, s_lj3, rowa, rowb, A, sp, sta, sat, src, fx, fy, fz, te,
+                                             tl, tn_pairs, ea, eb);
+    } else {
+      record_packed<false, COUNT, TRI, false>(P, S, s_lj, s_lj3, rowa, rowb, A, sp, sta, sat, src, fx, fy, fz, te,
+                                              tl, tn_pairs, ea, eb);
+    }
+    gia[0] += to_fix_f(fx.x, P.status);
+    gia[1] += to_fix_f(fy.x, P.status);
+    gia[2] += to_fix_f(fz.x, P.status);
+    gib[0] += to_fix_f(fx.y, P.status);
+    gib[1] += to_fix_f(fy.y, P.status);
+    gib[2] += to_fix_f(fz.y, P.status);
+    eel += to_fix(te, kEneScale, P.status);
+    elj += to_fix(tl * (1.0 / 6.0), kEneScale, P.status);
+    if (COUNT) npair += tn_pairs;
+    t = tn;
+    tn = t2;
+    b ^= 1;
+  }
+  flush_i();
+  flush_block<8>(P, cur_rep, eel, elj, npair, COUNT, CLS);
+  // a copy still in flight (only after a timed-out wait) must land before the block exits
+  for (int k = 0; k < 2; ++k)
+    if ((pend >> k) & 1u) mbar_wait(&S.bar[k], (phase >> k) & 1u, wlim);
 }
 
 // what a lane gathers for a record pair before computing it: its two j entries a = l and
@@ -284,26 +674,25 @@ __device__ __forceinline__ void pair_scalar(float4 pi, float xj, float yj, float
   elj = in ? e2 : 0.f;
 }
 
-// One record in the scalar form (ALSD, CMM and partial-McMD variants), the two entries of a
-// step one after the other, same staging and rotation as tile_mixed2.  ALSD: ci = cluster bit
-// of the i atom; a pair with nA cluster atoms has its force times f2 (nA = 2, class AA), f1
-// (AB) or f0 (BB: 1 but while per-class outputs are evaluated), and its energy also goes to
-// ea (AA) / eb (AB).  SPLIT (partial McMD): the pair's class from the regions of its atoms
-// (bit cj of trow: class 1), the class-1 forces in accumulators of their own (fi[3..5],
-// gj[6..11], rotated like the others) and the class-1 energy in ea.  CMM: no cut-off (rc2 is
-// huge) and the Coulomb term only for the pairs of `me`.  gj[0..5]: entries a and b.
-template <bool MINIMG, bool COUNT, bool ALSD, bool CMM, bool SPLIT>
+// One record in the scalar form (CMM and partial-McMD variants): at step k (k < 16) lane l of
+// the half-warp meets entries a = (l + k) & 15 and b = 16 + a, staged at sidx + k (sidx =
+// 32 h + l), one after the other.  The j-force accumulators of a and b move one lane per step
+// (from lane src = l + 1 of the same half); after 16 steps lane l holds those of entries l and
+// 16 + l.  SPLIT (partial McMD): the pair's class from the regions of its atoms (bit cj of
+// trow: class 1), the class-1 forces in accumulators of their own (fi[3..5], gj[6..11],
+// rotated like the others) and the class-1 energy in ea.  CMM: no cut-off (rc2 is huge) and
+// the Coulomb term only for the pairs of `me`.  gj[0..5]: entries a and b.
+template <bool MINIMG, bool COUNT, bool CMM, bool SPLIT>
 __device__ __forceinline__ void tile_scalar(const MixStage& S, const float2* __restrict__ s_lj, int row,
                                             float4 pi, unsigned m, unsigned me, int sidx, int src, float bx,
                                             float by, float bz, float ibx, float iby, float ibz, float rc2,
                                             float zb, float zf, float zc, float (&fi)[6], float (&gj)[12],
-                                            double& te, double& tl, int& tn, int ci, float f0, float f1,
-                                            float f2, unsigned trow, double& ea, double& eb) {
+                                            double& te, double& tl, int& tn, unsigned trow, double& ea) {
   const unsigned full = 0xffffffffu;
   constexpr int NG = SPLIT ? 12 : 6;
 #pragma unroll 1
   for (int k0 = 0; k0 < 16; k0 += 4) {
-    float te4 = 0.f, tl4 = 0.f, ea4 = 0.f, eb4 = 0.f;
+    float te4 = 0.f, tl4 = 0.f, ea4 = 0.f;
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
       const float4 a = S.p2[sidx + k0 + k];
@@ -313,7 +702,7 @@ __device__ __forceinline__ void tile_scalar(const MixStage& S, const float2* __r
       for (int e = 0; e < 2; ++e) {
         const int tj = e ? t.y : t.x;
         const int sh = k0 + k + 16 * e;
-        const float2 lj = s_lj[row + ((ALSD || SPLIT) ? (tj & kTypeMask) : tj)];
+        const float2 lj = s_lj[row + (SPLIT ? (tj & kTypeMask) : tj)];
         float dx, dy, dz, fs, eel, elj;
         bool in;
         pair_scalar<MINIMG, CMM>(pi, e ? a.y : a.x, e ? a.w : a.z, e ? b.y : b.x, e ? b.w : b.z, lj,
@@ -327,11 +716,6 @@ __device__ __forceinline__ void tile_scalar(const MixStage& S, const float2* __r
           ea4 += c1 ? eel + elj : 0.f;
           fs1 = c1 ? fs : 0.f;
           fs -= fs1;
-        } else if (ALSD) {
-          const int na = ci + ((tj >> 30) & 1);
-          ea4 += na == 2 ? eel + elj : 0.f;
-          eb4 += na == 1 ? eel + elj : 0.f;
-          fs *= na == 2 ? f2 : (na == 1 ? f1 : f0);
         }
         const float fx = dx * fs, fy = dy * fs, fz = dz * fs;
         fi[0] -= fx; fi[1] -= fy; fi[2] -= fz;
@@ -348,34 +732,18 @@ __device__ __forceinline__ void tile_scalar(const MixStage& S, const float2* __r
     }
     te += (double)te4;
     tl += (double)tl4;
-    if (ALSD || SPLIT) {
-      ea += (double)ea4;
-      eb += (double)eb4;
-    }
+    if (SPLIT) ea += (double)ea4;
   }
 }
 
-// dynamic shared memory of the mixed kernel: the type-pair (C6, C12) table, and with TRI the
-// type-triple table after it (16-byte aligned)
-__host__ __device__ constexpr size_t lj_pair_bytes(int nt1) { return ((size_t)nt1 * nt1 * 8 + 15) / 16 * 16; }
-__host__ __device__ constexpr size_t lj_tri_bytes(int nt1) { return (size_t)nt1 * nt1 * nt1 * 16; }
-constexpr int kTriMaxTypes = 16;   // the triple table up to 16 types (64 KiB)
-
-template <bool COUNT, bool ALSD, bool CMM, bool SPLIT = false, bool TRI = false>
+template <bool COUNT, bool CMM, bool SPLIT>
 __global__ void __launch_bounds__(kPairThreads, 2)
 k_pair_mixed(DevPtrs P, ZdConst z) {
   extern __shared__ float2 s_lj[];
   __shared__ MixStage s_stage[kPairWarps];
   const unsigned full = 0xffffffffu;
   const int nlj = z.nt1 * z.nt1;
-  float4* s_lj3 = reinterpret_cast<float4*>(reinterpret_cast<char*>(s_lj) + lj_pair_bytes(z.nt1));
   for (int i = threadIdx.x; i < nlj; i += blockDim.x) s_lj[i] = P.lj_f[i];
-  if (TRI)
-    for (int i = threadIdx.x; i < nlj * z.nt1; i += blockDim.x) {
-      const int ti = i / nlj, ta = (i / z.nt1) % z.nt1, tb = i % z.nt1;
-      const float2 a = P.lj_f[ti * z.nt1 + ta], b = P.lj_f[ti * z.nt1 + tb];
-      s_lj3[i] = make_float4(a.x, b.x, a.y, b.y);
-    }
   const int lane = threadIdx.x & 31;
   const int hw = lane >> 4, lp = lane & (kHalf - 1);   // half-warp, lane inside it
   const int sidx = 32 * hw + lp;                        // this lane's staging slot
@@ -426,16 +794,14 @@ k_pair_mixed(DevPtrs P, ZdConst z) {
     pend |= 1u << b;
   };
   auto gather1 = [&](float4 e, bool valid, float4& p, int& ty, int& at) {
-    const int sj = valid ? __float_as_int(e.w) : -1;
-    if (sj >= 0) {
-      const float4 q = P.pos_f[sj];
+    at = valid ? __float_as_int(e.w) : -1;
+    if (at >= 0) {
+      const float4 q = P.pos_f[at];
       p = make_float4(q.x - e.x, q.y - e.y, q.z - e.z, q.w);   // into the i block's frame
-      ty = P.styp[sj];
-      at = P.satom[sj];
+      ty = P.typ[at];
     } else {
       p = make_float4(0.f, 0.f, 0.f, 0.f);
       ty = z.nt1 - 1;   // the zero dummy type
-      at = -1;
     }
   };
   // pair t's copy has landed in buffer b: start the gathers of this lane's two entries
@@ -460,11 +826,10 @@ k_pair_mixed(DevPtrs P, ZdConst z) {
   float4 pi = make_float4(0.f, 0.f, 0.f, 0.f);
   long long gix = 0, giy = 0, giz = 0;
   long long gix1 = 0, giy1 = 0, giz1 = 0;   // partial McMD: class-1 i forces
-  long long eel = 0, elj = 0, eaa = 0, eab = 0;
+  long long eel = 0, elj = 0, eaa = 0;
   long long npair = 0;
   bool mi = false;
   float bx = 0.f, by = 0.f, bz = 0.f, ibx = 0.f, iby = 0.f, ibz = 0.f;
-  float f0 = 1.f, f1 = 1.f, f2 = 1.f;
   unsigned tab = 0u;
 
   int t = claim(), tn = TU;
@@ -482,7 +847,7 @@ k_pair_mixed(DevPtrs P, ZdConst z) {
     {
       const float4 p2 = make_float4(G.pa.x, G.pb.x, G.pa.y, G.pb.y);
       const float4 q2 = make_float4(G.pa.z, G.pb.z, G.pa.w, G.pb.w);
-      const int2 t2 = TRI ? make_int2(G.ta * z.nt1 + G.tb, 0) : make_int2(G.ta, G.tb);
+      const int2 t2 = make_int2(G.ta, G.tb);
       S.p2[sidx] = p2;
       S.p2[sidx + kHalf] = p2;
       S.q2[sidx] = q2;
@@ -509,9 +874,9 @@ k_pair_mixed(DevPtrs P, ZdConst z) {
       cur_unit = unit;
       if (unit >= 0) {
         const int si = (unit >> 1) * kTile + (unit & 1) * kHalf + lp;
-        pi = P.pos_f[si];
         ti = P.styp[si];
         ai = P.satom[si];
+        pi = ai >= 0 ? P.pos_f[ai] : make_float4(0.f, 0.f, 0.f, 0.f);
         rep = P.blk_rep[unit >> 1];
       } else {
         pi = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -521,20 +886,14 @@ k_pair_mixed(DevPtrs P, ZdConst z) {
     }
     // a new replica in either half: both halves' energies go to their replicas so far
     if (__any_sync(full, rep != cur_rep)) {
-      flush_fix(P, cur_rep, eel, elj, eaa, eab, npair, COUNT, ALSD || SPLIT);
-      eel = elj = eaa = eab = 0;
+      flush_fix<16>(P, cur_rep, eel, elj, eaa, 0, npair, COUNT, SPLIT);
+      eel = elj = eaa = 0;
       npair = 0;
       if (rep != cur_rep) {
         cur_rep = rep;
         const Rep& R = P.reps[rep];
         bx = (float)R.box[0]; by = (float)R.box[1]; bz = (float)R.box[2];
         ibx = (float)R.invbox[0]; iby = (float)R.invbox[1]; ibz = (float)R.invbox[2];
-        if (ALSD) {
-          const double lam = P.lam[2 * rep];
-          f0 = (float)cls_weight(R, lam, 2);
-          f1 = (float)cls_weight(R, lam, 1);
-          f2 = (float)cls_weight(R, lam, 0);
-        }
         if (SPLIT) tab = R.split ? R.cls_tab : 0u;
         // Per-pair minimum image is needed only where a pair within the cut-off can have
         // another image than its tile's.  Per axis the tile's image puts the two block
@@ -562,42 +921,18 @@ k_pair_mixed(DevPtrs P, ZdConst z) {
     }
     Gather Gn;
     if (tn < TU) fetch(tn, b ^ 1, Gn);
-    float fix = 0.f, fiy = 0.f, fiz = 0.f;
-    float3 gja = make_float3(0.f, 0.f, 0.f), gjb = gja, gja1 = gja, gjb1 = gja;
-    double te = 0.0, tl = 0.0, ea = 0.0, eb = 0.0;
+    double te = 0.0, tl = 0.0, ea = 0.0;
     int tn_pairs = 0;
-    const int ci = ALSD ? ((ti >> 30) & 1) : 0;
-    const int row = ((ALSD || SPLIT) ? (ti & kTypeMask) : ti) * z.nt1;
-    if (ALSD || CMM || SPLIT) {
-      float fi6[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-      float gj[12] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-      const unsigned trow = SPLIT ? tab >> (3 * ((ti >> kRegionShift) & 3)) : 0u;
-      if (wmi)
-        tile_scalar<true, COUNT, ALSD, CMM, SPLIT>(S, s_lj, row, pi, m, me, sidx, src, bx, by, bz, ibx, iby,
-                                                   ibz, rc2, zb, zf, zc, fi6, gj, te, tl, tn_pairs, ci, f0,
-                                                   f1, f2, trow, ea, eb);
-      else
-        tile_scalar<false, COUNT, ALSD, CMM, SPLIT>(S, s_lj, row, pi, m, me, sidx, src, bx, by, bz, ibx, iby,
-                                                    ibz, rc2, zb, zf, zc, fi6, gj, te, tl, tn_pairs, ci, f0,
-                                                    f1, f2, trow, ea, eb);
-      fix = fi6[0]; fiy = fi6[1]; fiz = fi6[2];
-      gja = make_float3(gj[0], gj[1], gj[2]);
-      gjb = make_float3(gj[3], gj[4], gj[5]);
-      if (SPLIT) {
-        gja1 = make_float3(gj[6], gj[7], gj[8]);
-        gjb1 = make_float3(gj[9], gj[10], gj[11]);
-        gix1 += to_fix_f(fi6[3], P.status);
-        giy1 += to_fix_f(fi6[4], P.status);
-        giz1 += to_fix_f(fi6[5], P.status);
-      }
-    } else if (wmi) {
-      tile_mixed2<true, COUNT, TRI>(S, s_lj, s_lj3, TRI ? ti * nlj : row, pi, m, sidx, src, bx, by, bz, ibx,
-                                    iby, ibz, rc2, zb, zf, zc, fix, fiy, fiz, gja, gjb, te, tl, tn_pairs);
-    } else {
-      tile_mixed2<false, COUNT, TRI>(S, s_lj, s_lj3, TRI ? ti * nlj : row, pi, m, sidx, src, bx, by, bz,
-                                     ibx, iby, ibz, rc2, zb, zf, zc, fix, fiy, fiz, gja, gjb, te, tl,
-                                     tn_pairs);
-    }
+    const int row = (SPLIT ? (ti & kTypeMask) : ti) * z.nt1;
+    float fi6[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    float gj[12] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    const unsigned trow = SPLIT ? tab >> (3 * ((ti >> kRegionShift) & 3)) : 0u;
+    if (wmi)
+      tile_scalar<true, COUNT, CMM, SPLIT>(S, s_lj, row, pi, m, me, sidx, src, bx, by, bz, ibx, iby, ibz, rc2, zb,
+                                           zf, zc, fi6, gj, te, tl, tn_pairs, trow, ea);
+    else
+      tile_scalar<false, COUNT, CMM, SPLIT>(S, s_lj, row, pi, m, me, sidx, src, bx, by, bz, ibx, iby, ibz, rc2,
+                                            zb, zf, zc, fi6, gj, te, tl, tn_pairs, trow, ea);
     auto add_j = [&](long long* f, int aj, float3 g) {
       if (aj >= 0 && (g.x != 0.f || g.y != 0.f || g.z != 0.f)) {
         atomic_add_ll(&f[3 * aj + 0], to_fix_f(g.x, P.status));
@@ -605,20 +940,20 @@ k_pair_mixed(DevPtrs P, ZdConst z) {
         atomic_add_ll(&f[3 * aj + 2], to_fix_f(g.z, P.status));
       }
     };
-    add_j(P.frc, aa, gja);
-    add_j(P.frc, ab, gjb);
-    if (SPLIT) {
-      add_j(P.frc1, aa, gja1);
-      add_j(P.frc1, ab, gjb1);
-    }
-    gix += to_fix_f(fix, P.status);
-    giy += to_fix_f(fiy, P.status);
-    giz += to_fix_f(fiz, P.status);
+    add_j(P.frc, aa, make_float3(gj[0], gj[1], gj[2]));
+    add_j(P.frc, ab, make_float3(gj[3], gj[4], gj[5]));
+    gix += to_fix_f(fi6[0], P.status);
+    giy += to_fix_f(fi6[1], P.status);
+    giz += to_fix_f(fi6[2], P.status);
     eel += to_fix(te, kEneScale, P.status);
     elj += to_fix(tl, kEneScale, P.status);
-    if (ALSD || SPLIT) {
+    if (SPLIT) {
+      add_j(P.frc1, aa, make_float3(gj[6], gj[7], gj[8]));
+      add_j(P.frc1, ab, make_float3(gj[9], gj[10], gj[11]));
+      gix1 += to_fix_f(fi6[3], P.status);
+      giy1 += to_fix_f(fi6[4], P.status);
+      giz1 += to_fix_f(fi6[5], P.status);
       eaa += to_fix(ea, kEneScale, P.status);
-      eab += to_fix(eb, kEneScale, P.status);
     }
     if (COUNT) npair += tn_pairs;
     t = tn;
@@ -636,7 +971,7 @@ k_pair_mixed(DevPtrs P, ZdConst z) {
     atomic_add_ll(&P.frc1[3 * ai + 1], giy1);
     atomic_add_ll(&P.frc1[3 * ai + 2], giz1);
   }
-  flush_fix(P, cur_rep, eel, elj, eaa, eab, npair, COUNT, ALSD || SPLIT);
+  flush_fix<16>(P, cur_rep, eel, elj, eaa, 0, npair, COUNT, SPLIT);
   // a copy still in flight (only after a timed-out wait) must land before the block exits
   for (int k = 0; k < 2; ++k)
     if ((pend >> k) & 1u) mbar_wait(&S.bar[k], (phase >> k) & 1u, wlim);
@@ -702,9 +1037,9 @@ k_pair_fp64(DevPtrs P, ZdConst z) {
       cur_unit = unit;
       if (unit >= 0) {
         const int si = (unit >> 1) * kTile + (unit & 1) * kHalf + lp;
-        pi = P.pos_d[si];
         ti = P.styp[si];
         ai = P.satom[si];
+        pi = ai >= 0 ? P.pos_d[ai] : make_double4(0, 0, 0, 0);
         rep = P.blk_rep[unit >> 1];
       } else {
         pi = make_double4(0, 0, 0, 0);
@@ -713,7 +1048,7 @@ k_pair_fp64(DevPtrs P, ZdConst z) {
       }
     }
     if (__any_sync(full, rep != cur_rep)) {
-      flush_fix(P, cur_rep, eel, elj, eaa, eab, npair, COUNT, ALSD || SPLIT);
+      flush_fix<16>(P, cur_rep, eel, elj, eaa, eab, npair, COUNT, ALSD || SPLIT);
       eel = elj = eaa = eab = 0;
       npair = 0;
       if (rep != cur_rep) {
@@ -734,10 +1069,10 @@ k_pair_fp64(DevPtrs P, ZdConst z) {
     int aj[2], tjv[2];
     double4 pj[2];
     for (int e = 0; e < 2; ++e) {
-      const int sj = valid ? __float_as_int(P.ct_j[(size_t)rec * 32 + kHalf * e + lp].w) : -1;
-      pj[e] = sj >= 0 ? P.pos_d[sj] : make_double4(0.0, 0.0, 0.0, 0.0);
-      tjv[e] = sj >= 0 ? P.styp[sj] : z.nt1 - 1;
-      aj[e] = sj >= 0 ? P.satom[sj] : -1;
+      const size_t o = (size_t)rec * 32 + kHalf * e + lp;
+      aj[e] = valid ? __float_as_int(P.ct_j[o].w) : -1;
+      tjv[e] = valid ? type_word(P.ct_ty[o]) : z.nt1 - 1;
+      pj[e] = aj[e] >= 0 ? P.pos_d[aj[e]] : make_double4(0.0, 0.0, 0.0, 0.0);
     }
     __syncwarp();
     S.pa[sidx] = pj[0];
@@ -823,56 +1158,77 @@ k_pair_fp64(DevPtrs P, ZdConst z) {
     if (ALSD || SPLIT) { eaa += to_fix(ta, kEneScale, P.status); eab += to_fix(tb, kEneScale, P.status); }
   }
   flush_i();
-  flush_fix(P, cur_rep, eel, elj, eaa, eab, npair, COUNT, ALSD || SPLIT);
+  flush_fix<16>(P, cur_rep, eel, elj, eaa, eab, npair, COUNT, ALSD || SPLIT);
 }
 
-// the mixed kernels that read the type-triple table need more than the default 48 KiB of
-// dynamic shared memory above 12 types: raised once, when a context is created
-static void allow_tri_smem(int nt1) {
-  const int b = (int)(lj_pair_bytes(nt1) + lj_tri_bytes(nt1));
-  cudaFuncSetAttribute(k_pair_mixed<false, false, false, false, true>,
-                       cudaFuncAttributeMaxDynamicSharedMemorySize, b);
-  cudaFuncSetAttribute(k_pair_mixed<true, false, false, false, true>,
-                       cudaFuncAttributeMaxDynamicSharedMemorySize, b);
+// the packed kernel's stages and table take more than the default 48 KiB of dynamic shared
+// memory: raised when a context is created
+template <bool TRI>
+static int packed_blocks_per_sm(int bytes) {
+  int per = 0;
+  cudaFuncSetAttribute(k_pair_packed<false, false, TRI>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  cudaFuncSetAttribute(k_pair_packed<true, false, TRI>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  cudaFuncSetAttribute(k_pair_packed<false, true, TRI>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  cudaFuncSetAttribute(k_pair_packed<true, true, TRI>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_pair_packed<false, false, TRI>, kPairThreads, bytes);
+  return per;
 }
 
-int pair_blocks_per_sm(bool fp64, int nt1) {
+// the LJ table of the packed kernel as it lies in shared memory: per type pair (-6 C6, 12 C12),
+// or per type triple (i, i', j) those of (i, j) and (i', j) side by side
+void pack_lj_table(const float2* lj, int nt1, std::vector<float>& out) {
+  out.assign(lj_bytes(nt1) / sizeof(float), 0.f);
+  size_t o = 0;
+  if (!lj_tri(nt1)) {
+    for (int i = 0; i < nt1 * nt1; ++i) {
+      out[o++] = -6.f * lj[i].x;
+      out[o++] = 12.f * lj[i].y;
+    }
+    return;
+  }
+  for (int a = 0; a < nt1; ++a)
+    for (int b = 0; b < nt1; ++b)
+      for (int j = 0; j < nt1; ++j) {
+        const float2 pa = lj[a * nt1 + j], pb = lj[b * nt1 + j];
+        out[o++] = -6.f * pa.x;
+        out[o++] = -6.f * pb.x;
+        out[o++] = 12.f * pa.y;
+        out[o++] = 12.f * pb.y;
+      }
+}
+
+int pair_blocks_per_sm(bool fp64, bool packed, int nt1) {
   int per = 0;
   if (fp64) {
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_pair_fp64<false, false, false>, kPairThreads,
                                                   sizeof(double2) * nt1 * nt1);
-  } else if (nt1 <= kTriMaxTypes) {
-    allow_tri_smem(nt1);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_pair_mixed<false, false, false, false, true>,
-                                                  kPairThreads, lj_pair_bytes(nt1) + lj_tri_bytes(nt1));
+  } else if (packed) {
+    const int bytes = (int)(kPackedStageBytes + lj_bytes(nt1));
+    per = lj_tri(nt1) ? packed_blocks_per_sm<true>(bytes) : packed_blocks_per_sm<false>(bytes);
   } else {
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_pair_mixed<false, false, false>, kPairThreads,
-                                                  lj_pair_bytes(nt1));
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_pair_mixed<false, true, false>, kPairThreads,
+                                                  sizeof(float2) * nt1 * nt1);
   }
   return per > 0 ? per : 1;
+}
+
+template <bool COUNT>
+static void launch_mixed(const DevPtrs& P, const ZdConst& z, int nb, bool alsd, bool split, cudaStream_t st) {
+  const size_t sh = sizeof(float2) * z.nt1 * z.nt1, shp = kPackedStageBytes + lj_bytes(z.nt1);
+  const bool tri = lj_tri(z.nt1);
+  if (split) k_pair_mixed<COUNT, false, true><<<nb, kPairThreads, sh, st>>>(P, z);
+  else if (z.cmm) k_pair_mixed<COUNT, true, false><<<nb, kPairThreads, sh, st>>>(P, z);
+  else if (alsd && tri) k_pair_packed<COUNT, true, true><<<nb, kPairThreads, shp, st>>>(P, z);
+  else if (alsd) k_pair_packed<COUNT, true, false><<<nb, kPairThreads, shp, st>>>(P, z);
+  else if (tri) k_pair_packed<COUNT, false, true><<<nb, kPairThreads, shp, st>>>(P, z);
+  else k_pair_packed<COUNT, false, false><<<nb, kPairThreads, shp, st>>>(P, z);
 }
 
 void launch_pair_mixed(const DevPtrs& P, const ZdConst& z, int nwarps, bool count, bool alsd, bool split,
                        cudaStream_t st) {
   const int nb = (nwarps + kPairWarps - 1) / kPairWarps;
-  const size_t sh = lj_pair_bytes(z.nt1);
-  if (split) {
-    if (count) k_pair_mixed<true, true, false, true><<<nb, kPairThreads, sh, st>>>(P, z);
-    else k_pair_mixed<false, true, false, true><<<nb, kPairThreads, sh, st>>>(P, z);
-  } else if (z.cmm) {
-    if (count) k_pair_mixed<true, false, true><<<nb, kPairThreads, sh, st>>>(P, z);
-    else k_pair_mixed<false, false, true><<<nb, kPairThreads, sh, st>>>(P, z);
-  } else if (alsd) {
-    if (count) k_pair_mixed<true, true, false><<<nb, kPairThreads, sh, st>>>(P, z);
-    else k_pair_mixed<false, true, false><<<nb, kPairThreads, sh, st>>>(P, z);
-  } else if (z.nt1 <= kTriMaxTypes) {   // LJ pairs from the type-triple table
-    const size_t sh3 = lj_pair_bytes(z.nt1) + lj_tri_bytes(z.nt1);
-    if (count) k_pair_mixed<true, false, false, false, true><<<nb, kPairThreads, sh3, st>>>(P, z);
-    else k_pair_mixed<false, false, false, false, true><<<nb, kPairThreads, sh3, st>>>(P, z);
-  } else {
-    if (count) k_pair_mixed<true, false, false><<<nb, kPairThreads, sh, st>>>(P, z);
-    else k_pair_mixed<false, false, false><<<nb, kPairThreads, sh, st>>>(P, z);
-  }
+  if (count) launch_mixed<true>(P, z, nb, alsd, split, st);
+  else launch_mixed<false>(P, z, nb, alsd, split, st);
 }
 
 void launch_pair_fp64(const DevPtrs& P, const ZdConst& z, int nwarps, bool count, bool alsd, bool split,
@@ -894,23 +1250,21 @@ void launch_pair_fp64(const DevPtrs& P, const ZdConst& z, int nwarps, bool count
   }
 }
 
-// slot positions from the master coordinates (after an external coordinate change)
-__global__ void k_update_pos(DevPtrs P, int nslot, int fp64, double qscale) {
-  int s = blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= nslot) return;
-  int a = P.satom[s];
-  if (a < 0) return;
+// kernel positions from the master coordinates (after an external coordinate change)
+__global__ void k_update_pos(DevPtrs P, int natom, int fp64, double qscale) {
+  const int a = blockIdx.x * blockDim.x + threadIdx.x;
+  if (a >= natom) return;
   const double x = P.x[3 * a], y = P.x[3 * a + 1], zz = P.x[3 * a + 2];
   if (fp64) {
-    P.pos_d[s] = make_double4(x, y, zz, qscale * P.chg[a]);
+    P.pos_d[a] = make_double4(x, y, zz, qscale * P.chg[a]);
   } else {
-    P.pos_f[s] = make_float4((float)(x - P.off[3 * s]), (float)(y - P.off[3 * s + 1]),
-                             (float)(zz - P.off[3 * s + 2]), (float)(qscale * P.chg[a]));
+    P.pos_f[a] = make_float4((float)(x - P.off[3 * a]), (float)(y - P.off[3 * a + 1]),
+                             (float)(zz - P.off[3 * a + 2]), (float)(qscale * P.chg[a]));
   }
 }
 
-void launch_update_pos(const DevPtrs& P, int nslot, bool fp64, double qscale, cudaStream_t st) {
-  k_update_pos<<<(nslot + 255) / 256, 256, 0, st>>>(P, nslot, fp64 ? 1 : 0, qscale);
+void launch_update_pos(const DevPtrs& P, int natom, bool fp64, double qscale, cudaStream_t st) {
+  k_update_pos<<<(natom + 255) / 256, 256, 0, st>>>(P, natom, fp64 ? 1 : 0, qscale);
 }
 
 }  // namespace jp
