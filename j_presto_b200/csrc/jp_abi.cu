@@ -1651,8 +1651,12 @@ int jp_create(const jp_system *sys, int32_t nrep, const jp_params *prm, jp_ctx *
   if (!e) P.tile_ctr = reinterpret_cast<int *>(P.ene_fix + 16 * (size_t)nrep);
   e |= dalloc(c, &P.kin_fix, (size_t)c->nkin * c->nsub);
   e |= dput(c, &P.nfr, hnfr);
+  std::vector<int> hsub_rep(c->nsub, 0);
+  for (int r = 0; r < nrep; ++r)
+    for (int q = 0; q < reps[r].nsub; ++q) hsub_rep[reps[r].sub0 + q] = r;
+  e |= dput(c, &P.sub_rep, hsub_rep);
   e |= dalloc(c, &P.scale, (size_t)nrep);
-  e |= dalloc(c, &P.done, (size_t)nrep);
+  e |= dalloc(c, &P.done, (size_t)nrep + 1);
   e |= dalloc(c, &P.rep_fail, (size_t)nrep);
   e |= dalloc(c, &P.lam_dew, (size_t)nrep);
   e |= dalloc(c, &P.lam_step, (size_t)5 * nrep);

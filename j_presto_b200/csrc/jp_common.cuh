@@ -248,8 +248,10 @@ struct DevPtrs {
   int *tile_ctr;                  // next unclaimed tile (zeroed with ene_fix every step)
   long long *kin_fix;             // [nslots_kin][nsub_total]
   double *nfr;                    // DOF per sub-system
+  int *sub_rep;                   // replica of each sub-system
   double *scale;                  // per replica force scale (GE / pseudo-T)
-  int *done;                      // per replica SHAKE-thermostat loop finished
+  int *done;                      // per replica: still in the SHAKE <-> thermostat loop (per-phase
+                                  // form, one pass at a time); [nrep]: any
   int *rep_fail;                  // per replica: a SHAKE group failed this step (1)
   // ALSD weight iteration, per replica: counts and sums of dE/dlambda of the cluster energy
   // per lambda bin [nrep][JP_ALSD_MAX_LBINS], and per (E, lambda) bin

@@ -24,8 +24,21 @@ constexpr int kCom = 16;   // centre-of-mass stop sums per replica and slot
 // the same over a 1-3 atom unit (the units of the small lanes: 4-atom groups take eight lanes)
 #define JP_SMALL_LOOP(q) _Pragma("unroll") for (int q = 0; q < 3; ++q) if (q < u.n)
 
+// Minimum image of a constraint's vector.  Adding and subtracting 1.5 * 2^52 rounds to the
+// nearest integer as anint does except at exact halves, which the ends of a bond never are
+// (they are angstroms apart); round() is 58 cycles of latency, the two additions 16, and a
+// water group images six vectors a SHAKE pass.
 __host__ __device__ __forceinline__ void mimg(const Rep& R, double* d) {
-  for (int k = 0; k < 3; ++k) d[k] -= R.box[k] * anint(d[k] * R.invbox[k]);
+  const double m = 6755399441055744.0;
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+#ifdef __CUDA_ARCH__
+    const double n = __dadd_rn(__dadd_rn(d[k] * R.invbox[k], m), -m);
+#else
+    const double n = anint(d[k] * R.invbox[k]);
+#endif
+    d[k] -= R.box[k] * n;
+  }
 }
 
 // A partial-McMD replica scales its class-1 gradient alone (verlet.f90:130-141,
@@ -370,6 +383,45 @@ __device__ bool cano_active(const DevPtrs& P, const IntConst& c, const Rep& R, i
   return true;
 }
 
+// The first converged pass of each of the first kActCache replicas among passes 1 .. last
+// (INT_MAX: none), evaluated by the whole block with one sub-system and pass per thread, so
+// that all their loads are in flight together.  One thread per replica that walks its
+// sub-systems and passes (the form above, kept for replicas beyond the cache) takes a memory
+// latency and a division for each: 3,000 cycles at the first pass of a solvated chain's step
+// and 5,000 at the second, so under
+// 1,300 either time.
+constexpr int kActCache = 1024;
+constexpr int kPassBits = 24;                 // passes a word holds at a time
+constexpr unsigned kHasSub = 0x80000000u;     // a thermostatted sub-system (else never converged)
+
+struct LoopState {
+  int first[kActCache];        // first converged pass
+  unsigned off[kActCache];     // passes with a sub-system out of tolerance
+};
+
+__device__ void loop_first(const DevPtrs& P, const IntConst& c, int last, double tt, LoopState& L) {
+  const int nr = min(c.nrep, kActCache);
+  const int ns = c.nrep <= kActCache ? c.nsub_total : P.reps[kActCache].sub0;   // sub-systems go by replica
+  for (int r = threadIdx.x; r < nr; r += blockDim.x) L.first[r] = 0x7fffffff;
+  for (int q0 = 1; q0 <= last; q0 += kPassBits) {
+    const int m = min(kPassBits, last - q0 + 1);
+    for (int r = threadIdx.x; r < nr; r += blockDim.x) L.off[r] = 0u;
+    __syncthreads();
+    for (int e = threadIdx.x; e < m * ns; e += blockDim.x) {
+      const int q = e / ns, sub = e % ns;
+      if (P.nfr[sub] <= 0.0) continue;
+      const bool off = !(fabs(sub_temp(P, c, 2 * (q0 + q) - 1, sub) - tt) < c.fcstol * tt);
+      atomicOr(&L.off[P.sub_rep[sub]], kHasSub | (off ? 1u << q : 0u));
+    }
+    __syncthreads();
+    for (int r = threadIdx.x; r < nr; r += blockDim.x) {
+      const unsigned on = (L.off[r] & kHasSub) ? ~L.off[r] & ((1u << m) - 1u) : 0u;
+      if (on && L.first[r] == 0x7fffffff) L.first[r] = q0 + __ffs(on) - 1;
+    }
+  }
+  __syncthreads();
+}
+
 // ---- per-replica preparation --------------------------------------------------------
 // force scale of replica r for this step: McMD weight (verlethe.f90:196-238) from the total
 // potential energy, or the pseudo-temperature factor (verlet.f90:118-142)
@@ -609,26 +661,37 @@ __device__ __forceinline__ bool grid_barrier(const DevPtrs& P, unsigned& epoch) 
   return s_ok != 0;
 }
 
-// end of step, one block after all others have finished: temperature of each replica (the kinetic
-// slot of the last SHAKE pass, i.e. of (v(t-dt/2)+v(t+dt/2))/2) and the step counters
-__device__ void finish_block(const DevPtrs& P, const IntConst& c, double tt) {
+// end of step, one block after all others have finished: temperature of each replica (the
+// kinetic slot of the last SHAKE pass, i.e. of (v(t-dt/2)+v(t+dt/2))/2) and the step counters
+__device__ void finish_block(const DevPtrs& P, const IntConst& c, double tt, LoopState* L) {
   const int h = P.step_ctr[1];
-  for (int r = threadIdx.x; r < c.nrep; r += blockDim.x) {
+  const bool loop = c.method > JP_METHOD_MICR && c.shake_method != JP_SHAKE_NONE;   // verlethe
+  if (loop) loop_first(P, c, c.icslop - 1, tt, *L);
+  // one warp per replica, a lane per sub-system; the sums in the order of the sub-systems
+  const int lane = threadIdx.x & 31;
+  for (int r = threadIdx.x >> 5; r < c.nrep; r += blockDim.x >> 5) {
     const Rep& R = P.reps[r];
     int ks = c.nkin - 1;   // MICR
-    if (c.method > JP_METHOD_MICR && c.shake_method != JP_SHAKE_NONE) {   // verlethe
-      int q = 1;
-      for (; q < c.icslop; ++q)
-        if (cano_conv(P, c, R, q, tt)) break;
+    if (loop) {
+      int q = c.icslop;
+      if (r < kActCache) q = min(q, L->first[r]);
+      else for (q = 1; q < c.icslop; ++q) if (cano_conv(P, c, R, q, tt)) break;
       ks = 2 * q - 1;
     }
     double ek = 0.0, nf = 0.0;
-    for (int s = R.sub0; s < R.sub0 + R.nsub; ++s) {
-      ek += (double)__ldcg(&P.kin_fix[(size_t)ks * c.nsub_total + s]) * kKinInv;
-      nf += P.nfr[s];
+    for (int s0 = 0; s0 < R.nsub; s0 += 32) {
+      const int sub = R.sub0 + s0 + lane;
+      const bool in = s0 + lane < R.nsub;
+      const double e = in ? (double)__ldcg(&P.kin_fix[(size_t)ks * c.nsub_total + sub]) * kKinInv : 0.0;
+      const double n = in ? P.nfr[sub] : 0.0;
+      for (int k = 0; k < min(32, R.nsub - s0); ++k) {
+        ek += __shfl_sync(0xffffffffu, e, k);
+        nf += __shfl_sync(0xffffffffu, n, k);
+      }
     }
-    P.temp_hist[(size_t)h * c.nrep + r] =
-        (c.method <= JP_METHOD_MICR || c.shake_method != JP_SHAKE_NONE) ? ek * 1.0e7 / (kGas * nf) : -1.0;
+    if (lane == 0)
+      P.temp_hist[(size_t)h * c.nrep + r] =
+          (c.method <= JP_METHOD_MICR || c.shake_method != JP_SHAKE_NONE) ? ek * 1.0e7 / (kGas * nf) : -1.0;
   }
   __syncthreads();
   // the next step starts from zero kinetic (and centre-of-mass) sums and a fresh barrier:
@@ -642,7 +705,7 @@ __device__ void finish_block(const DevPtrs& P, const IntConst& c, double tt) {
     for (int i = threadIdx.x; i < c.ncom * c.nrep * kCom; i += blockDim.x) P.com[i] = 0.0;
   if (threadIdx.x == 0) {
     P.step_ctr[0] += 1;
-    P.step_ctr[1] += 1;
+    P.step_ctr[1] = h + 1;
     P.bar[0] = 0u;
     P.bar[1] = 0u;
     P.bar[2] = 0u;
@@ -651,30 +714,24 @@ __device__ void finish_block(const DevPtrs& P, const IntConst& c, double tt) {
 }
 
 // is any replica still iterating the SHAKE <-> thermostat loop at pass `it`?  The same answer
-// in every block: all read the kinetic sums completed before the last grid barrier.
-// The block also keeps each replica's answer in s_act (replicas below kActCache), so the
-// lanes of the pass read a shared flag instead of re-reading the kinetic sums.
-constexpr int kActCache = 1024;
-
-__device__ bool any_active(const DevPtrs& P, const IntConst& c, int it, double tt,
-                           unsigned char* s_act) {
+// in every block: all read the kinetic sums completed before the last grid barrier.  The lanes
+// of the pass read their replica's first converged pass from the block's state.
+__device__ bool any_active(const DevPtrs& P, const IntConst& c, int it, double tt, LoopState& L) {
+  loop_first(P, c, it, tt, L);
   int act = 0;
-  for (int r = threadIdx.x; r < c.nrep; r += blockDim.x) {
-    const bool a = cano_active(P, c, P.reps[r], it, true, tt);
-    if (r < kActCache) s_act[r] = a ? 1 : 0;
-    act |= a ? 1 : 0;
-  }
-  return __syncthreads_or(act) != 0;   // also publishes s_act to the block
+  for (int r = threadIdx.x; r < c.nrep; r += blockDim.x)
+    act |= r < kActCache ? L.first[r] > it : cano_active(P, c, P.reps[r], it, true, tt);
+  return __syncthreads_or(act) != 0;
 }
 
-// is replica r still iterating at pass `it` (after any_active filled s_act)?
-__device__ __forceinline__ bool rep_active(const DevPtrs& P, const IntConst& c, const unsigned char* s_act,
-                                           int r, int it, double tt) {
-  return r < kActCache ? s_act[r] != 0 : cano_active(P, c, P.reps[r], it, true, tt);
+// is replica r still iterating at pass `it` (after any_active filled the state)?
+__device__ __forceinline__ bool rep_active(const DevPtrs& P, const IntConst& c, const LoopState& L, int r, int it,
+                                           double tt) {
+  return r < kActCache ? L.first[r] > it : cano_active(P, c, P.reps[r], it, true, tt);
 }
 
 // the last block to finish the step computes the temperatures and advances the step counters
-__device__ void finish_last(const DevPtrs& P, const IntConst& c, double tt) {
+__device__ void finish_last(const DevPtrs& P, const IntConst& c, double tt, LoopState* L) {
   __shared__ int s_last;
   __syncthreads();
   if (threadIdx.x == 0) {
@@ -683,7 +740,7 @@ __device__ void finish_last(const DevPtrs& P, const IntConst& c, double tt) {
     __threadfence();
   }
   __syncthreads();
-  if (s_last) finish_block(P, c, tt);
+  if (s_last) finish_block(P, c, tt, L);
 }
 
 // ---- centre-of-mass stop (remotv.f90:2-131) ----------------------------------------------
@@ -1000,7 +1057,7 @@ __global__ void __launch_bounds__(64) k_micr_fused(DevPtrs P, IntConst c, int nu
       add_kin(P, c.nsub_total, c.nkin - 1, sub, ke);
     }
   }
-  finish_last(P, c, c.temp);
+  finish_last(P, c, c.temp, nullptr);   // no loop in verlet
 }
 
 // ---- METHOD= CANO / GE: verlethe.f90 ----------------------------------------------------
@@ -1511,11 +1568,97 @@ __device__ __forceinline__ void add_kin_quad(const DevPtrs& P, int nsub_total, i
   }
 }
 
-// shake4 (shake.f90:333-562) for one group spread over its 8 lanes: each constraint lane
-// builds its row of the Newton matrix, the LU with partial pivoting (simulu) eliminates the
-// rows held by the lanes that are not yet pivots, and back substitution broadcasts G one
-// entry at a time.  Same iteration, pivot rule, elimination arithmetic and convergence test
-// as the serial form.  x (in/out) and x0 are this lane's atom (lanes 0-3).  Returns 0, 1 (not
+// A group's Newton system with partial pivoting (simulu): each constraint lane holds its row, the
+// rows of the lanes that are not yet pivots are eliminated, and back substitution broadcasts
+// the solution one entry at a time.  Every lane of the warp runs the shuffles.  lu_ok: no pivot
+// of the group vanishes (simulu's 1e-30).  Out of line: quad_solve below takes nearly every
+// system.
+__device__ __noinline__ void quad_solve_pivot(const double (&row)[6], double B, bool con, int sl, double (&G)[6],
+                                              bool& lu_ok) {
+  const unsigned full = 0xffffffffu;
+  double A[6];
+#pragma unroll
+  for (int j = 0; j < 6; ++j) A[j] = row[j];
+  bool used = !con;
+  int perm[6];
+  lu_ok = true;
+#pragma unroll
+  for (int k = 0; k < 6; ++k) {
+    double bv = used ? -1.0 : fabs(A[k]);
+    int bl = sl;
+#pragma unroll
+    for (int off = 4; off > 0; off >>= 1) {
+      const double ov = __shfl_xor_sync(full, bv, off, 8);
+      const int ol = __shfl_xor_sync(full, bl, off, 8);
+      if (ov > bv || (ov == bv && ol < bl)) { bv = ov; bl = ol; }
+    }
+    perm[k] = bl;
+    double pk[6];
+#pragma unroll
+    for (int j = k; j < 6; ++j) pk[j] = __shfl_sync(full, A[j], bl, 8);
+    const double pb = __shfl_sync(full, B, bl, 8);
+    if (fabs(pk[k]) < 1.0e-30) lu_ok = false;
+    const double piv = recip_nr(pk[k]);
+    if (sl == bl) {
+      used = true;
+      A[k] = piv;
+    } else if (!used) {
+      const double f = A[k] * piv;
+#pragma unroll
+      for (int j = k + 1; j < 6; ++j) A[j] -= f * pk[j];
+      B -= f * pb;
+    }
+  }
+#pragma unroll
+  for (int i = 5; i >= 0; --i) {   // every lane keeps its row's right-hand side up to date
+    G[i] = __shfl_sync(full, B * A[i], perm[i], 8);
+    B -= A[i] * G[i];
+  }
+}
+
+// The same system in the natural pivot order, every lane of the group solving all of it: one
+// gather of the six rows (42 doubles), then no lane waits for another.  A pivot search and a
+// broadcast before each elimination step were 26-cycle shuffles in a serial chain, 2,400 cycles
+// a Newton step against 1,700.  The gradient matrix is close to symmetric and positive definite
+// (it is where the bonds point as they did before the step), so the natural order is stable;
+// false, the same in every lane of the warp, if an entry below a pivot of an unfinished group
+// is more than 16 times that pivot (1.6 times on methyl groups) or a pivot vanishes.
+__device__ __forceinline__ bool quad_solve(const double (&row)[6], double B0, bool done, double (&G)[6]) {
+  const unsigned full = 0xffffffffu;
+  double A[6][6], B[6];
+#pragma unroll
+  for (int i = 0; i < 6; ++i) {
+#pragma unroll
+    for (int j = 0; j < 6; ++j) A[i][j] = __shfl_sync(full, row[j], i, 8);
+    B[i] = __shfl_sync(full, B0, i, 8);
+  }
+  bool weak = false;
+#pragma unroll
+  for (int k = 0; k < 6; ++k) {
+    const double lim = 16.0 * fabs(A[k][k]);
+    weak |= !(lim >= 1.6e-29);
+    const double piv = recip_nr(A[k][k]);
+#pragma unroll
+    for (int i = k + 1; i < 6; ++i) {
+      weak |= !(fabs(A[i][k]) <= lim);
+      const double f = A[i][k] * piv;
+#pragma unroll
+      for (int j = k + 1; j < 6; ++j) A[i][j] -= f * A[k][j];
+      B[i] -= f * B[k];
+    }
+    A[k][k] = piv;
+  }
+#pragma unroll
+  for (int i = 5; i >= 0; --i) {
+    G[i] = B[i] * A[i][i];
+#pragma unroll
+    for (int j = 0; j < i; ++j) B[j] -= A[j][i] * G[i];
+  }
+  return !__any_sync(full, weak && !done);
+}
+
+// shake4 (shake.f90:333-562) for one group spread over its 8 lanes: the same Newton iteration
+// and convergence test as the serial form.  x (in/out) and x0 are this lane's atom (lanes 0-3).  Returns 0, 1 (not
 // converged) or -2 (singular), the same value in all lanes of the group.
 __device__ int quad_shake(const Rep& R, const QLane& q, double x[3], const double x0[3], double tol,
                           int maxit) {
@@ -1535,15 +1678,22 @@ __device__ int quad_shake(const Rep& R, const QLane& q, double x[3], const doubl
   }
   mimg(R, d1);
   mimg(R, d2);
-  double D2[6][3], im4[4], cr[6];
+  double D2[6][3], cr[6];
 #pragma unroll
   for (int ig = 0; ig < 6; ++ig)
 #pragma unroll
     for (int k = 0; k < 3; ++k) D2[ig][k] = __shfl_sync(full, d2[k], ig, 8);
+  // this constraint's row of coeg (cg4): +-1/m of an end that constraint ig shares, by selects
+  // (cg4's switch with a lane-dependent row ran its cases one after the other, 6,000 cycles)
+  const double imi = __shfl_sync(full, q.im, pi_, 8), imj = __shfl_sync(full, q.im, pj_, 8);
 #pragma unroll
-  for (int a = 0; a < 4; ++a) im4[a] = __shfl_sync(full, q.im, a, 8);
-#pragma unroll
-  for (int ig = 0; ig < 6; ++ig) cr[ig] = sl < 6 ? cg4(sl, ig, im4) : 0.0;
+  for (int ig = 0; ig < 6; ++ig) {
+    const int a = ig == 0 ? 0 : ig == 1 ? 1 : ig == 2 ? 2 : ig == 3 ? 3 : ig == 4 ? 2 : 1;
+    const int b = ig == 0 ? 1 : ig == 1 ? 2 : ig == 2 ? 0 : ig == 3 ? 0 : 3;
+    const double ci = pi_ == a ? imi : pi_ == b ? -imi : 0.0;
+    const double cj = pj_ == a ? imj : pj_ == b ? -imj : 0.0;
+    cr[ig] = sl < 6 ? ci - cj : 0.0;
+  }
   double wk[3] = {d1[0], d1[1], d1[2]};
   double G[6] = {0, 0, 0, 0, 0, 0};
   bool done = !q.grp;
@@ -1569,57 +1719,18 @@ __device__ int quad_shake(const Rep& R, const QLane& q, double x[3], const doubl
       }
     }
     if (__all_sync(full, done)) return q.grp ? ret : 0;
-    // gradient matrix row of this constraint and the right-hand side
-    double A[6];
+    // the Newton step's increment of G from this constraint's row and residual (md_run solves
+    // for G itself, from the residual plus the row times the last G: the same step)
+    double row[6], dG[6];
 #pragma unroll
     for (int ig = 0; ig < 6; ++ig)
-      A[ig] = 2.0 * cr[ig] * (wk[0] * D2[ig][0] + wk[1] * D2[ig][1] + wk[2] * D2[ig][2]);
-    double B = B0;
-#pragma unroll
-    for (int ig = 0; ig < 6; ++ig) B += A[ig] * G[ig];
-    // LU with partial pivoting over the constraint lanes
-    bool used = !con;
+      row[ig] = 2.0 * cr[ig] * (wk[0] * D2[ig][0] + wk[1] * D2[ig][1] + wk[2] * D2[ig][2]);
     bool lu_ok = true;
-    int perm[6];
-#pragma unroll
-    for (int k = 0; k < 6; ++k) {
-      double bv = used ? -1.0 : fabs(A[k]);
-      int bl = sl;
-#pragma unroll
-      for (int off = 4; off > 0; off >>= 1) {
-        const double ov = __shfl_xor_sync(full, bv, off, 8);
-        const int ol = __shfl_xor_sync(full, bl, off, 8);
-        if (ov > bv || (ov == bv && ol < bl)) { bv = ov; bl = ol; }
-      }
-      perm[k] = bl;
-      double pk[6];
-#pragma unroll
-      for (int j = k; j < 6; ++j) pk[j] = __shfl_sync(full, A[j], bl, 8);
-      const double pb = __shfl_sync(full, B, bl, 8);
-      if (fabs(pk[k]) < 1.0e-30) lu_ok = false;
-      const double piv = recip_nr(pk[k]);
-      if (sl == bl) {
-        used = true;
-        A[k] = piv;
-      } else if (!used) {
-        const double f = A[k] * piv;
-#pragma unroll
-        for (int j = k + 1; j < 6; ++j) A[j] -= f * pk[j];
-        B -= f * pb;
-      }
-    }
-    // back substitution: every lane of the warp runs the shuffles (lu_ok and done differ
-    // between the groups of a warp); only a live group with a regular matrix takes the result
-    const bool take = lu_ok && !done;
+    if (!quad_solve(row, B0, done, dG)) quad_solve_pivot(row, B0, con, sl, dG, lu_ok);
     if (!lu_ok && !done) singular = true;
+    if (lu_ok && !done)
 #pragma unroll
-    for (int i = 5; i >= 0; --i) {
-      double t = B;
-#pragma unroll
-      for (int j = i + 1; j < 6; ++j) t -= A[j] * G[j];
-      const double gi = __shfl_sync(full, t * A[i], perm[i], 8);
-      if (take) G[i] = gi;
-    }
+      for (int i = 0; i < 6; ++i) G[i] += dG[i];
     if (!done) {
 #pragma unroll
       for (int k = 0; k < 3; ++k) {
@@ -1899,7 +2010,7 @@ __device__ __forceinline__ void fix_unit(const DevPtrs& P, const IntConst& c, in
 template <bool FP64, bool STOP>
 __global__ void __launch_bounds__(kIntThreads) k_cano_fused(DevPtrs P, IntConst c) {
   __shared__ UnitSmem S;
-  __shared__ unsigned char s_act[kActCache];   // replicas still in the SHAKE<->thermostat loop
+  __shared__ LoopState s_act;   // the SHAKE<->thermostat loop of each replica
   const int gt = blockIdx.x * blockDim.x + threadIdx.x;
   const int tid = threadIdx.x;
   const double tt = target_temp(c, (long long)P.step_ctr[0] + 1);
@@ -2089,7 +2200,7 @@ __global__ void __launch_bounds__(kIntThreads) k_cano_fused(DevPtrs P, IntConst 
     P.lam[2 * gt] = L.lam;
     P.lam[2 * gt + 1] = L.lv;
   }
-  finish_last(P, c, tt);
+  finish_last(P, c, tt, &s_act);
 }
 
 // ---- METHOD= CANO / GE, streaming form: one launch per phase -------------------------------
@@ -2131,10 +2242,20 @@ __device__ __forceinline__ void lam_load(const DevPtrs& P, int r, LamStep& L) {
 // KIND 0: the 1-3 atom units [0, nsmall) and the per-replica threads (energy record,
 // lambda); KIND 1: the 4-atom group lanes [qbase, nvirt) (a launch of its own, as their
 // SHAKE needs several times the registers); KIND 2 (PH_END only): every lane.
+// which replicas still iterate at pass `it` (done[r]; done[nrep]: any), once for the pass's
+// launches.  With the test in every block of every launch, a batch of 64 replicas spent 1.5 us
+// more in each of them than this launch takes in all.
+__global__ void __launch_bounds__(1024) k_cano_loop(DevPtrs P, IntConst c, int it) {
+  __shared__ LoopState s_act;
+  const double tt = target_temp(c, (long long)P.step_ctr[0] + 1);
+  const bool any = any_active(P, c, it, tt, s_act);
+  for (int r = threadIdx.x; r < c.nrep; r += blockDim.x) P.done[r] = rep_active(P, c, s_act, r, it, tt) ? 1 : 0;
+  if (threadIdx.x == 0) P.done[c.nrep] = any ? 1 : 0;
+}
+
 template <bool FP64, bool STOP, int PH, int KIND>
 __global__ void __launch_bounds__(kIntThreads, KIND == 1 ? 4 : kPhaseBlocks) k_cano_phase(DevPtrs P, IntConst c, int it) {
   __shared__ QuadSmem S;
-  __shared__ unsigned char s_act[kActCache];
   const int v = (KIND == 1 ? c.qbase : 0) + blockIdx.x * blockDim.x + threadIdx.x;
   const int tid = threadIdx.x;
   const double tt = target_temp(c, (long long)P.step_ctr[0] + 1);
@@ -2207,11 +2328,11 @@ __global__ void __launch_bounds__(kIntThreads, KIND == 1 ? 4 : kPhaseBlocks) k_c
     }
   } else if (PH == PH_FIX) {
     // after phase 2 (it = 0, every replica) or after phase 5 of pass it
-    if (it > 0 && !any_active(P, c, it, tt, s_act)) return;
+    if (it > 0 && !P.done[c.nrep]) return;
     const int ks = it == 0 ? 1 : 2 * it + 1;
     if (quad) {
       const QLane q = ql_make(P, c, v);
-      const bool act = it == 0 || (q.grp && rep_active(P, c, s_act, q.rep, it, tt));
+      const bool act = it == 0 || (q.grp && P.done[q.rep]);
       q_fetch(P, q, S, tid, false);
       if (act) fix_quad(P, c, it, q, S, tid);
       const double ke = q_cano3(P, c, q, S, tid);
@@ -2222,7 +2343,7 @@ __global__ void __launch_bounds__(kIntThreads, KIND == 1 ? 4 : kPhaseBlocks) k_c
       int sub = -1;
       if (small) {
         const Unit u = P.units[P.small_idx[v]];
-        if (it == 0 || rep_active(P, c, s_act, u.rep, it, tt)) {
+        if (it == 0 || P.done[u.rep]) {
           fix_unit(P, c, it, u, shk, FP64);
           if (shk) {
             sub = u.sub;
@@ -2233,9 +2354,9 @@ __global__ void __launch_bounds__(kIntThreads, KIND == 1 ? 4 : kPhaseBlocks) k_c
       if (shk) add_kin(P, c.nsub_total, ks, sub, ke);
     }
   } else if (PH == PH_CORR) {
-    if (!any_active(P, c, it, tt, s_act)) return;
+    if (!P.done[c.nrep]) return;
     // lambda's velocity stays (v_back + v)/2 through the loop (verlethe.f90:529)
-    if (lam_thread && rep_active(P, c, s_act, v, it, tt)) {
+    if (lam_thread && P.done[v]) {
       LamStep L;
       lam_load(P, v, L);
       lam_add_ke(P, c, P.reps[v], 2 * it, L.lvt);
@@ -2243,7 +2364,7 @@ __global__ void __launch_bounds__(kIntThreads, KIND == 1 ? 4 : kPhaseBlocks) k_c
     }
     if (quad) {
       const QLane q = ql_make(P, c, v);
-      const bool act = q.grp && rep_active(P, c, s_act, q.rep, it, tt);
+      const bool act = q.grp && P.done[q.rep];
       q_fetch(P, q, S, tid, false);
       const double ke = q_cano4<FP64>(P, c, q, S, tid, rep_scale(P, c, q.rep));
       if (act) q_spill(P, c, q, S, tid, FP64);
@@ -2253,7 +2374,7 @@ __global__ void __launch_bounds__(kIntThreads, KIND == 1 ? 4 : kPhaseBlocks) k_c
       int sub = -1;
       if (small) {
         const Unit u = P.units[P.small_idx[v]];
-        if (rep_active(P, c, s_act, u.rep, it, tt)) {
+        if (P.done[u.rep]) {
           sub = u.sub;
           ke = cano4_unit<FP64>(P, c, u, rep_scale(P, c, u.rep));
         }
@@ -2261,13 +2382,13 @@ __global__ void __launch_bounds__(kIntThreads, KIND == 1 ? 4 : kPhaseBlocks) k_c
       add_kin(P, c.nsub_total, 2 * it, sub, ke);
     }
   } else if (PH == PH_RESCALE) {
-    if (!any_active(P, c, it, tt, s_act)) return;
+    if (!P.done[c.nrep]) return;
     if (split) {
       double w[kCom];
       int rep = -1;
       if (quad) {
         const QLane q = ql_make(P, c, v);
-        if (q.grp && rep_active(P, c, s_act, q.rep, it, tt)) {
+        if (q.grp && P.done[q.rep]) {
           q_fetch(P, q, S, tid, false);
           q_cano5<FP64>(P, c, q, S, tid, rep_scale(P, c, q.rep), sqrt(tt / sub_temp(P, c, 2 * it, q.sub)));
           rep = com_quad(P, c, q, S, tid, w);
@@ -2275,7 +2396,7 @@ __global__ void __launch_bounds__(kIntThreads, KIND == 1 ? 4 : kPhaseBlocks) k_c
         }
       } else if (small) {
         const Unit u = P.units[P.small_idx[v]];
-        if (rep_active(P, c, s_act, u.rep, it, tt)) {
+        if (P.done[u.rep]) {
           cano5_unit<FP64>(P, c, u, rep_scale(P, c, u.rep), it, tt);
           rep = com_unit(P, c, u, w);
         }
@@ -2283,7 +2404,7 @@ __global__ void __launch_bounds__(kIntThreads, KIND == 1 ? 4 : kPhaseBlocks) k_c
       com_add(P, c, it, rep, w);
     } else if (quad) {
       const QLane q = ql_make(P, c, v);
-      const bool act = q.grp && rep_active(P, c, s_act, q.rep, it, tt);
+      const bool act = q.grp && P.done[q.rep];
       q_fetch(P, q, S, tid, false);
       if (act)
         q_cano5<FP64>(P, c, q, S, tid, rep_scale(P, c, q.rep), sqrt(tt / sub_temp(P, c, 2 * it, q.sub)));
@@ -2295,7 +2416,7 @@ __global__ void __launch_bounds__(kIntThreads, KIND == 1 ? 4 : kPhaseBlocks) k_c
       int sub = -1;
       if (small) {
         const Unit u = P.units[P.small_idx[v]];
-        if (rep_active(P, c, s_act, u.rep, it, tt)) {
+        if (P.done[u.rep]) {
           sub = u.sub;
           ke = cano53_unit<FP64>(P, c, u, rep_scale(P, c, u.rep), it, tt);
         }
@@ -2316,7 +2437,8 @@ __global__ void __launch_bounds__(kIntThreads, KIND == 1 ? 4 : kPhaseBlocks) k_c
       P.lam[2 * v] = L.lam;
       P.lam[2 * v + 1] = L.lv;
     }
-    finish_last(P, c, tt);
+    __shared__ LoopState s_act;
+    finish_last(P, c, tt, &s_act);
   }
 }
 
@@ -2409,6 +2531,7 @@ static void launch_cano_phases(const DevPtrs& P, const IntConst& c, cudaStream_t
   if (STOP) launch_phase<FP64, STOP, PH_FIX>(P, c, 0, st);
   if (shk) {
     for (int it = 1; it < c.icslop; ++it) {
+      k_cano_loop<<<1, 1024, 0, st>>>(P, c, it);
       launch_phase<FP64, STOP, PH_CORR>(P, c, it, st);
       launch_phase<FP64, STOP, PH_RESCALE>(P, c, it, st);
       if (STOP) launch_phase<FP64, STOP, PH_FIX>(P, c, it, st);
@@ -2424,6 +2547,7 @@ int integrate_launches(const IntConst& c, int grid_max) {
   int phases = 2 + (stop ? 1 : 0);
   if (shk) phases += std::max(0, c.icslop - 1) * (stop ? 3 : 2);
   int n = phases * (c.nvirt > c.qbase ? 2 : 1) + 1;            // + PH_END
+  if (shk) n += std::max(0, c.icslop - 1);                     // k_cano_loop
   if (c.method == JP_METHOD_GE && !c.ge_prescaled) n += 1;   // k_ge_scale
   return n;
 }
