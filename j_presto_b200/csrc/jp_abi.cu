@@ -58,7 +58,7 @@ struct jp_ctx {
   int device = 0;
   int natom = 0, nblk = 0, nslot = 0, nunit = 0, nterm = 0, nsub = 0, nkeys = 0, nkin = 8;
   int ncol = 0;
-  int tile_cap_total = 0, nchunk = 0;
+  size_t tile_cap_total = 0;        // block pairs of all replicas: every one could be a tile
   std::vector<Rep> reps;
   std::vector<int> rep_natom;
   DevPtrs P{};
@@ -72,6 +72,7 @@ struct jp_ctx {
   bool alsd = false;                // some replica has ALSD classes (lambda)
   bool split = false;               // some replica keeps partial-McMD class-1 forces apart
   bool classes = false;             // alsd or split: class energies are kept
+  bool every_cls = false;           // class weights set to one class at a time (jp_energy_grad_cls)
   bool cmm = false;                 // CAL15M= CMM
   bool hbond = false;               // some type pair has the 10-12 H-bond term
   int hb_cap = 0;                   // capacity of the H-bond pair list
@@ -178,6 +179,9 @@ void enqueue_rebuild(jp_ctx *c, bool count_only = false) {
   cudaMemsetAsync(P.hist, 0, sizeof(int) * (c->nkeys + 1), st);
   cudaMemsetAsync(P.cursor, 0, sizeof(int) * (c->nkeys + 1), st);
   cudaMemsetAsync(P.rep_hmax, 0, sizeof(float) * 3 * c->nrep, st);
+  cudaMemsetAsync(P.nctiles, 0, 2 * sizeof(int), st);
+  cudaMemsetAsync(P.ext_pos, 0, sizeof(int), st);
+  if (c->hbond) cudaMemsetAsync(P.ntiles, 0, sizeof(int), st);
   int ncmm = 0;
   if (c->cmm) {   // celpar_CB + celoth + celpol: cells and multipoles at this rebuild
     int ntot = 0;
@@ -189,7 +193,7 @@ void enqueue_rebuild(jp_ctx *c, bool count_only = false) {
     ncmm = 3 + std::max(0, c->cmm_nlev - 1);
   }
   k_cell_key<<<(c->natom + nt - 1) / nt, nt, 0, st>>>(P, c->natom);
-  int nl = 10;   // the single kernels below
+  int nl = 9;   // the single kernels below
   nl += scan_exclusive(P.hist, P.hist_scan, c->nkeys + 1, c->scan_scratch, nullptr, st);
   k_scatter<<<(c->natom + nt - 1) / nt, nt, 0, st>>>(P, c->natom);
   k_sort_bins<<<(c->nkeys + nt - 1) / nt, nt, 0, st>>>(P, c->nkeys);
@@ -201,14 +205,8 @@ void enqueue_rebuild(jp_ctx *c, bool count_only = false) {
   k_block_setup<<<(c->nblk * 32 + nt - 1) / nt, nt, 0, st>>>(P, c->nblk, c->qscale);
   const double rlim = c->zc.rlim;   // rc + 1.5; CMM: the farthest near-field pair
   const double rc = c->prm.cutoff;
-  const int nwb = (c->nchunk * 32 + 127) / 128;
-  launch_tile_scan(P, c->nchunk, rlim * rlim, (float)rlim, rc * rc, c->cmm, st);
-  nl += scan_exclusive(P.chunk_cnt, P.chunk_off, c->nchunk + 1, c->scan_scratch, P.ntiles, st);
-  for (int h = 0; h < 2; ++h)   // the entries of each half block
-    nl += scan_exclusive(P.chunk_ent + h * (c->nchunk + 1), P.chunk_eoff + h * (c->nchunk + 1), c->nchunk + 1,
-                         c->scan_scratch, nullptr, st);
-  k_tile_emit<<<nwb, 128, 0, st>>>(P, c->nchunk, c->cmm ? 1 : 0);
-  nl += launch_compact_tiles(P, c->nblk, c->nchunk, c->nsm, c->cmm, c->zc.nt1 - 1, c->scan_scratch, count_only, st);
+  launch_block_list(P, c->nblk, c->nsm, rlim * rlim, (float)rlim, rc * rc, c->cmm, c->zc.nt1 - 1, count_only,
+                    c->hbond, c->alsd && !c->fp64, st);
   if (count_only) return;
   if (c->hbond) launch_hb_list(P, c->hb_cap, c->zc.nt1, c->nblk, st);
   c->launches_rebuild = nl + ncmm + (c->hbond ? 1 : 0);
@@ -231,7 +229,7 @@ void enqueue_zero(jp_ctx *c, bool count) {
 // steps by the step counter, or always with force_far: a single-point evaluation)
 void enqueue_pair(jp_ctx *c, bool count, bool force_far = false) {
   if (c->fp64) launch_pair_fp64(c->P, c->zc, c->pair_warps, count, c->alsd, c->split, c->st);
-  else launch_pair_mixed(c->P, c->zc, c->pair_warps, count, c->alsd, c->split, c->st);
+  else launch_pair_mixed(c->P, c->zc, c->pair_warps, count, c->alsd, c->every_cls, c->split, c->st);
   if (c->hbond) launch_hbond(c->P, c->hb_cap, c->zc.rc2, c->zc.nt1, c->fp64, c->classes, c->st);
   if (c->cmm) launch_cmm_far(c->P, c->natom, c->nrep, c->fp64, force_far, c->qscale * c->qscale, c->st);
 }
@@ -265,6 +263,7 @@ int launches_per_step(const jp_ctx *c) {
   n += c->ic.ge_prescaled ? 1 : 0; // k_ge_scale
   n += c->cmm ? 2 : 0;             // k_cmm_far, k_cmm_energy
   n += c->hbond ? 1 : 0;           // k_hbond
+  n += c->alsd && !c->fp64 ? 1 : 0;   // the records with cluster atoms
   n += c->nres > 0 ? 1 : 0;        // k_restraints
   return n;
 }
@@ -1522,19 +1521,13 @@ int jp_create(const jp_system *sys, int32_t nrep, const jp_params *prm, jp_ctx *
   std::vector<int> hblk_rep(c->nblk);
   for (int r = 0; r < nrep; ++r)
     for (int bb = 0; bb < reps[r].nblk; ++bb) hblk_rep[reps[r].blk0 + bb] = r;
-  // tile-list chunks: (i-block, j0) for j0 = i, i+32, ... inside the replica
-  std::vector<int> chunk_i, chunk_j0, blk_chunk0(c->nblk + 1, 0);
+  // possible tiles: an i-block with itself and every later block of its replica
+  std::vector<long long> blk_tile0(c->nblk);
   for (int bb = 0; bb < c->nblk; ++bb) {
     const Rep &R = reps[hblk_rep[bb]];
-    blk_chunk0[bb] = (int)chunk_i.size();
-    for (int j0 = bb; j0 < R.blk0 + R.nblk; j0 += 32) {
-      chunk_i.push_back(bb);
-      chunk_j0.push_back(j0);
-    }
+    blk_tile0[bb] = (long long)c->tile_cap_total;
+    c->tile_cap_total += R.blk0 + R.nblk - bb;
   }
-  blk_chunk0[c->nblk] = (int)chunk_i.size();
-  c->nchunk = (int)chunk_i.size();
-  c->tile_cap_total = c->nchunk * 32;   // every candidate could be a tile: no overflow
 
   // ---- device allocation ---------------------------------------------------------------
   DevPtrs &P = c->P;
@@ -1570,35 +1563,29 @@ int jp_create(const jp_system *sys, int32_t nrep, const jp_params *prm, jp_ctx *
   e |= dalloc(c, &P.blk_ctr, (size_t)c->nblk);
   e |= dalloc(c, &P.blk_half, (size_t)c->nblk);
   e |= dalloc(c, &P.blk_ref, 3 * (size_t)c->nblk);
-  e |= dput(c, &P.chunk_i, chunk_i);
-  e |= dput(c, &P.chunk_j0, chunk_j0);
-  e |= dalloc(c, &P.chunk_nz, (size_t)c->nchunk);
-  e |= dalloc(c, &P.chunk_cnt, (size_t)c->nchunk + 1);
-  e |= dalloc(c, &P.chunk_off, (size_t)c->nchunk + 1);
-  e |= dalloc(c, &P.tmp_masks, (size_t)c->tile_cap_total * 32);
-  e |= dalloc(c, &P.tiles, (size_t)c->tile_cap_total);
-  e |= dalloc(c, &P.tile_src, (size_t)c->tile_cap_total);
-  // compact tiles: at most one per tile (an i-block's j entries never outnumber 32 per tile)
-  e |= dput(c, &P.blk_chunk0, blk_chunk0);
+  e |= dput(c, &P.blk_tile0, blk_tile0);
+  e |= dalloc(c, &P.blk_tiles, c->tile_cap_total);
+  e |= dalloc(c, &P.tmp_masks, c->tile_cap_total * 32);
+  if (c->hbond) {
+    e |= dalloc(c, &P.tiles, c->tile_cap_total);
+    e |= dalloc(c, &P.tile_src, c->tile_cap_total);
+  }
   // pair records: at most one per tile and half (a unit's records never outnumber the tiles
   // of its block), plus padding so that the kernels' record groups (up to four) stay inside
-  const size_t rec_cap = 2 * (size_t)c->tile_cap_total + 4;
-  e |= dalloc(c, &P.ct_cnt, 2 * (size_t)c->nblk + 1);
-  e |= dalloc(c, &P.ct_off, 2 * (size_t)c->nblk + 1);
+  const size_t rec_cap = 2 * c->tile_cap_total + 8;
+  P.rec_cap = rec_cap;
+  e |= dalloc(c, &P.ct_cnt, 2 * (size_t)c->nblk);
   e |= dalloc(c, &P.ct_blk, rec_cap);
-  e |= dalloc(c, &P.tmp_occ, (size_t)c->nchunk * 32 * 2);
-  e |= dalloc(c, &P.chunk_ent, 2 * ((size_t)c->nchunk + 1));
-  e |= dalloc(c, &P.chunk_eoff, 2 * ((size_t)c->nchunk + 1));
-  e |= dalloc(c, &P.tile_eoff, 2 * (size_t)c->tile_cap_total);
   e |= dalloc(c, &P.ct_j, rec_cap * 32);
   e |= dalloc(c, &P.ct_ty, rec_cap * 32);
   e |= dalloc(c, &P.ct_mask, rec_cap * kHalf);
-  e |= dalloc(c, &P.nctiles, 1);
+  e |= dalloc(c, &P.nctiles, 2);
+  e |= dalloc(c, &P.ext_pos, 1);
   if (c->cmm) e |= dalloc(c, &P.ct_mask_el, rec_cap * kHalf);
   if (c->cmm) {
     int ntot = 0;
     for (int l = 1; l <= 5; ++l) ntot += c->cmm_ncell[l];
-    e |= dalloc(c, &P.tmp_masks_el, (size_t)c->tile_cap_total * 32);
+    e |= dalloc(c, &P.tmp_masks_el, c->tile_cap_total * 32);
     e |= dalloc(c, &P.cmm_cell, (size_t)N);
     if (!hres_cmm.empty()) e |= dput(c, &P.cmm_res, hres_cmm);
     e |= dalloc(c, &P.gwk, 3 * (size_t)N);
@@ -1699,7 +1686,7 @@ int jp_create(const jp_system *sys, int32_t nrep, const jp_params *prm, jp_ctx *
     e |= dalloc(c, &P.hb_n, 1);
   }
   e |= dalloc(c, &c->scan_scratch,
-              (size_t)std::max(std::max(c->nkeys, c->ncol), c->nchunk) / 1024 + 4);
+              (size_t)std::max(c->nkeys, c->ncol) / 1024 + 4);
   if (e) { jp_destroy(c); return JP_E_CUDA; }
   // the tile-row prefix must cover the sentinel entry; row_cnt[nblk] stays 0
   // ---- constants ---------------------------------------------------------------------------
@@ -1765,6 +1752,7 @@ int jp_create(const jp_system *sys, int32_t nrep, const jp_params *prm, jp_ctx *
   CK(cudaEventCreateWithFlags(&c->ev_join, cudaEventDisableTiming));
   CK(cudaEventCreate(&c->ev_a));
   CK(cudaEventCreate(&c->ev_b));
+  init_block_list();
   if (c->fp64) launch_update_pos(P, N, true, c->qscale, c->st);   // the mixed path's: at each list build
   int rs = tune_blocks(c, prm->tune_blocks != 0);
   if (rs < 0) { jp_destroy(c); return rs; }
@@ -1906,6 +1894,7 @@ int jp_energy_grad(jp_ctx *c, int32_t r, const double *cord, double *eneval, dou
 int set_cls_override(jp_ctx *c, int32_t r, int cls) {
   Rep &R = c->reps[r];
   R.cls_over = cls >= 0 ? 1 : 0;
+  c->every_cls = cls >= 0;
   for (int k = 0; k < 3; ++k) R.cls_w[k] = k == cls ? 1.0 : 0.0;
   CK(cudaMemcpyAsync(c->P.reps + r, &R, sizeof(Rep), cudaMemcpyHostToDevice, c->st));
   CK(cudaStreamSynchronize(c->st));
@@ -2319,13 +2308,17 @@ int jp_list_stats(jp_ctx *c, int64_t *ntiles, int64_t *npairs_listed, int64_t *n
   CK(cudaSetDevice(c->device));
   if (int e = flush_rebuild(c)) return e;
   CK(cudaStreamSynchronize(c->st));
-  int nt = 0;
-  CK(cudaMemcpy(&nt, c->P.nctiles, sizeof(int), cudaMemcpyDeviceToHost));
+  int n2[2] = {0, 0};   // records from the start and from the end of the arrays
+  CK(cudaMemcpy(n2, c->P.nctiles, sizeof(n2), cudaMemcpyDeviceToHost));
+  const int nt = n2[0] + n2[1];
   if (ntiles) *ntiles = nt;
   if (nslots) *nslots = c->nslot;
   if (npairs_listed) {
     std::vector<unsigned> m((size_t)nt * kHalf);
-    if (nt) CK(cudaMemcpy(m.data(), c->P.ct_mask, sizeof(unsigned) * m.size(), cudaMemcpyDeviceToHost));
+    const size_t m0 = (size_t)n2[0] * kHalf, m1 = (size_t)n2[1] * kHalf;
+    if (m0) CK(cudaMemcpy(m.data(), c->P.ct_mask, sizeof(unsigned) * m0, cudaMemcpyDeviceToHost));
+    if (m1) CK(cudaMemcpy(m.data() + m0, c->P.ct_mask + c->P.rec_cap * kHalf - m1, sizeof(unsigned) * m1,
+                          cudaMemcpyDeviceToHost));
     int64_t s = 0;
     for (unsigned v : m) s += __builtin_popcount(v);
     *npairs_listed = s;

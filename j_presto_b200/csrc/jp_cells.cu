@@ -7,13 +7,10 @@
 //   3. k_scatter       bin atoms; k_sort_bins makes the order within a bin deterministic
 //   4. k_fill_slots    compact order -> 32-atom blocks padded per replica
 //   5. k_block_setup   per-block bounding box, frame origin, block-local coordinates
-//   6. k_tile_scan_chunks  one warp per (i-block, 32 candidate j-blocks): bounding-box test
-//                      of the 32 candidates at once, warp-ballot compaction of the
-//                      survivors, then the exact 32x32 interaction mask in FP64:
-//                      r^2 <= (rc+1.5)^2 at build time (cutatm `dd .le. rlim2`), minus
-//                      1-2/1-3/1-4 partners (cutoff.f90:50-96).
-//   7. scan of the per-chunk tile counts, k_tile_emit writes one dense list in row-major,
-//      ascending-j order (deterministic).
+//   6. k_block_list    one thread block per i-block: bounding-box tests of the later blocks,
+//                      the exact 32x32 interaction mask of the survivors (r^2 <= (rc+1.5)^2 at
+//                      build time, cutatm `dd .le. rlim2`, minus 1-2/1-3/1-4 partners,
+//                      cutoff.f90:50-96), and the pair records of its two halves.
 #include "jp_common.cuh"
 #include "jp_kernels.h"
 
@@ -164,25 +161,80 @@ __global__ void k_excl_slots(DevPtrs P, int natom) {
   for (int p = P.excl_ptr[a]; p < P.excl_ptr[a + 1]; ++p) P.excl_slot[p] = P.slot_of[P.excl_idx[p]];
 }
 
-constexpr int kExclReg = 8;   // exclusion partners held in registers per i-atom
+// ---- pair list: one thread block per i-block ---------------------------------------------------
+// k_block_list does everything that belongs to one 32-atom i-block: the bounding-box test of
+// the later blocks of its replica, the exact 32x32 interaction mask of every survivor, and the
+// pair records of its two halves.  The masks and what belongs to a tile stay in shared memory
+// (in global memory beyond kTileCache tiles), and a unit's records are placed by one atomic
+// counter: which records stand where varies from run to run, what a record holds does not, and
+// the sums of the pair kernels do not depend on it.
+// Before, a warp scanned 32 candidates one after the other, and eleven more launches (three
+// scans of per-chunk counts, tile emit, unit counts, their scan, record index, record emit)
+// passed the tiles on through memory.  A whole list build, before and now: 64 replicas 4,380 and
+// 2,303 us, 99,200 atoms 534 and 358, 22,700 atoms 216 and 139, 2,200 atoms 196 and 105.
+//
+// Pair record: a half block (16 i atoms: rows 0-15 or 16-31 of an i-block, unit u = 2 i-block +
+// half) with 32 j entries, the j atoms of that block's tiles that at least one of the 16 i
+// atoms lists, taken in tile order (ascending j block, ascending slot).  A 32 x 32 tile of two
+// blocks holds ~26 % listed pairs at the md_run list radius; keeping only the j atoms a half
+// block lists raises that to ~55 %, because 16 atoms span a smaller volume than 32 (within the
+// cut-off: 32 % of the slots with whole blocks, 39 % with half blocks), and the pair kernels'
+// work per pair falls in proportion.  Each entry carries its tile's image shift (into the i
+// block's frame) and its atom, with the atom's type beside it; the mask of i atom l (0..15)
+// has bit k = entry (l + k) & 15 and bit 16 + k = entry 16 + ((l + k) & 15).
 
-// Tile list, pass A: one warp per chunk = (i-block, 32 consecutive candidate j-blocks
-// starting at j0 >= i, same replica).  Bounding-box test of the 32 candidates at once, then
-// for each survivor the exact mask; non-empty masks go to the chunk's scratch slots.
-// CMM: level-1 cells ci / cj (packed 0-based x | y << 8 | z << 16, -1 = off the grid);
-// neighbours (neartb.f90 first table) set mask and mel, cells up to idelay apart with
+constexpr int kListWarps = 8;     // warps of a block, at most
+constexpr int kTileListImg = 1 << 30, kTilePairImg = 1 << 29, kTileBlock = kTilePairImg - 1;   // BlkTile.j
+constexpr int kSegment = 512;     // candidate blocks tested at a time
+constexpr int kTileCache = 96;    // tiles of an i-block kept in shared memory (water: 65 on average)
+constexpr int kWindow = 40;       // records of a half emitted at a time (water: 27 on average)
+
+struct __align__(16) ListShared {
+  double x[kTile], y[kTile], z[kTile];     // the i block, wrapped
+  // a candidate's live j atoms, compacted, two per element: x, x', y, y' and z, z', mask bits
+  float4 lxy[kListWarps][kTile / 2], lzb[kListWarps][kTile / 2];
+  unsigned ball[kSegment / 32];            // survivors of the bounding-box test
+  unsigned excl[kSegment / 32];            // blocks that hold an exclusion partner
+  int wsum[kListWarps][2];
+  int carry[2];
+  int base;
+  // ALSD: which of a window's records hold a class but BB, and each one's place
+  unsigned char rcls[2 * kWindow];
+  size_t rpos[2 * kWindow];
+  BlkTile tile[kTileCache];
+  unsigned elist[2][kWindow * 32];         // entry -> tile << 5 | j lane, of each half's window
+};
+
+// 1-2/1-3/1-4 partners (cutoff.f90:50-96) of this lane's i atom that sit in block bj out of its
+// mask row: lane l sees slot bj * 32 + ((l + k) & 31) at bit k
+__device__ __forceinline__ unsigned drop_excluded(const DevPtrs& P, int bj, int lane, int ai, unsigned mask) {
+  if (ai >= 0)
+    for (int p = P.excl_ptr[ai]; p < P.excl_ptr[ai + 1]; ++p) {
+      const int sp = P.excl_slot[p];
+      if ((sp >> 5) == bj) mask &= ~(1u << (((sp & 31) - lane) & 31));
+    }
+  return mask;
+}
+
+// (the two FP64 forms are out of line and take plain pointers: a reference to the kernel's
+// parameter block would have it copied to local memory)
+// General form of a tile's mask in FP64, per-pair minimum image: lane = i atom, bit k = j lane
+// (lane + k) & 31.  CMM: level-1 cells ci / cj (packed 0-based x | y << 8 | z << 16, -1 = off the
+// grid); neighbours (neartb.f90 first table) set mask and mel, cells up to idelay apart with
 // r^2 < rc2 at the rebuild (neartb.f90:330-370, the LJ-only table) set mask only
 template <bool CMM>
-__device__ __forceinline__ unsigned tile_mask(const DevPtrs& P, const Rep& R, int bi, int bj, int lane,
-                                              int ai, double xi, double yi, double zi,
-                                              const int (&ps)[kExclReg], int pb, int pe,
-                                              double rlim2, int ci, double rc2, unsigned& mel) {
-  const int aj = P.satom[bj * kTile + lane];
-  double xj = 0, yj = 0, zj = 0;
-  int cj = -1;
+__device__ __noinline__ unsigned tile_mask(const int* satom, const double* x, const int* cmm_cell, const Rep& R, int bi,
+                                           int bj, int lane, int ai, double rlim2, double rc2, unsigned& mel) {
+  const int aj = satom[bj * kTile + lane];
+  double xi = 0, yi = 0, zi = 0, xj = 0, yj = 0, zj = 0;
+  int ci = -1, cj = -1;
+  if (ai >= 0) {
+    xi = x[3 * ai]; yi = x[3 * ai + 1]; zi = x[3 * ai + 2];
+    if (CMM) ci = cmm_cell[ai];
+  }
   if (aj >= 0) {
-    xj = P.x[3 * aj]; yj = P.x[3 * aj + 1]; zj = P.x[3 * aj + 2];
-    if (CMM) cj = P.cmm_cell[aj];
+    xj = x[3 * aj]; yj = x[3 * aj + 1]; zj = x[3 * aj + 2];
+    if (CMM) cj = cmm_cell[aj];
   }
   unsigned mask = 0;
   mel = 0;
@@ -198,152 +250,42 @@ __device__ __forceinline__ unsigned tile_mask(const DevPtrs& P, const Rep& R, in
     const int ck = CMM ? __shfl_sync(0xffffffffu, cj, src) : 0;
     if (ai < 0 || ak < 0) continue;
     if (bj == bi && (k == 0 || k > 16 || (k == 16 && lane >= 16))) continue;
+    int cheb = 0;
+    if (CMM) {
+      if (ci < 0 || ck < 0) continue;
+      cheb = max(abs((ci & 255) - (ck & 255)),
+                 max(abs(((ci >> 8) & 255) - ((ck >> 8) & 255)), abs((ci >> 16) - (ck >> 16))));
+      if (cheb <= 1) {
+        mask |= 1u << k;
+        mel |= 1u << k;
+        continue;
+      }
+      if (!(idelay > 1 && cheb <= idelay)) continue;
+    }
     double dx = xi - xk, dy = yi - yk, dz = zi - zk;
     dx -= bx * anint(dx * ibx);
     dy -= by * anint(dy * iby);
     dz -= bz * anint(dz * ibz);
     const double d2 = dx * dx + dy * dy + dz * dz;
-    if (CMM) {
-      if (ci < 0 || ck < 0) continue;
-      const int cheb = max(abs((ci & 255) - (ck & 255)),
-                           max(abs(((ci >> 8) & 255) - ((ck >> 8) & 255)), abs((ci >> 16) - (ck >> 16))));
-      if (cheb <= 1) {
-        mask |= 1u << k;
-        mel |= 1u << k;
-      } else if (idelay > 1 && cheb <= idelay && d2 < rc2) {
-        mask |= 1u << k;
-      }
-    } else if (d2 <= rlim2) {
-      mask |= 1u << k;
-    }
+    if (CMM ? d2 < rc2 : d2 <= rlim2) mask |= 1u << k;
   }
-  // 1-2/1-3/1-4 partners of the i-atom that sit in block bj: lane l sees slot
-  // bj*32 + ((l+k)&31) at bit k
-  if (mask) {
-#pragma unroll
-    for (int q = 0; q < kExclReg; ++q)
-      if ((ps[q] >> 5) == bj) mask &= ~(1u << (((ps[q] & 31) - lane) & 31));
-    for (int p = pb + kExclReg; p < pe; ++p) {
-      const int sp = P.excl_slot[p];
-      if ((sp >> 5) == bj) mask &= ~(1u << (((sp & 31) - lane) & 31));
-    }
-  }
-  mel &= mask;
   return mask;
 }
 
-// Fast form of the mask (no CMM, large box): lane = j atom; the i block is read from shared
+// The FP64 form where the tile's image serves every listed pair (no CMM): lane = j atom; the i block is read from shared
 // memory one atom per step (a broadcast) and a ballot gives that i atom's row of the tile at
-// once; lane i keeps row i and rotates it into the kernels' layout (bit k = j (i + k) & 31).
-// Coordinates are wrapped (x - box floor(x / box)) and the tile's image is the block
-// references' minimum image n, exact for every pair the list can hold when box/2 > list
-// radius + block extents (the condition of the pair kernels' per-tile shift).
-struct IStage {
-  double x[kTile], y[kTile], z[kTile];
-  float xf[kTile], yf[kTile], zf[kTile];   // the same relative to the i block's reference
-  float4 live[kTile];                      // a candidate's live i atoms, compacted (x, y, z, lane)
-};
-
-// The exact list radius decides in FP64, but almost every pair is far from it: the mask is
-// first built in FP32 on coordinates relative to the i block's reference (|x| <~ 25 A, so
-// d^2 is good to ~3e-4 A^2), and a tile with any pair within `band` of rlim^2 is redone by
-// tile_mask_fast in FP64; the FP32 mask is returned only where every decision is certain,
-// so the list is the FP64 list.  `unsure` is warp-uniform.
-// A j atom in the i frame is its block-local position (pos_f, relative to its block's
-// reference in the wrapped frame) plus block bj's reference shifted by the tiles' image into
-// the i block's frame.  Only the i atoms within the list radius of block bj's bounding box
-// (with a margin of 1e-4 rlim^2 + 1e-3 A^2, far wider than `band` and the FP32 rounding) can
-// list a pair; the rows of the others are certainly empty, and the loop skips them.
-// PIMG (a box at most twice the list radius plus two block extents): the tiles' image is not
-// every pair's, so each pair takes its own minimum image in FP32 and no i atom is culled.
-template <bool PIMG>
-__device__ __forceinline__ unsigned tile_row_f32(const DevPtrs& P, const Rep& R, int bi, int bj, int lane,
-                                                 IStage& S, float rlim2f, float band, bool& unsure) {
-  const int aj = P.satom[bj * kTile + lane];
-  float cj[3];   // block bj's reference (its bounding-box centre) in the i block's frame
-  for (int k = 0; k < 3; ++k) {
-    const double d = P.blk_ref[3 * bi + k] - P.blk_ref[3 * bj + k];
-    cj[k] = (float)(R.box[k] * anint(d * R.invbox[k]) - d);
-  }
-  const float4 pj = aj >= 0 ? P.pos_f[aj] : make_float4(0.f, 0.f, 0.f, 0.f);
-  const float r[3] = {pj.x + cj[0], pj.y + cj[1], pj.z + cj[2]};
-  unsigned live;
-  if (PIMG) {   // every real i atom (padding slots sit at 1e18)
-    live = __ballot_sync(0xffffffffu, S.xf[lane] < 1.0e17f);
-  } else {
-    const float4 hj = P.blk_half[bj];
-    const float gx = fmaxf(fabsf(S.xf[lane] - cj[0]) - hj.x, 0.f);
-    const float gy = fmaxf(fabsf(S.yf[lane] - cj[1]) - hj.y, 0.f);
-    const float gz = fmaxf(fabsf(S.zf[lane] - cj[2]) - hj.z, 0.f);
-    live = __ballot_sync(0xffffffffu, fmaf(gx, gx, fmaf(gy, gy, gz * gz)) <= rlim2f * 1.0001f + 1e-3f);
-  }
-  const float bx = (float)R.box[0], by = (float)R.box[1], bz = (float)R.box[2];
-  const float ibx = (float)R.invbox[0], iby = (float)R.invbox[1], ibz = (float)R.invbox[2];
-  unsigned row = 0;
-  bool u = false;
-  // the live i atoms compacted in shared memory, so each pass reads two of them by
-  // position instead of scanning the bit mask (bit scans run on the XU pipe); two i atoms
-  // per pass: two independent distance chains and ballots
-  const int nlive = __popc(live);
-  __syncwarp();   // the previous candidate's passes are done with S.live
-  if ((live >> lane) & 1u)
-    S.live[__popc(live & ((1u << lane) - 1u))] = make_float4(S.xf[lane], S.yf[lane], S.zf[lane], __int_as_float(lane));
-  __syncwarp();
-  auto d2of = [&](float4 a) {
-    float dx = a.x - r[0], dy = a.y - r[1], dz = a.z - r[2];
-    if (PIMG) {
-      dx = fmaf(-bx, rintf(dx * ibx), dx);
-      dy = fmaf(-by, rintf(dy * iby), dy);
-      dz = fmaf(-bz, rintf(dz * ibz), dz);
-    }
-    return fmaf(dx, dx, fmaf(dy, dy, dz * dz));
-  };
-  for (int q = 0; q < nlive; q += 2) {   // warp-uniform
-    const bool has2 = q + 1 < nlive;
-    const float4 a = S.live[q];
-    const float4 c = S.live[has2 ? q + 1 : q];
-    const float d2 = d2of(a), e2 = d2of(c);
-    const bool in = aj >= 0 && d2 <= rlim2f;
-    const bool in2 = aj >= 0 && has2 && e2 <= rlim2f;
-    u |= aj >= 0 && fabsf(d2 - rlim2f) < band;
-    u |= aj >= 0 && has2 && fabsf(e2 - rlim2f) < band;
-    const unsigned b = __ballot_sync(0xffffffffu, in);
-    const unsigned b2 = __ballot_sync(0xffffffffu, in2);
-    if (lane == __float_as_int(a.w)) row = b;
-    if (has2 && lane == __float_as_int(c.w)) row = b2;
-  }
-  unsure = __any_sync(0xffffffffu, u);
-  return row;
-}
-
-// row i of a tile (bit j: pair (i, j) within the list radius) into the kernels' rotated
-// layout, each unordered pair once, exclusions removed
-__device__ __forceinline__ unsigned finish_mask(const DevPtrs& P, int bi, int bj, int lane, unsigned row,
-                                                const int (&ps)[kExclReg], int pb, int pe) {
-  unsigned mask = __funnelshift_r(row, row, lane);
-  if (bj == bi) mask &= lane < 16 ? 0x1fffeu : 0xfffeu;   // each unordered pair once, no self pair
-  if (mask) {
-#pragma unroll
-    for (int q = 0; q < kExclReg; ++q)
-      if ((ps[q] >> 5) == bj) mask &= ~(1u << (((ps[q] & 31) - lane) & 31));
-    for (int p = pb + kExclReg; p < pe; ++p) {
-      const int sp = P.excl_slot[p];
-      if ((sp >> 5) == bj) mask &= ~(1u << (((sp & 31) - lane) & 31));
-    }
-  }
-  return mask;
-}
-
-__device__ __forceinline__ unsigned tile_mask_fast(const DevPtrs& P, const Rep& R, int bi, int bj, int lane,
-                                                   int ai, const IStage& S, const int (&ps)[kExclReg],
-                                                   int pb, int pe, double rlim2) {
-  const int aj = P.satom[bj * kTile + lane];
+// once; lane i keeps row i.  Coordinates are wrapped (x - box floor(x / box)) and the tile's
+// image is the block references' minimum image n.
+__device__ __noinline__ unsigned tile_row_fast(const int* satom, const double* xm, const double* blk_ref, const Rep& R,
+                                               int bi, int bj, int lane, int ai, const ListShared& S,
+                                               double rlim2) {
+  const int aj = satom[bj * kTile + lane];
   double xj = 0.0, yj = 0.0, zj = 0.0;
   if (aj >= 0) {
     double w[3];
     for (int k = 0; k < 3; ++k) {
-      const double x = P.x[3 * aj + k];
-      const double n = anint((P.blk_ref[3 * bi + k] - P.blk_ref[3 * bj + k]) * R.invbox[k]);
+      const double x = xm[3 * aj + k];
+      const double n = anint((blk_ref[3 * bi + k] - blk_ref[3 * bj + k]) * R.invbox[k]);
       w[k] = (x - R.box[k] * floor(x * R.invbox[k])) + R.box[k] * n;
     }
     xj = w[0]; yj = w[1]; zj = w[2];
@@ -356,211 +298,94 @@ __device__ __forceinline__ unsigned tile_mask_fast(const DevPtrs& P, const Rep& 
     const unsigned b = __ballot_sync(0xffffffffu, in);
     if (lane == i) row = b;
   }
-  if (ai < 0) row = 0;
-  return finish_mask(P, bi, bj, lane, row, ps, pb, pe);
+  return ai >= 0 ? row : 0u;
 }
 
-template <bool CMM>
-__global__ void __launch_bounds__(128, 6) k_tile_scan_chunks(DevPtrs P, int nchunk, double rlim2, float rlimf,
-                                                          double rc2) {
-  const float rlim2f = (float)rlim2;
-  __shared__ IStage s_i[4];
-  const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  if (w >= nchunk) return;
-  const int bi = P.chunk_i[w], j0 = P.chunk_j0[w];
-  const int rep = P.blk_rep[bi];
-  const Rep& R = P.reps[rep];
-  // exact when a pair within the list radius cannot be another image than the blocks':
-  // box/2 > list radius + the two blocks' half extents (largest of the replica)
-  bool fast = !CMM;
-  for (int k = 0; k < 3; ++k)
-    if (!(0.5 * R.box[k] > sqrt(rlim2) + 2.0 * (double)P.rep_hmax[3 * rep + k] + 0.01)) fast = false;
-  const int bend = R.blk0 + R.nblk;
-  const float4 ci = P.blk_ctr[bi], hi = P.blk_half[bi];
-  const int bj = j0 + lane;
-  bool cand = false;
-  if (bj < bend) {
-    const float4 cj = P.blk_ctr[bj], hj = P.blk_half[bj];
-    float dx = ci.x - cj.x, dy = ci.y - cj.y, dz = ci.z - cj.z;
-    dx -= (float)R.box[0] * rintf(dx * (float)R.invbox[0]);
-    dy -= (float)R.box[1] * rintf(dy * (float)R.invbox[1]);
-    dz -= (float)R.box[2] * rintf(dz * (float)R.invbox[2]);
-    const float gx = fmaxf(fabsf(dx) - hi.x - hj.x, 0.f);
-    const float gy = fmaxf(fabsf(dy) - hi.y - hj.y, 0.f);
-    const float gz = fmaxf(fabsf(dz) - hi.z - hj.z, 0.f);
-    cand = gx * gx + gy * gy + gz * gz <= rlimf * rlimf * 1.0001f + 1e-3f;
+// The exact list radius decides in FP64, but almost every pair is far from it: the mask is
+// first built in FP32 on coordinates relative to the i block's reference (|x| <~ 25 A, so
+// d^2 is good to ~3e-4 A^2), and a tile with any pair within `band` of rlim^2 is redone in
+// FP64; the FP32 mask is returned only where every decision is certain, so the list is the
+// FP64 list.  `unsure` is warp-uniform.
+// Lane = i atom (xi, in its block's frame).  A j atom in the i frame is its block-local position
+// pj (relative to its block's reference in the wrapped frame) plus c, block bj's reference
+// shifted by the tiles' image into the i block's frame.  Only the j atoms within the list
+// radius of the i block's bounding box (half extents hi; with a margin of 1e-4 rlim^2 +
+// 1e-3 A^2, far wider than `band` and the FP32 rounding) can be listed, and the loop takes only
+// them: compacted in shared memory with their mask bits, two per pass in packed arithmetic.
+// (With a j atom a lane and the i atoms in the loop every pass also needed a ballot and a
+// select per row: 24 instructions for two atoms, so 17.)
+// PIMG (two blocks nearly half a small box apart): the tile's image is not every pair's, so each
+// pair takes its own minimum image in FP32 and no j atom is culled.  Decided per tile: with one
+// rule per replica from its largest block, boxes up to 51 A imaged every pair.
+template <bool PIMG>
+__device__ __forceinline__ unsigned tile_row_f32(const Rep& R, float3 c, float4 hi, int lane, float3 xi, bool ireal,
+                                                 float4 pj, bool jreal, ListShared& S, float rlim2f, float band,
+                                                 bool& unsure) {
+  const unsigned full = 0xffffffffu;
+  const int w = threadIdx.x >> 5;
+  const float rx = pj.x + c.x, ry = pj.y + c.y, rz = pj.z + c.z;
+  bool lv = jreal;
+  if (!PIMG) {
+    const float gx = fmaxf(fabsf(rx) - hi.x, 0.f);
+    const float gy = fmaxf(fabsf(ry) - hi.y, 0.f);
+    const float gz = fmaxf(fabsf(rz) - hi.z, 0.f);
+    lv = lv && fmaf(gx, gx, fmaf(gy, gy, gz * gz)) <= rlim2f * 1.0001f + 1e-3f;
   }
-  unsigned ball = __ballot_sync(0xffffffffu, cand);
-  unsigned nz = 0;
-  int nent0 = 0, nent1 = 0;   // entries of the two half blocks (rows 0-15, 16-31)
-  if (ball) {
-    const int ai = P.satom[bi * kTile + lane];
-    double xi = 0, yi = 0, zi = 0;
-    int pb = 0, pe = 0, ci = -1;
-    int ps[kExclReg];
-    if (ai >= 0) {
-      xi = P.x[3 * ai]; yi = P.x[3 * ai + 1]; zi = P.x[3 * ai + 2];
-      pb = P.excl_ptr[ai];
-      pe = P.excl_ptr[ai + 1];
-      if (CMM) ci = P.cmm_cell[ai];
+  const unsigned live = __ballot_sync(full, lv);
+  const int nlive = __popc(live);
+  __syncwarp();   // the previous tile's passes are done with the compacted atoms
+  {
+    float* xy = reinterpret_cast<float*>(S.lxy[w]);
+    float* zb = reinterpret_cast<float*>(S.lzb[w]);
+    if (lv) {
+      const int t = __popc(live & ((1u << lane) - 1u));
+      const int o = 4 * (t >> 1) + (t & 1);
+      xy[o] = rx;
+      xy[o + 2] = ry;
+      zb[o] = rz;
+      zb[o + 2] = __uint_as_float(1u << lane);
     }
-#pragma unroll
-    for (int q = 0; q < kExclReg; ++q) ps[q] = pb + q < pe ? P.excl_slot[pb + q] : -64;
-    IStage& S = s_i[threadIdx.x >> 5];
-    if (!CMM) {   // the i block, wrapped, for the broadcast reads
-      S.x[lane] = xi - R.box[0] * floor(xi * R.invbox[0]);
-      S.y[lane] = yi - R.box[1] * floor(yi * R.invbox[1]);
-      S.z[lane] = zi - R.box[2] * floor(zi * R.invbox[2]);
-      // padding slots far away: they never list a pair nor make a tile uncertain
-      S.xf[lane] = ai >= 0 ? (float)(S.x[lane] - P.blk_ref[3 * bi + 0]) : 1.0e18f;
-      S.yf[lane] = ai >= 0 ? (float)(S.y[lane] - P.blk_ref[3 * bi + 1]) : 1.0e18f;
-      S.zf[lane] = ai >= 0 ? (float)(S.z[lane] - P.blk_ref[3 * bi + 2]) : 1.0e18f;
-      __syncwarp();
-    }
-    // the FP32 mask's uncertainty band: every coordinate tile_row_f32 works with is below
-    // M = rlim + 3 h_max in magnitude (h_max: the replica's largest block half extent) and
-    // carries at most 2.5 roundings of 2^-24 M, a difference one more, so |error of d^2| <=
-    // 2 sqrt(3) rlim 5 2^-24 M + 3 2^-24 rlim^2; pairs within 4 times that of rlim^2 are
-    // decided in FP64 (about 1.5e-3 A^2 for water blocks at rc = 12 A)
-    const float hm = fmaxf(P.rep_hmax[3 * rep], fmaxf(P.rep_hmax[3 * rep + 1], P.rep_hmax[3 * rep + 2]));
-    // with per-pair images (a small box) the coordinates before imaging reach the box edge
-    const float mb = fast ? rlimf + 3.f * hm
-                          : fmaxf(rlimf + 3.f * hm, (float)fmax(R.box[0], fmax(R.box[1], R.box[2])) + 3.f * hm);
-    const float band = 4.f * 5.9604645e-8f * (17.33f * rlimf * mb + 3.f * rlimf * rlimf);
-    while (ball) {
-      const int b = __ffs(ball) - 1;
-      ball &= ball - 1;
-      unsigned mel = 0;
-      unsigned m;
-      bool unsure = true;
-      if (!CMM) {
-        unsigned row = fast ? tile_row_f32<false>(P, R, bi, j0 + b, lane, S, rlim2f, band, unsure)
-                            : tile_row_f32<true>(P, R, bi, j0 + b, lane, S, rlim2f, band, unsure);
-        if (!unsure) {
-          if (ai < 0) row = 0;
-          m = finish_mask(P, bi, j0 + b, lane, row, ps, pb, pe);
-        }
-      }
-      if (unsure)
-        m = fast ? tile_mask_fast(P, R, bi, j0 + b, lane, ai, S, ps, pb, pe, rlim2)
-                 : tile_mask<CMM>(P, R, bi, j0 + b, lane, ai, xi, yi, zi, ps, pb, pe, rlim2, ci, rc2, mel);
-      if (__any_sync(0xffffffffu, m != 0)) {
-        P.tmp_masks[((size_t)w * 32 + b) * 32 + lane] = m;
-        if (CMM) P.tmp_masks_el[((size_t)w * 32 + b) * 32 + lane] = mel;
-        // the j lanes some i atom of each half block lists: the entries this tile
-        // contributes to the two halves' pair records
-        const unsigned rowj = __funnelshift_l(m, m, lane);
-        const unsigned occ0 = __reduce_or_sync(0xffffffffu, lane < kHalf ? rowj : 0u);
-        const unsigned occ1 = __reduce_or_sync(0xffffffffu, lane < kHalf ? 0u : rowj);
-        if (lane == 0) {
-          P.tmp_occ[((size_t)w * 32 + b) * 2 + 0] = occ0;
-          P.tmp_occ[((size_t)w * 32 + b) * 2 + 1] = occ1;
-        }
-        nent0 += __popc(occ0);
-        nent1 += __popc(occ1);
-        nz |= 1u << b;
-      }
+    if (lane == 0 && (nlive & 1)) {   // the odd one's partner lists nothing: no comparison holds for a NaN
+      const int o = 4 * (nlive >> 1) + 1;
+      xy[o] = xy[o + 2] = zb[o] = __int_as_float(0x7fffffff);
+      zb[o + 2] = 0.f;
     }
   }
-  if (lane == 0) {
-    P.chunk_nz[w] = nz;
-    P.chunk_cnt[w] = __popc(nz);
-    P.chunk_ent[w] = nent0;
-    P.chunk_ent[nchunk + 1 + w] = nent1;
+  __syncwarp();
+  const float bx = (float)R.box[0], by = (float)R.box[1], bz = (float)R.box[2];
+  const float ibx = (float)R.invbox[0], iby = (float)R.invbox[1], ibz = (float)R.invbox[2];
+  const float2 nx = make_float2(-xi.x, -xi.x), ny = make_float2(-xi.y, -xi.y), nz = make_float2(-xi.z, -xi.z);
+  const float2 ml = make_float2(-rlim2f, -rlim2f);
+  unsigned row = 0;
+  bool u = false;
+#pragma unroll 4
+  for (int q = 0; 2 * q < nlive; ++q) {   // warp-uniform
+    const float4 xy = S.lxy[w][q], zb = S.lzb[w][q];
+    float2 dx = __fadd2_rn(make_float2(xy.x, xy.y), nx);
+    float2 dy = __fadd2_rn(make_float2(xy.z, xy.w), ny);
+    float2 dz = __fadd2_rn(make_float2(zb.x, zb.y), nz);
+    if (PIMG) {
+      dx.x = fmaf(-bx, rintf(dx.x * ibx), dx.x);
+      dx.y = fmaf(-bx, rintf(dx.y * ibx), dx.y);
+      dy.x = fmaf(-by, rintf(dy.x * iby), dy.x);
+      dy.y = fmaf(-by, rintf(dy.y * iby), dy.y);
+      dz.x = fmaf(-bz, rintf(dz.x * ibz), dz.x);
+      dz.y = fmaf(-bz, rintf(dz.y * ibz), dz.y);
+    }
+    // d^2 - rlim^2 has the sign of the comparison (a difference rounds to zero only if it is)
+    const float2 e = __fadd2_rn(__ffma2_rn(dx, dx, __ffma2_rn(dy, dy, __fmul2_rn(dz, dz))), ml);
+    u |= fabsf(e.x) < band;
+    u |= fabsf(e.y) < band;
+    if (e.x <= 0.f) row |= __float_as_uint(zb.z);
+    if (e.y <= 0.f) row |= __float_as_uint(zb.w);
   }
+  unsure = __any_sync(full, u && ireal);
+  return ireal ? row : 0u;
 }
 
-// pass C: copy non-empty tiles to the dense list at the scanned offsets (row-major, j order)
-void launch_tile_scan(const DevPtrs& P, int nchunk, double rlim2, float rlimf, double rc2, bool cmm,
-                      cudaStream_t st) {
-  const int nwb = (nchunk * 32 + 127) / 128;
-  if (cmm) k_tile_scan_chunks<true><<<nwb, 128, 0, st>>>(P, nchunk, rlim2, rlimf, rc2);
-  else k_tile_scan_chunks<false><<<nwb, 128, 0, st>>>(P, nchunk, rlim2, rlimf, rc2);
-}
-
-__global__ void k_tile_emit(DevPtrs P, int nchunk, int cmm) {
-  const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  if (w >= nchunk) return;
-  const unsigned nz = P.chunk_nz[w];
-  if (!nz) return;
-  const int bi = P.chunk_i[w], j0 = P.chunk_j0[w];
-  const int t0 = P.chunk_off[w];
-  const int cnt = __popc(nz);
-  // lane q: the chunk's q-th tile's occupied j lanes of each half block and its first entry
-  // in that half's entry order (global)
-  for (int h = 0; h < 2; ++h) {
-    const int b = lane < cnt ? (int)__fns(nz, 0, lane + 1) : 0;
-    const unsigned occ = lane < cnt ? P.tmp_occ[((size_t)w * 32 + b) * 2 + h] : 0u;
-    int e = __popc(occ);
-    for (int o = 1; o < 32; o <<= 1) {   // inclusive scan over the lanes
-      const int y = __shfl_up_sync(0xffffffffu, e, o);
-      if (lane >= o) e += y;
-    }
-    if (lane < cnt) {
-      P.tile_eoff[2 * (size_t)(t0 + lane) + h] = P.chunk_eoff[h * (nchunk + 1) + w] + e - __popc(occ);
-    }
-  }
-  if (lane < cnt) {   // lane q: the chunk's q-th tile and its block pair
-    const int bj = j0 + (int)__fns(nz, 0, lane + 1);
-    P.tiles[t0 + lane] = make_int2(bi, bj);
-    P.tile_src[t0 + lane] = w * 32 + (bj - j0);   // its mask rows stay where the scan wrote them
-  }
-}
-
-// ---- pair records ------------------------------------------------------------------------
-// The pair kernels run on pair records: a half block (16 i atoms: rows 0-15 or 16-31 of an
-// i-block, unit u = 2 i-block + half) with 32 j entries, the j atoms of that block's tiles
-// that at least one of the 16 i atoms lists, taken in tile order (ascending j block,
-// ascending slot).  A 32 x 32 tile of two blocks holds ~26 % listed pairs at the md_run list
-// radius; keeping only the j atoms a half block lists raises that to ~55 %, because 16 atoms
-// span a smaller volume than 32 (within the cut-off: 32 % of the slots with whole blocks,
-// 39 % with half blocks), and the pair kernels' work per pair falls in proportion.  The
-// listed pair set is unchanged.  Each entry carries its tile's image shift (into the i
-// block's frame) and its atom, with the atom's type beside it; the mask of i atom l (0..15) has bit k = entry (l + k) & 15
-// and bit 16 + k = entry 16 + ((l + k) & 15), the order in which the kernels meet them.
-
-// tiles of i-block bi: [chunk_off[blk_chunk0[bi]], chunk_off[blk_chunk0[bi + 1]]); the
-// entries of its half h: [eoff_h[blk_chunk0[bi]], eoff_h[blk_chunk0[bi + 1]]) in global
-// order, eoff_h = chunk_eoff + h (nchunk + 1) (the tile scan counts each tile's occupied j
-// lanes per half, the tile emit places each tile's entries)
-
-// per unit (one thread each): the pair records it needs
-__global__ void k_ct_count(DevPtrs P, int nblk, int nchunk) {
-  const int u = blockIdx.x * blockDim.x + threadIdx.x;
-  if (u >= 2 * nblk) return;
-  const int b = u >> 1, h = u & 1;
-  const int* eoff = P.chunk_eoff + h * (nchunk + 1);
-  const int ne = eoff[P.blk_chunk0[b + 1]] - eoff[P.blk_chunk0[b]];
-  P.ct_cnt[u] = (ne + 31) >> 5;
-}
-
-// per tile (one thread each, after the scan of ct_cnt) and half: the records of the unit
-// whose first slot falls among the tile's entries of that half get their unit and, for the
-// emit, the tile as their first source tile, their first slot's global entry, the end of the
-// unit's entries and of the block's tiles (a tile holds at most 32 entries, so at most two
-// records start in it)
-__global__ void k_ct_index(DevPtrs P, int nchunk) {
-  const int T = *P.ntiles;
-  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < T; t += gridDim.x * blockDim.x) {
-    const int b = P.tiles[t].x;
-    const int c0 = P.blk_chunk0[b], c1 = P.blk_chunk0[b + 1];
-    const int tl = P.chunk_off[c1] - 1;   // the block's last tile
-    for (int h = 0; h < 2; ++h) {
-      const int* eoff = P.chunk_eoff + h * (nchunk + 1);
-      const int e0 = eoff[c0];
-      const int lo = P.tile_eoff[2 * (size_t)t + h] - e0;
-      const int hi = t < tl ? P.tile_eoff[2 * (size_t)(t + 1) + h] - e0 : eoff[c1] - e0;
-      const int u = 2 * b + h;
-      for (int k = (lo + 31) >> 5; 32 * k < hi; ++k) {
-        P.ct_blk[P.ct_off[u] + k] = u;
-        // kept in the record's own entry space until the emit, which fills that
-        reinterpret_cast<int4*>(P.ct_j)[(size_t)(P.ct_off[u] + k) * 32] =
-            make_int4(t, e0 + 32 * k, eoff[c1], ((tl + 1) << 1) | h);
-      }
-    }
-  }
+// where tile c of i-block b keeps its mask rows and its record
+__device__ __forceinline__ BlkTile& blk_tile(const DevPtrs& P, ListShared& S, long long t0, int c) {
+  return c < kTileCache ? S.tile[c] : P.blk_tiles[t0 + c];
 }
 
 // a record row (bit e: entry e) into the kernels' order for i atom l: each 16-bit half
@@ -572,110 +397,341 @@ __device__ __forceinline__ unsigned record_row(unsigned row, int l) {
   return rl | (rh << 16);
 }
 
-// One warp per record, lane p for slot p.  The record's source tiles are consecutive from
-// k_ct_index's first tile and at most 32 (each holds at least one entry and the first covers
-// slot 0), so lane q reads source tile q's entry offset, occupancy, j block, image shift and
-// mask rows' place in one coalesced pass; each slot finds its tile and its rank among the
-// tile's entries by shuffles, and writes its entry.  Record row r (i atom 16 h + r) is then
-// one ballot: every slot contributes the bit of its j lane in row 16 h + r of its tile, so no
-// lane packs bits and lane r keeps row r.
-__global__ void k_ct_emit(DevPtrs P, int nchunk, int cmm, int dummy_type) {
+// 16 mask rows (64 bytes) of a half block's record slots: every slot contributes, per row, the
+// bit of its j lane (stored rotated: bit k of row ri is j lane (ri + k) & 31), one ballot a row;
+// lane r keeps row r
+__device__ __forceinline__ unsigned record_rows(const unsigned* rows, bool live, int jl, int h, int lane) {
+  unsigned cur = 0u;
+  uint4 m[4];
+#pragma unroll
+  for (int q = 0; q < 4; ++q) m[q] = live ? reinterpret_cast<const uint4*>(rows)[q] : make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    const unsigned v[4] = {m[q].x, m[q].y, m[q].z, m[q].w};
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const int r = 4 * q + k;
+      const unsigned row = __ballot_sync(0xffffffffu, (v[k] >> ((jl - kHalf * h - r) & 31)) & 1u);
+      if (lane == r) cur = row;
+    }
+  }
+  return cur;
+}
+
+// count_only: as far as the records per unit (the block-shape tuner needs no more); keep: leave
+// the masks in global memory and list the tiles (the H-bond list reads them); split_cls (ALSD,
+// mixed path): records with a cluster atom go to the top end of the record arrays, downwards,
+// as their pairs take class weights and class energies in a launch of their own
+template <bool CMM>
+__global__ void __launch_bounds__(32 * kListWarps, CMM ? 3 : 4) k_block_list(DevPtrs P, double rlim2, float rlimf,
+                                                                             double rc2, int dummy_type, int count_only,
+                                                                             int keep, int split_cls) {
+  extern __shared__ __align__(16) unsigned char s_dyn[];
+  ListShared& S = *reinterpret_cast<ListShared*>(s_dyn);
+  unsigned* s_mask = reinterpret_cast<unsigned*>(s_dyn + sizeof(ListShared));   // [kTileCache][32], CMM: twice
   const unsigned full = 0xffffffffu;
-  const int lane = threadIdx.x & 31;
-  const int nw = (gridDim.x * blockDim.x) >> 5;
-  const int T = *P.nctiles;
-  for (int ct = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; ct < T; ct += nw) {
-    const int4 info = reinterpret_cast<const int4*>(P.ct_j)[(size_t)ct * 32];   // k_ct_index's
-    __syncwarp();   // read by every lane before the entries overwrite it
-    const int ts = info.x, s0 = info.y, e1 = info.z, t1 = info.w >> 1, h = info.w & 1;
-    const int tq = ts + lane;   // lane q: source tile q
-    int qb = 32, qy = 0, qs = 0;
-    unsigned qocc = 0u;
-    float4 qsh = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (tq < t1) {
-      qb = P.tile_eoff[2 * (size_t)tq + h] - s0;   // slot of the tile's first entry (may be < 0)
-      if (qb < 32) {
-        qs = P.tile_src[tq];
-        qocc = P.tmp_occ[2 * (size_t)qs + h];
-        const int2 ij = P.tiles[tq];
-        qy = ij.y;
-        const Rep& R = P.reps[P.blk_rep[ij.x]];   // image shift of block j into the i block's frame
-        float sh[3];
+  const int bi = blockIdx.x, lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  const int ai = P.satom[bi * kTile + lane];
+  // a block fills from its first slot: this one is not used by the present sort
+  if (!__any_sync(full, ai >= 0)) {
+    if (threadIdx.x < 2) P.ct_cnt[2 * bi + threadIdx.x] = 0;
+    return;
+  }
+  const int rep = P.blk_rep[bi];
+  const Rep& R = P.reps[rep];
+  const long long t0 = P.blk_tile0[bi];
+  const float rlim2f = (float)rlim2;
+  // the FP32 mask's uncertainty band: every coordinate tile_row_f32 works with is below
+  // M = rlim + 3 h_max in magnitude (h_max: the replica's largest block half extent) and
+  // carries at most 2.5 roundings of 2^-24 M, a difference one more, so |error of d^2| <=
+  // 2 sqrt(3) rlim 5 2^-24 M + 3 2^-24 rlim^2; pairs within 4 times that of rlim^2 are
+  // decided in FP64 (about 1.5e-3 A^2 for water blocks at rc = 12 A)
+  const float hm = fmaxf(P.rep_hmax[3 * rep], fmaxf(P.rep_hmax[3 * rep + 1], P.rep_hmax[3 * rep + 2]));
+  // (with per-pair images, in a box below twice that, the coordinates before imaging reach the
+  // box edge)
+  const float lmax = (float)fmax(R.box[0], fmax(R.box[1], R.box[2]));
+  const float mb = (0.5f * lmax > rlimf + 2.f * hm ? rlimf : fmaxf(rlimf, lmax)) + 3.f * hm;
+  const float band = 4.f * 5.9604645e-8f * (17.33f * rlimf * mb + 3.f * rlimf * rlimf);
+  float3 xi = make_float3(0.f, 0.f, 0.f);   // this lane's i atom relative to its block's reference
+  if (!CMM) {   // the i block, wrapped, for the broadcast reads of the FP64 form
+    double q[3] = {0.0, 0.0, 0.0};
+    for (int k = 0; k < 3; ++k)
+      if (ai >= 0) {
+        const double x = P.x[3 * ai + k];
+        q[k] = x - R.box[k] * floor(x * R.invbox[k]);
+      }
+    if (w == 0) {
+      S.x[lane] = q[0];
+      S.y[lane] = q[1];
+      S.z[lane] = q[2];
+    }
+    xi = make_float3((float)(q[0] - P.blk_ref[3 * bi]), (float)(q[1] - P.blk_ref[3 * bi + 1]),
+                     (float)(q[2] - P.blk_ref[3 * bi + 2]));
+  }
+  const float4 ci = P.blk_ctr[bi], hi = P.blk_half[bi];
+  const float bx = (float)R.box[0], by = (float)R.box[1], bz = (float)R.box[2];
+  const float ibx = (float)R.invbox[0], iby = (float)R.invbox[1], ibz = (float)R.invbox[2];
+  const int ncand = R.blk0 + R.nblk - bi;   // later blocks of the replica, itself included
+  auto mask_rows = [&](int c, bool el) -> unsigned* {
+    if (c < kTileCache && !keep) return s_mask + (size_t)(el ? kTileCache + c : c) * 32;
+    return (el ? P.tmp_masks_el : P.tmp_masks) + (size_t)(t0 + c) * 32;
+  };
+
+  int nt = 0;   // tiles so far
+  for (int seg = 0; seg < ncand; seg += kSegment) {
+    const int nb = min(kSegment, ncand - seg);
+    for (int k = threadIdx.x; k < kSegment / 32; k += blockDim.x) S.ball[k] = S.excl[k] = 0u;
+    __syncthreads();
+    // bounding boxes, 32 candidates a warp at once
+    for (int g = w; 32 * g < nb; g += nw) {
+      const int bj = bi + seg + 32 * g + lane;
+      bool cand = false;
+      if (32 * g + lane < nb) {
+        const float4 cj = P.blk_ctr[bj], hj = P.blk_half[bj];
+        float dx = ci.x - cj.x, dy = ci.y - cj.y, dz = ci.z - cj.z;
+        dx -= bx * rintf(dx * ibx);
+        dy -= by * rintf(dy * iby);
+        dz -= bz * rintf(dz * ibz);
+        const float gx = fmaxf(fabsf(dx) - hi.x - hj.x, 0.f);
+        const float gy = fmaxf(fabsf(dy) - hi.y - hj.y, 0.f);
+        const float gz = fmaxf(fabsf(dz) - hi.z - hj.z, 0.f);
+        cand = gx * gx + gy * gy + gz * gz <= rlimf * rlimf * 1.0001f + 1e-3f;
+      }
+      const unsigned ball = __ballot_sync(full, cand);
+      if (lane == 0) S.ball[g] = ball;
+    }
+    // blocks of the segment that hold an exclusion partner of the i block (partners by atom,
+    // the atoms' lists spread over the warps)
+    for (int i = w; i < kTile; i += nw) {
+      const int a = __shfl_sync(full, ai, i);
+      if (a < 0) continue;
+      for (int p = P.excl_ptr[a] + lane; p < P.excl_ptr[a + 1]; p += 32) {
+        const int rel = (P.excl_slot[p] >> 5) - bi - seg;
+        if (rel >= 0 && rel < nb) atomicOr(&S.excl[rel >> 5], 1u << (rel & 31));
+      }
+    }
+    __syncthreads();
+    // the survivors in order, each with its block reference in the i block's frame
+    int n = 0;
+    for (int g = 0; 32 * g < nb; ++g) {
+      const unsigned ball = S.ball[g];
+      if (g % nw == w && ((ball >> lane) & 1u)) {
+        BlkTile& T = blk_tile(P, S, t0, nt + n + __popc(ball & ((1u << lane) - 1u)));
+        const int bj = bi + seg + 32 * g + lane;
+        // Per axis a pair's separation in the tile's image is at most |c| + h_i + h_j, so in any
+        // other image it is at least the box edge minus that.  The tile's image serves every
+        // listed pair if that is beyond the list radius; it serves every pair the kernels meet
+        // until the next build if, with 2 A for the atoms' motion, it is beyond the cut-off
+        // (CMM, no cut-off: beyond the farthest near-field pair)
+        const float4 hj = P.blk_half[bj];
+        const float hh[3] = {hi.x + hj.x, hi.y + hj.y, hi.z + hj.z};
+        const float rk = CMM ? rlimf : (float)sqrt(rc2);
+        float c[3];
+        int img = 0;
         for (int k = 0; k < 3; ++k) {
-          const double d = P.blk_ref[3 * ij.x + k] - P.blk_ref[3 * ij.y + k];
-          sh[k] = (float)(d - R.box[k] * anint(d * R.invbox[k]));
+          const double d = P.blk_ref[3 * bi + k] - P.blk_ref[3 * bj + k];
+          c[k] = (float)(R.box[k] * anint(d * R.invbox[k]) - d);
+          const float other = (float)R.box[k] - (fabsf(c[k]) + hh[k]);
+          if (!(other > rlimf + 0.01f)) img |= kTileListImg;
+          if (!(other > rk + 2.f)) img |= kTilePairImg;
         }
-        qsh = make_float4(sh[0], sh[1], sh[2], 0.f);
+        T.j = bj | img;
+        T.cx = c[0]; T.cy = c[1]; T.cz = c[2];
       }
+      n += __popc(ball);
     }
-    const int nt = __popc(__ballot_sync(full, tq < t1 && qb < 32));   // lanes 0 .. nt-1
-    unsigned cur = 0u, cur_el = 0u;
-    int src = -1, kk = 0;   // this slot's source tile and its rank among the tile's entries
-    for (int j = 0; j < nt; ++j) {   // warp-uniform: every lane looks for its slot
-      const int base = __shfl_sync(full, qb, j);
-      const int n = __popc(__shfl_sync(full, qocc, j));   // both shuffles by every lane
-      const int k = lane - base;
-      if (k >= 0 && k < n) {
-        src = j;
-        kk = k;
+    __syncthreads();
+    // one warp a tile: its mask, and the j lanes some i atom of each half lists.  The next
+    // tile's j atoms are gathered before this one's pairs
+    int an = -1;
+    float4 pn = make_float4(0.f, 0.f, 0.f, 0.f);
+    auto gather = [&](int c) {
+      an = c < nt + n ? P.satom[(blk_tile(P, S, t0, c).j & kTileBlock) * kTile + lane] : -1;
+      if (an >= 0) pn = P.pos_f[an];
+    };
+    if (!CMM) gather(nt + w);
+    for (int c = nt + w; c < nt + n; c += nw) {
+      BlkTile& T = blk_tile(P, S, t0, c);
+      const int bj = T.j & kTileBlock;
+      const bool fast = !CMM && !(T.j & kTileListImg);
+      unsigned mask = 0, mel = 0;
+      bool unsure = true;
+      if (!CMM) {
+        const float3 cc = make_float3(T.cx, T.cy, T.cz);
+        const bool jreal = an >= 0;
+        const float4 pj = pn;
+        gather(c + nw);
+        const unsigned row =
+            fast ? tile_row_f32<false>(R, cc, hi, lane, xi, ai >= 0, pj, jreal, S, rlim2f, band, unsure)
+                 : tile_row_f32<true>(R, cc, hi, lane, xi, ai >= 0, pj, jreal, S, rlim2f, band, unsure);
+        if (!unsure) mask = __funnelshift_r(row, row, lane);
       }
-    }
-    const int sy = __shfl_sync(full, qy, src & 31);
-    const unsigned socc = __shfl_sync(full, qocc, src & 31);
-    const int sm = __shfl_sync(full, qs, src & 31);   // the source tile's rows in tmp_masks
-    const float shx = __shfl_sync(full, qsh.x, src & 31);
-    const float shy = __shfl_sync(full, qsh.y, src & 31);
-    const float shz = __shfl_sync(full, qsh.z, src & 31);
-    const bool live = src >= 0 && s0 + lane < e1;
-    const int jl = live ? (int)__fns(socc, 0, kk + 1) : 0;   // the slot's j lane in its tile
-    float4 ent = make_float4(0.f, 0.f, 0.f, __int_as_float(-1));
-    int ty = dummy_type;
-    if (live) {
-      const int slot = sy * kTile + jl;
-      ent = make_float4(shx, shy, shz, __int_as_float(P.satom[slot]));
-      ty = P.styp[slot];
-    }
-    P.ct_j[(size_t)ct * 32 + lane] = ent;
-    P.ct_ty[(size_t)ct * 32 + lane] = type_half(ty);
-    // record row r (bit p: slot p) is one ballot: slot p's bit is bit jl of row 16 h + r of its
-    // source tile (stored rotated: bit k is j lane (row + k) & 31); lane r keeps row r
-    {
-      const unsigned* rows = P.tmp_masks + (size_t)(live ? sm : 0) * 32 + kHalf * h;
-      unsigned m[kHalf];
-#pragma unroll
-      for (int r = 0; r < kHalf; ++r) m[r] = live ? rows[r] : 0u;
-#pragma unroll
-      for (int r = 0; r < kHalf; ++r) {
-        const unsigned row = __ballot_sync(full, (m[r] >> ((jl - kHalf * h - r) & 31)) & 1u);
-        if (lane == r) cur = row;
-      }
-      if (cmm) {
-        const unsigned* rows_el = P.tmp_masks_el + (size_t)(live ? sm : 0) * 32 + kHalf * h;
-#pragma unroll
-        for (int r = 0; r < kHalf; ++r) m[r] = live ? rows_el[r] : 0u;
-#pragma unroll
-        for (int r = 0; r < kHalf; ++r) {
-          const unsigned row = __ballot_sync(full, (m[r] >> ((jl - kHalf * h - r) & 31)) & 1u);
-          if (lane == r) cur_el = row;
+      if (unsure) {
+        if (fast) {
+          const unsigned row = tile_row_fast(P.satom, P.x, P.blk_ref, R, bi, bj, lane, ai, S, rlim2);
+          mask = __funnelshift_r(row, row, lane);
+        } else {
+          mask = tile_mask<CMM>(P.satom, P.x, P.cmm_cell, R, bi, bj, lane, ai, rlim2, rc2, mel);
         }
       }
+      if (bj == bi) mask &= lane < 16 ? 0x1fffeu : 0xfffeu;   // each unordered pair once, no self pair
+      const int rel = bj - bi - seg;
+      if ((S.excl[rel >> 5] >> (rel & 31)) & 1u) mask = drop_excluded(P, bj, lane, ai, mask);
+      mask_rows(c, false)[lane] = mask;
+      if (CMM) mask_rows(c, true)[lane] = mel & mask;
+      const unsigned rowj = __funnelshift_l(mask, mask, lane);
+      const unsigned o0 = __reduce_or_sync(full, lane < kHalf ? rowj : 0u);
+      const unsigned o1 = __reduce_or_sync(full, lane < kHalf ? 0u : rowj);
+      if (lane == 0) {
+        T.occ[0] = o0;
+        T.occ[1] = o1;
+        if (keep && !count_only && (o0 | o1)) {
+          const int t = atomicAdd(P.ntiles, 1);
+          P.tiles[t] = make_int2(bi, bj);
+          P.tile_src[t] = t0 + c;
+        }
+      }
     }
-    if (lane < kHalf) {
-      P.ct_mask[(size_t)ct * kHalf + lane] = record_row(cur, lane);
-      if (cmm) P.ct_mask_el[(size_t)ct * kHalf + lane] = record_row(cur_el, lane);
+    nt += n;
+    __syncthreads();
+  }
+
+  // entries of each half: exclusive sums over the tiles
+  if (threadIdx.x < 2) S.carry[threadIdx.x] = 0;
+  for (int c0 = 0; c0 < nt; c0 += blockDim.x) {
+    const int c = c0 + threadIdx.x;
+    int n0 = 0, n1 = 0;
+    if (c < nt) {
+      const BlkTile& T = blk_tile(P, S, t0, c);
+      n0 = __popc(T.occ[0]);
+      n1 = __popc(T.occ[1]);
+    }
+    int s0 = n0, s1 = n1;
+    for (int o = 1; o < 32; o <<= 1) {
+      const int y0 = __shfl_up_sync(full, s0, o), y1 = __shfl_up_sync(full, s1, o);
+      if (lane >= o) { s0 += y0; s1 += y1; }
+    }
+    if (lane == 31) { S.wsum[w][0] = s0; S.wsum[w][1] = s1; }
+    __syncthreads();
+    int b0 = S.carry[0], b1 = S.carry[1];
+    for (int v = 0; v < w; ++v) { b0 += S.wsum[v][0]; b1 += S.wsum[v][1]; }
+    if (c < nt) {
+      BlkTile& T = blk_tile(P, S, t0, c);
+      T.eoff[0] = b0 + s0 - n0;
+      T.eoff[1] = b1 + s1 - n1;
+    }
+    __syncthreads();
+    if (threadIdx.x == blockDim.x - 1) { S.carry[0] = b0 + s0; S.carry[1] = b1 + s1; }
+  }
+  __syncthreads();
+  const int E[2] = {S.carry[0], S.carry[1]};
+  const int nr0 = (E[0] + 31) >> 5, nr1 = (E[1] + 31) >> 5;
+  if (threadIdx.x == 0) {
+    P.ct_cnt[2 * bi] = nr0;
+    P.ct_cnt[2 * bi + 1] = nr1;
+    if (!count_only && !split_cls) S.base = atomicAdd(P.nctiles, nr0 + nr1);
+  }
+  if (count_only) return;
+
+  // the records, kWindow of each half at a time: every tile spreads its entries over the
+  // window's list, then a warp takes a record, lane p slot p
+  for (int w0 = 0; w0 < max(nr0, nr1); w0 += kWindow) {
+    __syncthreads();
+    for (int c = w; c < nt; c += nw) {
+      const BlkTile& T = blk_tile(P, S, t0, c);
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const unsigned occ = T.occ[h];
+        const int e = T.eoff[h] + __popc(occ & ((1u << lane) - 1u)) - 32 * w0;
+        if (((occ >> lane) & 1u) && e >= 0 && e < 32 * kWindow) S.elist[h][e] = ((unsigned)c << 5) | lane;
+      }
+    }
+    __syncthreads();
+    const int m0 = max(0, min(kWindow, nr0 - w0)), m1 = max(0, min(kWindow, nr1 - w0));
+    if (split_cls) {
+      for (int q = w; q < m0 + m1; q += nw) {
+        const int h = q < m0 ? 0 : 1, r = q < m0 ? q : q - m0;
+        int ty = 0;
+        if (32 * (w0 + r) + lane < E[h]) {
+          const unsigned v = S.elist[h][32 * r + lane];
+          ty = P.styp[(blk_tile(P, S, t0, (int)(v >> 5)).j & kTileBlock) * kTile + (int)(v & 31u)];
+        }
+        if (lane < kHalf) ty |= P.styp[bi * kTile + kHalf * h + lane];
+        const bool cls = __any_sync(full, (ty >> 30) & 1);
+        if (lane == 0) S.rcls[q] = cls ? 1 : 0;
+      }
+      __syncthreads();
+      if (w == 0) {   // places of the window's records in their two sequences
+        int n[2] = {0, 0};
+        for (int pass = 0; pass < 2; ++pass) {
+          int b[2] = {0, 0};
+          if (pass) {
+            if (lane < 2) b[0] = atomicAdd(&P.nctiles[lane], lane ? n[1] : n[0]);
+            b[1] = __shfl_sync(full, b[0], 1);
+            b[0] = __shfl_sync(full, b[0], 0);
+            n[0] = n[1] = 0;
+          }
+          for (int q0 = 0; q0 < m0 + m1; q0 += 32) {
+            const bool in = q0 + lane < m0 + m1;
+            const bool cls = in && S.rcls[q0 + lane];
+            const unsigned mc = __ballot_sync(full, cls), mp = __ballot_sync(full, in && !cls);
+            const unsigned below = (1u << lane) - 1u;
+            if (pass && in)
+              S.rpos[q0 + lane] = cls ? P.rec_cap - 1 - (size_t)(b[1] + n[1] + __popc(mc & below))
+                                      : (size_t)(b[0] + n[0] + __popc(mp & below));
+            n[0] += __popc(mp);
+            n[1] += __popc(mc);
+          }
+        }
+      }
+      __syncthreads();
+    }
+    for (int q = w; q < m0 + m1; q += nw) {
+      const int h = q < m0 ? 0 : 1, r = q < m0 ? q : q - m0;   // record r of the window of half h
+      const size_t ct = split_cls ? S.rpos[q] : (size_t)S.base + (h ? nr0 : 0) + w0 + r;
+      const bool live = 32 * (w0 + r) + lane < E[h];
+      const unsigned v = live ? S.elist[h][32 * r + lane] : 0u;
+      const int c = (int)(v >> 5), jl = (int)(v & 31u);
+      float4 ent = make_float4(0.f, 0.f, 0.f, __int_as_float(-1));
+      int ty = dummy_type;
+      bool img = false;
+      if (live) {
+        const BlkTile& T = blk_tile(P, S, t0, c);
+        img = (T.j & kTilePairImg) != 0;
+        const int slot = (T.j & kTileBlock) * kTile + jl;
+        ent = make_float4(-T.cx, -T.cy, -T.cz, __int_as_float(P.satom[slot]));
+        ty = P.styp[slot];
+      }
+      P.ct_j[ct * 32 + lane] = ent;
+      P.ct_ty[ct * 32 + lane] = type_half(ty);
+      const unsigned cur = record_rows(mask_rows(c, false) + kHalf * h, live, jl, h, lane);
+      if (lane < kHalf) P.ct_mask[ct * kHalf + lane] = record_row(cur, lane);
+      if (CMM) {
+        const unsigned cel = record_rows(mask_rows(c, true) + kHalf * h, live, jl, h, lane);
+        if (lane < kHalf) P.ct_mask_el[ct * kHalf + lane] = record_row(cel, lane);
+      }
+      const bool any_img = __any_sync(full, img);
+      if (lane == 0) P.ct_blk[ct] = (2 * bi + h) | (any_img ? kRecImg : 0);
     }
   }
 }
 
-int launch_compact_tiles(const DevPtrs& P, int nblk, int nchunk, int nsm, bool cmm, int dummy_type,
-                         int* scan_scratch, bool count_only, cudaStream_t st) {
-  const int nb = (2 * nblk + 127) / 128;
-  k_ct_count<<<nb, 128, 0, st>>>(P, nblk, nchunk);
-  if (count_only) return 1;
-  const int ns = scan_exclusive(P.ct_cnt, P.ct_off, 2 * nblk + 1, scan_scratch, P.nctiles, st);
-  k_ct_index<<<nsm * 4, 256, 0, st>>>(P, nchunk);
-  k_ct_emit<<<nsm * 8, 256, 0, st>>>(P, nchunk, cmm ? 1 : 0, dummy_type);
-  return 3 + ns;
+static size_t list_smem(bool cmm) { return sizeof(ListShared) + (size_t)kTileCache * 128 * (cmm ? 2 : 1); }
+
+void init_block_list() {
+  cudaFuncSetAttribute(k_block_list<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)list_smem(false));
+  cudaFuncSetAttribute(k_block_list<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)list_smem(true));
+}
+
+void launch_block_list(const DevPtrs& P, int nblk, int nsm, double rlim2, float rlimf, double rc2, bool cmm,
+                       int dummy_type, bool count_only, bool keep, bool split_cls, cudaStream_t st) {
+  // eight warps a block where the blocks alone do not fill the chip (each i-block's tiles in fewer
+  // rounds), four where they do (64 replicas: 2,994 us a build with four, 3,287 with eight)
+  const int nt = 32 * (nblk < 8 * nsm ? 8 : 4);
+  if (cmm)
+    k_block_list<true><<<nblk, nt, list_smem(true), st>>>(P, rlim2, rlimf, rc2, dummy_type, count_only, keep, split_cls);
+  else
+    k_block_list<false><<<nblk, nt, list_smem(false), st>>>(P, rlim2, rlimf, rc2, dummy_type, count_only, keep, split_cls);
 }
 
 // ---- deterministic exclusive scan (3 passes) --------------------------------------------

@@ -20,6 +20,7 @@ namespace jp {
 
 constexpr int kTile = 32;
 constexpr int kHalf = 16;   // i atoms of a pair record: half a block
+constexpr int kRecImg = 1 << 30;   // in ct_blk: a record with a tile whose pairs take their own images
 // fixed-point scales: forces 2^32 per kcal/mol/A, energies 2^32 per kcal/mol,
 // kinetic sums (m v^2, amu A^2/fs^2) 2^40.
 constexpr double kFrcScale = 4294967296.0;
@@ -165,6 +166,15 @@ struct MinState {
   double ene[JP_MAXENE];    // energies of the last evaluation
 };
 
+// a tile of an i-block's list: its j block, that block's reference in the i block's frame, the
+// j lanes each half lists and the first entry of each half it contributes
+struct BlkTile {
+  int j;                    // and its image flags (jp_cells.cu)
+  float cx, cy, cz;
+  unsigned occ[2];
+  int eoff[2];
+};
+
 struct DevPtrs {
   // bound of every grid-barrier wait of the cooperative integration, in SM clock cycles
   long long wait_cycles;
@@ -187,30 +197,25 @@ struct DevPtrs {
   int *blk_rep;
   float4 *blk_ctr, *blk_half;     // bbox (wrapped frame) centre / half extent
   double *blk_ref;                // [B][3]
-  // tile-list build: chunk = (i-block, 32 candidate j-blocks from j0)
-  int *chunk_i, *chunk_j0;        // static per context
-  unsigned *chunk_nz;             // non-empty candidates of the chunk (bit b = j0+b)
-  int *chunk_cnt, *chunk_off;     // their count and its exclusive scan [nchunk+1]
-  unsigned *tmp_masks;            // [nchunk*32][32] masks of the chunk candidates
-  // tiles
-  int2 *tiles;                    // dense (i-block, j-block)
-  int *tile_src;                  // [T] where each tile's mask rows are in tmp_masks: chunk * 32 + candidate
+  // pair list build: an i-block's tiles (its candidate j blocks that passed the bounding-box
+  // test) start at blk_tile0 in the arrays that hold one element per possible tile
+  long long *blk_tile0;           // [nblk] (static)
+  BlkTile *blk_tiles;             // tiles beyond a block's shared-memory cache
+  unsigned *tmp_masks;            // [tile][32] their mask rows: bit k of row i is j lane (i + k) & 31
+  // the tiles themselves, listed only for the H-bond list
+  int2 *tiles;                    // (i-block, j-block)
+  long long *tile_src;            // where each tile's mask rows are in tmp_masks
   int *ntiles;                    // device scalar
-  // compact tiles (what the pair kernels run on): an i-block and 32 j entries
-  int *blk_chunk0;                // [nblk+1] first chunk of each i-block (static)
-  int *ct_cnt, *ct_off;           // pair records per unit (2 i-block + half) and their scan [2 nblk+1]
-  int *ct_blk;                    // [CT] unit of each pair record
-  unsigned *tmp_occ;              // [nchunk*32][2] occupied j lanes of each chunk candidate, per half
-  int *chunk_ent, *chunk_eoff;    // per half [2][nchunk+1]: entries per chunk, their exclusive scan
-  int *tile_eoff;                 // [T][2] first entry of each tile in its half's order (global)
-  float4 *ct_j;                   // [CT][32] (image shift into the i frame, atom bits; -1 = empty).
-                                  // Between k_ct_index and the emit, entry 0 holds what the emit
-                                  // needs: the record's first source tile, the global entry of its
-                                  // slot 0, the end of its unit's entries, and (end of its block's
-                                  // tiles) << 1 | half
+  // pair records (what the pair kernels run on): half an i-block and 32 j entries
+  int *ct_cnt;                    // records per unit (2 i-block + half)
+  int *ct_blk;                    // [CT] unit of each pair record, with kRecImg
+  int *ext_pos;                   // coordinates were replaced since the last list build: the records'
+                                  // image flags, made for the motion between builds, don't hold
+  float4 *ct_j;                   // [CT][32] (image shift into the i frame, atom bits; -1 = empty)
   unsigned short *ct_ty;          // [CT][32] type word of each entry (type_half; empty: dummy type)
   unsigned *ct_mask, *ct_mask_el; // [CT][32] rotated masks (listed pairs; CMM Coulomb pairs)
-  int *nctiles;                   // device scalar
+  int *nctiles;                   // records from the start of the arrays, and (ALSD, mixed) from their end
+  size_t rec_cap;                 // length of the record arrays
   // cell sort
   unsigned *key;                  // per atom
   int *hist, *hist_scan, *cursor; // per key
@@ -245,7 +250,7 @@ struct DevPtrs {
   double *ext_pot;                // their 13 coefficients
   // accumulators
   long long *ene_fix;             // [nrep][16], then the pair kernels' tile counter
-  int *tile_ctr;                  // next unclaimed tile (zeroed with ene_fix every step)
+  int *tile_ctr;                  // [2] next unclaimed tile of each sequence (zeroed with ene_fix every step)
   long long *kin_fix;             // [nslots_kin][nsub_total]
   double *nfr;                    // DOF per sub-system
   int *sub_rep;                   // replica of each sub-system

@@ -15,15 +15,14 @@ __global__ void k_clear_slots(DevPtrs P, int nslot, int dummy_type);
 __global__ void k_fill_slots(DevPtrs P, int natom);
 __global__ void k_excl_slots(DevPtrs P, int natom);
 __global__ void k_block_setup(DevPtrs P, int nblk, double qscale);
-// CMM: masks from the level-1 cells (neighbours: Coulomb + LJ into masks and masks_el;
-// cells up to idelay apart and r^2 < rc2: LJ only) instead of the list radius
-void launch_tile_scan(const DevPtrs& P, int nchunk, double rlim2, float rlimf, double rc2, bool cmm,
-                      cudaStream_t st);
-__global__ void k_tile_emit(DevPtrs P, int nchunk, int cmm);
-// pair records of every i-block from the tile list (count, scan, emit; with count_only the
-// records per unit alone); returns the launches
-int launch_compact_tiles(const DevPtrs& P, int nblk, int nchunk, int nsm, bool cmm, int dummy_type,
-                         int* scan_scratch, bool count_only, cudaStream_t st);
+// tiles and pair records of every i-block.  CMM: masks from the level-1 cells (neighbours:
+// Coulomb + LJ into masks and masks_el; cells up to idelay apart and r^2 < rc2: LJ only) instead
+// of the list radius.  count_only: the records per unit alone; keep: masks left in global
+// memory and the tiles listed (for the H-bond list); split_cls: records with ALSD cluster atoms
+// apart (k_block_list).  init_block_list: once per context.
+void init_block_list();
+void launch_block_list(const DevPtrs& P, int nblk, int nsm, double rlim2, float rlimf, double rc2, bool cmm,
+                       int dummy_type, bool count_only, bool keep, bool split_cls, cudaStream_t st);
 // deterministic exclusive scan of n ints (total: the sum, or null); returns the launches
 int scan_exclusive(const int* in, int* out, int n, int* scratch, int* total, cudaStream_t st);
 
@@ -43,10 +42,11 @@ void launch_cmm_far(const DevPtrs& P, int natom, int nrep, bool fp64, bool force
                     cudaStream_t st);
 
 // pair kernels (jp_pair.cu)
-// alsd: some replica has ALSD classes; split: some replica keeps partial-McMD class-1 forces
+// alsd: some replica has ALSD classes (every_cls: class weights that are not lambda's, so the
+// records without cluster atoms are weighted too); split: some replica keeps partial-McMD class-1 forces
 // apart (frc1 / grd1)
-void launch_pair_mixed(const DevPtrs& P, const ZdConst& z, int nwarps, bool count, bool alsd, bool split,
-                       cudaStream_t st);
+void launch_pair_mixed(const DevPtrs& P, const ZdConst& z, int nwarps, bool count, bool alsd, bool every_cls,
+                       bool split, cudaStream_t st);
 void launch_pair_fp64(const DevPtrs& P, const ZdConst& z, int nwarps, bool count, bool alsd, bool split,
                       cudaStream_t st);
 // co-resident blocks per SM of the (non-counting) pair kernel: the grid is one full wave

@@ -157,20 +157,24 @@ __device__ __forceinline__ float rint1(float v) {
 // of them per lane group (19,000 atomics) a launch on 24,000 atoms took 59.1 us, so 52.0.
 // Called by all threads of the block.
 template <int W>
-__device__ __forceinline__ void flush_block(const DevPtrs& P, int rep, long long eel, long long elj, long long npair,
-                                            bool count, bool cls) {
-  __shared__ long long s_sum[kPairWarps][3];
+__device__ __forceinline__ void flush_block(const DevPtrs& P, int rep, long long eel, long long elj, long long eaa,
+                                            long long eab, long long npair, bool count, bool cls) {
+  __shared__ long long s_sum[kPairWarps][5];
   __shared__ int s_rep[kPairWarps];
   const unsigned full = 0xffffffffu;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   int r = __reduce_max_sync(full, rep);
   if (!__all_sync(full, rep < 0 || rep == r)) {   // lane groups of several replicas
-    flush_fix<W>(P, rep, eel, elj, 0, 0, npair, count, cls);
+    flush_fix<W>(P, rep, eel, elj, eaa, eab, npair, count, cls);
     r = -1;
   }
   for (int o = 16; o > 0; o >>= 1) {
     eel += __shfl_xor_sync(full, eel, o);
     elj += __shfl_xor_sync(full, elj, o);
+    if (cls) {
+      eaa += __shfl_xor_sync(full, eaa, o);
+      eab += __shfl_xor_sync(full, eab, o);
+    }
     if (count) npair += __shfl_xor_sync(full, npair, o);
   }
   if (lane == 0) {
@@ -178,32 +182,42 @@ __device__ __forceinline__ void flush_block(const DevPtrs& P, int rep, long long
     s_sum[warp][0] = eel;
     s_sum[warp][1] = elj;
     s_sum[warp][2] = count ? npair : 0;
+    s_sum[warp][3] = eaa;
+    s_sum[warp][4] = eab;
   }
   __syncthreads();
   if (threadIdx.x == 0) {
     for (int w = 0; w < kPairWarps; ++w) {
       const int rw = s_rep[w];
       if (rw < 0) continue;
-      long long a = 0, b = 0, n = 0;   // the warps of this replica, taken together
+      long long a = 0, b = 0, n = 0, ca = 0, cb = 0;   // the warps of this replica, taken together
       for (int v = w; v < kPairWarps; ++v)
         if (s_rep[v] == rw) {
           a += s_sum[v][0];
           b += s_sum[v][1];
           n += s_sum[v][2];
+          ca += s_sum[v][3];
+          cb += s_sum[v][4];
           s_rep[v] = -1;
         }
       atomic_add_ll(&P.ene_fix[rw * 16 + JP_E_ELE15], a);
       atomic_add_ll(&P.ene_fix[rw * 16 + JP_E_VDW15], b);
-      if (cls) atomic_add_ll(&P.ene_cls[rw * 4 + 2], a + b);
+      if (cls) {
+        if (ca) atomic_add_ll(&P.ene_cls[rw * 4 + 0], ca);
+        if (cb) atomic_add_ll(&P.ene_cls[rw * 4 + 1], cb);
+        atomic_add_ll(&P.ene_cls[rw * 4 + 2], a + b - ca - cb);
+      }
       if (count) atomic_add_ll(&P.pair_cnt[rw], n);
     }
   }
 }
 
 // ---- packed kernel: four records a warp, eight lanes and two i atoms a lane -----------------
-// In ALSD contexts (CLS) a group whose records hold no cluster atom takes the plain loop; the
-// others add class weights and class energies to it (32 replicas of 9,100 atoms with four
-// cluster residues each: 897 us with the classes in every record, 686 so).
+// In ALSD contexts the records that hold a cluster atom stand apart (k_block_list) and take a
+// launch of their own with class weights and class energies (CLS); the others take the plain
+// kernel.  Both forms in one kernel, chosen per group, spilled the class state and ran the rare
+// form's instructions through the others' cache (32 replicas of 9,100 atoms with four cluster
+// residues each: 897 us with the classes in every record, 717 chosen per group, 573 so).
 // Per-warp shared memory: two bulk-copy buffers (entries, their atoms and types, and masks of a
 // record group: record q in entries 32 q and masks 16 q), and the staged j atoms of the group
 // being computed.  The position of entry 8 g + e of record q is staged twice, at 64 q + 16 g + e
@@ -384,8 +398,10 @@ __host__ __device__ constexpr size_t lj_bytes(int nt1) {
 }
 constexpr size_t kPackedStageBytes = sizeof(QuadStage) * kPairWarps;
 
+// CLS: every record with class weights and energies, from the sequence at the arrays' end
+// (seq = 1) or the one at their start; without it cls_sum adds the energies to class BB
 template <bool COUNT, bool CLS, bool TRI>
-__global__ void __launch_bounds__(kPairThreads, 2) k_pair_packed(DevPtrs P, ZdConst z) {
+__global__ void __launch_bounds__(kPairThreads, CLS ? 1 : 2) k_pair_packed(DevPtrs P, ZdConst z, int seq, int cls_sum) {
   extern __shared__ __align__(16) unsigned char s_dyn[];
   __shared__ unsigned long long s_tab_bar;
   const unsigned full = 0xffffffffu;
@@ -408,7 +424,10 @@ __global__ void __launch_bounds__(kPairThreads, 2) k_pair_packed(DevPtrs P, ZdCo
     bulk_load(s_dyn + kPackedStageBytes, P.lj_tab, (unsigned)lj_bytes(z.nt1), &s_tab_bar);
   }
   __syncthreads();
-  const int T = *P.nctiles;         // records
+  const int T = P.nctiles[seq];     // records
+  // record of lane group qd in group t, and the first record of the group's copies
+  auto rec0 = [&](int t) { return seq ? P.rec_cap - 4 * (size_t)(t + 1) : 4 * (size_t)t; };
+  const bool ext = *P.ext_pos != 0;
   const int TU = (T + 3) >> 2;      // record groups: a warp's work units
   // a 2.5-KiB copy lands in microseconds; the bound (about a second of SM clock) only ends
   // the wait on a broken device, and it is not the integrator's adjustable barrier bound:
@@ -428,22 +447,23 @@ __global__ void __launch_bounds__(kPairThreads, 2) k_pair_packed(DevPtrs P, ZdCo
     if (run_next >= run_end) {
       if (nw * run >= TU) return TU;
       int t = 0;
-      if (lane == 0) t = atomicAdd(P.tile_ctr, run);
+      if (lane == 0) t = atomicAdd(&P.tile_ctr[seq], run);
       t = __shfl_sync(full, t, 0) + nw * run;
       run_next = t;
       run_end = min(t + run, TU);
     }
     return run_next < run_end ? run_next++ : TU;
   };
-  // the entries, types and masks of records 4t .. 4t + 3 into buffer b (up to three past
-  // the last record are padding inside the arrays: read, never used)
+  // the entries, types and masks of group t's four records into buffer b (up to three past
+  // the last record of the sequence lie inside the arrays: read, never used)
   auto issue = [&](int t, int b) {
     if (lane == 0) {
+      const size_t r0 = rec0(t);
       fence_proxy_async();
       mbar_expect(&S.bar[b], 2560u);
-      bulk_load(S.ent[b], P.ct_j + (size_t)t * 128, 2048u, &S.bar[b]);
-      bulk_load(S.ty[b], P.ct_ty + (size_t)t * 128, 256u, &S.bar[b]);
-      bulk_load(S.msk[b], P.ct_mask + (size_t)t * 64, 256u, &S.bar[b]);
+      bulk_load(S.ent[b], P.ct_j + r0 * 32, 2048u, &S.bar[b]);
+      bulk_load(S.ty[b], P.ct_ty + r0 * 32, 256u, &S.bar[b]);
+      bulk_load(S.msk[b], P.ct_mask + r0 * kHalf, 256u, &S.bar[b]);
     }
     pend |= 1u << b;
   };
@@ -456,9 +476,8 @@ __global__ void __launch_bounds__(kPairThreads, 2) k_pair_packed(DevPtrs P, ZdCo
     }
     phase ^= 1u << b;
     pend &= ~(1u << b);
-    const int rec = 4 * t + qd;
-    const bool valid = rec < T;
-    G.unit = valid ? P.ct_blk[rec] : -1;
+    const bool valid = 4 * t + (seq ? 3 - qd : qd) < T;   // the sequence at the end runs downwards
+    G.unit = valid ? P.ct_blk[rec0(t) + qd] : -1;
 #pragma unroll
     for (int g = 0; g < 4; ++g) {
       const int aj = valid ? __float_as_int(S.ent[b][32 * qd + 8 * g + lp].w) : -1;
@@ -475,7 +494,7 @@ __global__ void __launch_bounds__(kPairThreads, 2) k_pair_packed(DevPtrs P, ZdCo
   A.w0 = A.w1 = make_float2(1.f, 1.f);   // set where a record holds classes
   int cur_unit = -2, cur_rep = -1, rep = -1, aia = -1, aib = -1, tia = z.nt1 - 1, tib = tia;
   long long gia[3] = {0, 0, 0}, gib[3] = {0, 0, 0};
-  long long eel = 0, elj = 0;
+  long long eel = 0, elj = 0, eaa = 0, eab = 0;
   long long npair = 0;
   bool mi = false;
   auto flush_i = [&]() {
@@ -517,7 +536,7 @@ __global__ void __launch_bounds__(kPairThreads, 2) k_pair_packed(DevPtrs P, ZdCo
       S.at[sta + 8 * g] = ta;
       if (CLS) jc |= ((__ballot_sync(full, (ta.y >> 30) & 1) >> (8 * qd)) & 0xffu) << (8 * g);
     }
-    const int unit = G.unit;
+    const int unit = G.unit >= 0 ? G.unit & ~kRecImg : -1;
     A.ma = unit >= 0 ? step_mask(S.msk[b][16 * qd + lp], lp) : 0u;
     A.mb = unit >= 0 ? step_mask(S.msk[b][16 * qd + 8 + lp], lp + 8) : 0u;
     // the lane's i atoms: a new unit flushes the last one's forces and loads the new atoms
@@ -545,8 +564,8 @@ __global__ void __launch_bounds__(kPairThreads, 2) k_pair_packed(DevPtrs P, ZdCo
     }
     // a new replica in any record: every record's energies go to its replica so far
     if (__any_sync(full, rep != cur_rep)) {
-      flush_fix<8>(P, cur_rep, eel, elj, 0, 0, npair, COUNT, CLS);
-      eel = elj = 0;
+      flush_fix<8>(P, cur_rep, eel, elj, eaa, eab, npair, COUNT, CLS || cls_sum);
+      eel = elj = eaa = eab = 0;
       npair = 0;
       if (rep != cur_rep) {
         cur_rep = rep;
@@ -554,21 +573,22 @@ __global__ void __launch_bounds__(kPairThreads, 2) k_pair_packed(DevPtrs P, ZdCo
         if (lp < 6) S.rep[qd][lp] = (float)(lp < 3 ? R.box[lp] : R.invbox[lp - 3]);
         if (CLS && lp < 3) S.rep[qd][6 + lp] = (float)cls_weight(R, P.lam[2 * rep], 2 - lp);
         // Per-pair minimum image is needed only where a pair within the cut-off can have
-        // another image than its tile's.  Per axis the tile's image puts the two block
-        // references at most box/2 apart, and a pair's separation differs from theirs by at
-        // most h_i + h_j <= 2 h_max plus the atoms' motion since the build (2 A margin), so
-        // in the tile's image |d| <= box/2 + 2 h_max + 2; in any other image |d| >= box - rc.
-        // Both hold at once only if box/2 <= rc + 2 h_max + 2.
+        // another image than its tile's: the list build flags the records with such a tile
+        // (k_block_list).  Coordinates replaced without a build since may have moved farther
+        // than its margin: then, by replica, as the largest block allows -- per axis the tile's
+        // image puts the two block references at most box/2 apart, and a pair's separation
+        // differs from theirs by at most h_i + h_j <= 2 h_max plus 2 A of motion, so in the
+        // tile's image |d| <= box/2 + 2 h_max + 2; in any other image |d| >= box - rc; both
+        // hold at once only if box/2 <= rc + 2 h_max + 2
         mi = false;
-        for (int k = 0; k < 3; ++k)
-          if (0.5 * R.box[k] < sqrt(z.rc2) + 2.0 * (double)P.rep_hmax[3 * rep + k] + 2.0) mi = true;
+        if (ext)
+          for (int k = 0; k < 3; ++k)
+            if (0.5 * R.box[k] < sqrt(z.rc2) + 2.0 * (double)P.rep_hmax[3 * rep + k] + 2.0) mi = true;
       }
     }
-    const bool wmi = __any_sync(full, mi);   // one image form for the whole warp
-    bool wcls = false;                       // does any record of the group hold a class but BB?
+    // one image form for the whole warp
+    const bool wmi = __any_sync(full, mi || (G.unit >= 0 && (G.unit & kRecImg)));
     __syncwarp();
-    if (CLS)   // BB records keep the plain form unless BB itself is weighted (per-class evaluation)
-      wcls = __any_sync(full, jc != 0u || (((tia | tib) >> 30) & 1) || S.rep[qd][6] != 1.f);
     // buffer b is free again: the group after next goes into it; the next group's gathers
     // are issued before this group's arithmetic
     int t2 = TU;
@@ -583,33 +603,24 @@ __global__ void __launch_bounds__(kPairThreads, 2) k_pair_packed(DevPtrs P, ZdCo
     const int ka = CLS ? (tia & kTypeMask) : tia, kb = CLS ? (tib & kTypeMask) : tib;
     const int rowa = TRI ? (ka * z.nt1 + kb) * z.nt1 : ka * z.nt1, rowb = kb * z.nt1;
     double ea = 0.0, eb = 0.0;
-    if (CLS && wcls) {
+    if (CLS) {
       const float f0 = S.rep[qd][6], f1 = S.rep[qd][7], f2 = S.rep[qd][8];
       A.ca = ((tia >> 30) & 1) != 0;
       A.cb = ((tib >> 30) & 1) != 0;
       A.jc = byte_rotr(jc, lp);
       A.w0 = make_float2(A.ca ? f1 : f0, A.cb ? f1 : f0);
       A.w1 = make_float2(A.ca ? f2 : f1, A.cb ? f2 : f1);
-      if (wmi)
-        record_packed<true, COUNT, TRI, CLS>(P, S, s_lj, s_lj3, rowa, rowb, A, sp, sta, sat, src, fx, fy, fz, te,
-                                             tl, tn_pairs, ea, eb);
-      else
-        record_packed<false, COUNT, TRI, CLS>(P, S, s_lj, s_lj3, rowa, rowb, A, sp, sta, sat, src, fx, fy, fz, te,
-                                              tl, tn_pairs, ea, eb);
-      // classes AA and AB of these few records go to their slots at once; BB, which the flush
-      // credits with everything, gives them back
-      const long long xa = to_fix(ea, kEneScale, P.status), xb = to_fix(eb, kEneScale, P.status);
-      if (cur_rep >= 0 && (xa | xb)) {
-        atomic_add_ll(&P.ene_cls[cur_rep * 4 + 0], xa);
-        atomic_add_ll(&P.ene_cls[cur_rep * 4 + 1], xb);
-        atomic_add_ll(&P.ene_cls[cur_rep * 4 + 2], -(xa + xb));
-      }
-    } else if (wmi) {
-      record_packed<true, COUNT, TRI, false>(P, S, s_lj, s_lj3, rowa, rowb, A, sp, sta, sat, src, fx, fy, fz, te,
-                                             tl, tn_pairs, ea, eb);
-    } else {
-      record_packed<false, COUNT, TRI, false>(P, S, s_lj, s_lj3, rowa, rowb, A, sp, sta, sat, src, fx, fy, fz, te,
-                                              tl, tn_pairs, ea, eb);
+    }
+    // (classes: with per-pair images always, which change nothing where they are not needed)
+    if (CLS || wmi)
+      record_packed<true, COUNT, TRI, CLS>(P, S, s_lj, s_lj3, rowa, rowb, A, sp, sta, sat, src, fx, fy, fz, te, tl,
+                                           tn_pairs, ea, eb);
+    else
+      record_packed<false, COUNT, TRI, CLS>(P, S, s_lj, s_lj3, rowa, rowb, A, sp, sta, sat, src, fx, fy, fz, te, tl,
+                                            tn_pairs, ea, eb);
+    if (CLS) {
+      eaa += to_fix(ea, kEneScale, P.status);
+      eab += to_fix(eb, kEneScale, P.status);
     }
     gia[0] += to_fix_f(fx.x, P.status);
     gia[1] += to_fix_f(fy.x, P.status);
@@ -625,7 +636,7 @@ __global__ void __launch_bounds__(kPairThreads, 2) k_pair_packed(DevPtrs P, ZdCo
     b ^= 1;
   }
   flush_i();
-  flush_block<8>(P, cur_rep, eel, elj, npair, COUNT, CLS);
+  flush_block<8>(P, cur_rep, eel, elj, eaa, eab, npair, COUNT, CLS || cls_sum);
   // a copy still in flight (only after a timed-out wait) must land before the block exits
   for (int k = 0; k < 2; ++k)
     if ((pend >> k) & 1u) mbar_wait(&S.bar[k], (phase >> k) & 1u, wlim);
@@ -817,7 +828,7 @@ k_pair_mixed(DevPtrs P, ZdConst z) {
     const bool valid = rec < T;
     G.m = valid ? S.msk[b][lane] : 0u;
     G.me = CMM && valid ? S.msk_el[b][lane] : 0u;
-    G.unit = valid ? P.ct_blk[rec] : -1;
+    G.unit = valid ? P.ct_blk[rec] & ~kRecImg : -1;
     gather1(S.ent[b][32 * hw + lp], valid, G.pa, G.ta, G.aa);
     gather1(S.ent[b][32 * hw + kHalf + lp], valid, G.pb, G.tb, G.ab);
   };
@@ -1031,7 +1042,7 @@ k_pair_fp64(DevPtrs P, ZdConst z) {
     if (t >= TU) break;
     const int rec = 2 * t + hw;
     const bool valid = rec < T;
-    const int unit = valid ? P.ct_blk[rec] : -1;
+    const int unit = valid ? P.ct_blk[rec] & ~kRecImg : -1;
     if (unit != cur_unit) {
       flush_i();
       cur_unit = unit;
@@ -1213,22 +1224,26 @@ int pair_blocks_per_sm(bool fp64, bool packed, int nt1) {
 }
 
 template <bool COUNT>
-static void launch_mixed(const DevPtrs& P, const ZdConst& z, int nb, bool alsd, bool split, cudaStream_t st) {
+static void launch_mixed(const DevPtrs& P, const ZdConst& z, int nb, bool alsd, bool every_cls, bool split,
+                         cudaStream_t st) {
   const size_t sh = sizeof(float2) * z.nt1 * z.nt1, shp = kPackedStageBytes + lj_bytes(z.nt1);
   const bool tri = lj_tri(z.nt1);
   if (split) k_pair_mixed<COUNT, false, true><<<nb, kPairThreads, sh, st>>>(P, z);
   else if (z.cmm) k_pair_mixed<COUNT, true, false><<<nb, kPairThreads, sh, st>>>(P, z);
-  else if (alsd && tri) k_pair_packed<COUNT, true, true><<<nb, kPairThreads, shp, st>>>(P, z);
-  else if (alsd) k_pair_packed<COUNT, true, false><<<nb, kPairThreads, shp, st>>>(P, z);
-  else if (tri) k_pair_packed<COUNT, false, true><<<nb, kPairThreads, shp, st>>>(P, z);
-  else k_pair_packed<COUNT, false, false><<<nb, kPairThreads, shp, st>>>(P, z);
+  else {
+    // the records with cluster atoms, and under every_cls the others too, by class
+    auto plain = tri ? k_pair_packed<COUNT, false, true> : k_pair_packed<COUNT, false, false>;
+    auto cls = tri ? k_pair_packed<COUNT, true, true> : k_pair_packed<COUNT, true, false>;
+    if (alsd) cls<<<nb, kPairThreads, shp, st>>>(P, z, 1, 0);
+    (every_cls ? cls : plain)<<<nb, kPairThreads, shp, st>>>(P, z, 0, alsd ? 1 : 0);
+  }
 }
 
-void launch_pair_mixed(const DevPtrs& P, const ZdConst& z, int nwarps, bool count, bool alsd, bool split,
-                       cudaStream_t st) {
+void launch_pair_mixed(const DevPtrs& P, const ZdConst& z, int nwarps, bool count, bool alsd, bool every_cls,
+                       bool split, cudaStream_t st) {
   const int nb = (nwarps + kPairWarps - 1) / kPairWarps;
-  if (count) launch_mixed<true>(P, z, nb, alsd, split, st);
-  else launch_mixed<false>(P, z, nb, alsd, split, st);
+  if (count) launch_mixed<true>(P, z, nb, alsd, every_cls, split, st);
+  else launch_mixed<false>(P, z, nb, alsd, every_cls, split, st);
 }
 
 void launch_pair_fp64(const DevPtrs& P, const ZdConst& z, int nwarps, bool count, bool alsd, bool split,
@@ -1253,14 +1268,23 @@ void launch_pair_fp64(const DevPtrs& P, const ZdConst& z, int nwarps, bool count
 // kernel positions from the master coordinates (after an external coordinate change)
 __global__ void k_update_pos(DevPtrs P, int natom, int fp64, double qscale) {
   const int a = blockIdx.x * blockDim.x + threadIdx.x;
+  if (a == 0) *P.ext_pos = 1;
   if (a >= natom) return;
-  const double x = P.x[3 * a], y = P.x[3 * a + 1], zz = P.x[3 * a + 2];
+  const double x[3] = {P.x[3 * a], P.x[3 * a + 1], P.x[3 * a + 2]};
   if (fp64) {
-    P.pos_d[a] = make_double4(x, y, zz, qscale * P.chg[a]);
-  } else {
-    P.pos_f[a] = make_float4((float)(x - P.off[3 * a]), (float)(y - P.off[3 * a + 1]),
-                             (float)(zz - P.off[3 * a + 2]), (float)(qscale * P.chg[a]));
+    P.pos_d[a] = make_double4(x[0], x[1], x[2], qscale * P.chg[a]);
+    return;
   }
+  // an atom put into another periodic image since the list build keeps to its block: its frame
+  // origin moves along, so that the FP32 position stays small
+  const Rep& R = P.reps[P.rep_of[a]];
+  float q[3];
+  for (int k = 0; k < 3; ++k) {
+    const double d = x[k] - P.off[3 * a + k], n = anint(d * R.invbox[k]);
+    q[k] = (float)(d - R.box[k] * n);
+    if (n != 0.0) P.off[3 * a + k] += R.box[k] * n;
+  }
+  P.pos_f[a] = make_float4(q[0], q[1], q[2], (float)(qscale * P.chg[a]));
 }
 
 void launch_update_pos(const DevPtrs& P, int natom, bool fp64, double qscale, cudaStream_t st) {

@@ -71,3 +71,17 @@ def test_few_records(eng_mod, natom):
         assert e.pair_count() == o.npairs_cut
     assert rms_rel(g, go) < 1e-5
     np.testing.assert_allclose(ene, eo, rtol=1e-5, atol=1e-2)
+
+
+@pytest.mark.parametrize("nwat", [700, 2900])
+def test_replaced_coordinates_without_a_build(eng_mod, nwat):
+    """Molecules put into other periodic images without a list build: the records' image flags no
+    longer hold, and pairs take their own images as the FP64 path does."""
+    top = systems.solvated_polymer(0, nwat, seed=23)
+    x = top["cord"] + np.repeat(np.random.default_rng(1).integers(-1, 2, (nwat, 3)), 3, axis=0) * top["box"]
+    out = []
+    for prec in (abi.JP_PREC_MIXED, abi.JP_PREC_FP64):
+        with eng_mod.Engine(top, precision=prec, method=abi.JP_METHOD_MICR) as e:
+            out.append(e.energy_grad(cord=x))
+    assert rms_rel(out[0][1], out[1][1]) < 1e-5
+    np.testing.assert_allclose(out[0][0], out[1][0], rtol=1e-5, atol=1e-2)
