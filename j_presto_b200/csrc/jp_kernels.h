@@ -50,7 +50,8 @@ void launch_pair_mixed(const DevPtrs& P, const ZdConst& z, int nwarps, bool coun
 void launch_pair_fp64(const DevPtrs& P, const ZdConst& z, int nwarps, bool count, bool alsd, bool split,
                       cudaStream_t st);
 // co-resident blocks per SM of the (non-counting) pair kernel: the grid is one full wave
-// (packed: the mixed path without CMM and partial McMD)
+// (packed: the kernels with two i atoms a lane -- the mixed path without CMM and partial McMD, the
+// FP64 path without those and ALSD)
 int pair_blocks_per_sm(bool fp64, bool packed, int nt1);
 // LJ table of the packed kernel (DevPtrs::lj_tab) from the type-pair (C6, C12)
 void pack_lj_table(const float2* lj, int nt1, std::vector<float>& out);

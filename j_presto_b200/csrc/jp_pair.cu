@@ -27,8 +27,8 @@
 // computes: the bulk-copy engine (cp.async.bulk, completion on an mbarrier) brings the
 // entries and masks of the group after next into shared memory, and the gathers of the next
 // group's j atoms are issued before the current group's arithmetic.
-// FP64 path: the same records in FP64 with absolute coordinates, per-pair minimum image and
-// FP64 force atomics.
+// FP64 path: the same records in FP64 with FP64 force atomics (k_pair_fp64q; k_pair_fp64 with
+// classes and CMM).
 #include <vector>
 
 #include "jp_kernels.h"
@@ -988,8 +988,221 @@ k_pair_mixed(DevPtrs P, ZdConst z) {
     if ((pend >> k) & 1u) mbar_wait(&S.bar[k], (phase >> k) & 1u, wlim);
 }
 
-// Per-warp shared memory of the FP64 kernel: each half-warp's record, entries a and b of
-// every lane, twice (see MixStage).
+// ---- FP64 kernel of the plain contexts ---------------------------------------------------------
+// Four records a warp, eight lanes each, two i atoms a lane, as k_pair_packed, in FP64.  The FP64
+// pipe bounds it (a warp instruction every 2.2 cycles of a scheduler), so the step holds
+// nothing that can be done once per atom or by fewer instructions:
+//  - Images.  Every atom is taken in its image nearest to the i block's reference.  A pair
+//    within the cut-off then is in the right image if box/2 exceeds the cut-off plus the i
+//    block's half extent plus the atoms' motion since the build (2 A): the j atom's image
+//    within the cut-off of the i atom lies within half a box of the reference on every axis.
+//    Else (a small box, or coordinates replaced without a build) each pair takes its own.
+//  - 1/r by rsqrt_h3; the cut-off test on r^2 itself; LJ from (-6 C6, 12 C12) as in record_packed.
+//  - Branch-free: a pair outside the mask or the cut-off has zero charge product and r^-1 = 0.
+// On 22,700 atoms 144 us with one i atom a lane and an image, a division and a square root per
+// pair, 93 with rsqrt() and the images per atom, 83 so (the FP64 pipe busy half the time).
+struct __align__(16) QuadStageD {
+  double2 pxy[256], pzq[256];   // entry 8 g + e of record q at 64 q + 16 g + e, and 8 further on
+  int2 at[4 * 36];              // (atom, type) of entry 8 g + e at 36 q + 8 g + e
+};
+
+// d's image nearest to zero (adding and subtracting 1.5 * 2^52 rounds to the nearest integer)
+__device__ __forceinline__ double near_image(double d, double box, double inv) {
+  const double n = __dadd_rn(__dadd_rn(d * inv, 6755399441055744.0), -6755399441055744.0);
+  return fma(-box, n, d);
+}
+
+// 1/sqrt(x) from the hardware's approximation y (its error e = 1 - x y^2 is about 2^-22) by
+// Householder's third-order step y + y e (1/2 + 3/8 e), whose error is of the order of e^3: full
+// double precision in five operations for the normal squared distances it is used on
+__device__ __forceinline__ double rsqrt_h3(double x) {
+  double y;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  const double e = fma(-(x * y), y, 1.0);
+  return fma(y * e, fma(e, 0.375, 0.5), y);
+}
+
+template <bool MINIMG, bool COUNT>
+__device__ __forceinline__ void record_fp64(const DevPtrs& P, const QuadStageD& S, const double2* __restrict__ s_lj,
+                                            int rowa, int rowb, const double (&xa)[4], const double (&xb)[4],
+                                            unsigned ma, unsigned mb, const double (&box)[3], const double (&inv)[3],
+                                            double rc2, double zb, double zf, double zc, int sp, int st, int sat,
+                                            int src, double (&fa)[3], double (&fb)[3], double& te, double& tl,
+                                            int& tn) {
+  const unsigned full = 0xffffffffu;
+#pragma unroll 1
+  for (int g = 0; g < 4; ++g) {
+    const double2* __restrict__ pxy = S.pxy + sp + 16 * g;
+    const double2* __restrict__ pzq = S.pzq + sp + 16 * g;
+    int tj = S.at[st + 8 * g].y;
+    double gx = 0.0, gy = 0.0, gz = 0.0;   // minus the j force of the entry this lane meets
+#pragma unroll 2
+    for (int k = 0; k < 8; ++k) {
+      const double2 jxy = pxy[k], jzq = pzq[k];
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        const double* xi = e ? xb : xa;
+        double dx = jxy.x - xi[0], dy = jxy.y - xi[1], dz = jzq.x - xi[2];   // x_j - x_i
+        if (MINIMG) {
+          dx = near_image(dx, box[0], inv[0]);
+          dy = near_image(dy, box[1], inv[1]);
+          dz = near_image(dz, box[2], inv[2]);
+        }
+        const double r2 = fma(dx, dx, fma(dy, dy, dz * dz));
+        const bool in = (((e ? mb : ma) >> (8 * g + k)) & 1u) && r2 <= rc2;
+        const double ri = in ? rsqrt_h3(r2) : 0.0;
+        const double qq = in ? xi[3] * jzq.y : 0.0;
+        const double2 lj = s_lj[(e ? rowb : rowa) + tj];   // -6 C6, 12 C12
+        const double r2i = ri * ri, r6 = r2i * r2i * r2i;
+        const double p = lj.y * r6;
+        te = fma(qq, ri + fma(zb, r2, -zc), te);
+        tl = fma(fma(p, 0.5, lj.x), r6, tl);
+        const double fs = fma(p + lj.x, r6 * r2i, qq * fma(ri, r2i, -zf));
+        double* fi = e ? fb : fa;
+        fi[0] = fma(dx, fs, fi[0]);
+        fi[1] = fma(dy, fs, fi[1]);
+        fi[2] = fma(dz, fs, fi[2]);
+        gx = fma(dx, fs, gx);
+        gy = fma(dy, fs, gy);
+        gz = fma(dz, fs, gz);
+        if (COUNT) tn += in ? 1 : 0;
+      }
+      if (k < 7) {
+        gx = __shfl_sync(full, gx, src);
+        gy = __shfl_sync(full, gy, src);
+        gz = __shfl_sync(full, gz, src);
+        tj = __shfl_sync(full, tj, src);
+      }
+    }
+    const int aj = S.at[sat + 8 * g].x;
+    if (aj >= 0 && (gx != 0.0 || gy != 0.0 || gz != 0.0)) {
+      atomicAdd(&P.grd[3 * aj + 0], -gx);
+      atomicAdd(&P.grd[3 * aj + 1], -gy);
+      atomicAdd(&P.grd[3 * aj + 2], -gz);
+    }
+  }
+}
+
+template <bool COUNT>
+__global__ void __launch_bounds__(kPairThreads, 2) k_pair_fp64q(DevPtrs P, ZdConst z) {
+  extern __shared__ __align__(16) unsigned char s_dynd[];
+  const unsigned full = 0xffffffffu;
+  QuadStageD& S = reinterpret_cast<QuadStageD*>(s_dynd)[threadIdx.x >> 5];
+  double2* s_lj = reinterpret_cast<double2*>(s_dynd + sizeof(QuadStageD) * kPairWarps);
+  for (int i = threadIdx.x; i < z.nt1 * z.nt1; i += blockDim.x) {
+    const double2 c = P.lj_d[i];
+    s_lj[i] = make_double2(-6.0 * c.x, 12.0 * c.y);
+  }
+  __syncthreads();
+  const int lane = threadIdx.x & 31, qd = lane >> 3, lp = lane & 7;
+  const int sp = 64 * qd + lp, sta = 36 * qd + lp, sat = 36 * qd + ((lp + 7) & 7);
+  const int src = (lane & 24) | ((lp + 1) & 7);
+  const int T = P.nctiles[0];
+  const bool ext = *P.ext_pos != 0;
+  const int TU = (T + 3) >> 2;
+  const int gw = blockIdx.x * kPairWarps + (threadIdx.x >> 5), nw = gridDim.x * kPairWarps;
+  int cur_unit = -2, cur_rep = -1, rep = -1, aia = -1, aib = -1, tia = z.nt1 - 1, tib = tia;
+  double xa[4] = {0, 0, 0, 0}, xb[4] = {0, 0, 0, 0}, fa[3] = {0, 0, 0}, fb[3] = {0, 0, 0};
+  double box[3] = {0, 0, 0}, inv[3] = {0, 0, 0}, ref[3] = {0, 0, 0};
+  long long eel = 0, elj = 0, npair = 0;
+  bool mi = false;
+  auto flush_i = [&]() {
+    if (aia >= 0)
+      for (int k = 0; k < 3; ++k) atomicAdd(&P.grd[3 * aia + k], fa[k]);
+    if (aib >= 0)
+      for (int k = 0; k < 3; ++k) atomicAdd(&P.grd[3 * aib + k], fb[k]);
+    for (int k = 0; k < 3; ++k) fa[k] = fb[k] = 0.0;
+  };
+  auto take = [&](int a, double (&x)[4]) {   // an atom in its image nearest to the i block's reference
+    x[0] = x[1] = x[2] = x[3] = 0.0;
+    if (a < 0) return;
+    const double4 p = P.pos_d[a];
+    x[0] = near_image(p.x - ref[0], box[0], inv[0]);
+    x[1] = near_image(p.y - ref[1], box[1], inv[1]);
+    x[2] = near_image(p.z - ref[2], box[2], inv[2]);
+    x[3] = p.w;
+  };
+  // the first group by the warp's index, the others from the counter
+  for (int t = gw; t < TU;) {
+    const int rec = 4 * t + qd;
+    const bool valid = rec < T;
+    const int unit = valid ? P.ct_blk[rec] & ~kRecImg : -1;
+    int aj[4], ty[4];
+#pragma unroll
+    for (int g = 0; g < 4; ++g) {
+      const size_t o = (size_t)rec * 32 + 8 * g + lp;
+      aj[g] = valid ? __float_as_int(P.ct_j[o].w) : -1;
+      ty[g] = valid ? type_word(P.ct_ty[o]) : z.nt1 - 1;
+    }
+    const unsigned ma = valid ? step_mask(P.ct_mask[(size_t)rec * kHalf + lp], lp) : 0u;
+    const unsigned mb = valid ? step_mask(P.ct_mask[(size_t)rec * kHalf + lp + 8], lp + 8) : 0u;
+    if (unit != cur_unit) {
+      flush_i();
+      cur_unit = unit;
+      aia = aib = -1;
+      tia = tib = z.nt1 - 1;
+      if (unit >= 0) {
+        const int si = unit * kHalf + lp, bi = unit >> 1;
+        aia = P.satom[si];
+        aib = P.satom[si + 8];
+        tia = P.styp[si];
+        tib = P.styp[si + 8];
+        rep = P.blk_rep[bi];
+        const Rep& R = P.reps[rep];
+        const float4 h = P.blk_half[bi];
+        const double hh[3] = {(double)h.x, (double)h.y, (double)h.z}, rc = sqrt(z.rc2);
+        mi = ext;
+        for (int k = 0; k < 3; ++k) {
+          box[k] = R.box[k];
+          inv[k] = R.invbox[k];
+          ref[k] = P.blk_ref[3 * bi + k];
+          if (!(0.5 * box[k] > rc + hh[k] + 2.0)) mi = true;
+        }
+      }
+      take(aia, xa);
+      take(aib, xb);
+    }
+    if (__any_sync(full, rep != cur_rep)) {
+      flush_fix<8>(P, cur_rep, eel, elj, 0, 0, npair, COUNT, false);
+      eel = elj = npair = 0;
+      cur_rep = rep;
+    }
+    __syncwarp();   // the last group's steps are done with the stage
+#pragma unroll
+    for (int g = 0; g < 4; ++g) {
+      double x[4];
+      take(aj[g], x);
+      const double2 xy = make_double2(x[0], x[1]), zq = make_double2(x[2], x[3]);
+      S.pxy[sp + 16 * g] = xy;
+      S.pxy[sp + 16 * g + 8] = xy;
+      S.pzq[sp + 16 * g] = zq;
+      S.pzq[sp + 16 * g + 8] = zq;
+      S.at[sta + 8 * g] = make_int2(aj[g], ty[g]);
+    }
+    __syncwarp();
+    double te = 0.0, tl = 0.0;
+    int tn = 0;
+    if (__any_sync(full, mi))
+      record_fp64<true, COUNT>(P, S, s_lj, tia * z.nt1, tib * z.nt1, xa, xb, ma, mb, box, inv, z.rc2, z.bcoeff,
+                               z.fcoeff, z.zcore, sp, sta, sat, src, fa, fb, te, tl, tn);
+    else
+      record_fp64<false, COUNT>(P, S, s_lj, tia * z.nt1, tib * z.nt1, xa, xb, ma, mb, box, inv, z.rc2, z.bcoeff,
+                                z.fcoeff, z.zcore, sp, sta, sat, src, fa, fb, te, tl, tn);
+    if (COUNT) npair += tn;
+    eel += to_fix(te, kEneScale, P.status);
+    elj += to_fix(tl * (1.0 / 6.0), kEneScale, P.status);
+    t = TU;
+    if (nw < TU) {
+      if (lane == 0) t = atomicAdd(P.tile_ctr, 1) + nw;
+      t = __shfl_sync(full, t, 0);
+    }
+  }
+  flush_i();
+  flush_block<8>(P, cur_rep, eel, elj, 0, 0, npair, COUNT, false);
+}
+
+// Per-warp shared memory of k_pair_fp64 (classes, CMM): each half-warp's record, entries a and b
+// of every lane, twice (see MixStage).
 struct __align__(16) F64Stage {
   double4 pa[64], pb[64];
   int2 t[64];
@@ -1208,10 +1421,17 @@ void pack_lj_table(const float2* lj, int nt1, std::vector<float>& out) {
       }
 }
 
+static size_t fp64q_bytes(int nt1) { return sizeof(QuadStageD) * kPairWarps + sizeof(double2) * nt1 * nt1; }
+
 int pair_blocks_per_sm(bool fp64, bool packed, int nt1) {
   int per = 0;
-  if (fp64) {
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_pair_fp64<false, false, false>, kPairThreads,
+  if (fp64 && packed) {
+    const int bytes = (int)fp64q_bytes(nt1);
+    cudaFuncSetAttribute(k_pair_fp64q<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    cudaFuncSetAttribute(k_pair_fp64q<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_pair_fp64q<false>, kPairThreads, bytes);
+  } else if (fp64) {
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_pair_fp64<false, true, false>, kPairThreads,
                                                   sizeof(double2) * nt1 * nt1);
   } else if (packed) {
     const int bytes = (int)(kPackedStageBytes + lj_bytes(nt1));
@@ -1260,8 +1480,8 @@ void launch_pair_fp64(const DevPtrs& P, const ZdConst& z, int nwarps, bool count
     if (count) k_pair_fp64<true, true, false><<<nb, kPairThreads, sh, st>>>(P, z);
     else k_pair_fp64<false, true, false><<<nb, kPairThreads, sh, st>>>(P, z);
   } else {
-    if (count) k_pair_fp64<true, false, false><<<nb, kPairThreads, sh, st>>>(P, z);
-    else k_pair_fp64<false, false, false><<<nb, kPairThreads, sh, st>>>(P, z);
+    if (count) k_pair_fp64q<true><<<nb, kPairThreads, fp64q_bytes(z.nt1), st>>>(P, z);
+    else k_pair_fp64q<false><<<nb, kPairThreads, fp64q_bytes(z.nt1), st>>>(P, z);
   }
 }
 
