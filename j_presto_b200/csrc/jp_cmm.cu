@@ -15,7 +15,7 @@
 // [q, p_x, p_y, p_z, Q_xx/2, Q_yy/2, Q_zz/2, Q_xx, Q_yy, Q_zz, Q_xy, Q_yz, Q_zx] with the
 // traceless Q_ab = sum q (3 d_a d_b - d^2 delta_ab).
 //
-// One thread per atom (assignment, far field) or per cell (moments, translation).  Sums into
+// One thread per atom (assignment; eight for the far field) or per cell (moments, translation).  Sums into
 // a cell are FP64 atomics (their order varies in the last bits); the far-field energy is
 // reduced per warp and added in 64-bit fixed point.
 #include "jp_kernels.h"
@@ -49,12 +49,24 @@ __device__ int cmm_cell_rep(const DevPtrs& P, int nrep, int l, int g, int& local
   return -1;
 }
 
+// a warp of one replica adds its sum (an atom at a time, the three addresses of a replica took
+// 25 us for 4,600 atoms)
 __global__ void k_cmm_centroid(DevPtrs P, int natom) {
+  const unsigned full = 0xffffffffu;
   const int a = blockIdx.x * blockDim.x + threadIdx.x;
-  if (a >= natom) return;
-  const int rep = P.rep_of[a];
-  if (!P.reps[rep].cmm || P.reps[rep].ext) return;
-  for (int k = 0; k < 3; ++k) atomicAdd(&P.cmm_c0[3 * rep + k], P.x[3 * a + k]);
+  int rep = a < natom ? P.rep_of[a] : -1;
+  if (rep >= 0 && (!P.reps[rep].cmm || P.reps[rep].ext)) rep = -1;
+  const int r0 = __reduce_max_sync(full, rep);
+  const bool one = __all_sync(full, rep < 0 || rep == r0);
+  for (int k = 0; k < 3; ++k) {
+    double v = rep >= 0 ? P.x[3 * a + k] : 0.0;
+    if (one) {
+      for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(full, v, o);
+      if (r0 >= 0 && (threadIdx.x & 31) == 0) atomicAdd(&P.cmm_c0[3 * r0 + k], v);
+    } else if (rep >= 0) {
+      atomicAdd(&P.cmm_c0[3 * rep + k], v);
+    }
+  }
 }
 
 // level-1 cell of each atom (celpar.f90:90-116), its population and raw moments
@@ -193,10 +205,12 @@ void launch_cmm_rebuild(const DevPtrs& P, int natom, int nrep, int ncell1, const
 }
 
 // far field of one atom (cmmdo.f90:181-290): the multipole expansion of every non-empty far
-// cell at every level; returns sum over levels of the potential, gradient in g (per unit
-// charge of the atom)
+// cell at every level, the cells of a level dealt to the kFarLanes lanes of the atom in turn;
+// returns this lane's share of the potential, of the gradient in g (per unit charge of the atom)
+constexpr int kFarLanes = 8;
+
 __device__ double cmm_far_atom(const DevPtrs& P, const Rep& R, const double* c0, int cell,
-                               const double* x, double* g) {
+                               const double* x, int sub, double* g) {
   int a[3] = {(cell & 255) + 1, ((cell >> 8) & 255) + 1, ((cell >> 16) & 255) + 1};
   double e = 0.0;
   g[0] = g[1] = g[2] = 0.0;
@@ -217,32 +231,27 @@ __device__ double cmm_far_atom(const DevPtrs& P, const Rep& R, const double* c0,
         hi[k] = m;
       }
     }
-    for (int kz = lo[2]; kz <= hi[2]; ++kz) {
+    const int wx = hi[0] - lo[0] + 1, wy = hi[1] - lo[1] + 1, n = wx * wy * (hi[2] - lo[2] + 1);
+    for (int c = sub; c < n; c += kFarLanes) {
+      const int kx = lo[0] + c % wx, ky = lo[1] + (c / wx) % wy, kz = lo[2] + c / (wx * wy);
+      if (kx >= nlo[0] && kx <= nhi[0] && ky >= nlo[1] && ky <= nhi[1] && kz >= nlo[2] && kz <= nhi[2]) continue;
+      const int id = R.cell_off[l] + ((kz - 1) * m + (ky - 1)) * m + (kx - 1);
+      if (__ldg(&P.cmm_pop[id]) == 0) continue;
+      const double* q = P.cmm_pot + (size_t)id * 13;
+      const double dx = x[0] - cmm_cen(R, c0, l, kx, 0);
+      const double dy = x[1] - cmm_cen(R, c0, l, ky, 1);
       const double dz = x[2] - cmm_cen(R, c0, l, kz, 2);
-      const bool nz = kz >= nlo[2] && kz <= nhi[2];
-      for (int ky = lo[1]; ky <= hi[1]; ++ky) {
-        const double dy = x[1] - cmm_cen(R, c0, l, ky, 1);
-        const bool nyz = nz && ky >= nlo[1] && ky <= nhi[1];
-        for (int kx = lo[0]; kx <= hi[0]; ++kx) {
-          if (nyz && kx >= nlo[0] && kx <= nhi[0]) continue;
-          const int id = R.cell_off[l] + ((kz - 1) * m + (ky - 1)) * m + (kx - 1);
-          if (__ldg(&P.cmm_pop[id]) == 0) continue;
-          const double* q = P.cmm_pot + (size_t)id * 13;
-          const double dx = x[0] - cmm_cen(R, c0, l, kx, 0);
-          const double dx2 = dx * dx, dy2 = dy * dy, dz2 = dz * dz;
-          const double dd2i = 1.0 / (dx2 + dy2 + dz2);
-          const double ddi = sqrt(dd2i);
-          const double dd3i = ddi * dd2i, dd5i = dd3i * dd2i;
-          const double aa1 = q[1] * dx + q[2] * dy + q[3] * dz;
-          const double aa2 = q[4] * dx2 + q[5] * dy2 + q[6] * dz2 + q[10] * dx * dy + q[11] * dy * dz +
-                             q[12] * dz * dx;
-          e += q[0] * ddi + aa1 * dd3i + aa2 * dd5i;
-          const double c4 = aa1 * 3.0 + aa2 * dd2i * 5.0;
-          g[0] += -(q[0] * dx - q[1]) * dd3i + (q[7] * dx + q[10] * dy + q[12] * dz - c4 * dx) * dd5i;
-          g[1] += -(q[0] * dy - q[2]) * dd3i + (q[10] * dx + q[8] * dy + q[11] * dz - c4 * dy) * dd5i;
-          g[2] += -(q[0] * dz - q[3]) * dd3i + (q[12] * dx + q[11] * dy + q[9] * dz - c4 * dz) * dd5i;
-        }
-      }
+      const double dx2 = dx * dx, dy2 = dy * dy, dz2 = dz * dz;
+      const double dd2i = 1.0 / (dx2 + dy2 + dz2);
+      const double ddi = sqrt(dd2i);
+      const double dd3i = ddi * dd2i, dd5i = dd3i * dd2i;
+      const double aa1 = q[1] * dx + q[2] * dy + q[3] * dz;
+      const double aa2 = q[4] * dx2 + q[5] * dy2 + q[6] * dz2 + q[10] * dx * dy + q[11] * dy * dz + q[12] * dz * dx;
+      e += q[0] * ddi + aa1 * dd3i + aa2 * dd5i;
+      const double c4 = aa1 * 3.0 + aa2 * dd2i * 5.0;
+      g[0] += -(q[0] * dx - q[1]) * dd3i + (q[7] * dx + q[10] * dy + q[12] * dz - c4 * dx) * dd5i;
+      g[1] += -(q[0] * dy - q[2]) * dd3i + (q[10] * dx + q[8] * dy + q[11] * dz - c4 * dy) * dd5i;
+      g[2] += -(q[0] * dz - q[3]) * dd3i + (q[12] * dx + q[11] * dy + q[9] * dz - c4 * dz) * dd5i;
     }
   }
   return e;
@@ -326,37 +335,51 @@ __device__ __forceinline__ bool cmm_due(const DevPtrs& P, const Rep& R, bool for
   return force || (P.step_ctr[0] % R.cmm_upd) == 0;
 }
 
-// far field of each atom when due (into gwk, energy into cmm_enew), then gwk into the forces
+// far field of each atom when due (into gwk, energy into cmm_enew), then gwk into the forces.
+// Eight lanes an atom: with one, a droplet of 4,600 atoms filled 145 warps, each a serial walk over
+// some 200 cells a level: 203 us, 48 so
 __global__ void k_cmm_far(DevPtrs P, int natom, int fp64, int force, double ccoef) {
-  const int a = blockIdx.x * blockDim.x + threadIdx.x;
+  const unsigned full = 0xffffffffu;
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  const int a = t / kFarLanes, sub = t % kFarLanes;
   int rep = -1, rep_x = -1;
-  double e = 0.0, ex = 0.0;
+  double e = 0.0, ex = 0.0, g[3] = {0.0, 0.0, 0.0}, x[3], c0[3], q2 = 0.0;
+  int cell = -1, r = 0;
+  bool due = false;
   if (a < natom) {
-    const int r = P.rep_of[a];
+    r = P.rep_of[a];
     const Rep& R = P.reps[r];
     if (R.cmm) {
-      const int cell = P.cmm_cell[a];
-      const double q2 = ccoef * P.chg[a];   // chgmod2 (inpcls.f90:223)
-      double c0[3], x[3], g[3];
-      cmm_centroid(P, R, r, c0);
-      for (int k = 0; k < 3; ++k) x[k] = P.x[3 * a + k];
-      if (cmm_due(P, R, force != 0) && cell >= 0) {
-        e = 0.5 * q2 * cmm_far_atom(P, R, c0, cell, x, g);
-        for (int k = 0; k < 3; ++k) P.gwk[3 * a + k] = g[k] * q2;
-        rep = r;
+      cell = P.cmm_cell[a];
+      q2 = ccoef * P.chg[a];   // chgmod2 (inpcls.f90:223)
+      due = cmm_due(P, R, force != 0) && cell >= 0;
+      if (due || R.ext) {
+        cmm_centroid(P, R, r, c0);
+        for (int k = 0; k < 3; ++k) x[k] = P.x[3 * a + k];
       }
-      if (cell >= 0) {
-        double gx[3] = {0.0, 0.0, 0.0};
-        if (R.ext) {   // the external environment, every step (cmmdo.f90:82)
-          ex = 0.5 * q2 * cmm_ext_atom(P, R, c0, cell, x, gx);
-          rep_x = r;
-        }
-        for (int k = 0; k < 3; ++k) {
-          const double gk = P.gwk[3 * a + k] + gx[k] * q2;
-          if (fp64) atomicAdd(&P.grd[3 * a + k], gk);
-          else atomic_add_ll(&P.frc[3 * a + k], to_fix(gk, kFrcScale, P.status));
-        }
-      }
+      if (due) e = cmm_far_atom(P, R, c0, cell, x, sub, g);
+    }
+  }
+  for (int o = kFarLanes / 2; o > 0; o >>= 1) {
+    e += __shfl_xor_sync(full, e, o);
+    for (int k = 0; k < 3; ++k) g[k] += __shfl_xor_sync(full, g[k], o);
+  }
+  if (cell >= 0 && sub == 0) {
+    const Rep& R = P.reps[r];
+    if (due) {
+      e *= 0.5 * q2;
+      for (int k = 0; k < 3; ++k) P.gwk[3 * a + k] = g[k] * q2;
+      rep = r;
+    }
+    double gx[3] = {0.0, 0.0, 0.0};
+    if (R.ext) {   // the external environment, every step (cmmdo.f90:82)
+      ex = 0.5 * q2 * cmm_ext_atom(P, R, c0, cell, x, gx);
+      rep_x = r;
+    }
+    for (int k = 0; k < 3; ++k) {
+      const double gk = P.gwk[3 * a + k] + gx[k] * q2;
+      if (fp64) atomicAdd(&P.grd[3 * a + k], gk);
+      else atomic_add_ll(&P.frc[3 * a + k], to_fix(gk, kFrcScale, P.status));
     }
   }
   // warp-level energy sums (one replica per warp as a rule; mixed warps add per lane)
@@ -381,7 +404,7 @@ __global__ void k_cmm_energy(DevPtrs P, int nrep, int force) {
 void launch_cmm_far(const DevPtrs& P, int natom, int nrep, bool fp64, bool force, double ccoef,
                     cudaStream_t st) {
   const int nt = 128;
-  k_cmm_far<<<(natom + nt - 1) / nt, nt, 0, st>>>(P, natom, fp64 ? 1 : 0, force ? 1 : 0, ccoef);
+  k_cmm_far<<<((long long)natom * kFarLanes + nt - 1) / nt, nt, 0, st>>>(P, natom, fp64 ? 1 : 0, force ? 1 : 0, ccoef);
   k_cmm_energy<<<1, 128, 0, st>>>(P, nrep, force ? 1 : 0);
 }
 
