@@ -1624,7 +1624,18 @@ int jp_create(const jp_system *sys, int32_t nrep, const jp_params *prm, jp_ctx *
   e |= dput(c, &P.units, units);
   std::vector<int> small_idx, quad_idx;
   for (int i = 0; i < (int)units.size(); ++i) (units[i].n == 4 ? quad_idx : small_idx).push_back(i);
-  e |= dput(c, &P.small_idx, small_idx);
+  std::vector<int4> hsu_atoms(small_idx.size());
+  std::vector<int2> hsu_own(small_idx.size());
+  std::vector<double> hsu_d2(3 * small_idx.size());
+  for (size_t i = 0; i < small_idx.size(); ++i) {
+    const Unit &u = units[small_idx[i]];
+    hsu_atoms[i] = make_int4(u.a[0], u.a[1], u.a[2], u.n);
+    hsu_own[i] = make_int2(u.sub, u.rep);
+    for (int q = 0; q < 3; ++q) hsu_d2[q * small_idx.size() + i] = u.d2[q];
+  }
+  e |= dput(c, &P.su_atoms, hsu_atoms);
+  e |= dput(c, &P.su_own, hsu_own);
+  e |= dput(c, &P.su_d2, hsu_d2);
   e |= dput(c, &P.quad_idx, quad_idx);
   e |= dput(c, &P.terms, terms);
   e |= dput(c, &P.reps, reps);

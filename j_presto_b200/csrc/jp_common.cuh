@@ -225,7 +225,10 @@ struct DevPtrs {
   float *rep_hmax;                // largest block half-extent per replica [nrep][3]
   // units / terms
   Unit *units;
-  int *small_idx, *quad_idx;      // units of 1-3 atoms / of 4 atoms, in unit order
+  int4 *su_atoms;                 // units of 1-3 atoms in unit order: atoms, atom count
+  int2 *su_own;                   // their sub-system, replica
+  double *su_d2;                  // their squared constraint lengths [3][nsmall]
+  int *quad_idx;                  // units of 4 atoms, in unit order
   Term *terms;
   // replicas
   Rep *reps;

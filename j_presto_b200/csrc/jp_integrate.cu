@@ -667,31 +667,51 @@ __device__ void finish_block(const DevPtrs& P, const IntConst& c, double tt, Loo
   const int h = P.step_ctr[1];
   const bool loop = c.method > JP_METHOD_MICR && c.shake_method != JP_SHAKE_NONE;   // verlethe
   if (loop) loop_first(P, c, c.icslop - 1, tt, *L);
-  // one warp per replica, a lane per sub-system; the sums in the order of the sub-systems
-  const int lane = threadIdx.x & 31;
-  for (int r = threadIdx.x >> 5; r < c.nrep; r += blockDim.x >> 5) {
-    const Rep& R = P.reps[r];
-    int ks = c.nkin - 1;   // MICR
-    if (loop) {
-      int q = c.icslop;
-      if (r < kActCache) q = min(q, L->first[r]);
-      else for (q = 1; q < c.icslop; ++q) if (cano_conv(P, c, R, q, tt)) break;
-      ks = 2 * q - 1;
-    }
-    double ek = 0.0, nf = 0.0;
-    for (int s0 = 0; s0 < R.nsub; s0 += 32) {
-      const int sub = R.sub0 + s0 + lane;
-      const bool in = s0 + lane < R.nsub;
-      const double e = in ? (double)__ldcg(&P.kin_fix[(size_t)ks * c.nsub_total + sub]) * kKinInv : 0.0;
-      const double n = in ? P.nfr[sub] : 0.0;
-      for (int k = 0; k < min(32, R.nsub - s0); ++k) {
-        ek += __shfl_sync(0xffffffffu, e, k);
-        nf += __shfl_sync(0xffffffffu, n, k);
+  auto last_slot = [&](int r) {
+    if (!loop) return c.nkin - 1;   // MICR
+    int q = c.icslop;
+    if (r < kActCache) q = min(q, L->first[r]);
+    else for (q = 1; q < c.icslop; ++q) if (cano_conv(P, c, P.reps[r], q, tt)) break;
+    return 2 * q - 1;
+  };
+  auto put = [&](int r, double ek, double nf) {
+    P.temp_hist[(size_t)h * c.nrep + r] =
+        (c.method <= JP_METHOD_MICR || c.shake_method != JP_SHAKE_NONE) ? ek * 1.0e7 / (kGas * nf) : -1.0;
+  };
+  // The sums in the order of the sub-systems.  One warp per replica, a lane per sub-system; a
+  // batch with more replicas a warp than sub-systems a replica takes a thread per replica
+  // instead (64 replicas of two sub-systems: 26 us
+  // against 62 for the launch that ends the step).
+  const int lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+  if ((long long)c.nrep * c.nrep > (long long)c.nsub_total * nw) {
+    for (int r = threadIdx.x; r < c.nrep; r += blockDim.x) {
+      const Rep& R = P.reps[r];
+      const long long* k = P.kin_fix + (size_t)last_slot(r) * c.nsub_total + R.sub0;
+      double ek = 0.0, nf = 0.0;
+#pragma unroll 4
+      for (int q = 0; q < R.nsub; ++q) {
+        ek += (double)__ldcg(&k[q]) * kKinInv;
+        nf += P.nfr[R.sub0 + q];
       }
+      put(r, ek, nf);
     }
-    if (lane == 0)
-      P.temp_hist[(size_t)h * c.nrep + r] =
-          (c.method <= JP_METHOD_MICR || c.shake_method != JP_SHAKE_NONE) ? ek * 1.0e7 / (kGas * nf) : -1.0;
+  } else {
+    for (int r = threadIdx.x >> 5; r < c.nrep; r += nw) {
+      const Rep& R = P.reps[r];
+      const int ks = last_slot(r);
+      double ek = 0.0, nf = 0.0;
+      for (int s0 = 0; s0 < R.nsub; s0 += 32) {
+        const int sub = R.sub0 + s0 + lane;
+        const bool in = s0 + lane < R.nsub;
+        const double e = in ? (double)__ldcg(&P.kin_fix[(size_t)ks * c.nsub_total + sub]) * kKinInv : 0.0;
+        const double n = in ? P.nfr[sub] : 0.0;
+        for (int k = 0; k < min(32, R.nsub - s0); ++k) {
+          ek += __shfl_sync(0xffffffffu, e, k);
+          nf += __shfl_sync(0xffffffffu, n, k);
+        }
+      }
+      if (lane == 0) put(r, ek, nf);
+    }
   }
   __syncthreads();
   // the next step starts from zero kinetic (and centre-of-mass) sums and a fresh barrier:
@@ -1068,6 +1088,20 @@ __global__ void __launch_bounds__(64) k_micr_fused(DevPtrs P, IntConst c, int nu
 // between two loads holds the later load back until the store's own inputs have arrived, and
 // a unit would wait for memory once per atom component instead of once.
 
+// The 1-3 atom unit of virtual lane v, from arrays with a lane's words side by side: a warp
+// reads its units in 12 wavefronts (the 80-byte Unit records of the lanes: 180).
+__device__ __forceinline__ Unit small_unit(const DevPtrs& P, const IntConst& c, int v) {
+  const int4 h = P.su_atoms[v];
+  const int2 o = P.su_own[v];
+  Unit u;
+  u.a[0] = h.x; u.a[1] = h.y; u.a[2] = h.z; u.a[3] = 0;
+  u.n = h.w;
+  u.sub = o.x; u.rep = o.y;
+#pragma unroll
+  for (int q = 0; q < 6; ++q) u.d2[q] = q < 3 ? P.su_d2[(size_t)q * c.nsmall + v] : 0.0;
+  return u;
+}
+
 // an atom's kernel-position record, read ahead of the update that rewrites it (write_slot)
 struct SlotRef {
   int s;            // the atom
@@ -1274,15 +1308,163 @@ __device__ __forceinline__ void cano5_unit(const DevPtrs& P, const IntConst& c, 
   }
 }
 
-// phase 2 then phase 3 with SHAKE and no centre-of-mass stop (the form of cano2_unit followed
-// by cano3_unit): phase 1 left x0 = x and vback = v, so both come from one read of x and v
+// ---- the same without the centre-of-mass stop and with SHAKE --------------------------------
+// x and v stay those of time t until the step's end: phase 1 only sums, a SHAKE pass leaves
+// the constrained positions in xback and the constraint forces so far in forcec, and the last
+// launch moves xback to x with v = (xback - x)/dt.  A step with one pass of the loop so moves
+// 608 bytes an atom instead of 800 (phase 1's copies, and x, v and the kernel positions written
+// by every pass, are gone).
+//
+// What bounded these launches was the load and store unit: a lane with a unit of three atoms
+// reads 72 consecutive bytes one double at a time, so each of a warp's accesses touched 18
+// lines.  Where the units of a warp are whole 3-atom groups with consecutive atoms of one
+// sub-system (solvent), the warp works on its 288 components side by side instead, lane l on
+// components l, l+32, ...; only the SHAKE pass needs a unit's components in one lane, and
+// gets them through shared memory (9 doubles a lane: no bank conflicts).  64 solvated
+// chains of 16,500 atoms: 397 -> 264 us a step, 32 of 9,000: 222 -> 160.
+constexpr int kWarpComp = 288;     // components of a warp's 32 three-atom units
+
+struct PassSmem {
+  double x1[kWarpComp], x0[kWarpComp], vb[kWarpComp];
+};
+
+// is the warp's work the 96 atoms from lane 0's on?  (every lane calls; v beyond nsmall: no)
+__device__ __forceinline__ bool warp_run(const Unit& u, int lane) {
+  const unsigned full = 0xffffffffu;
+  const int a0 = __shfl_sync(full, u.a[0], 0), s0 = __shfl_sync(full, u.sub, 0);
+  return __all_sync(full, u.n == 3 && u.a[0] == a0 + 3 * lane && u.a[1] == u.a[0] + 1 && u.a[2] == u.a[0] + 2 &&
+                              u.sub == s0);
+}
+
+// component i of the scaled gradient (load_grad and split_grad for one component)
 template <bool FP64>
-__device__ __forceinline__ double cano23_unit(const DevPtrs& P, const IntConst& c, const Unit& u, double s,
-                                              double tt) {
-  const double chi = sqrt(tt / sub_temp(P, c, 0, u.sub));
-  const double a1 = chi * c.dt * kConvcv, b1 = 2.0 * chi - 1.0;
-  double x1[3][3], x0[3][3], vb[3][3], g[3][3], im[3], m[3];
-  SlotRef sl[3];
+__device__ __forceinline__ double comp_grad(const DevPtrs& P, int i, double s, bool part) {
+  const double g = FP64 ? P.grd[i] : (double)P.frc[i] * kFrcInv;
+  if (!part) return g * s;
+  const double g1 = FP64 ? P.grd1[i] : (double)P.frc1[i] * kFrcInv;
+  return g1 * s + g;
+}
+
+template <bool FP64>
+__device__ __forceinline__ bool part_grad(const DevPtrs& P, int rep) {
+  return (FP64 ? P.grd1 != nullptr : P.frc1 != nullptr) && P.reps[rep].split;
+}
+
+// phase 1 (verlethe.f90:380-398): KE of v - dt/2 c g/m; phase 4 (verlethe.f90:625-640): KE of
+// v(t-dt/2) + dt/2 (-c g/m + forcec)
+template <bool FP64, bool CORR>
+__device__ __forceinline__ double half_ke(const DevPtrs& P, const IntConst& c, const Unit& u, bool run, int lane,
+                                          double s) {
+  const double h = 0.5 * c.dt, rt = h * kConvcv;
+  double ke = 0.0;
+  if (run) {
+    const bool part = part_grad<FP64>(P, u.rep);
+    const int i0 = 3 * __shfl_sync(0xffffffffu, u.a[0], 0) + lane;
+    double g[9], v[9], f[9], im[9], m[9];
+#pragma unroll
+    for (int j = 0; j < 9; ++j) {
+      const int i = i0 + 32 * j;
+      g[j] = comp_grad<FP64>(P, i, s, part);
+      v[j] = P.v[i];
+      f[j] = CORR ? P.forcec[i] : 0.0;
+      im[j] = P.imass[i / 3];
+      m[j] = P.mass[i / 3];
+    }
+#pragma unroll
+    for (int j = 0; j < 9; ++j) {
+      const double vt = CORR ? h * (-kConvcv * g[j] * im[j] + f[j]) + v[j] : v[j] - rt * g[j] * im[j];
+      ke += m[j] * (vt * vt);
+    }
+    return ke;
+  }
+  double g[3][3], v[3][3], f[3][3], im[3], m[3];
+  JP_SMALL_LOOP(q) {
+    const int a = u.a[q];
+    load_grad<FP64>(P, a, s, g[q]);
+    im[q] = P.imass[a];
+    m[q] = P.mass[a];
+    for (int k = 0; k < 3; ++k) {
+      v[q][k] = P.v[3 * a + k];
+      f[q][k] = CORR ? P.forcec[3 * a + k] : 0.0;
+    }
+  }
+  JP_SMALL_LOOP(q) {
+    double vv = 0.0;
+    for (int k = 0; k < 3; ++k) {
+      const double vt = CORR ? h * (-kConvcv * g[q][k] * im[q] + f[q][k]) + v[q][k]
+                             : v[q][k] - rt * g[q][k] * im[q];
+      vv += vt * vt;
+    }
+    ke += m[q] * vv;
+  }
+  return ke;
+}
+
+// phases 2 and 3 (verlethe.f90:400-612; chi from kinetic slot 0, forcec still zero) or phases 5
+// and 3 (RESC, verlethe.f90:641-718; chi from slot 2 it): the velocity update from time t, SHAKE
+// of the moved positions, forcec += shift/dt^2; returns the kinetic term of (vb + v)/2
+template <bool FP64, bool RESC>
+__device__ __forceinline__ double shake_pass(const DevPtrs& P, const IntConst& c, const Unit& u, bool run, int lane,
+                                             PassSmem& S, double s, int it, double tt) {
+  const double chi = sqrt(tt / sub_temp(P, c, RESC ? 2 * it : 0, u.sub));
+  const double a1 = RESC ? chi * c.dt : chi * c.dt * kConvcv, b1 = 2.0 * chi - 1.0;
+  const double r2 = 1.0 / (c.dt * c.dt), ri = 1.0 / c.dt;
+  double x1[3][3], x0[3][3], im[3], m[3];
+  if (run) {
+    const int c0 = 3 * __shfl_sync(0xffffffffu, u.a[0], 0) + lane;
+    const bool part = part_grad<FP64>(P, u.rep);
+    double g[9], v[9], x[9], f[9], w[9];
+#pragma unroll
+    for (int j = 0; j < 9; ++j) {
+      const int i = c0 + 32 * j;
+      g[j] = comp_grad<FP64>(P, i, s, part);
+      v[j] = P.v[i];
+      x[j] = P.x[i];
+      f[j] = RESC ? P.forcec[i] : 0.0;
+      w[j] = P.imass[i / 3];
+    }
+#pragma unroll
+    for (int j = 0; j < 9; ++j) {
+      const double vn = RESC ? (-kConvcv * g[j] * w[j] + f[j]) * a1 + v[j] * b1 : b1 * v[j] - a1 * g[j] * w[j];
+      S.x1[lane + 32 * j] = x[j] + c.dt * vn;
+      S.x0[lane + 32 * j] = x[j];
+      S.vb[lane + 32 * j] = v[j];
+    }
+    __syncwarp();
+#pragma unroll
+    for (int q = 0; q < 3; ++q) {
+      im[q] = P.imass[u.a[q]];
+      m[q] = P.mass[u.a[q]];
+      for (int k = 0; k < 3; ++k) {
+        x1[q][k] = S.x1[9 * lane + 3 * q + k];
+        x0[q][k] = S.x0[9 * lane + 3 * q + k];
+      }
+    }
+    const int ier = shake_small(P.reps[u.rep], 3, u.d2, im, x1, x0, c.shake_method, c.shake_tol, c.shake_maxit);
+    if (ier) shake_status(P, ier, u.rep);
+    double ke = 0.0;
+#pragma unroll
+    for (int q = 0; q < 3; ++q) {
+      double vv = 0.0;
+      for (int k = 0; k < 3; ++k) {
+        const int e = 9 * lane + 3 * q + k;
+        const double vt = 0.5 * (S.vb[e] + (x1[q][k] - x0[q][k]) * ri);
+        vv += vt * vt;
+        S.x0[e] = x1[q][k];                    // a lane's own components until the next sync
+        S.x1[e] = x1[q][k] - S.x1[e];
+      }
+      ke += m[q] * vv;
+    }
+    __syncwarp();
+#pragma unroll
+    for (int j = 0; j < 9; ++j) {
+      const int i = c0 + 32 * j;
+      P.xback[i] = S.x0[lane + 32 * j];
+      P.forcec[i] = (RESC ? P.forcec[i] : 0.0) + r2 * S.x1[lane + 32 * j];
+    }
+    return ke;
+  }
+  double g[3][3], vb[3][3], f[3][3], xb[3][3];
   JP_SMALL_LOOP(q) {
     const int a = u.a[q];
     load_grad<FP64>(P, a, s, g[q]);
@@ -1291,45 +1473,89 @@ __device__ __forceinline__ double cano23_unit(const DevPtrs& P, const IntConst& 
     for (int k = 0; k < 3; ++k) {
       vb[q][k] = P.v[3 * a + k];
       x0[q][k] = P.x[3 * a + k];
+      f[q][k] = RESC ? P.forcec[3 * a + k] : 0.0;
     }
-    slot_load<FP64>(P, a, sl[q]);
   }
   JP_SMALL_LOOP(q)
     for (int k = 0; k < 3; ++k) {
-      const double v = b1 * vb[q][k] - a1 * g[q][k] * im[q];
-      x1[q][k] = x0[q][k] + c.dt * v;
-      P.forcec[3 * u.a[q] + k] = 0.0;
+      const double vn = RESC ? (-kConvcv * g[q][k] * im[q] + f[q][k]) * a1 + vb[q][k] * b1
+                             : b1 * vb[q][k] - a1 * g[q][k] * im[q];
+      xb[q][k] = x1[q][k] = x0[q][k] + c.dt * vn;
     }
-  return shake_finish_unit<FP64>(P, c, u, im, m, sl, x1, x0, vb);
-}
-
-// phase 5 then phase 3 (cano5_unit followed by cano3_unit), no centre-of-mass stop
-template <bool FP64>
-__device__ __forceinline__ double cano53_unit(const DevPtrs& P, const IntConst& c, const Unit& u, double s,
-                                              int it, double tt) {
-  const double chi = sqrt(tt / sub_temp(P, c, 2 * it, u.sub));
-  const double a1 = chi * c.dt, b1 = 2.0 * chi - 1.0;
-  double x1[3][3], x0[3][3], vb[3][3], g[3][3], fc[3][3], im[3], m[3];
-  SlotRef sl[3];
+  if (u.n >= 2) {
+    const int ier = shake_small(P.reps[u.rep], u.n, u.d2, im, x1, x0, c.shake_method, c.shake_tol, c.shake_maxit);
+    if (ier) shake_status(P, ier, u.rep);
+  }
+  double ke = 0.0;
   JP_SMALL_LOOP(q) {
     const int a = u.a[q];
-    load_grad<FP64>(P, a, s, g[q]);
-    im[q] = P.imass[a];
-    m[q] = P.mass[a];
+    double vv = 0.0;
     for (int k = 0; k < 3; ++k) {
-      const int i = 3 * a + k;
-      vb[q][k] = P.vback[i];
-      x0[q][k] = P.x0[i];
-      fc[q][k] = P.forcec[i];
+      const double vt = 0.5 * (vb[q][k] + (x1[q][k] - x0[q][k]) * ri);
+      vv += vt * vt;
+      P.xback[3 * a + k] = x1[q][k];
+      P.forcec[3 * a + k] = f[q][k] + r2 * (x1[q][k] - xb[q][k]);
     }
-    slot_load<FP64>(P, a, sl[q]);
+    ke += m[q] * vv;
   }
-  JP_SMALL_LOOP(q)
-    for (int k = 0; k < 3; ++k) {
-      const double v = (-kConvcv * g[q][k] * im[q] + fc[q][k]) * a1 + vb[q][k] * b1;
-      x1[q][k] = x0[q][k] + c.dt * v;
+  return ke;
+}
+
+// the step's end: x, v and the kernel positions from the last pass's xback, forces cleared
+template <bool FP64>
+__device__ __forceinline__ void move_unit(const DevPtrs& P, const IntConst& c, const Unit& u, bool run, int lane) {
+  const double ri = 1.0 / c.dt;
+  bool bad = false;
+  if (run) {
+    const int i0 = 3 * __shfl_sync(0xffffffffu, u.a[0], 0) + lane;
+    double x1[9], x0[9], o[9];
+#pragma unroll
+    for (int j = 0; j < 9; ++j) {
+      const int i = i0 + 32 * j;
+      x1[j] = P.xback[i];
+      x0[j] = P.x[i];
+      o[j] = FP64 ? 0.0 : P.off[i];
     }
-  return shake_finish_unit<FP64>(P, c, u, im, m, sl, x1, x0, vb);
+#pragma unroll
+    for (int j = 0; j < 9; ++j) {
+      const int i = i0 + 32 * j;
+      const int p = i + i / 3;                 // component of the 4-word position records
+      P.v[i] = (x1[j] - x0[j]) * ri;
+      P.x[i] = x1[j];
+      if (FP64) {
+        reinterpret_cast<double*>(P.pos_d)[p] = x1[j];
+        P.grd[i] = 0.0;
+        if (P.grd1) P.grd1[i] = 0.0;
+      } else {
+        reinterpret_cast<float*>(P.pos_f)[p] = (float)(x1[j] - o[j]);
+        P.frc[i] = 0;
+        if (P.frc1) P.frc1[i] = 0;
+      }
+      bad |= !isfinite(x1[j]);
+    }
+  } else {
+    double x1[3][3], x0[3][3];
+    SlotRef sl[3];
+    JP_SMALL_LOOP(q) {
+      const int a = u.a[q];
+      for (int k = 0; k < 3; ++k) {
+        x1[q][k] = P.xback[3 * a + k];
+        x0[q][k] = P.x[3 * a + k];
+      }
+      slot_load<FP64>(P, a, sl[q]);
+    }
+    JP_SMALL_LOOP(q) {
+      const int a = u.a[q];
+      for (int k = 0; k < 3; ++k) {
+        P.v[3 * a + k] = (x1[q][k] - x0[q][k]) * ri;
+        P.x[3 * a + k] = x1[q][k];
+        bad |= !isfinite(x1[q][k]);
+      }
+      slot_store<FP64>(P, sl[q], x1[q]);
+      zero_force<FP64>(P, a);
+    }
+  }
+  if (bad) atomicOr(P.status, ERR_NONFINITE);
 }
 
 // Resident form: a 1-3 atom unit keeps its state through every phase of the step on chip:
@@ -2028,7 +2254,7 @@ __global__ void __launch_bounds__(kIntThreads) k_cano_fused(DevPtrs P, IntConst 
   const bool quad = gt >= c.qbase && gt < c.nvirt;
   double s = 1.0;
   if (small) {
-    const Unit u = P.units[P.small_idx[gt]];
+    const Unit u = small_unit(P, c, gt);
     ru_load(P, u, U, S, tid);
     s = rep_scale(P, c, u.rep);
   } else if (quad) {
@@ -2208,7 +2434,8 @@ __global__ void __launch_bounds__(kIntThreads) k_cano_fused(DevPtrs P, IntConst 
 // a chain of ordinary launches with one virtual lane per thread, so that every lane's loads
 // are in flight together: each launch is one phase of the form above, the launch boundary
 // stands where that form has a grid barrier, and a lane's state is in the atom arrays between
-// launches (x, x0, v, vback, xback, forcec).  A launch for a SHAKE <-> thermostat pass that no
+// launches (with the stop and for 4-atom groups x, x0, v, vback, xback, forcec; without it x, v
+// of time t, xback, forcec).  A launch for a SHAKE <-> thermostat pass that no
 // replica still runs returns at once.  Lambda's state through the step is kept in lam_step.
 enum : int {
   PH_BEGIN = 0,     // energy record, lambda force; phase 1
@@ -2220,7 +2447,8 @@ enum : int {
 };
 
 // blocks per SM the unit-lane launches are compiled for (their registers: 65,536 / (64 x this));
-// on C4 a bound of 8 (128 registers, with spills) measured 3 % slower than 4 (no spills)
+// 64 chains take 264 us a step with 4, 262 with 6 and 265 with 8 (spills), 32 take 160, 160
+// and 170
 constexpr int kPhaseBlocks = 4;
 
 // shared-memory state of the 4-atom group lanes of a launch (component 0-2)
@@ -2255,7 +2483,8 @@ __global__ void __launch_bounds__(1024) k_cano_loop(DevPtrs P, IntConst c, int i
 
 template <bool FP64, bool STOP, int PH, int KIND>
 __global__ void __launch_bounds__(kIntThreads, KIND == 1 ? 4 : kPhaseBlocks) k_cano_phase(DevPtrs P, IntConst c, int it) {
-  __shared__ QuadSmem S;
+  __shared__ QuadSmem S;                          // 4-atom group lanes
+  __shared__ PassSmem W[kIntThreads / 32];        // unit lanes, without the stop
   const int v = (KIND == 1 ? c.qbase : 0) + blockIdx.x * blockDim.x + threadIdx.x;
   const int tid = threadIdx.x;
   const double tt = target_temp(c, (long long)P.step_ctr[0] + 1);
@@ -2264,6 +2493,15 @@ __global__ void __launch_bounds__(kIntThreads, KIND == 1 ? 4 : kPhaseBlocks) k_c
   const bool small = KIND != 1 && v < c.nsmall;
   const bool quad = KIND != 0 && v >= c.qbase && v < c.nvirt;   // warp-uniform (multiples of 32)
   constexpr bool split = STOP;
+  // (warp-uniform conditions: the warp's lanes take the unit phases together)
+  const int lane = tid & 31;
+  Unit u;
+  bool run = false;
+  if (KIND != 1) {
+    u.n = 0; u.a[0] = 0; u.a[1] = 0; u.a[2] = 0; u.sub = -1; u.rep = 0;
+    if (small) u = small_unit(P, c, v);
+    if (!STOP) run = warp_run(u, lane);
+  }
   if (PH == PH_BEGIN) {
     if (KIND == 0 && v < c.nrep) write_ene_hist(P, c, v);
     if (lam_thread) {
@@ -2282,9 +2520,9 @@ __global__ void __launch_bounds__(kIntThreads, KIND == 1 ? 4 : kPhaseBlocks) k_c
       double ke = 0.0;
       int sub = -1;
       if (small) {
-        const Unit u = P.units[P.small_idx[v]];
         sub = u.sub;
-        ke = cano1_unit<FP64>(P, c, u, rep_scale(P, c, u.rep));
+        const double s = rep_scale(P, c, u.rep);
+        ke = STOP ? cano1_unit<FP64>(P, c, u, s) : half_ke<FP64, false>(P, c, u, run, lane, s);
       }
       add_kin(P, c.nsub_total, 0, sub, ke);
     }
@@ -2314,13 +2552,12 @@ __global__ void __launch_bounds__(kIntThreads, KIND == 1 ? 4 : kPhaseBlocks) k_c
       double ke = 0.0;
       int sub = -1, rep = -1;
       if (small) {
-        const Unit u = P.units[P.small_idx[v]];
         if (split || !shk) {
           cano2_unit<FP64>(P, c, u, rep_scale(P, c, u.rep), tt);
           if (split) rep = com_unit(P, c, u, w);
         } else {
           sub = u.sub;
-          ke = cano23_unit<FP64>(P, c, u, rep_scale(P, c, u.rep), tt);
+          ke = shake_pass<FP64, false>(P, c, u, run, lane, W[tid >> 5], rep_scale(P, c, u.rep), 0, tt);
         }
       }
       if (split) com_add(P, c, 0, rep, w);
@@ -2342,7 +2579,6 @@ __global__ void __launch_bounds__(kIntThreads, KIND == 1 ? 4 : kPhaseBlocks) k_c
       double ke = 0.0;
       int sub = -1;
       if (small) {
-        const Unit u = P.units[P.small_idx[v]];
         if (it == 0 || P.done[u.rep]) {
           fix_unit(P, c, it, u, shk, FP64);
           if (shk) {
@@ -2373,10 +2609,10 @@ __global__ void __launch_bounds__(kIntThreads, KIND == 1 ? 4 : kPhaseBlocks) k_c
       double ke = 0.0;
       int sub = -1;
       if (small) {
-        const Unit u = P.units[P.small_idx[v]];
         if (P.done[u.rep]) {
           sub = u.sub;
-          ke = cano4_unit<FP64>(P, c, u, rep_scale(P, c, u.rep));
+          const double s = rep_scale(P, c, u.rep);
+          ke = STOP ? cano4_unit<FP64>(P, c, u, s) : half_ke<FP64, true>(P, c, u, run, lane, s);
         }
       }
       add_kin(P, c.nsub_total, 2 * it, sub, ke);
@@ -2395,7 +2631,6 @@ __global__ void __launch_bounds__(kIntThreads, KIND == 1 ? 4 : kPhaseBlocks) k_c
           q_spill(P, c, q, S, tid, FP64);
         }
       } else if (small) {
-        const Unit u = P.units[P.small_idx[v]];
         if (P.done[u.rep]) {
           cano5_unit<FP64>(P, c, u, rep_scale(P, c, u.rep), it, tt);
           rep = com_unit(P, c, u, w);
@@ -2415,10 +2650,9 @@ __global__ void __launch_bounds__(kIntThreads, KIND == 1 ? 4 : kPhaseBlocks) k_c
       double ke = 0.0;
       int sub = -1;
       if (small) {
-        const Unit u = P.units[P.small_idx[v]];
         if (P.done[u.rep]) {
           sub = u.sub;
-          ke = cano53_unit<FP64>(P, c, u, rep_scale(P, c, u.rep), it, tt);
+          ke = shake_pass<FP64, true>(P, c, u, run, lane, W[tid >> 5], rep_scale(P, c, u.rep), it, tt);
         }
       }
       add_kin(P, c.nsub_total, 2 * it + 1, sub, ke);
@@ -2427,9 +2661,10 @@ __global__ void __launch_bounds__(kIntThreads, KIND == 1 ? 4 : kPhaseBlocks) k_c
     if (quad) {
       const QLane q = ql_make(P, c, v);
       if (q.a >= 0) zero_force<FP64>(P, q.a);
+    } else if (small && (STOP || !shk)) {
+      JP_SMALL_LOOP(q) zero_force<FP64>(P, u.a[q]);
     } else if (small) {
-      const Unit u = P.units[P.small_idx[v]];
-      JP_UNIT_LOOP(q) zero_force<FP64>(P, u.a[q]);
+      move_unit<FP64>(P, c, u, run, lane);
     }
     if (lam_thread) {
       LamStep L;

@@ -94,7 +94,7 @@ struct IntConst {
   int nsub_total;
   int natom;
   int nkin;                // kinetic-sum slots; the last one is MICR's
-  // virtual lanes of the CANO/GE kernel: [0, nsmall) one 1-3 atom unit each (small_idx),
+  // virtual lanes of the CANO/GE kernel: [0, nsmall) one 1-3 atom unit each (su_atoms),
   // [qbase, nvirt) eight lanes per 4-atom group (quad_idx); qbase and nvirt are multiples of 32
   int nsmall, nquad, qbase, nvirt;
   int ge_prescaled;        // force scales computed by k_ge_scale before the integration kernel
