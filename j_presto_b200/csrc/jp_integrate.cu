@@ -1321,7 +1321,8 @@ __device__ __forceinline__ void cano5_unit(const DevPtrs& P, const IntConst& c, 
 // sub-system (solvent), the warp works on its 288 components side by side instead, lane l on
 // components l, l+32, ...; only the SHAKE pass needs a unit's components in one lane, and
 // gets them through shared memory (9 doubles a lane: no bank conflicts).  64 solvated
-// chains of 16,500 atoms: 397 -> 264 us a step, 32 of 9,000: 222 -> 160.
+// chains of 16,500 atoms: 397 -> 264 us a step, 32 of 9,000: 222 -> 160 (with the groups in
+// launches of their own, see quad_blocks).
 constexpr int kWarpComp = 288;     // components of a warp's 32 three-atom units
 
 struct PassSmem {
@@ -2467,9 +2468,15 @@ __device__ __forceinline__ void lam_load(const DevPtrs& P, int r, LamStep& L) {
   L.lam = d[0]; L.lv = d[1]; L.lvback = d[2]; L.lf = d[3]; L.lvt = d[4];
 }
 
-// KIND 0: the 1-3 atom units [0, nsmall) and the per-replica threads (energy record,
-// lambda); KIND 1: the 4-atom group lanes [qbase, nvirt) (a launch of its own, as their
-// SHAKE needs several times the registers); KIND 2 (PH_END only): every lane.
+// The first quad_blocks(c) blocks take the 4-atom group lanes [qbase, nvirt), the others the
+// 1-3 atom units [0, nsmall) and the per-replica threads (energy record, lambda).  The group
+// blocks are few and each is one long chain (their SHAKE), so they start first and run beside
+// the units' blocks; in launches of their own a
+// step of 64 chains (1.06 M atoms) took 264 us against 229, of 32 (290 k) 160 against 119.
+__host__ __device__ __forceinline__ int quad_blocks(const IntConst& c) {
+  return (c.nvirt - c.qbase + kIntThreads - 1) / kIntThreads;
+}
+
 // which replicas still iterate at pass `it` (done[r]; done[nrep]: any), once for the pass's
 // launches.  With the test in every block of every launch, a batch of 64 replicas spent 1.5 us
 // more in each of them than this launch takes in all.
@@ -2481,29 +2488,34 @@ __global__ void __launch_bounds__(1024) k_cano_loop(DevPtrs P, IntConst c, int i
   if (threadIdx.x == 0) P.done[c.nrep] = any ? 1 : 0;
 }
 
-template <bool FP64, bool STOP, int PH, int KIND>
-__global__ void __launch_bounds__(kIntThreads, KIND == 1 ? 4 : kPhaseBlocks) k_cano_phase(DevPtrs P, IntConst c, int it) {
-  __shared__ QuadSmem S;                          // 4-atom group lanes
-  __shared__ PassSmem W[kIntThreads / 32];        // unit lanes, without the stop
-  const int v = (KIND == 1 ? c.qbase : 0) + blockIdx.x * blockDim.x + threadIdx.x;
+template <bool FP64, bool STOP, int PH>
+__global__ void __launch_bounds__(kIntThreads, kPhaseBlocks) k_cano_phase(DevPtrs P, IntConst c, int it) {
+  __shared__ union {
+    QuadSmem S;                          // 4-atom group lanes
+    PassSmem W[kIntThreads / 32];        // unit lanes, without the stop
+  } sm;
+  QuadSmem& S = sm.S;
+  PassSmem* W = sm.W;
+  const int gq = quad_blocks(c), b = blockIdx.x;
+  const int v = (b < gq ? c.qbase + b * kIntThreads : (b - gq) * kIntThreads) + threadIdx.x;
   const int tid = threadIdx.x;
   const double tt = target_temp(c, (long long)P.step_ctr[0] + 1);
   const bool shk = c.shake_method != JP_SHAKE_NONE;
-  const bool lam_thread = KIND != 1 && c.alsd && v < c.nrep && P.reps[v].lam_mode != 0;
-  const bool small = KIND != 1 && v < c.nsmall;
-  const bool quad = KIND != 0 && v >= c.qbase && v < c.nvirt;   // warp-uniform (multiples of 32)
+  const bool lam_thread = b >= gq && c.alsd && v < c.nrep && P.reps[v].lam_mode != 0;
+  const bool small = b >= gq && v < c.nsmall;
+  const bool quad = b < gq && v < c.nvirt;   // warp-uniform (multiples of 32)
   constexpr bool split = STOP;
   // (warp-uniform conditions: the warp's lanes take the unit phases together)
   const int lane = tid & 31;
   Unit u;
   bool run = false;
-  if (KIND != 1) {
+  if (b >= gq) {
     u.n = 0; u.a[0] = 0; u.a[1] = 0; u.a[2] = 0; u.sub = -1; u.rep = 0;
     if (small) u = small_unit(P, c, v);
     if (!STOP) run = warp_run(u, lane);
   }
   if (PH == PH_BEGIN) {
-    if (KIND == 0 && v < c.nrep) write_ene_hist(P, c, v);
+    if (b >= gq && v < c.nrep) write_ene_hist(P, c, v);
     if (lam_thread) {
       LamStep L{};
       lam_begin(P, c, v, L, shk);
@@ -2749,13 +2761,10 @@ static bool cano_streaming(const IntConst& c, int grid_max) {
   return want > grid_max;
 }
 
-// one phase: the unit lanes (and per-replica threads), then the 4-atom group lanes
 template <bool FP64, bool STOP, int PH>
 static void launch_phase(const DevPtrs& P, const IntConst& c, int it, cudaStream_t st) {
-  const int g0 = (std::max(c.nsmall, c.nrep) + kIntThreads - 1) / kIntThreads;
-  const int g1 = (c.nvirt - c.qbase + kIntThreads - 1) / kIntThreads;
-  k_cano_phase<FP64, STOP, PH, 0><<<g0, kIntThreads, 0, st>>>(P, c, it);
-  if (g1 > 0) k_cano_phase<FP64, STOP, PH, 1><<<g1, kIntThreads, 0, st>>>(P, c, it);
+  const int grid = quad_blocks(c) + (std::max(c.nsmall, c.nrep) + kIntThreads - 1) / kIntThreads;
+  k_cano_phase<FP64, STOP, PH><<<grid, kIntThreads, 0, st>>>(P, c, it);
 }
 
 template <bool FP64, bool STOP>
@@ -2772,8 +2781,7 @@ static void launch_cano_phases(const DevPtrs& P, const IntConst& c, cudaStream_t
       if (STOP) launch_phase<FP64, STOP, PH_FIX>(P, c, it, st);
     }
   }
-  const int grid = (std::max(c.nvirt, c.nrep) + kIntThreads - 1) / kIntThreads;
-  k_cano_phase<FP64, STOP, PH_END, 2><<<grid, kIntThreads, 0, st>>>(P, c, 0);
+  launch_phase<FP64, STOP, PH_END>(P, c, 0, st);
 }
 
 int integrate_launches(const IntConst& c, int grid_max) {
@@ -2781,7 +2789,7 @@ int integrate_launches(const IntConst& c, int grid_max) {
   const bool stop = c.stop != 0, shk = c.shake_method != JP_SHAKE_NONE;
   int phases = 2 + (stop ? 1 : 0);
   if (shk) phases += std::max(0, c.icslop - 1) * (stop ? 3 : 2);
-  int n = phases * (c.nvirt > c.qbase ? 2 : 1) + 1;            // + PH_END
+  int n = phases + 1;                                          // + PH_END
   if (shk) n += std::max(0, c.icslop - 1);                     // k_cano_loop
   if (c.method == JP_METHOD_GE && !c.ge_prescaled) n += 1;   // k_ge_scale
   return n;
