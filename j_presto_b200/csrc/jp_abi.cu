@@ -1564,6 +1564,7 @@ int jp_create(const jp_system *sys, int32_t nrep, const jp_params *prm, jp_ctx *
   e |= dalloc(c, &P.blk_half, (size_t)c->nblk);
   e |= dalloc(c, &P.blk_ref, 3 * (size_t)c->nblk);
   e |= dput(c, &P.blk_tile0, blk_tile0);
+  e |= dalloc(c, &P.blk_kind, (size_t)c->nblk);
   e |= dalloc(c, &P.blk_tiles, c->tile_cap_total);
   e |= dalloc(c, &P.tmp_masks, c->tile_cap_total * 32);
   if (c->hbond) {
@@ -1675,6 +1676,10 @@ int jp_create(const jp_system *sys, int32_t nrep, const jp_params *prm, jp_ctx *
   std::vector<float> ljtab;
   pack_lj_table(ljf.data(), nt1, ljtab);
   e |= dput(c, &P.lj_tab, ljtab);
+  std::vector<unsigned char> ljfree(nt1, 1);
+  for (int q = 0; q < nt1 * nt1; ++q)
+    if (!(ljd[q].x == 0.0 && ljd[q].y == 0.0)) ljfree[q % nt1] = 0;
+  e |= dput(c, &P.lj_free, ljfree);
   e |= dput(c, &P.lj_d, ljd);
   e |= dput(c, &P.lj14, lj14);
   c->nres = (int)hres.size();

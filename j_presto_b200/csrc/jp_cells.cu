@@ -104,6 +104,10 @@ __global__ void k_block_setup(DevPtrs P, int nblk, double qscale) {
   const int slot = warp * kTile + lane;
   const int a = P.satom[slot];
   const Rep& R = P.reps[P.blk_rep[warp]];
+  const int ty = P.styp[slot];
+  const unsigned lj = __ballot_sync(0xffffffffu, a >= 0 && !P.lj_free[ty & kTypeMask]);
+  const unsigned cls = __ballot_sync(0xffffffffu, a >= 0 && ((ty >> 30) & 1));
+  if (lane == 0) P.blk_kind[warp] = make_uint2(lj, cls);
   double w[3] = {0, 0, 0}, img[3] = {0, 0, 0};
   double lo[3], hi[3];
   for (int k = 0; k < 3; ++k) {
@@ -175,7 +179,8 @@ __global__ void k_excl_slots(DevPtrs P, int natom) {
 //
 // Pair record: a half block (16 i atoms: rows 0-15 or 16-31 of an i-block, unit u = 2 i-block +
 // half) with 32 j entries, the j atoms of that block's tiles that at least one of the 16 i
-// atoms lists, taken in tile order (ascending j block, ascending slot).  A 32 x 32 tile of two
+// atoms lists, by kind (below) and in tile order (ascending j block, ascending slot).
+// A 32 x 32 tile of two
 // blocks holds ~26 % listed pairs at the md_run list radius; keeping only the j atoms a half
 // block lists raises that to ~55 %, because 16 atoms span a smaller volume than 32 (within the
 // cut-off: 32 % of the slots with whole blocks, 39 % with half blocks), and the pair kernels'
@@ -183,6 +188,14 @@ __global__ void k_excl_slots(DevPtrs P, int natom) {
 // block's frame) and its atom, with the atom's type beside it; the mask of i atom l (0..15)
 // has bit k = entry (l + k) & 15 and bit 16 + k = entry 16 + ((l + k) & 15).
 
+// The four kinds of entries (0 .. 3), in their order in the first half of a block (in the second half the other
+// way round, so that a unit ends with the kind that the next one begins with): with an LJ term,
+// without, and the same two, without first, of the entries that make a record take per-pair
+// images or ALSD classes.  The pair kernels leave the LJ term out over eight entries of a
+// warp's records that have none (in waters two thirds of the entries), and few records mix
+// the forms.  Pair kernel with entries in tile order and so: LJNOTE.  With the LJ order alone
+// the entries of image tiles, scattered over more records, cost 64 replicas more than it gave
+// (1,480 us).
 constexpr int kListWarps = 8;     // warps of a block, at most
 constexpr int kTileListImg = 1 << 30, kTilePairImg = 1 << 29, kTileBlock = kTilePairImg - 1;   // BlkTile.j
 constexpr int kSegment = 512;     // candidate blocks tested at a time
@@ -191,18 +204,25 @@ constexpr int kWindow = 40;       // records of a half emitted at a time (water:
 
 struct __align__(16) ListShared {
   double x[kTile], y[kTile], z[kTile];     // the i block, wrapped
-  // a candidate's live j atoms, compacted, two per element: x, x', y, y' and z, z', mask bits
-  float4 lxy[kListWarps][kTile / 2], lzb[kListWarps][kTile / 2];
+  union {
+    // a candidate's live j atoms, compacted, two per element: x, x', y, y' and z, z', mask bits
+    struct {
+      float4 xy[kListWarps][kTile / 2], zb[kListWarps][kTile / 2];
+    } l;
+    // afterwards, entry -> tile << 5 | j lane of each half's window (beyond 2,048 tiles in 32
+    // bits, half the window)
+    unsigned short e16[2][kWindow * 32];
+    unsigned e32[2][kWindow * 16];
+  };
   unsigned ball[kSegment / 32];            // survivors of the bounding-box test
   unsigned excl[kSegment / 32];            // blocks that hold an exclusion partner
-  int wsum[kListWarps][2];
-  int carry[2];
+  int carry[8];                            // entries by half and kind
+  int first[2][4];                         // a half's first entry of each kind
   int base;
   // ALSD: which of a window's records hold a class but BB, and each one's place
   unsigned char rcls[2 * kWindow];
   size_t rpos[2 * kWindow];
   BlkTile tile[kTileCache];
-  unsigned elist[2][kWindow * 32];         // entry -> tile << 5 | j lane, of each half's window
 };
 
 // 1-2/1-3/1-4 partners (cutoff.f90:50-96) of this lane's i atom that sit in block bj out of its
@@ -335,8 +355,8 @@ __device__ __forceinline__ unsigned tile_row_f32(const Rep& R, float3 c, float4 
   const int nlive = __popc(live);
   __syncwarp();   // the previous tile's passes are done with the compacted atoms
   {
-    float* xy = reinterpret_cast<float*>(S.lxy[w]);
-    float* zb = reinterpret_cast<float*>(S.lzb[w]);
+    float* xy = reinterpret_cast<float*>(S.l.xy[w]);
+    float* zb = reinterpret_cast<float*>(S.l.zb[w]);
     if (lv) {
       const int t = __popc(live & ((1u << lane) - 1u));
       const int o = 4 * (t >> 1) + (t & 1);
@@ -360,7 +380,7 @@ __device__ __forceinline__ unsigned tile_row_f32(const Rep& R, float3 c, float4 
   bool u = false;
 #pragma unroll 4
   for (int q = 0; 2 * q < nlive; ++q) {   // warp-uniform
-    const float4 xy = S.lxy[w][q], zb = S.lzb[w][q];
+    const float4 xy = S.l.xy[w][q], zb = S.l.zb[w][q];
     float2 dx = __fadd2_rn(make_float2(xy.x, xy.y), nx);
     float2 dy = __fadd2_rn(make_float2(xy.z, xy.w), ny);
     float2 dz = __fadd2_rn(make_float2(zb.x, zb.y), nz);
@@ -524,6 +544,7 @@ __global__ void __launch_bounds__(32 * kListWarps, CMM ? 3 : 4) k_block_list(Dev
         // until the next build if, with 2 A for the atoms' motion, it is beyond the cut-off
         // (CMM, no cut-off: beyond the farthest near-field pair)
         const float4 hj = P.blk_half[bj];
+        const uint2 kind = P.blk_kind[bj];
         const float hh[3] = {hi.x + hj.x, hi.y + hj.y, hi.z + hj.z};
         const float rk = CMM ? rlimf : (float)sqrt(rc2);
         float c[3];
@@ -536,6 +557,8 @@ __global__ void __launch_bounds__(32 * kListWarps, CMM ? 3 : 4) k_block_list(Dev
           if (!(other > rk + 2.f)) img |= kTilePairImg;
         }
         T.j = bj | img;
+        T.lj = kind.x;
+        T.sp = (img & kTilePairImg) ? 0xffffffffu : kind.y;
         T.cx = c[0]; T.cy = c[1]; T.cz = c[2];
       }
       n += __popc(ball);
@@ -596,35 +619,33 @@ __global__ void __launch_bounds__(32 * kListWarps, CMM ? 3 : 4) k_block_list(Dev
     __syncthreads();
   }
 
-  // entries of each half: exclusive sums over the tiles
-  if (threadIdx.x < 2) S.carry[threadIdx.x] = 0;
-  for (int c0 = 0; c0 < nt; c0 += blockDim.x) {
-    const int c = c0 + threadIdx.x;
-    int n0 = 0, n1 = 0;
-    if (c < nt) {
-      const BlkTile& T = blk_tile(P, S, t0, c);
-      n0 = __popc(T.occ[0]);
-      n1 = __popc(T.occ[1]);
+  // entries of each half and kind, a warp a sum: exclusive sums over the tiles
+  for (int key = w; key < 8; key += nw) {
+    const int h = key >> 2, k = key & 3;
+    int sum = 0;
+    for (int c0 = 0; c0 < nt; c0 += 32) {
+      const bool in = c0 + lane < nt;
+      BlkTile& T = blk_tile(P, S, t0, min(c0 + lane, nt - 1));
+      const int n = in ? __popc(T.occ[h] & (k & 2 ? T.sp : ~T.sp) & (k == 0 || k == 3 ? T.lj : ~T.lj)) : 0;
+      int s = n;
+      for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(full, s, o);
+        if (lane >= o) s += y;
+      }
+      if (in) T.eoff[h][k] = sum + s - n;
+      sum += __shfl_sync(full, s, 31);
     }
-    int s0 = n0, s1 = n1;
-    for (int o = 1; o < 32; o <<= 1) {
-      const int y0 = __shfl_up_sync(full, s0, o), y1 = __shfl_up_sync(full, s1, o);
-      if (lane >= o) { s0 += y0; s1 += y1; }
-    }
-    if (lane == 31) { S.wsum[w][0] = s0; S.wsum[w][1] = s1; }
-    __syncthreads();
-    int b0 = S.carry[0], b1 = S.carry[1];
-    for (int v = 0; v < w; ++v) { b0 += S.wsum[v][0]; b1 += S.wsum[v][1]; }
-    if (c < nt) {
-      BlkTile& T = blk_tile(P, S, t0, c);
-      T.eoff[0] = b0 + s0 - n0;
-      T.eoff[1] = b1 + s1 - n1;
-    }
-    __syncthreads();
-    if (threadIdx.x == blockDim.x - 1) { S.carry[0] = b0 + s0; S.carry[1] = b1 + s1; }
+    if (lane == 0) S.carry[key] = sum;
   }
   __syncthreads();
-  const int E[2] = {S.carry[0], S.carry[1]};
+  const int E[2] = {S.carry[0] + S.carry[1] + S.carry[2] + S.carry[3], S.carry[4] + S.carry[5] + S.carry[6] + S.carry[7]};
+  if (threadIdx.x < 8) {   // half h: kinds 0 1 2 3, or 3 2 1 0
+    const int h = threadIdx.x >> 2, k = threadIdx.x & 3;
+    int f = 0;
+    for (int q = 0; q < 4; ++q)
+      if (h ? q > k : q < k) f += S.carry[4 * h + q];
+    S.first[h][k] = f;
+  }
   const int nr0 = (E[0] + 31) >> 5, nr1 = (E[1] + 31) >> 5;
   if (threadIdx.x == 0) {
     P.ct_cnt[2 * bi] = nr0;
@@ -633,27 +654,36 @@ __global__ void __launch_bounds__(32 * kListWarps, CMM ? 3 : 4) k_block_list(Dev
   }
   if (count_only) return;
 
-  // the records, kWindow of each half at a time: every tile spreads its entries over the
+  const bool wide = nt > 2048;
+  const int win = wide ? kWindow / 2 : kWindow;
+  auto entry = [&](int h, int e) { return wide ? S.e32[h][e] : (unsigned)S.e16[h][e]; };
+  // the records, `win` of each half at a time: every tile spreads its entries over the
   // window's list, then a warp takes a record, lane p slot p
-  for (int w0 = 0; w0 < max(nr0, nr1); w0 += kWindow) {
+  for (int w0 = 0; w0 < max(nr0, nr1); w0 += win) {
     __syncthreads();
     for (int c = w; c < nt; c += nw) {
       const BlkTile& T = blk_tile(P, S, t0, c);
+      const bool sp = (T.sp >> lane) & 1u, lj = (T.lj >> lane) & 1u;
+      const int k = sp ? (lj ? 3 : 2) : (lj ? 0 : 1);
+      const unsigned same = (sp ? T.sp : ~T.sp) & (lj ? T.lj : ~T.lj) & ((1u << lane) - 1u);   // of this kind, before
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
         const unsigned occ = T.occ[h];
-        const int e = T.eoff[h] + __popc(occ & ((1u << lane) - 1u)) - 32 * w0;
-        if (((occ >> lane) & 1u) && e >= 0 && e < 32 * kWindow) S.elist[h][e] = ((unsigned)c << 5) | lane;
+        const int e = S.first[h][k] + T.eoff[h][k] + __popc(occ & same) - 32 * w0;
+        if (((occ >> lane) & 1u) && e >= 0 && e < 32 * win) {
+          if (wide) S.e32[h][e] = ((unsigned)c << 5) | lane;
+          else S.e16[h][e] = (unsigned short)((c << 5) | lane);
+        }
       }
     }
     __syncthreads();
-    const int m0 = max(0, min(kWindow, nr0 - w0)), m1 = max(0, min(kWindow, nr1 - w0));
+    const int m0 = max(0, min(win, nr0 - w0)), m1 = max(0, min(win, nr1 - w0));
     if (split_cls) {
       for (int q = w; q < m0 + m1; q += nw) {
         const int h = q < m0 ? 0 : 1, r = q < m0 ? q : q - m0;
         int ty = 0;
         if (32 * (w0 + r) + lane < E[h]) {
-          const unsigned v = S.elist[h][32 * r + lane];
+          const unsigned v = entry(h, 32 * r + lane);
           ty = P.styp[(blk_tile(P, S, t0, (int)(v >> 5)).j & kTileBlock) * kTile + (int)(v & 31u)];
         }
         if (lane < kHalf) ty |= P.styp[bi * kTile + kHalf * h + lane];
@@ -690,13 +720,14 @@ __global__ void __launch_bounds__(32 * kListWarps, CMM ? 3 : 4) k_block_list(Dev
       const int h = q < m0 ? 0 : 1, r = q < m0 ? q : q - m0;   // record r of the window of half h
       const size_t ct = split_cls ? S.rpos[q] : (size_t)S.base + (h ? nr0 : 0) + w0 + r;
       const bool live = 32 * (w0 + r) + lane < E[h];
-      const unsigned v = live ? S.elist[h][32 * r + lane] : 0u;
+      const unsigned v = live ? entry(h, 32 * r + lane) : 0u;
       const int c = (int)(v >> 5), jl = (int)(v & 31u);
       float4 ent = make_float4(0.f, 0.f, 0.f, __int_as_float(-1));
       int ty = dummy_type;
-      bool img = false;
+      bool img = false, has_lj = false;
       if (live) {
         const BlkTile& T = blk_tile(P, S, t0, c);
+        has_lj = (T.lj >> jl) & 1u;
         img = (T.j & kTilePairImg) != 0;
         const int slot = (T.j & kTileBlock) * kTile + jl;
         ent = make_float4(-T.cx, -T.cy, -T.cz, __int_as_float(P.satom[slot]));
@@ -711,7 +742,11 @@ __global__ void __launch_bounds__(32 * kListWarps, CMM ? 3 : 4) k_block_list(Dev
         if (lane < kHalf) P.ct_mask_el[ct * kHalf + lane] = record_row(cel, lane);
       }
       const bool any_img = __any_sync(full, img);
-      if (lane == 0) P.ct_blk[ct] = (2 * bi + h) | (any_img ? kRecImg : 0);
+      const unsigned lj = __ballot_sync(full, has_lj);
+      int fl = any_img ? kRecImg : 0;
+#pragma unroll
+      for (int g = 0; g < 4; ++g) fl |= ((lj >> (8 * g)) & 0xffu) ? 0 : 1 << (kRecFree + g);
+      if (lane == 0) P.ct_blk[ct] = (2 * bi + h) | fl;
     }
   }
 }

@@ -20,7 +20,9 @@ namespace jp {
 
 constexpr int kTile = 32;
 constexpr int kHalf = 16;   // i atoms of a pair record: half a block
-constexpr int kRecImg = 1 << 30;   // in ct_blk: a record with a tile whose pairs take their own images
+// ct_blk: a record's unit, kRecImg if one of its tiles' pairs take their own images, and from bit
+// kRecFree on a bit for each eight entries that have no LJ term with anything
+constexpr int kRecImg = 1 << 30, kRecFree = 26, kRecUnit = (1 << kRecFree) - 1;
 // fixed-point scales: forces 2^32 per kcal/mol/A, energies 2^32 per kcal/mol,
 // kinetic sums (m v^2, amu A^2/fs^2) 2^40.
 constexpr double kFrcScale = 4294967296.0;
@@ -167,12 +169,14 @@ struct MinState {
 };
 
 // a tile of an i-block's list: its j block, that block's reference in the i block's frame, the
-// j lanes each half lists and the first entry of each half it contributes
+// j lanes each half lists and, per half and kind of entry (jp_cells.cu), the entries before its own
 struct BlkTile {
   int j;                    // and its image flags (jp_cells.cu)
   float cx, cy, cz;
   unsigned occ[2];
-  int eoff[2];
+  int eoff[2][4];
+  unsigned lj, sp;          // j lanes with an LJ term, with per-pair images or an ALSD class
+  int pad;                  // (an odd number of words: lanes with a tile each read without conflicts)
 };
 
 struct DevPtrs {
@@ -200,6 +204,8 @@ struct DevPtrs {
   // pair list build: an i-block's tiles (its candidate j blocks that passed the bounding-box
   // test) start at blk_tile0 in the arrays that hold one element per possible tile
   long long *blk_tile0;           // [nblk] (static)
+  uint2 *blk_kind;                // the lanes of each block with an LJ term, with an ALSD cluster atom
+  unsigned char *lj_free;         // types without an LJ term with any type
   BlkTile *blk_tiles;             // tiles beyond a block's shared-memory cache
   unsigned *tmp_masks;            // [tile][32] their mask rows: bit k of row i is j lane (i + k) & 31
   // the tiles themselves, listed only for the H-bond list
@@ -208,7 +214,7 @@ struct DevPtrs {
   int *ntiles;                    // device scalar
   // pair records (what the pair kernels run on): half an i-block and 32 j entries
   int *ct_cnt;                    // records per unit (2 i-block + half)
-  int *ct_blk;                    // [CT] unit of each pair record, with kRecImg
+  int *ct_blk;                    // [CT] unit of each pair record and its flags (kRecImg, kRecFree)
   int *ext_pos;                   // coordinates were replaced since the last list build: the records'
                                   // image flags, made for the motion between builds, don't hold
   float4 *ct_j;                   // [CT][32] (image shift into the i frame, atom bits; -1 = empty)

@@ -275,12 +275,12 @@ struct PackedArgs {
 // one i atom a lane, 1,494 so; 190 and 179 us on 99,200 atoms, 59 and 52 us on 22,700.  Now 59 % of the issue slots and
 // 70 % of that pipe are busy (24 % of it staging, 17 % the force atomics), the FMA pipe 45 %.
 // Half or quarter groups as work units of small lists measured slower (the per-record work).
-template <bool MINIMG, bool COUNT, bool TRI, bool CLS>
-__device__ __forceinline__ void record_packed(const DevPtrs& P, const QuadStage& S, const float2* __restrict__ s_lj,
+template <bool MINIMG, bool COUNT, bool TRI, bool CLS, bool LJ>
+__device__ __forceinline__ void group_packed(const DevPtrs& P, const QuadStage& S, const float2* __restrict__ s_lj,
                                               const float4* __restrict__ s_lj3, int rowa, int rowb,
-                                              const PackedArgs& A, int sp, int st, int sat, int src,
-                                              float2& fx, float2& fy, float2& fz, double& te, double& tl,
-                                              int& tn, double& ea, double& eb) {
+                                             const PackedArgs& A, int g, int sp, int st, int sat, int src,
+                                             float2& fx, float2& fy, float2& fz, double& te, double& tl,
+                                             int& tn, double& ea, double& eb) {
   const unsigned full = 0xffffffffu;
   const float2 zb2 = make_float2(A.zb, A.zb), mzc = make_float2(-A.zc, -A.zc), mzf = make_float2(-A.zf, -A.zf);
   const float2 half2 = make_float2(0.5f, 0.5f);
@@ -290,34 +290,33 @@ __device__ __forceinline__ void record_packed(const DevPtrs& P, const QuadStage&
     bx = rp[0]; by = rp[1]; bz = rp[2];
     ibx = rp[3]; iby = rp[4]; ibz = rp[5];
   }
-#pragma unroll 1
-  for (int g = 0; g < 4; ++g) {
-    const float4* __restrict__ pp = S.p + sp + 16 * g;
-    int tj = S.at[st + 8 * g].y;
-    if (CLS) tj &= kTypeMask;
-    const unsigned ma = A.ma >> (8 * g), mb = A.mb >> (8 * g);
-    const unsigned jc = CLS ? A.jc >> (8 * g) : 0u;
-    float gx = 0.f, gy = 0.f, gz = 0.f;   // minus the j force of the entry this lane meets
-    float2 te4 = make_float2(0.f, 0.f), tl4 = te4;
-    float ea4 = 0.f, eb4 = 0.f;
+  const float4* __restrict__ pp = S.p + sp + 16 * g;
+  int tj = LJ ? S.at[st + 8 * g].y : 0;
+  if (CLS && LJ) tj &= kTypeMask;
+  const unsigned ma = A.ma >> (8 * g), mb = A.mb >> (8 * g);
+  const unsigned jc = CLS ? A.jc >> (8 * g) : 0u;
+  float gx = 0.f, gy = 0.f, gz = 0.f;   // minus the j force of the entry this lane meets
+  float2 te4 = make_float2(0.f, 0.f), tl4 = te4;
+  float ea4 = 0.f, eb4 = 0.f;
 #pragma unroll
-    for (int k = 0; k < 8; ++k) {
-      const float4 j = pp[k];
-      float2 dx = __fadd2_rn(make_float2(j.x, j.x), A.nx);   // x_j - x_i
-      float2 dy = __fadd2_rn(make_float2(j.y, j.y), A.ny);
-      float2 dz = __fadd2_rn(make_float2(j.z, j.z), A.nz);
-      if (MINIMG) {
-        dx = __ffma2_rn(make_float2(-bx, -bx), rint2(__fmul2_rn(dx, make_float2(ibx, ibx))), dx);
-        dy = __ffma2_rn(make_float2(-by, -by), rint2(__fmul2_rn(dy, make_float2(iby, iby))), dy);
-        dz = __ffma2_rn(make_float2(-bz, -bz), rint2(__fmul2_rn(dz, make_float2(ibz, ibz))), dz);
-      }
-      const float2 r2 = __ffma2_rn(dx, dx, __ffma2_rn(dy, dy, __fmul2_rn(dz, dz)));
-      const bool ia = ((ma >> k) & 1u) && r2.x <= A.rc2;
-      const bool ib = ((mb >> k) & 1u) && r2.y <= A.rc2;
-      const float2 rinv = make_float2(rsqrt_ftz(ia ? r2.x : 1e30f), rsqrt_ftz(ib ? r2.y : 1e30f));
-      const float2 r2i = __fmul2_rn(rinv, rinv);
-      const float2 r6 = __fmul2_rn(__fmul2_rn(r2i, r2i), r2i);
-      float2 m6, p12;   // -6 C6, 12 C12
+  for (int k = 0; k < 8; ++k) {
+    const float4 j = pp[k];
+    float2 dx = __fadd2_rn(make_float2(j.x, j.x), A.nx);   // x_j - x_i
+    float2 dy = __fadd2_rn(make_float2(j.y, j.y), A.ny);
+    float2 dz = __fadd2_rn(make_float2(j.z, j.z), A.nz);
+    if (MINIMG) {
+      dx = __ffma2_rn(make_float2(-bx, -bx), rint2(__fmul2_rn(dx, make_float2(ibx, ibx))), dx);
+      dy = __ffma2_rn(make_float2(-by, -by), rint2(__fmul2_rn(dy, make_float2(iby, iby))), dy);
+      dz = __ffma2_rn(make_float2(-bz, -bz), rint2(__fmul2_rn(dz, make_float2(ibz, ibz))), dz);
+    }
+    const float2 r2 = __ffma2_rn(dx, dx, __ffma2_rn(dy, dy, __fmul2_rn(dz, dz)));
+    const bool ia = ((ma >> k) & 1u) && r2.x <= A.rc2;
+    const bool ib = ((mb >> k) & 1u) && r2.y <= A.rc2;
+    const float2 rinv = make_float2(rsqrt_ftz(ia ? r2.x : 1e30f), rsqrt_ftz(ib ? r2.y : 1e30f));
+    const float2 r2i = __fmul2_rn(rinv, rinv);
+    float2 r6 = make_float2(0.f, 0.f), m6 = r6, p12 = r6;   // -6 C6, 12 C12
+    if (LJ) {
+      r6 = __fmul2_rn(__fmul2_rn(r2i, r2i), r2i);
       if (TRI) {
         const float4 lj = s_lj3[rowa + tj];
         m6 = make_float2(lj.x, lj.y);
@@ -327,57 +326,80 @@ __device__ __forceinline__ void record_packed(const DevPtrs& P, const QuadStage&
         m6 = make_float2(lja.x, ljb.x);
         p12 = make_float2(lja.y, ljb.y);
       }
-      const float2 qf = __fmul2_rn(A.qi, make_float2(j.w, j.w));
-      const float2 qq = make_float2(ia ? qf.x : 0.f, ib ? qf.y : 0.f);
-      const float2 p = __fmul2_rn(p12, r6);
-      const float2 h = __ffma2_rn(p, half2, m6);
-      const float2 c = __fadd2_rn(rinv, __ffma2_rn(zb2, r2, mzc));
-      const float2 el = __fmul2_rn(qq, __ffma2_rn(rinv, r2i, mzf));
-      float2 fs = __ffma2_rn(__fadd2_rn(p, m6), __fmul2_rn(r6, r2i), el);
-      if (CLS) {   // the pair's class from the number of cluster atoms in it
-        const float2 eel = __fmul2_rn(qq, c), elj = __fmul2_rn(h, r6);
-        te4 = __fadd2_rn(te4, eel);
-        tl4 = __fadd2_rn(tl4, elj);
-        const bool cj = ((jc >> k) & 1u) != 0u;
-        const float2 e2 = __ffma2_rn(elj, make_float2(1.f / 6.f, 1.f / 6.f), eel);
-        ea4 += (cj && A.ca ? e2.x : 0.f) + (cj && A.cb ? e2.y : 0.f);
-        eb4 += (cj != A.ca ? e2.x : 0.f) + (cj != A.cb ? e2.y : 0.f);
-        fs = __fmul2_rn(fs, cj ? A.w1 : A.w0);
-      } else {
-        te4 = __ffma2_rn(qq, c, te4);
-        tl4 = __ffma2_rn(h, r6, tl4);
-      }
-      fx = __ffma2_rn(dx, fs, fx);
-      fy = __ffma2_rn(dy, fs, fy);
-      fz = __ffma2_rn(dz, fs, fz);
-      gx = fmaf(dx.y, fs.y, fmaf(dx.x, fs.x, gx));
-      gy = fmaf(dy.y, fs.y, fmaf(dy.x, fs.x, gy));
-      gz = fmaf(dz.y, fs.y, fmaf(dz.x, fs.x, gz));
-      if (COUNT) tn += (ia ? 1 : 0) + (ib ? 1 : 0);
-      if (k < 7) {
-        gx = __shfl_sync(full, gx, src);
-        gy = __shfl_sync(full, gy, src);
-        gz = __shfl_sync(full, gz, src);
-        tj = __shfl_sync(full, tj, src);
-      }
-      if (k == 3 || k == 7) {   // energies: FP32 over 4 steps, then FP64
-        te += (double)te4.x + (double)te4.y;
-        tl += (double)tl4.x + (double)tl4.y;
-        te4 = tl4 = make_float2(0.f, 0.f);
-        if (CLS) {
-          ea += (double)ea4;
-          eb += (double)eb4;
-          ea4 = eb4 = 0.f;
-        }
-      }
     }
-    const int aj = S.at[sat + 8 * g].x;
-    if (aj >= 0 && (gx != 0.f || gy != 0.f || gz != 0.f)) {
-      atomic_add_ll(&P.frc[3 * aj + 0], to_fix_f(-gx, P.status));
-      atomic_add_ll(&P.frc[3 * aj + 1], to_fix_f(-gy, P.status));
-      atomic_add_ll(&P.frc[3 * aj + 2], to_fix_f(-gz, P.status));
+    const float2 qf = __fmul2_rn(A.qi, make_float2(j.w, j.w));
+    const float2 qq = make_float2(ia ? qf.x : 0.f, ib ? qf.y : 0.f);
+    const float2 p = __fmul2_rn(p12, r6);
+    const float2 h = __ffma2_rn(p, half2, m6);
+    const float2 c = __fadd2_rn(rinv, __ffma2_rn(zb2, r2, mzc));
+    const float2 el = __fmul2_rn(qq, __ffma2_rn(rinv, r2i, mzf));
+    float2 fs = LJ ? __ffma2_rn(__fadd2_rn(p, m6), __fmul2_rn(r6, r2i), el) : el;
+    if (CLS) {   // the pair's class from the number of cluster atoms in it
+      const float2 eel = __fmul2_rn(qq, c), elj = LJ ? __fmul2_rn(h, r6) : make_float2(0.f, 0.f);
+      te4 = __fadd2_rn(te4, eel);
+      if (LJ) tl4 = __fadd2_rn(tl4, elj);
+      const bool cj = ((jc >> k) & 1u) != 0u;
+      const float2 e2 = LJ ? __ffma2_rn(elj, make_float2(1.f / 6.f, 1.f / 6.f), eel) : eel;
+      ea4 += (cj && A.ca ? e2.x : 0.f) + (cj && A.cb ? e2.y : 0.f);
+      eb4 += (cj != A.ca ? e2.x : 0.f) + (cj != A.cb ? e2.y : 0.f);
+      fs = __fmul2_rn(fs, cj ? A.w1 : A.w0);
+    } else {
+      te4 = __ffma2_rn(qq, c, te4);
+      if (LJ) tl4 = __ffma2_rn(h, r6, tl4);
+    }
+    fx = __ffma2_rn(dx, fs, fx);
+    fy = __ffma2_rn(dy, fs, fy);
+    fz = __ffma2_rn(dz, fs, fz);
+    gx = fmaf(dx.y, fs.y, fmaf(dx.x, fs.x, gx));
+    gy = fmaf(dy.y, fs.y, fmaf(dy.x, fs.x, gy));
+    gz = fmaf(dz.y, fs.y, fmaf(dz.x, fs.x, gz));
+    if (COUNT) tn += (ia ? 1 : 0) + (ib ? 1 : 0);
+    if (k < 7) {
+      gx = __shfl_sync(full, gx, src);
+      gy = __shfl_sync(full, gy, src);
+      gz = __shfl_sync(full, gz, src);
+      if (LJ) tj = __shfl_sync(full, tj, src);
+    }
+    if (k == 3 || k == 7) {   // energies: FP32 over 4 steps, then FP64
+      te += (double)te4.x + (double)te4.y;
+      if (LJ) tl += (double)tl4.x + (double)tl4.y;
+      te4 = tl4 = make_float2(0.f, 0.f);
+      if (CLS) {
+        ea += (double)ea4;
+        eb += (double)eb4;
+        ea4 = eb4 = 0.f;
+      }
     }
   }
+  const int aj = S.at[sat + 8 * g].x;
+  if (aj >= 0 && (gx != 0.f || gy != 0.f || gz != 0.f)) {
+    atomic_add_ll(&P.frc[3 * aj + 0], to_fix_f(-gx, P.status));
+    atomic_add_ll(&P.frc[3 * aj + 1], to_fix_f(-gy, P.status));
+    atomic_add_ll(&P.frc[3 * aj + 2], to_fix_f(-gz, P.status));
+  }
+}
+
+// ljg: bit g set if some entry 8 g .. 8 g + 7 of the warp's four records has an LJ term
+template <bool MINIMG, bool COUNT, bool TRI, bool CLS>
+__device__ __forceinline__ void record_packed(const DevPtrs& P, const QuadStage& S, const float2* __restrict__ s_lj,
+                                              const float4* __restrict__ s_lj3, int rowa, int rowb,
+                                              const PackedArgs& A, unsigned ljg, int sp, int st, int sat, int src,
+                                              float2& fx, float2& fy, float2& fz, double& te, double& tl,
+                                              int& tn, double& ea, double& eb) {
+  // in the groups' order whatever the neighbouring records are (the sums must not depend on
+  // where a record stands); a run of groups of one form is a loop of its own
+  int g = 0;
+#pragma unroll 1
+  do {
+#pragma unroll 1
+    for (; (ljg >> g) & 1u; ++g)
+      group_packed<MINIMG, COUNT, TRI, CLS, true>(P, S, s_lj, s_lj3, rowa, rowb, A, g, sp, st, sat, src, fx, fy, fz,
+                                                  te, tl, tn, ea, eb);
+#pragma unroll 1
+    for (; g < 4 && !((ljg >> g) & 1u); ++g)
+      group_packed<MINIMG, COUNT, TRI, CLS, false>(P, S, s_lj, s_lj3, rowa, rowb, A, g, sp, st, sat, src, fx, fy, fz,
+                                                   te, tl, tn, ea, eb);
+  } while (g < 4);
 }
 
 // what a lane gathers for a record group before computing it: the positions (in their own
@@ -536,7 +558,7 @@ __global__ void __launch_bounds__(kPairThreads, CLS ? 1 : 2) k_pair_packed(DevPt
       S.at[sta + 8 * g] = ta;
       if (CLS) jc |= ((__ballot_sync(full, (ta.y >> 30) & 1) >> (8 * qd)) & 0xffu) << (8 * g);
     }
-    const int unit = G.unit >= 0 ? G.unit & ~kRecImg : -1;
+    const int unit = G.unit >= 0 ? G.unit & kRecUnit : -1;
     A.ma = unit >= 0 ? step_mask(S.msk[b][16 * qd + lp], lp) : 0u;
     A.mb = unit >= 0 ? step_mask(S.msk[b][16 * qd + 8 + lp], lp + 8) : 0u;
     // the lane's i atoms: a new unit flushes the last one's forces and loads the new atoms
@@ -588,6 +610,8 @@ __global__ void __launch_bounds__(kPairThreads, CLS ? 1 : 2) k_pair_packed(DevPt
     }
     // one image form for the whole warp
     const bool wmi = __any_sync(full, mi || (G.unit >= 0 && (G.unit & kRecImg)));
+    // (a record past the last one, -1, has every flag set)
+    const unsigned ljg = (~__reduce_and_sync(full, (unsigned)G.unit) >> kRecFree) & 0xfu;
     __syncwarp();
     // buffer b is free again: the group after next goes into it; the next group's gathers
     // are issued before this group's arithmetic
@@ -613,10 +637,10 @@ __global__ void __launch_bounds__(kPairThreads, CLS ? 1 : 2) k_pair_packed(DevPt
     }
     // (classes: with per-pair images always, which change nothing where they are not needed)
     if (CLS || wmi)
-      record_packed<true, COUNT, TRI, CLS>(P, S, s_lj, s_lj3, rowa, rowb, A, sp, sta, sat, src, fx, fy, fz, te, tl,
+      record_packed<true, COUNT, TRI, CLS>(P, S, s_lj, s_lj3, rowa, rowb, A, ljg, sp, sta, sat, src, fx, fy, fz, te, tl,
                                            tn_pairs, ea, eb);
     else
-      record_packed<false, COUNT, TRI, CLS>(P, S, s_lj, s_lj3, rowa, rowb, A, sp, sta, sat, src, fx, fy, fz, te, tl,
+      record_packed<false, COUNT, TRI, CLS>(P, S, s_lj, s_lj3, rowa, rowb, A, ljg, sp, sta, sat, src, fx, fy, fz, te, tl,
                                             tn_pairs, ea, eb);
     if (CLS) {
       eaa += to_fix(ea, kEneScale, P.status);
@@ -828,7 +852,7 @@ k_pair_mixed(DevPtrs P, ZdConst z) {
     const bool valid = rec < T;
     G.m = valid ? S.msk[b][lane] : 0u;
     G.me = CMM && valid ? S.msk_el[b][lane] : 0u;
-    G.unit = valid ? P.ct_blk[rec] & ~kRecImg : -1;
+    G.unit = valid ? P.ct_blk[rec] & kRecUnit : -1;
     gather1(S.ent[b][32 * hw + lp], valid, G.pa, G.ta, G.aa);
     gather1(S.ent[b][32 * hw + kHalf + lp], valid, G.pb, G.tb, G.ab);
   };
@@ -1126,7 +1150,7 @@ __global__ void __launch_bounds__(kPairThreads, 2) k_pair_fp64q(DevPtrs P, ZdCon
   for (int t = gw; t < TU;) {
     const int rec = 4 * t + qd;
     const bool valid = rec < T;
-    const int unit = valid ? P.ct_blk[rec] & ~kRecImg : -1;
+    const int unit = valid ? P.ct_blk[rec] & kRecUnit : -1;
     int aj[4], ty[4];
 #pragma unroll
     for (int g = 0; g < 4; ++g) {
@@ -1255,7 +1279,7 @@ k_pair_fp64(DevPtrs P, ZdConst z) {
     if (t >= TU) break;
     const int rec = 2 * t + hw;
     const bool valid = rec < T;
-    const int unit = valid ? P.ct_blk[rec] & ~kRecImg : -1;
+    const int unit = valid ? P.ct_blk[rec] & kRecUnit : -1;
     if (unit != cur_unit) {
       flush_i();
       cur_unit = unit;
