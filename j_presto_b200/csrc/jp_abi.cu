@@ -176,12 +176,8 @@ void enqueue_rebuild(jp_ctx *c, bool count_only = false) {
   DevPtrs &P = c->P;
   cudaStream_t st = c->st;
   const int nt = 256;
-  cudaMemsetAsync(P.hist, 0, sizeof(int) * (c->nkeys + 1), st);
-  cudaMemsetAsync(P.cursor, 0, sizeof(int) * (c->nkeys + 1), st);
-  cudaMemsetAsync(P.rep_hmax, 0, sizeof(float) * 3 * c->nrep, st);
-  cudaMemsetAsync(P.nctiles, 0, 2 * sizeof(int), st);
-  cudaMemsetAsync(P.ext_pos, 0, sizeof(int), st);
-  if (c->hbond) cudaMemsetAsync(P.ntiles, 0, sizeof(int), st);
+  const int nreset = std::max(std::max(c->nkeys + 1, c->nslot), 3 * c->nrep);
+  k_list_reset<<<(nreset + nt - 1) / nt, nt, 0, st>>>(P, c->nkeys, c->nslot, c->nrep, c->zc.nt1 - 1, c->hbond);
   int ncmm = 0;
   if (c->cmm) {   // celpar_CB + celoth + celpol: cells and multipoles at this rebuild
     int ntot = 0;
@@ -193,16 +189,13 @@ void enqueue_rebuild(jp_ctx *c, bool count_only = false) {
     ncmm = 3 + std::max(0, c->cmm_nlev - 1);
   }
   k_cell_key<<<(c->natom + nt - 1) / nt, nt, 0, st>>>(P, c->natom);
-  int nl = 9;   // the single kernels below
+  int nl = 6;   // the single kernels below
   nl += scan_exclusive(P.hist, P.hist_scan, c->nkeys + 1, c->scan_scratch, nullptr, st);
-  k_scatter<<<(c->natom + nt - 1) / nt, nt, 0, st>>>(P, c->natom);
-  k_sort_bins<<<(c->nkeys + nt - 1) / nt, nt, 0, st>>>(P, c->nkeys);
-  k_col_count<<<(c->ncol + nt - 1) / nt, nt, 0, st>>>(P, c->ncol);
+  k_scatter<<<(std::max(c->natom, c->ncol) + nt - 1) / nt, nt, 0, st>>>(P, c->natom, c->ncol);
   nl += scan_exclusive(P.col_nb, P.col_blk, c->ncol + 1, c->scan_scratch, nullptr, st);
-  k_clear_slots<<<(c->nslot + nt - 1) / nt, nt, 0, st>>>(P, c->nslot, c->zc.nt1 - 1);
   k_fill_slots<<<(c->natom + nt - 1) / nt, nt, 0, st>>>(P, c->natom);
-  k_excl_slots<<<(c->natom + nt - 1) / nt, nt, 0, st>>>(P, c->natom);
-  k_block_setup<<<(c->nblk * 32 + nt - 1) / nt, nt, 0, st>>>(P, c->nblk, c->qscale);
+  const int nsetup = (c->nblk * 32 + nt - 1) / nt;
+  k_block_setup<<<nsetup + (c->natom + nt - 1) / nt, nt, 0, st>>>(P, c->nblk, c->qscale, nsetup, c->natom);
   const double rlim = c->zc.rlim;   // rc + 1.5; CMM: the farthest near-field pair
   const double rc = c->prm.cutoff;
   launch_block_list(P, c->nblk, c->nsm, rlim * rlim, (float)rlim, rc * rc, c->cmm, c->zc.nt1 - 1, count_only,
@@ -1616,7 +1609,7 @@ int jp_create(const jp_system *sys, int32_t nrep, const jp_params *prm, jp_ctx *
   e |= dalloc(c, &P.key, (size_t)N);
   e |= dalloc(c, &P.hist, (size_t)c->nkeys + 1);        // +1: sentinel for the scan
   e |= dalloc(c, &P.hist_scan, (size_t)c->nkeys + 1);
-  e |= dalloc(c, &P.cursor, (size_t)c->nkeys + 1);
+  e |= dalloc(c, &P.rank, (size_t)N);
   e |= dput(c, &P.col_rep, hcol_rep);
   e |= dalloc(c, &P.col_nb, (size_t)c->ncol + 1);
   e |= dalloc(c, &P.col_blk, (size_t)c->ncol + 1);

@@ -4,7 +4,7 @@
 // Pipeline (every UPDATE steps, all replicas in one pass):
 //   1. k_cell_key      radix binning: wrapped position -> fine cell -> Morton key per replica
 //   2. scan            counting-sort offsets (deterministic exclusive scan)
-//   3. k_scatter       bin atoms; k_sort_bins makes the order within a bin deterministic
+//   3. k_scatter       atoms to their bins; blocks per column
 //   4. k_fill_slots    compact order -> 32-atom blocks padded per replica
 //   5. k_block_setup   per-block bounding box, frame origin, block-local coordinates
 //   6. k_block_list    one thread block per i-block: bounding-box tests of the later blocks,
@@ -35,48 +35,35 @@ __global__ void k_cell_key(DevPtrs P, int natom) {
   if (out) atomicOr(P.status, ERR_FREE_WINDOW);
   const unsigned key = (unsigned)(R.key0 + (c[1] * R.grid[0] + c[0]) * R.grid[2] + c[2]);
   P.key[a] = key;
-  atomicAdd(&P.hist[key], 1);
+  P.rank[a] = atomicAdd(&P.hist[key], 1);
 }
 
-__global__ void k_scatter(DevPtrs P, int natom) {
-  int a = blockIdx.x * blockDim.x + threadIdx.x;
-  if (a >= natom) return;
-  unsigned key = P.key[a];
-  int pos = P.hist_scan[key] + atomicAdd(&P.cursor[key], 1);
-  P.sorted[pos] = a;
-}
-
-// deterministic order inside each bin: ascending atom index (bins hold a few atoms)
-__global__ void k_sort_bins(DevPtrs P, int nkeys) {
-  int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= nkeys) return;
-  int n = P.hist[k];
-  if (n < 2) return;
-  int* s = P.sorted + P.hist_scan[k];
-  for (int i = 1; i < n; ++i) {
-    int v = s[i];
-    int j = i - 1;
-    while (j >= 0 && s[j] > v) { s[j + 1] = s[j]; --j; }
-    s[j + 1] = v;
-  }
-}
-
-// blocks each column needs: ceil(atoms in column / 32)
-__global__ void k_col_count(DevPtrs P, int ncol) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= ncol) return;
-  const int r = P.col_rep[c];
-  const Rep& R = P.reps[r];
-  const int k0 = R.key0 + (c - R.col0) * R.grid[2];
+// an atom to its place of its bin; and the blocks each column needs: ceil(atoms in column / 32)
+__global__ void k_scatter(DevPtrs P, int natom, int ncol) {
+  const int a = blockIdx.x * blockDim.x + threadIdx.x;
+  if (a < natom) P.sorted[P.hist_scan[P.key[a]] + P.rank[a]] = a;
+  if (a >= ncol) return;
+  const Rep& R = P.reps[P.col_rep[a]];
+  const int k0 = R.key0 + (a - R.col0) * R.grid[2];
   const int n = P.hist_scan[k0 + R.grid[2]] - P.hist_scan[k0];
-  P.col_nb[c] = (n + kTile - 1) / kTile;
+  P.col_nb[a] = (n + kTile - 1) / kTile;
 }
 
-__global__ void k_clear_slots(DevPtrs P, int nslot, int dummy_type) {
-  int s = blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= nslot) return;
-  P.satom[s] = -1;
-  P.styp[s] = dummy_type;
+// what a list build starts from: empty bins and slots, no records, no block extents (a small
+// system's build is a chain of launches of 2-4 us each: with this for six memsets and a launch,
+// with the sort within bins, the column counts and the exclusion slots inside their
+// neighbours' launches, 2,200 atoms took 80 us instead of 104, 22,700 atoms 118 instead of 141)
+__global__ void k_list_reset(DevPtrs P, int nkeys, int nslot, int nrep, int dummy_type, int hbond) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i <= nkeys) P.hist[i] = 0;
+  if (i < nslot) {
+    P.satom[i] = -1;
+    P.styp[i] = dummy_type;
+  }
+  if (i < 3 * nrep) P.rep_hmax[i] = 0.f;
+  if (i < 2) P.nctiles[i] = 0;
+  if (i == 0) *P.ext_pos = 0;
+  if (i == 0 && hbond) *P.ntiles = 0;
 }
 
 // sorted position -> slot: block = replica's first block + blocks of the columns before this
@@ -88,7 +75,12 @@ __global__ void k_fill_slots(DevPtrs P, int natom) {
   const Rep& R = P.reps[P.rep_of[a]];
   const int col = R.col0 + ((int)P.key[a] - R.key0) / R.grid[2];
   const int kcol = R.key0 + (col - R.col0) * R.grid[2];
-  const int rank = pos - P.hist_scan[kcol];
+  // within a bin (a few atoms) by ascending atom index, so that the order does not depend on the
+  // arrival that k_cell_key counted
+  const int bin = (int)P.key[a], b0 = P.hist_scan[bin], b1 = b0 + P.hist[bin];
+  int place = b0;
+  for (int q = b0; q < b1; ++q) place += P.sorted[q] < a ? 1 : 0;
+  const int rank = place - P.hist_scan[kcol];
   const int blk = R.blk0 + (P.col_blk[col] - P.col_blk[R.col0]) + rank / kTile;
   const int slot = blk * kTile + (rank % kTile);
   P.slot_of[a] = slot;
@@ -96,8 +88,15 @@ __global__ void k_fill_slots(DevPtrs P, int natom) {
   P.styp[slot] = P.typ[a];
 }
 
-// one warp per block
-__global__ void k_block_setup(DevPtrs P, int nblk, double qscale) {
+// one warp per block; the blocks from nsetup on: the slot of every exclusion partner (lets the
+// tile build clear excluded pairs per partner instead of searching the partner list per pair)
+__global__ void k_block_setup(DevPtrs P, int nblk, double qscale, int nsetup, int natom) {
+  if ((int)blockIdx.x >= nsetup) {
+    const int a = (blockIdx.x - nsetup) * blockDim.x + threadIdx.x;
+    if (a < natom)
+      for (int p = P.excl_ptr[a]; p < P.excl_ptr[a + 1]; ++p) P.excl_slot[p] = P.slot_of[P.excl_idx[p]];
+    return;
+  }
   int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   int lane = threadIdx.x & 31;
   if (warp >= nblk) return;
@@ -141,9 +140,12 @@ __global__ void k_block_setup(DevPtrs P, int nblk, double qscale) {
     if (lo[0] <= hi[0]) {   // largest block half-extent per replica (non-negative floats
                             // order like their bit patterns)
       const int r = P.blk_rep[warp];
-      for (int k = 0; k < 3; ++k)
-        atomicMax(reinterpret_cast<int*>(&P.rep_hmax[3 * r + k]),
-                  __float_as_int((float)(0.5 * (hi[k] - lo[k]))));
+      for (int k = 0; k < 3; ++k) {
+        // (only where it still grows: the blocks of 64 replicas waited 50 us for each other)
+        const float h = (float)(0.5 * (hi[k] - lo[k]));
+        if (__ldcg(&P.rep_hmax[3 * r + k]) < h)
+          atomicMax(reinterpret_cast<int*>(&P.rep_hmax[3 * r + k]), __float_as_int(h));
+      }
     }
   }
   double o[3];
@@ -157,14 +159,6 @@ __global__ void k_block_setup(DevPtrs P, int nblk, double qscale) {
                            (float)(P.x[3 * a + 2] - o[2]), q);
 }
 
-// slot of every exclusion partner, refreshed after each sort: lets the tile build clear
-// excluded pairs per partner instead of searching the partner list per pair
-__global__ void k_excl_slots(DevPtrs P, int natom) {
-  const int a = blockIdx.x * blockDim.x + threadIdx.x;
-  if (a >= natom) return;
-  for (int p = P.excl_ptr[a]; p < P.excl_ptr[a + 1]; ++p) P.excl_slot[p] = P.slot_of[P.excl_idx[p]];
-}
-
 // ---- pair list: one thread block per i-block ---------------------------------------------------
 // k_block_list does everything that belongs to one 32-atom i-block: the bounding-box test of
 // the later blocks of its replica, the exact 32x32 interaction mask of every survivor, and the
@@ -175,7 +169,8 @@ __global__ void k_excl_slots(DevPtrs P, int natom) {
 // Before, a warp scanned 32 candidates one after the other, and eleven more launches (three
 // scans of per-chunk counts, tile emit, unit counts, their scan, record index, record emit)
 // passed the tiles on through memory.  A whole list build, before and now: 64 replicas 4,380 and
-// 2,303 us, 99,200 atoms 534 and 358, 22,700 atoms 216 and 139, 2,200 atoms 196 and 105.
+// 2,361 us, 99,200 atoms 534 and 352, 22,700 atoms 216 and 118, 2,200 atoms 196 and 80.  Its
+// shared memory counts: 4.6 KB more a block took 64 replicas 170 us longer.
 //
 // Pair record: a half block (16 i atoms: rows 0-15 or 16-31 of an i-block, unit u = 2 i-block +
 // half) with 32 j entries, the j atoms of that block's tiles that at least one of the 16 i

@@ -224,7 +224,8 @@ struct DevPtrs {
   size_t rec_cap;                 // length of the record arrays
   // cell sort
   unsigned *key;                  // per atom
-  int *hist, *hist_scan, *cursor; // per key
+  int *hist, *hist_scan;          // per key
+  int *rank;                      // of each atom in its key, by arrival
   int *sorted;                    // compact order -> atom
   int *col_rep;                   // replica of each xy column (static)
   int *col_nb, *col_blk;          // blocks per column and their exclusive scan [ncol+1]

@@ -8,13 +8,10 @@ namespace jp {
 
 // cells / tiles (jp_cells.cu)
 __global__ void k_cell_key(DevPtrs P, int natom);
-__global__ void k_scatter(DevPtrs P, int natom);
-__global__ void k_sort_bins(DevPtrs P, int nkeys);
-__global__ void k_col_count(DevPtrs P, int ncol);
-__global__ void k_clear_slots(DevPtrs P, int nslot, int dummy_type);
+__global__ void k_list_reset(DevPtrs P, int nkeys, int nslot, int nrep, int dummy_type, int hbond);
+__global__ void k_scatter(DevPtrs P, int natom, int ncol);
 __global__ void k_fill_slots(DevPtrs P, int natom);
-__global__ void k_excl_slots(DevPtrs P, int natom);
-__global__ void k_block_setup(DevPtrs P, int nblk, double qscale);
+__global__ void k_block_setup(DevPtrs P, int nblk, double qscale, int nsetup, int natom);
 // tiles and pair records of every i-block.  CMM: masks from the level-1 cells (neighbours:
 // Coulomb + LJ into masks and masks_el; cells up to idelay apart and r^2 < rc2: LJ only) instead
 // of the list radius.  count_only: the records per unit alone; keep: masks left in global
