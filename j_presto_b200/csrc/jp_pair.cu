@@ -1024,7 +1024,8 @@ k_pair_mixed(DevPtrs P, ZdConst z) {
 //  - 1/r by rsqrt_h3; the cut-off test on r^2 itself; LJ from (-6 C6, 12 C12) as in record_packed.
 //  - Branch-free: a pair outside the mask or the cut-off has zero charge product and r^-1 = 0.
 // On 22,700 atoms 144 us with one i atom a lane and an image, a division and a square root per
-// pair, 93 with rsqrt() and the images per atom, 83 so (the FP64 pipe busy half the time).
+// pair, 93 with rsqrt() and the images per atom, 83 so (the FP64 pipe busy half the time), 72
+// with the LJ term left out where a record group has none.
 struct __align__(16) QuadStageD {
   double2 pxy[256], pzq[256];   // entry 8 g + e of record q at 64 q + 16 g + e, and 8 further on
   int2 at[4 * 36];              // (atom, type) of entry 8 g + e at 36 q + 8 g + e
@@ -1046,65 +1047,87 @@ __device__ __forceinline__ double rsqrt_h3(double x) {
   return fma(y * e, fma(e, 0.375, 0.5), y);
 }
 
+template <bool MINIMG, bool COUNT, bool LJ>
+__device__ __forceinline__ void group_fp64(const DevPtrs& P, const QuadStageD& S, const double2* __restrict__ s_lj,
+                                           int rowa, int rowb, const double (&xa)[4], const double (&xb)[4],
+                                           unsigned ma, unsigned mb, int g, const double (&box)[3], const double (&inv)[3],
+                                           double rc2, double zb, double zf, double zc, int sp, int st, int sat,
+                                           int src, double (&fa)[3], double (&fb)[3], double& te, double& tl,
+                                           int& tn) {
+  const unsigned full = 0xffffffffu;
+  const double2* __restrict__ pxy = S.pxy + sp + 16 * g;
+  const double2* __restrict__ pzq = S.pzq + sp + 16 * g;
+  int tj = LJ ? S.at[st + 8 * g].y : 0;
+  double gx = 0.0, gy = 0.0, gz = 0.0;   // minus the j force of the entry this lane meets
+#pragma unroll 2
+  for (int k = 0; k < 8; ++k) {
+    const double2 jxy = pxy[k], jzq = pzq[k];
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      const double* xi = e ? xb : xa;
+      double dx = jxy.x - xi[0], dy = jxy.y - xi[1], dz = jzq.x - xi[2];   // x_j - x_i
+      if (MINIMG) {
+        dx = near_image(dx, box[0], inv[0]);
+        dy = near_image(dy, box[1], inv[1]);
+        dz = near_image(dz, box[2], inv[2]);
+      }
+      const double r2 = fma(dx, dx, fma(dy, dy, dz * dz));
+      const bool in = (((e ? mb : ma) >> (8 * g + k)) & 1u) && r2 <= rc2;
+      const double ri = in ? rsqrt_h3(r2) : 0.0;
+      const double qq = in ? xi[3] * jzq.y : 0.0;
+      const double r2i = ri * ri;
+      te = fma(qq, ri + fma(zb, r2, -zc), te);
+      double fs = qq * fma(ri, r2i, -zf);
+      if (LJ) {
+        const double2 lj = s_lj[(e ? rowb : rowa) + tj];   // -6 C6, 12 C12
+        const double r6 = r2i * r2i * r2i, p = lj.y * r6;
+        tl = fma(fma(p, 0.5, lj.x), r6, tl);
+        fs = fma(p + lj.x, r6 * r2i, fs);
+      }
+      double* fi = e ? fb : fa;
+      fi[0] = fma(dx, fs, fi[0]);
+      fi[1] = fma(dy, fs, fi[1]);
+      fi[2] = fma(dz, fs, fi[2]);
+      gx = fma(dx, fs, gx);
+      gy = fma(dy, fs, gy);
+      gz = fma(dz, fs, gz);
+      if (COUNT) tn += in ? 1 : 0;
+    }
+    if (k < 7) {
+      gx = __shfl_sync(full, gx, src);
+      gy = __shfl_sync(full, gy, src);
+      gz = __shfl_sync(full, gz, src);
+      if (LJ) tj = __shfl_sync(full, tj, src);
+    }
+  }
+  const int aj = S.at[sat + 8 * g].x;
+  if (aj >= 0 && (gx != 0.0 || gy != 0.0 || gz != 0.0)) {
+    atomicAdd(&P.grd[3 * aj + 0], -gx);
+    atomicAdd(&P.grd[3 * aj + 1], -gy);
+    atomicAdd(&P.grd[3 * aj + 2], -gz);
+  }
+}
+
+// (ljg as in record_packed)
 template <bool MINIMG, bool COUNT>
 __device__ __forceinline__ void record_fp64(const DevPtrs& P, const QuadStageD& S, const double2* __restrict__ s_lj,
                                             int rowa, int rowb, const double (&xa)[4], const double (&xb)[4],
-                                            unsigned ma, unsigned mb, const double (&box)[3], const double (&inv)[3],
-                                            double rc2, double zb, double zf, double zc, int sp, int st, int sat,
-                                            int src, double (&fa)[3], double (&fb)[3], double& te, double& tl,
-                                            int& tn) {
-  const unsigned full = 0xffffffffu;
+                                            unsigned ma, unsigned mb, unsigned ljg, const double (&box)[3],
+                                            const double (&inv)[3], double rc2, double zb, double zf, double zc, int sp,
+                                            int st, int sat, int src, double (&fa)[3], double (&fb)[3], double& te,
+                                            double& tl, int& tn) {
+  int g = 0;
 #pragma unroll 1
-  for (int g = 0; g < 4; ++g) {
-    const double2* __restrict__ pxy = S.pxy + sp + 16 * g;
-    const double2* __restrict__ pzq = S.pzq + sp + 16 * g;
-    int tj = S.at[st + 8 * g].y;
-    double gx = 0.0, gy = 0.0, gz = 0.0;   // minus the j force of the entry this lane meets
-#pragma unroll 2
-    for (int k = 0; k < 8; ++k) {
-      const double2 jxy = pxy[k], jzq = pzq[k];
-#pragma unroll
-      for (int e = 0; e < 2; ++e) {
-        const double* xi = e ? xb : xa;
-        double dx = jxy.x - xi[0], dy = jxy.y - xi[1], dz = jzq.x - xi[2];   // x_j - x_i
-        if (MINIMG) {
-          dx = near_image(dx, box[0], inv[0]);
-          dy = near_image(dy, box[1], inv[1]);
-          dz = near_image(dz, box[2], inv[2]);
-        }
-        const double r2 = fma(dx, dx, fma(dy, dy, dz * dz));
-        const bool in = (((e ? mb : ma) >> (8 * g + k)) & 1u) && r2 <= rc2;
-        const double ri = in ? rsqrt_h3(r2) : 0.0;
-        const double qq = in ? xi[3] * jzq.y : 0.0;
-        const double2 lj = s_lj[(e ? rowb : rowa) + tj];   // -6 C6, 12 C12
-        const double r2i = ri * ri, r6 = r2i * r2i * r2i;
-        const double p = lj.y * r6;
-        te = fma(qq, ri + fma(zb, r2, -zc), te);
-        tl = fma(fma(p, 0.5, lj.x), r6, tl);
-        const double fs = fma(p + lj.x, r6 * r2i, qq * fma(ri, r2i, -zf));
-        double* fi = e ? fb : fa;
-        fi[0] = fma(dx, fs, fi[0]);
-        fi[1] = fma(dy, fs, fi[1]);
-        fi[2] = fma(dz, fs, fi[2]);
-        gx = fma(dx, fs, gx);
-        gy = fma(dy, fs, gy);
-        gz = fma(dz, fs, gz);
-        if (COUNT) tn += in ? 1 : 0;
-      }
-      if (k < 7) {
-        gx = __shfl_sync(full, gx, src);
-        gy = __shfl_sync(full, gy, src);
-        gz = __shfl_sync(full, gz, src);
-        tj = __shfl_sync(full, tj, src);
-      }
-    }
-    const int aj = S.at[sat + 8 * g].x;
-    if (aj >= 0 && (gx != 0.0 || gy != 0.0 || gz != 0.0)) {
-      atomicAdd(&P.grd[3 * aj + 0], -gx);
-      atomicAdd(&P.grd[3 * aj + 1], -gy);
-      atomicAdd(&P.grd[3 * aj + 2], -gz);
-    }
-  }
+  do {
+#pragma unroll 1
+    for (; (ljg >> g) & 1u; ++g)
+      group_fp64<MINIMG, COUNT, true>(P, S, s_lj, rowa, rowb, xa, xb, ma, mb, g, box, inv, rc2, zb, zf, zc, sp, st, sat,
+                                      src, fa, fb, te, tl, tn);
+#pragma unroll 1
+    for (; g < 4 && !((ljg >> g) & 1u); ++g)
+      group_fp64<MINIMG, COUNT, false>(P, S, s_lj, rowa, rowb, xa, xb, ma, mb, g, box, inv, rc2, zb, zf, zc, sp, st, sat,
+                                       src, fa, fb, te, tl, tn);
+  } while (g < 4);
 }
 
 template <bool COUNT>
@@ -1150,7 +1173,8 @@ __global__ void __launch_bounds__(kPairThreads, 2) k_pair_fp64q(DevPtrs P, ZdCon
   for (int t = gw; t < TU;) {
     const int rec = 4 * t + qd;
     const bool valid = rec < T;
-    const int unit = valid ? P.ct_blk[rec] & kRecUnit : -1;
+    const int word = valid ? P.ct_blk[rec] : -1, unit = valid ? word & kRecUnit : -1;
+    const unsigned ljg = (~__reduce_and_sync(full, (unsigned)word) >> kRecFree) & 0xfu;
     int aj[4], ty[4];
 #pragma unroll
     for (int g = 0; g < 4; ++g) {
@@ -1207,10 +1231,10 @@ __global__ void __launch_bounds__(kPairThreads, 2) k_pair_fp64q(DevPtrs P, ZdCon
     double te = 0.0, tl = 0.0;
     int tn = 0;
     if (__any_sync(full, mi))
-      record_fp64<true, COUNT>(P, S, s_lj, tia * z.nt1, tib * z.nt1, xa, xb, ma, mb, box, inv, z.rc2, z.bcoeff,
+      record_fp64<true, COUNT>(P, S, s_lj, tia * z.nt1, tib * z.nt1, xa, xb, ma, mb, ljg, box, inv, z.rc2, z.bcoeff,
                                z.fcoeff, z.zcore, sp, sta, sat, src, fa, fb, te, tl, tn);
     else
-      record_fp64<false, COUNT>(P, S, s_lj, tia * z.nt1, tib * z.nt1, xa, xb, ma, mb, box, inv, z.rc2, z.bcoeff,
+      record_fp64<false, COUNT>(P, S, s_lj, tia * z.nt1, tib * z.nt1, xa, xb, ma, mb, ljg, box, inv, z.rc2, z.bcoeff,
                                 z.fcoeff, z.zcore, sp, sta, sat, src, fa, fb, te, tl, tn);
     if (COUNT) npair += tn;
     eel += to_fix(te, kEneScale, P.status);

@@ -55,3 +55,17 @@ def test_lj_free_entries_vs_oracle(eng_mod, kind, alsd):
         assert e.pair_count() == o.npairs_cut
     assert rms_rel(g, go) < 1e-5
     np.testing.assert_allclose(ene, eo, rtol=1e-5, atol=1e-2)
+
+
+@pytest.mark.parametrize("kind", ["some", "none", "all", "one"])
+def test_lj_free_entries_fp64(eng_mod, kind):
+    """The FP64 kernel's groups without the LJ term: the suite's FP64 tolerances."""
+    top = _top(kind)
+    kw = dict(method=abi.JP_METHOD_CANO, cutoff=8.0)
+    o = oracle.Oracle(top, **kw)
+    eo, go = o.energy_grad()
+    with eng_mod.Engine(top, precision=abi.JP_PREC_FP64, **kw) as e:
+        ene, g = e.energy_grad()
+        assert e.pair_count() == o.npairs_cut
+    assert rms_rel(g, go) < 1e-12
+    np.testing.assert_allclose(ene, eo, rtol=1e-8, atol=1e-7)
