@@ -194,8 +194,8 @@ void enqueue_rebuild(jp_ctx *c, bool count_only = false) {
   k_scatter<<<(std::max(c->natom, c->ncol) + nt - 1) / nt, nt, 0, st>>>(P, c->natom, c->ncol);
   nl += scan_exclusive(P.col_nb, P.col_blk, c->ncol + 1, c->scan_scratch, nullptr, st);
   k_fill_slots<<<(c->natom + nt - 1) / nt, nt, 0, st>>>(P, c->natom);
-  const int nsetup = (c->nblk * 32 + nt - 1) / nt;
-  k_block_setup<<<nsetup + (c->natom + nt - 1) / nt, nt, 0, st>>>(P, c->nblk, c->qscale, nsetup, c->natom);
+  const int nsu = 32 * kSetupWarps, nsetup = (c->nblk * 32 + nsu - 1) / nsu;
+  k_block_setup<<<nsetup + (c->natom + nsu - 1) / nsu, nsu, 0, st>>>(P, c->nblk, c->qscale, nsetup, c->natom);
   const double rlim = c->zc.rlim;   // rc + 1.5; CMM: the farthest near-field pair
   const double rc = c->prm.cutoff;
   launch_block_list(P, c->nblk, c->nsm, rlim * rlim, (float)rlim, rc * rc, c->cmm, c->zc.nt1 - 1, count_only,

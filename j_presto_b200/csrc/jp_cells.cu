@@ -97,66 +97,76 @@ __global__ void k_block_setup(DevPtrs P, int nblk, double qscale, int nsetup, in
       for (int p = P.excl_ptr[a]; p < P.excl_ptr[a + 1]; ++p) P.excl_slot[p] = P.slot_of[P.excl_idx[p]];
     return;
   }
-  int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  int lane = threadIdx.x & 31;
-  if (warp >= nblk) return;
-  const int slot = warp * kTile + lane;
-  const int a = P.satom[slot];
-  const Rep& R = P.reps[P.blk_rep[warp]];
-  const int ty = P.styp[slot];
-  const unsigned lj = __ballot_sync(0xffffffffu, a >= 0 && !P.lj_free[ty & kTypeMask]);
-  const unsigned cls = __ballot_sync(0xffffffffu, a >= 0 && ((ty >> 30) & 1));
-  if (lane == 0) P.blk_kind[warp] = make_uint2(lj, cls);
-  double w[3] = {0, 0, 0}, img[3] = {0, 0, 0};
-  double lo[3], hi[3];
-  for (int k = 0; k < 3; ++k) {
-    if (a >= 0) {
-      double x = P.x[3 * a + k];
-      img[k] = floor(x * R.invbox[k]);
-      w[k] = x - R.box[k] * img[k];
-      lo[k] = w[k];
-      hi[k] = w[k];
-    } else {
-      lo[k] = 1e300;
-      hi[k] = -1e300;
-    }
-    for (int o = 16; o > 0; o >>= 1) {
-      lo[k] = fmin(lo[k], __shfl_xor_sync(0xffffffffu, lo[k], o));
-      hi[k] = fmax(hi[k], __shfl_xor_sync(0xffffffffu, hi[k], o));
-    }
-  }
-  double ref[3];
-  for (int k = 0; k < 3; ++k) ref[k] = 0.5 * (lo[k] + hi[k]);
-  if (lane == 0) {
-    P.blk_ref[3 * warp + 0] = ref[0];
-    P.blk_ref[3 * warp + 1] = ref[1];
-    P.blk_ref[3 * warp + 2] = ref[2];
-    P.blk_ctr[warp] = make_float4((float)ref[0], (float)ref[1], (float)ref[2], 0.f);
-    // an empty block (capacity not used this rebuild) gets a -inf extent: it never passes
-    // the bounding-box test
-    P.blk_half[warp] = make_float4((float)(0.5 * (hi[0] - lo[0])) + 1e-4f,
-                                   (float)(0.5 * (hi[1] - lo[1])) + 1e-4f,
-                                   (float)(0.5 * (hi[2] - lo[2])) + 1e-4f, 0.f);
-    if (lo[0] <= hi[0]) {   // largest block half-extent per replica (non-negative floats
-                            // order like their bit patterns)
-      const int r = P.blk_rep[warp];
-      for (int k = 0; k < 3; ++k) {
-        // (only where it still grows: the blocks of 64 replicas waited 50 us for each other)
-        const float h = (float)(0.5 * (hi[k] - lo[k]));
-        if (__ldcg(&P.rep_hmax[3 * r + k]) < h)
-          atomicMax(reinterpret_cast<int*>(&P.rep_hmax[3 * r + k]), __float_as_int(h));
+  // largest extents and replica of the thread block's warps: one atomic per replica among them
+  // (with one per warp the blocks of 64 replicas waited for each other: a list build of theirs
+  // took 2,364 us, and 2,303 so)
+  __shared__ float s_h[kSetupWarps][3];
+  __shared__ int s_rep[kSetupWarps];
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int blk = blockIdx.x * kSetupWarps + w;
+  if (lane == 0) s_rep[w] = -1;
+  if (blk < nblk) {
+    const int slot = blk * kTile + lane;
+    const int a = P.satom[slot];
+    const int r = P.blk_rep[blk];
+    const Rep& R = P.reps[r];
+    const int ty = P.styp[slot];
+    const unsigned lj = __ballot_sync(0xffffffffu, a >= 0 && !P.lj_free[ty & kTypeMask]);
+    const unsigned cls = __ballot_sync(0xffffffffu, a >= 0 && ((ty >> 30) & 1));
+    if (lane == 0) P.blk_kind[blk] = make_uint2(lj, cls);
+    double x[3] = {0, 0, 0}, img[3] = {0, 0, 0};
+    double lo[3], hi[3], ref[3];
+    for (int k = 0; k < 3; ++k) {
+      if (a >= 0) {
+        x[k] = P.x[3 * a + k];
+        img[k] = floor(x[k] * R.invbox[k]);
+        lo[k] = hi[k] = x[k] - R.box[k] * img[k];
+      } else {
+        lo[k] = 1e300;
+        hi[k] = -1e300;
       }
     }
+    for (int o = 16; o > 0; o >>= 1)
+      for (int k = 0; k < 3; ++k) {
+        lo[k] = fmin(lo[k], __shfl_xor_sync(0xffffffffu, lo[k], o));
+        hi[k] = fmax(hi[k], __shfl_xor_sync(0xffffffffu, hi[k], o));
+      }
+    for (int k = 0; k < 3; ++k) ref[k] = 0.5 * (lo[k] + hi[k]);
+    if (lane == 0) {
+      P.blk_ref[3 * blk + 0] = ref[0];
+      P.blk_ref[3 * blk + 1] = ref[1];
+      P.blk_ref[3 * blk + 2] = ref[2];
+      P.blk_ctr[blk] = make_float4((float)ref[0], (float)ref[1], (float)ref[2], 0.f);
+      // an empty block (capacity not used this rebuild) gets a -inf extent: it never passes
+      // the bounding-box test
+      P.blk_half[blk] = make_float4((float)(0.5 * (hi[0] - lo[0])) + 1e-4f,
+                                    (float)(0.5 * (hi[1] - lo[1])) + 1e-4f,
+                                    (float)(0.5 * (hi[2] - lo[2])) + 1e-4f, 0.f);
+      if (lo[0] <= hi[0]) {
+        s_rep[w] = r;
+        for (int k = 0; k < 3; ++k) s_h[w][k] = (float)(0.5 * (hi[k] - lo[k]));
+      }
+    }
+    if (a >= 0) {
+      double o[3];
+      for (int k = 0; k < 3; ++k) {
+        o[k] = ref[k] + R.box[k] * img[k];
+        P.off[3 * a + k] = o[k];
+      }
+      const float q = (float)((double)qscale * P.chg[a]);
+      P.pos_f[a] = make_float4((float)(x[0] - o[0]), (float)(x[1] - o[1]), (float)(x[2] - o[2]), q);
+    }
   }
-  double o[3];
-  if (a < 0) return;
-  for (int k = 0; k < 3; ++k) o[k] = ref[k] + R.box[k] * img[k];
-  P.off[3 * a + 0] = o[0];
-  P.off[3 * a + 1] = o[1];
-  P.off[3 * a + 2] = o[2];
-  const float q = (float)((double)qscale * P.chg[a]);
-  P.pos_f[a] = make_float4((float)(P.x[3 * a] - o[0]), (float)(P.x[3 * a + 1] - o[1]),
-                           (float)(P.x[3 * a + 2] - o[2]), q);
+  __syncthreads();
+  if (w == 0 && lane < kSetupWarps) {
+    const unsigned all = (1u << kSetupWarps) - 1u;
+    const int r = s_rep[lane];
+    const unsigned same = __match_any_sync(all, r);
+    for (int k = 0; k < 3; ++k) {   // (non-negative floats order like their bit patterns)
+      const unsigned h = __reduce_max_sync(same, r >= 0 ? __float_as_uint(s_h[lane][k]) : 0u);
+      if (r >= 0 && lane == __ffs(same) - 1) atomicMax(reinterpret_cast<int*>(&P.rep_hmax[3 * r + k]), (int)h);
+    }
+  }
 }
 
 // ---- pair list: one thread block per i-block ---------------------------------------------------
@@ -169,7 +179,7 @@ __global__ void k_block_setup(DevPtrs P, int nblk, double qscale, int nsetup, in
 // Before, a warp scanned 32 candidates one after the other, and eleven more launches (three
 // scans of per-chunk counts, tile emit, unit counts, their scan, record index, record emit)
 // passed the tiles on through memory.  A whole list build, before and now: 64 replicas 4,380 and
-// 2,361 us, 99,200 atoms 534 and 352, 22,700 atoms 216 and 118, 2,200 atoms 196 and 80.  Its
+// 2,303 us, 99,200 atoms 534 and 344, 22,700 atoms 216 and 118, 2,200 atoms 196 and 80.  Its
 // shared memory counts: 4.6 KB more a block took 64 replicas 170 us longer.
 //
 // Pair record: a half block (16 i atoms: rows 0-15 or 16-31 of an i-block, unit u = 2 i-block +

@@ -11,6 +11,7 @@ __global__ void k_cell_key(DevPtrs P, int natom);
 __global__ void k_list_reset(DevPtrs P, int nkeys, int nslot, int nrep, int dummy_type, int hbond);
 __global__ void k_scatter(DevPtrs P, int natom, int ncol);
 __global__ void k_fill_slots(DevPtrs P, int natom);
+constexpr int kSetupWarps = 8;   // warps of a thread block of k_block_setup
 __global__ void k_block_setup(DevPtrs P, int nblk, double qscale, int nsetup, int natom);
 // tiles and pair records of every i-block.  CMM: masks from the level-1 cells (neighbours:
 // Coulomb + LJ into masks and masks_el; cells up to idelay apart and r^2 < rc2: LJ only) instead
