@@ -44,7 +44,7 @@ METRIC = "aggregate ns/day & pairs/s: mixed vs FP64 GPU path at ≤1e-5 RMS forc
 DT_FS = 2.0
 FLOPS_PER_PAIR = 52          # FP32 flops per pair interaction within rc (FMA = 2)
 L2_FLUSH_BYTES = 256 << 20   # > 126 MB L2
-PAIR_PROFILE = os.path.join(ROOT, "profiles", "k_pair_mixed_c4.md")
+PAIR_PROFILE = os.path.join(ROOT, "profiles", "k_pair_packed_c4.md")
 
 
 def c4_name(natoms):
@@ -505,7 +505,7 @@ def main():
                 "timing": "host wall clock around jp_step_io(1): all replicas' x, v in from pinned "
                           "memory, one step, x, v and energies out, one synchronisation"},
         "gpu_launches": args.steps * per_step + nreb * per_rebuild,
-        "roofline": {"bound": "fp32", "kernel": "k_pair_mixed", "achieved": achieved,
+        "roofline": {"bound": "fp32", "kernel": "k_pair_packed", "achieved": achieved,
                      "peak": peak, "unit": "TFLOP/s", "frac": achieved / peak,
                      "traffic": traffic, "traffic_source": tsrc,
                      "hbm": None if traffic is None or not hbm_peak else
