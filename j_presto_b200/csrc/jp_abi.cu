@@ -94,7 +94,7 @@ struct jp_ctx {
   Timing tm;
   int launches_step = 0, launches_rebuild = 0;
   bool rebuild_pending = false;     // the list rebuild due after the last step taken
-  // block-shape tuning: per replica and candidate the xy column grid, the compact tiles
+  // block-shape tuning: per replica and candidate the xy column grid, the pair records
   // the list needed with it, and the candidate kept
   std::vector<int> tune_grid;       // [nrep][JP_TUNE_CANDIDATES][2]
   std::vector<long long> tune_tiles;  // [nrep][JP_TUNE_CANDIDATES]
@@ -826,9 +826,9 @@ int minimize_conj(jp_ctx *c, int r, const jp_min_params *mp, int32_t *iters, dou
 int flush_rebuild(jp_ctx *c);   // below, beside the step loop
 
 // Block-shape tuning (the role of md_run's SIMD_check.f90:1-42 for its vector length): the
-// pair kernels' work is proportional to the compact tiles of the list, so each replica's
-// list is built with every candidate column grid and the grid needing the fewest compact
-// tiles is kept (ties to the unit factor, then to the smaller factor).  The count is exact
+// pair kernels' work is proportional to the pair records of the list, so each replica's
+// list is built with every candidate column grid and the grid needing the fewest
+// records is kept (ties to the unit factor, then to the smaller factor).  The count is exact
 // and deterministic, so the choice does not depend on timing noise, and a replica's choice
 // depends on its own atoms only (batched with others it chooses as it would alone).
 // Without tuning every replica keeps the unit factor.  Ends with the list built for the

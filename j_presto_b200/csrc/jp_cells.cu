@@ -131,11 +131,7 @@ __global__ void k_block_setup(DevPtrs P, int nblk, double qscale, int nsetup, in
         lo[k] = fmin(lo[k], __shfl_xor_sync(0xffffffffu, lo[k], o));
         hi[k] = fmax(hi[k], __shfl_xor_sync(0xffffffffu, hi[k], o));
       }
-    // the middle of the block, on a grid of 1/512 A: the references' differences, the shifts of
-    // the j atoms into an i block's frame, then are exact in FP32 (but for a box edge in them).
-    // Their rounding was common to a tile's pairs and as large as the staged position's: the
-    // mixed forces' error against FP64 on 15,200 atoms was 1.15e-6 (RMS, relative), 1.06e-6 so
-    for (int k = 0; k < 3; ++k) ref[k] = floor(256.0 * (lo[k] + hi[k]) + 0.5) * (1.0 / 512.0);
+    for (int k = 0; k < 3; ++k) ref[k] = 0.5 * (lo[k] + hi[k]);
     if (lane == 0) {
       P.blk_ref[3 * blk + 0] = ref[0];
       P.blk_ref[3 * blk + 1] = ref[1];
@@ -143,13 +139,12 @@ __global__ void k_block_setup(DevPtrs P, int nblk, double qscale, int nsetup, in
       P.blk_ctr[blk] = make_float4((float)ref[0], (float)ref[1], (float)ref[2], 0.f);
       // an empty block (capacity not used this rebuild) gets a -inf extent: it never passes
       // the bounding-box test
-      // (the reference is up to 1/1024 A off the middle)
-      P.blk_half[blk] = make_float4((float)(0.5 * (hi[0] - lo[0])) + 1.1e-3f,
-                                    (float)(0.5 * (hi[1] - lo[1])) + 1.1e-3f,
-                                    (float)(0.5 * (hi[2] - lo[2])) + 1.1e-3f, 0.f);
+      P.blk_half[blk] = make_float4((float)(0.5 * (hi[0] - lo[0])) + 1e-4f,
+                                    (float)(0.5 * (hi[1] - lo[1])) + 1e-4f,
+                                    (float)(0.5 * (hi[2] - lo[2])) + 1e-4f, 0.f);
       if (lo[0] <= hi[0]) {
         s_rep[w] = r;
-        for (int k = 0; k < 3; ++k) s_h[w][k] = (float)(0.5 * (hi[k] - lo[k])) + 1e-3f;
+        for (int k = 0; k < 3; ++k) s_h[w][k] = (float)(0.5 * (hi[k] - lo[k]));
       }
     }
     if (a >= 0) {
@@ -203,7 +198,7 @@ __global__ void k_block_setup(DevPtrs P, int nblk, double qscale, int nsetup, in
 // without, and the same two, without first, of the entries that make a record take per-pair
 // images or ALSD classes.  The pair kernels leave the LJ term out over eight entries of a
 // warp's records that have none (in waters two thirds of the entries), and few records mix
-// the forms.  Pair kernel with entries in tile order and so: 64 replicas (1.06 M
+// the forms.  Pair kernel with entries in tile order and so: 64 replicas (883,000
 // atoms) 1,345 and 1,290 us, 99,200 atoms 181 and 166, 22,700 atoms 54 and 51.  With the LJ order alone
 // the entries of image tiles, scattered over more records, cost 64 replicas more than it gave
 // (1,480 us).

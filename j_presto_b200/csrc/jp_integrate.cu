@@ -1321,7 +1321,7 @@ __device__ __forceinline__ void cano5_unit(const DevPtrs& P, const IntConst& c, 
 // sub-system (solvent), the warp works on its 288 components side by side instead, lane l on
 // components l, l+32, ...; only the SHAKE pass needs a unit's components in one lane, and
 // gets them through shared memory (9 doubles a lane: no bank conflicts).  64 solvated
-// chains of 16,500 atoms: 397 -> 264 us a step, 32 of 9,000: 222 -> 160 (with the groups in
+// chains of 13,800 atoms: 397 -> 264 us a step, 32 of 9,000: 222 -> 160 (with the groups in
 // launches of their own, see quad_blocks).
 constexpr int kWarpComp = 288;     // components of a warp's 32 three-atom units
 
@@ -2472,7 +2472,7 @@ __device__ __forceinline__ void lam_load(const DevPtrs& P, int r, LamStep& L) {
 // 1-3 atom units [0, nsmall) and the per-replica threads (energy record, lambda).  The group
 // blocks are few and each is one long chain (their SHAKE), so they start first and run beside
 // the units' blocks; in launches of their own a
-// step of 64 chains (1.06 M atoms) took 264 us against 229, of 32 (290 k) 160 against 119.
+// step of 64 chains (883,000 atoms) took 264 us against 229, of 32 (290 k) 160 against 119.
 __host__ __device__ __forceinline__ int quad_blocks(const IntConst& c) {
   return (c.nvirt - c.qbase + kIntThreads - 1) / kIntThreads;
 }

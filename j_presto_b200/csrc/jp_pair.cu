@@ -271,9 +271,14 @@ struct PackedArgs {
 // Why two i atoms a lane: the shared-memory and shuffle pipe (one 128-byte wavefront a cycle
 // per SM) bounds the loop.  A step of 64 pairs reads one j position (4 wavefronts), one type
 // (1), one LJ record (4) and shuffles one force (3): 12, where one i atom and two entries a
-// lane took 20 (two positions, two forces).  Measured on 64 replicas (883,000 atoms): 1,612 us with
-// one i atom a lane, 1,494 so; 190 and 179 us on 99,200 atoms, 59 and 52 us on 22,700.  Now 59 % of the issue slots and
-// 70 % of that pipe are busy (24 % of it staging, 17 % the force atomics), the FMA pipe 45 %.
+// lane took 20 (two positions, two forces); without the LJ term (LJ = false) it is 7.  Measured
+// on 64 replicas (883,000 atoms): 1,612 us with one i atom a lane, 1,494 so, 1,346 with images
+// by tile and 1,290 with the groups without an LJ term; on 99,200 atoms 190, 179, 180 and 165,
+// on 22,700 atoms 59, 52, 54 and 51 (the third with the positions by atom).  62 % of the issue
+// slots and 71 % of that pipe are busy, the FMA pipe 44 %.  Sums of an i atom by group and then
+// over the groups, instead of 32 terms in a row, cost registers (1,365, 171 and 52 us) and keep
+// the forces' error against FP64 at 1.05e-6 instead of 1.11e-6 (RMS, relative, mean of eight
+// systems of 3,000 to 15,200 atoms; one i atom a lane with 16 terms a sum: 1.02e-6).
 // Half or quarter groups as work units of small lists measured slower (the per-record work).
 template <bool MINIMG, bool COUNT, bool TRI, bool CLS, bool LJ>
 __device__ __forceinline__ void group_packed(const DevPtrs& P, const QuadStage& S, const float2* __restrict__ s_lj,
@@ -387,18 +392,29 @@ __device__ __forceinline__ void record_packed(const DevPtrs& P, const QuadStage&
                                               float2& fx, float2& fy, float2& fz, double& te, double& tl,
                                               int& tn, double& ea, double& eb) {
   // in the groups' order whatever the neighbouring records are (the sums must not depend on
-  // where a record stands); a run of groups of one form is a loop of its own
+  // where a record stands); a run of groups of one form is a loop of its own.  An i atom's
+  // force is summed by group, 8 terms, and then over the groups
   int g = 0;
 #pragma unroll 1
   do {
 #pragma unroll 1
-    for (; (ljg >> g) & 1u; ++g)
-      group_packed<MINIMG, COUNT, TRI, CLS, true>(P, S, s_lj, s_lj3, rowa, rowb, A, g, sp, st, sat, src, fx, fy, fz,
+    for (; (ljg >> g) & 1u; ++g) {
+      float2 lx = make_float2(0.f, 0.f), ly = lx, lz = lx;
+      group_packed<MINIMG, COUNT, TRI, CLS, true>(P, S, s_lj, s_lj3, rowa, rowb, A, g, sp, st, sat, src, lx, ly, lz,
                                                   te, tl, tn, ea, eb);
+      fx = __fadd2_rn(fx, lx);
+      fy = __fadd2_rn(fy, ly);
+      fz = __fadd2_rn(fz, lz);
+    }
 #pragma unroll 1
-    for (; g < 4 && !((ljg >> g) & 1u); ++g)
-      group_packed<MINIMG, COUNT, TRI, CLS, false>(P, S, s_lj, s_lj3, rowa, rowb, A, g, sp, st, sat, src, fx, fy, fz,
+    for (; g < 4 && !((ljg >> g) & 1u); ++g) {
+      float2 lx = make_float2(0.f, 0.f), ly = lx, lz = lx;
+      group_packed<MINIMG, COUNT, TRI, CLS, false>(P, S, s_lj, s_lj3, rowa, rowb, A, g, sp, st, sat, src, lx, ly, lz,
                                                    te, tl, tn, ea, eb);
+      fx = __fadd2_rn(fx, lx);
+      fy = __fadd2_rn(fy, ly);
+      fz = __fadd2_rn(fz, lz);
+    }
   } while (g < 4);
 }
 
