@@ -1449,16 +1449,33 @@ k_pair_fp64(DevPtrs P, ZdConst z) {
   flush_fix<16>(P, cur_rep, eel, elj, eaa, eab, npair, COUNT, ALSD || SPLIT);
 }
 
-// the packed kernel's stages and table take more than the default 48 KiB of dynamic shared
-// memory: raised when a context is created
+// The packed kernels' stages and tables take more than the default 48 KiB of dynamic shared memory.
+// The limit belongs to the function on its device, not to a context, so every context raises it
+// to the same value, all that the device allows: with the context's own size there, one of
+// fewer types created later lowered it below what an earlier context launches with.
+// Resident blocks of the kernel an SM, 0 if `bytes` do not fit.
+template <class Kernel>
+static int raise_smem_limit(Kernel kernel, int bytes) {
+  int dev = 0, optin = 0, per = 0;
+  cudaFuncAttributes fa{};
+  if (cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess ||
+      cudaFuncGetAttributes(&fa, kernel) != cudaSuccess)
+    return 0;
+  const int limit = optin - (int)fa.sharedSizeBytes;
+  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, limit) != cudaSuccess) return 0;
+  if (bytes > limit ||
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kernel, kPairThreads, bytes) != cudaSuccess)
+    return 0;
+  return per;
+}
+
 template <bool TRI>
 static int packed_blocks_per_sm(int bytes) {
-  int per = 0;
-  cudaFuncSetAttribute(k_pair_packed<false, false, TRI>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-  cudaFuncSetAttribute(k_pair_packed<true, false, TRI>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-  cudaFuncSetAttribute(k_pair_packed<false, true, TRI>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-  cudaFuncSetAttribute(k_pair_packed<true, true, TRI>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_pair_packed<false, false, TRI>, kPairThreads, bytes);
+  const int per = raise_smem_limit(k_pair_packed<false, false, TRI>, bytes);
+  raise_smem_limit(k_pair_packed<true, false, TRI>, bytes);
+  raise_smem_limit(k_pair_packed<false, true, TRI>, bytes);
+  raise_smem_limit(k_pair_packed<true, true, TRI>, bytes);
   return per;
 }
 
@@ -1491,9 +1508,8 @@ int pair_blocks_per_sm(bool fp64, bool packed, int nt1) {
   int per = 0;
   if (fp64 && packed) {
     const int bytes = (int)fp64q_bytes(nt1);
-    cudaFuncSetAttribute(k_pair_fp64q<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-    cudaFuncSetAttribute(k_pair_fp64q<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_pair_fp64q<false>, kPairThreads, bytes);
+    per = raise_smem_limit(k_pair_fp64q<false>, bytes);
+    raise_smem_limit(k_pair_fp64q<true>, bytes);
   } else if (fp64) {
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_pair_fp64<false, true, false>, kPairThreads,
                                                   sizeof(double2) * nt1 * nt1);
@@ -1504,6 +1520,8 @@ int pair_blocks_per_sm(bool fp64, bool packed, int nt1) {
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_pair_mixed<false, true, false>, kPairThreads,
                                                   sizeof(float2) * nt1 * nt1);
   }
+  // (tables that fit no block: the first evaluation's launch is refused and says so)
+  if (per <= 0) cudaGetLastError();
   return per > 0 ? per : 1;
 }
 
