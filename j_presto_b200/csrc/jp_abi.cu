@@ -1753,7 +1753,7 @@ int jp_create(const jp_system *sys, int32_t nrep, const jp_params *prm, jp_ctx *
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, c->device);
   c->nsm = std::max(1, nsm);
   // one wave: every warp resident at once, each with an equal share of the tiles
-  c->pair_warps = std::max(1, nsm) * (256 / 32) * pair_blocks_per_sm(c->fp64, !c->split && !c->cmm && !(c->fp64 && c->alsd), c->zc.nt1);
+  c->pair_warps = std::max(1, nsm) * kPairWarps * pair_blocks_per_sm(c->fp64, !c->split && !c->cmm && !(c->fp64 && c->alsd), c->zc.nt1);
   c->cano_grid = cano_grid(c->fp64, c->device);
   CK(cudaStreamCreateWithFlags(&c->st, cudaStreamNonBlocking));
   CK(cudaStreamCreateWithFlags(&c->st2, cudaStreamNonBlocking));

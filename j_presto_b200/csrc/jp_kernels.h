@@ -40,6 +40,7 @@ void launch_cmm_far(const DevPtrs& P, int natom, int nrep, bool fp64, bool force
                     cudaStream_t st);
 
 // pair kernels (jp_pair.cu)
+constexpr int kPairWarps = 6;    // warps of a thread block
 // alsd: some replica has ALSD classes (every_cls: class weights that are not lambda's, so the
 // records without cluster atoms are weighted too); split: some replica keeps partial-McMD class-1 forces
 // apart (frc1 / grd1)

@@ -19,8 +19,8 @@
 // records, a half-warp each, one i atom a lane, the two entries of a step in scalar
 // arithmetic.  FP32 pair arithmetic on block-local coordinates (|x| < ~30 A), every step of a
 // record branch-free (a pair outside the mask or the cut-off contributes an exact zero);
-// forces summed per record in FP32, energies in FP32 over 4 steps then in FP64, both added
-// as 64-bit fixed point (2^-32 kcal/mol/A) with integer atomics -- order independent, so
+// an i atom's forces summed over eight entries and a j atom's over the record's i atoms in FP32,
+// energies in FP32 over 4 steps then in FP64, all added as 64-bit fixed point (2^-32 kcal/mol/A) with integer atomics -- order independent, so
 // results are bit-identical run to run.  Warps take short runs of consecutive record groups,
 // the first by their own index and the next from a global counter, so all finish together
 // whatever their records hold.  A warp keeps two groups in flight ahead of the one it
@@ -35,9 +35,11 @@
 
 namespace jp {
 
-constexpr int kPairThreads = 256;
+// Six warps a block, two blocks an SM: 168 registers a thread, which the packed kernel's sums
+// need.  With eight warps (128 registers) they spilled: 64 replicas (883,000 atoms) 1,390 us, so
+// 1,307, 99,200 atoms 174 and 163, 2,200 atoms 21 and 17.
+constexpr int kPairThreads = 32 * kPairWarps;
 constexpr long long kCopyWaitCycles = 2000000000LL;
-constexpr int kPairWarps = kPairThreads / 32;
 
 // ---- bulk copies into shared memory (TMA engine, no tensor map) -------------------------
 __device__ __forceinline__ unsigned smem_addr(const void* p) {
@@ -248,6 +250,37 @@ __device__ __forceinline__ unsigned step_mask(unsigned w, int r) {
   return byte_rotr(((lo << r) >> 16) | ((hi << r) & 0xffff0000u), r & 7);
 }
 
+// a group's sums over its entries, (i atom, i atom + 8) side by side, into the lane's fixed-point
+// forces; a value outside the fixed-point range (2^24 kcal/mol/A) or not finite is reported
+__device__ __noinline__ void report_force(unsigned* status, float2 x, float2 y, float2 z) {
+  to_fix_f(x.x, status); to_fix_f(x.y, status);
+  to_fix_f(y.x, status); to_fix_f(y.y, status);
+  to_fix_f(z.x, status); to_fix_f(z.y, status);
+}
+
+__device__ __forceinline__ float max_nan(float a, float b) {   // NaN if either is
+  float m;
+  asm("max.NaN.f32 %0, %1, %2;" : "=f"(m) : "f"(a), "f"(b));
+  return m;
+}
+
+__device__ __forceinline__ void add_forces(unsigned* status, float2 x, float2 y, float2 z, long long (&ga)[3],
+                                           long long (&gb)[3]) {
+  const float m = max_nan(max_nan(max_nan(fabsf(x.x), fabsf(x.y)), max_nan(fabsf(y.x), fabsf(y.y))),
+                          max_nan(fabsf(z.x), fabsf(z.y)));
+  if (!(m < 16777216.f)) report_force(status, x, y, z);
+  const float2 k = make_float2(4294967296.f, 4294967296.f);
+  x = __fmul2_rn(x, k);
+  y = __fmul2_rn(y, k);
+  z = __fmul2_rn(z, k);
+  ga[0] += __float2ll_rn(x.x);
+  gb[0] += __float2ll_rn(x.y);
+  ga[1] += __float2ll_rn(y.x);
+  gb[1] += __float2ll_rn(y.y);
+  ga[2] += __float2ll_rn(z.x);
+  gb[2] += __float2ll_rn(z.y);
+}
+
 // what the inner loop reads of a lane's replica and classes
 struct PackedArgs {
   float2 nx, ny, nz, qi;                 // minus the two i positions, their charges
@@ -274,17 +307,21 @@ struct PackedArgs {
 // lane took 20 (two positions, two forces); without the LJ term (LJ = false) it is 7.  Measured
 // on 64 replicas (883,000 atoms): 1,612 us with one i atom a lane, 1,494 so, 1,346 with images
 // by tile and 1,290 with the groups without an LJ term; on 99,200 atoms 190, 179, 180 and 165,
-// on 22,700 atoms 59, 52, 54 and 51 (the third with the positions by atom).  62 % of the issue
-// slots and 71 % of that pipe are busy, the FMA pipe 44 %.  Sums of an i atom by group and then
-// over the groups, instead of 32 terms in a row, cost registers (1,365, 171 and 52 us) and keep
-// the forces' error against FP64 at 1.05e-6 instead of 1.11e-6 (RMS, relative, mean of eight
-// systems of 3,000 to 15,200 atoms; one i atom a lane with 16 terms a sum: 1.02e-6).
+// on 22,700 atoms 59, 52, 54 and 51 (the third with the positions by atom), each with the i
+// atoms' sums over a record's 32 terms.
+// The i atoms' sums: a group's eight entries stand close together and are of one kind (hydrogens,
+// say), so their forces on an atom mostly have one sign and a sum of many of them is large
+// before the other kind takes it back.  So four terms, plus four, then into fixed point: the
+// forces' error against FP64 (RMS, relative, mean of 27 systems of 2,100 to 15,300 atoms) is
+// 1.016e-6; 1.018e-6 with one i atom a lane and 16 terms a sum, 1.023e-6 with eight terms in a
+// row, 1.043e-6 with those groups added in FP32 (64 replicas 1,365 us, 99,200 atoms 171, 22,700
+// atoms 52; in this form 1,307, 163 and 50).
 // Half or quarter groups as work units of small lists measured slower (the per-record work).
 template <bool MINIMG, bool COUNT, bool TRI, bool CLS, bool LJ>
 __device__ __forceinline__ void group_packed(const DevPtrs& P, const QuadStage& S, const float2* __restrict__ s_lj,
                                               const float4* __restrict__ s_lj3, int rowa, int rowb,
                                              const PackedArgs& A, int g, int sp, int st, int sat, int src,
-                                             float2& fx, float2& fy, float2& fz, double& te, double& tl,
+                                             long long (&gia)[3], long long (&gib)[3], double& te, double& tl,
                                              int& tn, double& ea, double& eb) {
   const unsigned full = 0xffffffffu;
   const float2 zb2 = make_float2(A.zb, A.zb), mzc = make_float2(-A.zc, -A.zc), mzf = make_float2(-A.zf, -A.zf);
@@ -300,6 +337,7 @@ __device__ __forceinline__ void group_packed(const DevPtrs& P, const QuadStage& 
   if (CLS && LJ) tj &= kTypeMask;
   const unsigned ma = A.ma >> (8 * g), mb = A.mb >> (8 * g);
   const unsigned jc = CLS ? A.jc >> (8 * g) : 0u;
+  float2 fx = make_float2(0.f, 0.f), fy = fx, fz = fx, hx = fx, hy = fx, hz = fx;   // minus the i forces
   float gx = 0.f, gy = 0.f, gz = 0.f;   // minus the j force of the entry this lane meets
   float2 te4 = make_float2(0.f, 0.f), tl4 = te4;
   float ea4 = 0.f, eb4 = 0.f;
@@ -337,8 +375,8 @@ __device__ __forceinline__ void group_packed(const DevPtrs& P, const QuadStage& 
     const float2 p = __fmul2_rn(p12, r6);
     const float2 h = __ffma2_rn(p, half2, m6);
     const float2 c = __fadd2_rn(rinv, __ffma2_rn(zb2, r2, mzc));
-    const float2 el = __fmul2_rn(qq, __ffma2_rn(rinv, r2i, mzf));
-    float2 fs = LJ ? __ffma2_rn(__fadd2_rn(p, m6), __fmul2_rn(r6, r2i), el) : el;
+    const float2 fc = __ffma2_rn(rinv, r2i, mzf);
+    float2 fs = LJ ? __ffma2_rn(qq, fc, __fmul2_rn(__fadd2_rn(p, m6), __fmul2_rn(r6, r2i))) : __fmul2_rn(qq, fc);
     if (CLS) {   // the pair's class from the number of cluster atoms in it
       const float2 eel = __fmul2_rn(qq, c), elj = LJ ? __fmul2_rn(h, r6) : make_float2(0.f, 0.f);
       te4 = __fadd2_rn(te4, eel);
@@ -365,6 +403,10 @@ __device__ __forceinline__ void group_packed(const DevPtrs& P, const QuadStage& 
       gz = __shfl_sync(full, gz, src);
       if (LJ) tj = __shfl_sync(full, tj, src);
     }
+    if (k == 3) {   // i forces: four terms plus four
+      hx = fx; hy = fy; hz = fz;
+      fx = fy = fz = make_float2(0.f, 0.f);
+    }
     if (k == 3 || k == 7) {   // energies: FP32 over 4 steps, then FP64
       te += (double)te4.x + (double)te4.y;
       if (LJ) tl += (double)tl4.x + (double)tl4.y;
@@ -376,6 +418,7 @@ __device__ __forceinline__ void group_packed(const DevPtrs& P, const QuadStage& 
       }
     }
   }
+  add_forces(P.status, __fadd2_rn(fx, hx), __fadd2_rn(fy, hy), __fadd2_rn(fz, hz), gia, gib);
   const int aj = S.at[sat + 8 * g].x;
   if (aj >= 0 && (gx != 0.f || gy != 0.f || gz != 0.f)) {
     atomic_add_ll(&P.frc[3 * aj + 0], to_fix_f(-gx, P.status));
@@ -389,32 +432,21 @@ template <bool MINIMG, bool COUNT, bool TRI, bool CLS>
 __device__ __forceinline__ void record_packed(const DevPtrs& P, const QuadStage& S, const float2* __restrict__ s_lj,
                                               const float4* __restrict__ s_lj3, int rowa, int rowb,
                                               const PackedArgs& A, unsigned ljg, int sp, int st, int sat, int src,
-                                              float2& fx, float2& fy, float2& fz, double& te, double& tl,
+                                              long long (&gia)[3], long long (&gib)[3], double& te, double& tl,
                                               int& tn, double& ea, double& eb) {
   // in the groups' order whatever the neighbouring records are (the sums must not depend on
-  // where a record stands); a run of groups of one form is a loop of its own.  An i atom's
-  // force is summed by group, 8 terms, and then over the groups
+  // where a record stands); a run of groups of one form is a loop of its own
   int g = 0;
 #pragma unroll 1
   do {
 #pragma unroll 1
-    for (; (ljg >> g) & 1u; ++g) {
-      float2 lx = make_float2(0.f, 0.f), ly = lx, lz = lx;
-      group_packed<MINIMG, COUNT, TRI, CLS, true>(P, S, s_lj, s_lj3, rowa, rowb, A, g, sp, st, sat, src, lx, ly, lz,
-                                                  te, tl, tn, ea, eb);
-      fx = __fadd2_rn(fx, lx);
-      fy = __fadd2_rn(fy, ly);
-      fz = __fadd2_rn(fz, lz);
-    }
+    for (; (ljg >> g) & 1u; ++g)
+      group_packed<MINIMG, COUNT, TRI, CLS, true>(P, S, s_lj, s_lj3, rowa, rowb, A, g, sp, st, sat, src, gia, gib, te,
+                                                  tl, tn, ea, eb);
 #pragma unroll 1
-    for (; g < 4 && !((ljg >> g) & 1u); ++g) {
-      float2 lx = make_float2(0.f, 0.f), ly = lx, lz = lx;
-      group_packed<MINIMG, COUNT, TRI, CLS, false>(P, S, s_lj, s_lj3, rowa, rowb, A, g, sp, st, sat, src, lx, ly, lz,
-                                                   te, tl, tn, ea, eb);
-      fx = __fadd2_rn(fx, lx);
-      fy = __fadd2_rn(fy, ly);
-      fz = __fadd2_rn(fz, lz);
-    }
+    for (; g < 4 && !((ljg >> g) & 1u); ++g)
+      group_packed<MINIMG, COUNT, TRI, CLS, false>(P, S, s_lj, s_lj3, rowa, rowb, A, g, sp, st, sat, src, gia, gib, te,
+                                                   tl, tn, ea, eb);
   } while (g < 4);
 }
 
@@ -637,7 +669,6 @@ __global__ void __launch_bounds__(kPairThreads, CLS ? 1 : 2) k_pair_packed(DevPt
       if (t2 < TU) issue(t2, b);
     }
     if (tn < TU) fetch(tn, b ^ 1, G);
-    float2 fx = make_float2(0.f, 0.f), fy = fx, fz = fx;
     double te = 0.0, tl = 0.0;
     int tn_pairs = 0;
     const int ka = CLS ? (tia & kTypeMask) : tia, kb = CLS ? (tib & kTypeMask) : tib;
@@ -653,21 +684,15 @@ __global__ void __launch_bounds__(kPairThreads, CLS ? 1 : 2) k_pair_packed(DevPt
     }
     // (classes: with per-pair images always, which change nothing where they are not needed)
     if (CLS || wmi)
-      record_packed<true, COUNT, TRI, CLS>(P, S, s_lj, s_lj3, rowa, rowb, A, ljg, sp, sta, sat, src, fx, fy, fz, te, tl,
+      record_packed<true, COUNT, TRI, CLS>(P, S, s_lj, s_lj3, rowa, rowb, A, ljg, sp, sta, sat, src, gia, gib, te, tl,
                                            tn_pairs, ea, eb);
     else
-      record_packed<false, COUNT, TRI, CLS>(P, S, s_lj, s_lj3, rowa, rowb, A, ljg, sp, sta, sat, src, fx, fy, fz, te, tl,
+      record_packed<false, COUNT, TRI, CLS>(P, S, s_lj, s_lj3, rowa, rowb, A, ljg, sp, sta, sat, src, gia, gib, te, tl,
                                             tn_pairs, ea, eb);
     if (CLS) {
       eaa += to_fix(ea, kEneScale, P.status);
       eab += to_fix(eb, kEneScale, P.status);
     }
-    gia[0] += to_fix_f(fx.x, P.status);
-    gia[1] += to_fix_f(fy.x, P.status);
-    gia[2] += to_fix_f(fz.x, P.status);
-    gib[0] += to_fix_f(fx.y, P.status);
-    gib[1] += to_fix_f(fy.y, P.status);
-    gib[2] += to_fix_f(fz.y, P.status);
     eel += to_fix(te, kEneScale, P.status);
     elj += to_fix(tl * (1.0 / 6.0), kEneScale, P.status);
     if (COUNT) npair += tn_pairs;
