@@ -377,7 +377,7 @@ int snap_copy(jp_ctx *c, Snap &S, bool to, int row) {
     CK(cp(S.acnt2, P.alsd_cnt2, n2 * sizeof(unsigned long long)));
     CK(cp(S.af2, P.alsd_f2, n2 * sizeof(double)));
   }
-  if (!to) launch_update_pos(P, c->natom, c->fp64, c->qscale, c->st);
+  if (!to) launch_update_pos(P, c->natom, c->nrep, c->fp64, c->qscale, c->prm.cutoff, c->st);
   return 0;
 }
 
@@ -409,7 +409,7 @@ int snap_copy_rep(jp_ctx *c, Snap &S, bool to, int r) {
     CK(cp(S.acnt2 + r * n2, P.alsd_cnt2 + r * n2, n2 * sizeof(unsigned long long)));
     CK(cp(S.af2 + r * n2, P.alsd_f2 + r * n2, n2 * sizeof(double)));
   }
-  if (!to) launch_update_pos(P, c->natom, c->fp64, c->qscale, c->st);
+  if (!to) launch_update_pos(P, c->natom, c->nrep, c->fp64, c->qscale, c->prm.cutoff, c->st);
   return 0;
 }
 
@@ -1762,7 +1762,7 @@ int jp_create(const jp_system *sys, int32_t nrep, const jp_params *prm, jp_ctx *
   CK(cudaEventCreate(&c->ev_a));
   CK(cudaEventCreate(&c->ev_b));
   init_block_list();
-  if (c->fp64) launch_update_pos(P, N, true, c->qscale, c->st);   // the mixed path's: at each list build
+  if (c->fp64) launch_update_pos(P, N, nrep, true, c->qscale, prm->cutoff, c->st);   // the mixed path's: at each list build
   int rs = tune_blocks(c, prm->tune_blocks != 0);
   if (rs < 0) { jp_destroy(c); return rs; }
   *out = c;
@@ -1804,7 +1804,7 @@ int jp_set_state(jp_ctx *c, int32_t r, const double *cord, const double *vel) {
                                cudaMemcpyHostToDevice, c->st));
   if (vel) CK(cudaMemcpyAsync(c->P.v + 3 * (size_t)R.atom0, vel, sizeof(double) * 3 * R.natom,
                               cudaMemcpyHostToDevice, c->st));
-  if (cord) launch_update_pos(c->P, c->natom, c->fp64, c->qscale, c->st);
+  if (cord) launch_update_pos(c->P, c->natom, c->nrep, c->fp64, c->qscale, c->prm.cutoff, c->st);
   CK(cudaStreamSynchronize(c->st));
   return JP_OK;
 }
@@ -1829,7 +1829,7 @@ int eval_forces(jp_ctx *c, int32_t r, const double *cord) {
   if (cord) {
     CK(cudaMemcpyAsync(c->P.x + 3 * (size_t)R.atom0, cord, sizeof(double) * 3 * R.natom,
                        cudaMemcpyHostToDevice, c->st));
-    launch_update_pos(c->P, c->natom, c->fp64, c->qscale, c->st);
+    launch_update_pos(c->P, c->natom, c->nrep, c->fp64, c->qscale, c->prm.cutoff, c->st);
   }
   enqueue_forces(c, true, true);
   enqueue_bonded(c);
@@ -2224,7 +2224,7 @@ int jp_minimize(jp_ctx *c, const jp_min_params *mp, int32_t *iters, double *enev
     launch_shake_only(P, c->ic, 0, c->nunit, st);
     launch_min_commit(P, c->natom, nmax, st);
   }
-  launch_update_pos(P, c->natom, c->fp64, c->qscale, st);
+  launch_update_pos(P, c->natom, c->nrep, c->fp64, c->qscale, c->prm.cutoff, st);
   enqueue_zero(c, false);
   enqueue_pair(c, false, true);   // CMM: the far field at every evaluation
   enqueue_bonded(c);
@@ -2518,7 +2518,7 @@ int jp_step_io(jp_ctx *c, int32_t nsteps, const double *cord_in, const double *v
   const size_t n3 = sizeof(double) * 3 * (size_t)c->natom;
   if (cord_in) CK(cudaMemcpyAsync(c->P.x, cord_in, n3, cudaMemcpyHostToDevice, c->st));
   if (vel_in) CK(cudaMemcpyAsync(c->P.v, vel_in, n3, cudaMemcpyHostToDevice, c->st));
-  if (cord_in) launch_update_pos(c->P, c->natom, c->fp64, c->qscale, c->st);
+  if (cord_in) launch_update_pos(c->P, c->natom, c->nrep, c->fp64, c->qscale, c->prm.cutoff, c->st);
   if (nsteps == 0) {
     if (cord_out) CK(cudaMemcpyAsync(cord_out, c->P.x, n3, cudaMemcpyDeviceToHost, c->st));
     if (vel_out) CK(cudaMemcpyAsync(vel_out, c->P.v, n3, cudaMemcpyDeviceToHost, c->st));

@@ -23,6 +23,8 @@ constexpr int kHalf = 16;   // i atoms of a pair record: half a block
 // ct_blk: a record's unit, kRecImg if one of its tiles' pairs take their own images, and from bit
 // kRecFree on a bit for each eight entries that have no LJ term with anything
 constexpr int kRecImg = 1 << 30, kRecFree = 26, kRecUnit = (1 << kRecFree) - 1;
+// DevPtrs::ext_pos: coordinates replaced since the last list build; and per-pair images can be needed
+constexpr int kExtPos = 1, kExtImg = 2;
 // fixed-point scales: forces 2^32 per kcal/mol/A, energies 2^32 per kcal/mol,
 // kinetic sums (m v^2, amu A^2/fs^2) 2^40.
 constexpr double kFrcScale = 4294967296.0;
@@ -215,8 +217,8 @@ struct DevPtrs {
   // pair records (what the pair kernels run on): half an i-block and 32 j entries
   int *ct_cnt;                    // records per unit (2 i-block + half)
   int *ct_blk;                    // [CT] unit of each pair record and its flags (kRecImg, kRecFree)
-  int *ext_pos;                   // coordinates were replaced since the last list build: the records'
-                                  // image flags, made for the motion between builds, don't hold
+  int *ext_pos;                   // kExtPos, kExtImg: kernel positions were written from outside the step
+                                  // since the last list build (k_update_pos)
   float4 *ct_j;                   // [CT][32] (image shift into the i frame, atom bits; -1 = empty)
   unsigned short *ct_ty;          // [CT][32] type word of each entry (type_half; empty: dummy type)
   unsigned *ct_mask, *ct_mask_el; // [CT][32] rotated masks (listed pairs; CMM Coulomb pairs)

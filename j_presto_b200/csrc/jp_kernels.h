@@ -54,7 +54,7 @@ void launch_pair_fp64(const DevPtrs& P, const ZdConst& z, int nwarps, bool count
 int pair_blocks_per_sm(bool fp64, bool packed, int nt1);
 // LJ table of the packed kernel (DevPtrs::lj_tab) from the type-pair (C6, C12)
 void pack_lj_table(const float2* lj, int nt1, std::vector<float>& out);
-void launch_update_pos(const DevPtrs& P, int natom, bool fp64, double qscale, cudaStream_t st);
+void launch_update_pos(const DevPtrs& P, int natom, int nrep, bool fp64, double qscale, double rc, cudaStream_t st);
 
 // H-bond 10-12 pairs (jp_hbond.cu): their list at a rebuild (after the tile list), their
 // term at every force evaluation

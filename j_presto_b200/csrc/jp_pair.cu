@@ -20,8 +20,8 @@
 // arithmetic.  FP32 pair arithmetic on block-local coordinates (|x| < ~30 A), every step of a
 // record branch-free (a pair outside the mask or the cut-off contributes an exact zero);
 // an i atom's forces summed over eight entries and a j atom's over the record's i atoms in FP32,
-// energies in FP32 over 4 steps then in FP64, all added as 64-bit fixed point (2^-32 kcal/mol/A) with integer atomics -- order independent, so
-// results are bit-identical run to run.  Warps take short runs of consecutive record groups,
+// energies in FP32 over 4 steps then in FP64, all added as 64-bit fixed point (2^-32 kcal/mol/A)
+// with integer atomics -- order independent, so results are bit-identical run to run.  Warps take short runs of consecutive record groups,
 // the first by their own index and the next from a global counter, so all finish together
 // whatever their records hold.  A warp keeps two groups in flight ahead of the one it
 // computes: the bulk-copy engine (cp.async.bulk, completion on an mbarrier) brings the
@@ -29,6 +29,7 @@
 // group's j atoms are issued before the current group's arithmetic.
 // FP64 path: the same records in FP64 with FP64 force atomics (k_pair_fp64q; k_pair_fp64 with
 // classes and CMM).
+#include <algorithm>
 #include <vector>
 
 #include "jp_kernels.h"
@@ -497,7 +498,7 @@ __global__ void __launch_bounds__(kPairThreads, CLS ? 1 : 2) k_pair_packed(DevPt
   const int T = P.nctiles[seq];     // records
   // record of lane group qd in group t, and the first record of the group's copies
   auto rec0 = [&](int t) { return seq ? P.rec_cap - 4 * (size_t)(t + 1) : 4 * (size_t)t; };
-  const bool ext = *P.ext_pos != 0;
+  const bool ext = (*P.ext_pos & kExtImg) != 0;
   const int TU = (T + 3) >> 2;      // record groups: a warp's work units
   // a 2.5-KiB copy lands in microseconds; the bound (about a second of SM clock) only ends
   // the wait on a broken device, and it is not the integrator's adjustable barrier bound:
@@ -566,7 +567,6 @@ __global__ void __launch_bounds__(kPairThreads, CLS ? 1 : 2) k_pair_packed(DevPt
   long long gia[3] = {0, 0, 0}, gib[3] = {0, 0, 0};
   long long eel = 0, elj = 0, eaa = 0, eab = 0;
   long long npair = 0;
-  bool mi = false;
   auto flush_i = [&]() {
     if (aia >= 0 && (gia[0] | gia[1] | gia[2]))
       for (int k = 0; k < 3; ++k) atomic_add_ll(&P.frc[3 * aia + k], gia[k]);
@@ -642,22 +642,14 @@ __global__ void __launch_bounds__(kPairThreads, CLS ? 1 : 2) k_pair_packed(DevPt
         const Rep& R = P.reps[rep];
         if (lp < 6) S.rep[qd][lp] = (float)(lp < 3 ? R.box[lp] : R.invbox[lp - 3]);
         if (CLS && lp < 3) S.rep[qd][6 + lp] = (float)cls_weight(R, P.lam[2 * rep], 2 - lp);
-        // Per-pair minimum image is needed only where a pair within the cut-off can have
-        // another image than its tile's: the list build flags the records with such a tile
-        // (k_block_list).  Coordinates replaced without a build since may have moved farther
-        // than its margin: then, by replica, as the largest block allows -- per axis the tile's
-        // image puts the two block references at most box/2 apart, and a pair's separation
-        // differs from theirs by at most h_i + h_j <= 2 h_max plus 2 A of motion, so in the
-        // tile's image |d| <= box/2 + 2 h_max + 2; in any other image |d| >= box - rc; both
-        // hold at once only if box/2 <= rc + 2 h_max + 2
-        mi = false;
-        if (ext)
-          for (int k = 0; k < 3; ++k)
-            if (0.5 * R.box[k] < sqrt(z.rc2) + 2.0 * (double)P.rep_hmax[3 * rep + k] + 2.0) mi = true;
       }
     }
-    // one image form for the whole warp
-    const bool wmi = __any_sync(full, mi || (G.unit >= 0 && (G.unit & kRecImg)));
+    // Per-pair minimum image is needed only where a pair within the cut-off can have another image
+    // than its tile's: the list build flags the records with such a tile (k_block_list).
+    // Coordinates replaced without a build since may have moved farther than its margin: then
+    // every pair takes its own, unless no box of the context can need it (k_update_pos).  One
+    // form for the whole warp.
+    const bool wmi = ext || __any_sync(full, G.unit >= 0 && (G.unit & kRecImg));
     // (a record past the last one, -1, has every flag set)
     const unsigned ljg = (~__reduce_and_sync(full, (unsigned)G.unit) >> kRecFree) & 0xfu;
     __syncwarp();
@@ -1592,10 +1584,24 @@ void launch_pair_fp64(const DevPtrs& P, const ZdConst& z, int nwarps, bool count
   }
 }
 
-// kernel positions from the master coordinates (after an external coordinate change)
-__global__ void k_update_pos(DevPtrs P, int natom, int fp64, double qscale) {
+// kernel positions from the master coordinates (after an external coordinate change).  The
+// records' image flags don't hold until the next build: kExtPos, and kExtImg if per-pair images
+// can then be needed in the box of some replica.  Per axis a tile's image puts the two block
+// references at most box/2 apart, and a pair's separation differs from theirs by at most h_i + h_j
+// <= 2 h_max plus 2 A of motion, so in the tile's image |d| <= box/2 + 2 h_max + 2; in any other
+// image |d| >= box - rc; both hold at once only if box/2 <= rc + 2 h_max + 2.  One answer for the
+// whole context: with one per replica both image forms of the packed kernel stood in the
+// instruction cache at once, and 64 replicas with boxes on both sides of that line took 1,920 us
+// a launch with 883,000 atoms and 2,647 with 1.06 M, where all in one form take 1,484 and 1,763.
+__global__ void k_update_pos(DevPtrs P, int natom, int nrep, int fp64, double qscale, double rc) {
   const int a = blockIdx.x * blockDim.x + threadIdx.x;
-  if (a == 0) *P.ext_pos = 1;
+  if (a < nrep) {
+    const Rep& R = P.reps[a];
+    int f = kExtPos;
+    for (int k = 0; k < 3; ++k)
+      if (0.5 * R.box[k] < rc + 2.0 * (double)P.rep_hmax[3 * a + k] + 2.0) f |= kExtImg;
+    atomicOr(P.ext_pos, f);
+  }
   if (a >= natom) return;
   const double x[3] = {P.x[3 * a], P.x[3 * a + 1], P.x[3 * a + 2]};
   if (fp64) {
@@ -1614,8 +1620,8 @@ __global__ void k_update_pos(DevPtrs P, int natom, int fp64, double qscale) {
   P.pos_f[a] = make_float4(q[0], q[1], q[2], (float)(qscale * P.chg[a]));
 }
 
-void launch_update_pos(const DevPtrs& P, int natom, bool fp64, double qscale, cudaStream_t st) {
-  k_update_pos<<<(natom + 255) / 256, 256, 0, st>>>(P, natom, fp64 ? 1 : 0, qscale);
+void launch_update_pos(const DevPtrs& P, int natom, int nrep, bool fp64, double qscale, double rc, cudaStream_t st) {
+  k_update_pos<<<(std::max(natom, nrep) + 255) / 256, 256, 0, st>>>(P, natom, nrep, fp64 ? 1 : 0, qscale, rc);
 }
 
 }  // namespace jp
