@@ -1795,62 +1795,14 @@ __device__ __forceinline__ void add_kin_quad(const DevPtrs& P, int nsub_total, i
   }
 }
 
-// A group's Newton system with partial pivoting (simulu): each constraint lane holds its row, the
-// rows of the lanes that are not yet pivots are eliminated, and back substitution broadcasts
-// the solution one entry at a time.  Every lane of the warp runs the shuffles.  lu_ok: no pivot
-// of the group vanishes (simulu's 1e-30).  Out of line: quad_solve below takes nearly every
-// system.
-__device__ __noinline__ void quad_solve_pivot(const double (&row)[6], double B, bool con, int sl, double (&G)[6],
-                                              bool& lu_ok) {
-  const unsigned full = 0xffffffffu;
-  double A[6];
-#pragma unroll
-  for (int j = 0; j < 6; ++j) A[j] = row[j];
-  bool used = !con;
-  int perm[6];
-  lu_ok = true;
-#pragma unroll
-  for (int k = 0; k < 6; ++k) {
-    double bv = used ? -1.0 : fabs(A[k]);
-    int bl = sl;
-#pragma unroll
-    for (int off = 4; off > 0; off >>= 1) {
-      const double ov = __shfl_xor_sync(full, bv, off, 8);
-      const int ol = __shfl_xor_sync(full, bl, off, 8);
-      if (ov > bv || (ov == bv && ol < bl)) { bv = ov; bl = ol; }
-    }
-    perm[k] = bl;
-    double pk[6];
-#pragma unroll
-    for (int j = k; j < 6; ++j) pk[j] = __shfl_sync(full, A[j], bl, 8);
-    const double pb = __shfl_sync(full, B, bl, 8);
-    if (fabs(pk[k]) < 1.0e-30) lu_ok = false;
-    const double piv = recip_nr(pk[k]);
-    if (sl == bl) {
-      used = true;
-      A[k] = piv;
-    } else if (!used) {
-      const double f = A[k] * piv;
-#pragma unroll
-      for (int j = k + 1; j < 6; ++j) A[j] -= f * pk[j];
-      B -= f * pb;
-    }
-  }
-#pragma unroll
-  for (int i = 5; i >= 0; --i) {   // every lane keeps its row's right-hand side up to date
-    G[i] = __shfl_sync(full, B * A[i], perm[i], 8);
-    B -= A[i] * G[i];
-  }
-}
-
-// The same system in the natural pivot order, every lane of the group solving all of it: one
-// gather of the six rows (42 doubles), then no lane waits for another.  A pivot search and a
-// broadcast before each elimination step were 26-cycle shuffles in a serial chain, 2,400 cycles
+// A group's Newton system (each constraint lane holds its row) in the natural pivot order, every
+// lane of the group solving all of it: one gather of the six rows (42 doubles), then no lane
+// waits for another.  A pivot search and a broadcast before each elimination step were 26-cycle shuffles in a serial chain, 2,400 cycles
 // a Newton step against 1,700.  The gradient matrix is close to symmetric and positive definite
 // (it is where the bonds point as they did before the step), so the natural order is stable;
-// false, the same in every lane of the warp, if an entry below a pivot of an unfinished group
-// is more than 16 times that pivot (1.6 times on methyl groups) or a pivot vanishes.
-__device__ __forceinline__ bool quad_solve(const double (&row)[6], double B0, bool done, double (&G)[6]) {
+// false, the same in every lane of the group, if an entry below a pivot is more than 16 times
+// that pivot (1.6 times on methyl groups) or a pivot vanishes.
+__device__ __forceinline__ bool quad_solve(const double (&row)[6], double B0, double (&G)[6]) {
   const unsigned full = 0xffffffffu;
   double A[6][6], B[6];
 #pragma unroll
@@ -1881,7 +1833,59 @@ __device__ __forceinline__ bool quad_solve(const double (&row)[6], double B0, bo
 #pragma unroll
     for (int j = 0; j < i; ++j) B[j] -= A[j][i] * G[i];
   }
-  return !__any_sync(full, weak && !done);
+  return !weak;
+}
+
+// The same system with partial pivoting (simulu) for the groups with `weak`, the natural order's
+// solution for the others: a group's solution must not depend on which groups share its warp, all
+// of whose lanes run the shuffles.  The rows of the lanes that are not yet pivots are
+// eliminated, and back substitution broadcasts the solution one entry at a time.  lu_ok: no
+// pivot of a weak group vanishes (simulu's 1e-30).  Out of line, and with the natural order
+// solved again: quad_solve takes nearly every system, and with its solution handed over (live
+// across the call) every step of 2,200 atoms took 1.2 us longer.
+__device__ __noinline__ void quad_solve_pivot(const double (&row)[6], double B0, bool con, int sl, bool weak,
+                                              double (&G)[6], bool& lu_ok) {
+  const unsigned full = 0xffffffffu;
+  quad_solve(row, B0, G);
+  lu_ok = true;
+  double A[6], B = B0;
+#pragma unroll
+  for (int j = 0; j < 6; ++j) A[j] = row[j];
+  bool used = !con;
+  int perm[6];
+#pragma unroll
+  for (int k = 0; k < 6; ++k) {
+    double bv = used ? -1.0 : fabs(A[k]);
+    int bl = sl;
+#pragma unroll
+    for (int off = 4; off > 0; off >>= 1) {
+      const double ov = __shfl_xor_sync(full, bv, off, 8);
+      const int ol = __shfl_xor_sync(full, bl, off, 8);
+      if (ov > bv || (ov == bv && ol < bl)) { bv = ov; bl = ol; }
+    }
+    perm[k] = bl;
+    double pk[6];
+#pragma unroll
+    for (int j = k; j < 6; ++j) pk[j] = __shfl_sync(full, A[j], bl, 8);
+    const double pb = __shfl_sync(full, B, bl, 8);
+    if (fabs(pk[k]) < 1.0e-30 && weak) lu_ok = false;
+    const double piv = recip_nr(pk[k]);
+    if (sl == bl) {
+      used = true;
+      A[k] = piv;
+    } else if (!used) {
+      const double f = A[k] * piv;
+#pragma unroll
+      for (int j = k + 1; j < 6; ++j) A[j] -= f * pk[j];
+      B -= f * pb;
+    }
+  }
+#pragma unroll
+  for (int i = 5; i >= 0; --i) {   // every lane keeps its row's right-hand side up to date
+    const double gi = __shfl_sync(full, B * A[i], perm[i], 8);
+    B -= A[i] * gi;
+    if (weak) G[i] = gi;
+  }
 }
 
 // shake4 (shake.f90:333-562) for one group spread over its 8 lanes: the same Newton iteration
@@ -1953,7 +1957,8 @@ __device__ int quad_shake(const Rep& R, const QLane& q, double x[3], const doubl
     for (int ig = 0; ig < 6; ++ig)
       row[ig] = 2.0 * cr[ig] * (wk[0] * D2[ig][0] + wk[1] * D2[ig][1] + wk[2] * D2[ig][2]);
     bool lu_ok = true;
-    if (!quad_solve(row, B0, done, dG)) quad_solve_pivot(row, B0, con, sl, dG, lu_ok);
+    const bool weak = !quad_solve(row, B0, dG) && !done;
+    if (__any_sync(full, weak)) quad_solve_pivot(row, B0, con, sl, weak, dG, lu_ok);
     if (!lu_ok && !done) singular = true;
     if (lu_ok && !done)
 #pragma unroll
