@@ -59,6 +59,7 @@ struct jp_ctx {
   int natom = 0, nblk = 0, nslot = 0, nunit = 0, nterm = 0, nsub = 0, nkeys = 0, nkin = 8;
   int ncol = 0;
   size_t tile_cap_total = 0;        // block pairs of all replicas: every one could be a tile
+  std::vector<int> list_part;       // i-blocks of the list build's launches: bounds
   std::vector<Rep> reps;
   std::vector<int> rep_natom;
   DevPtrs P{};
@@ -198,11 +199,16 @@ void enqueue_rebuild(jp_ctx *c, bool count_only = false) {
   k_block_setup<<<nsetup + (c->natom + nsu - 1) / nsu, nsu, 0, st>>>(P, c->nblk, c->qscale, nsetup, c->natom);
   const double rlim = c->zc.rlim;   // rc + 1.5; CMM: the farthest near-field pair
   const double rc = c->prm.cutoff;
-  launch_block_list(P, c->nblk, c->nsm, rlim * rlim, (float)rlim, rc * rc, c->cmm, c->zc.nt1 - 1, count_only,
-                    c->hbond, c->alsd && !c->fp64, st);
+  const int parts = (int)c->list_part.size() - 1;
+  for (int q = 0; q < parts; ++q) {
+    const int b0 = c->list_part[q], nb = c->list_part[q + 1] - b0;
+    if (q > 0 && c->hbond) cudaMemsetAsync(P.ntiles, 0, sizeof(int), st);
+    launch_block_list(P, b0, nb, c->nsm, rlim * rlim, (float)rlim, rc * rc, c->cmm, c->zc.nt1 - 1, count_only,
+                      c->hbond, c->alsd && !c->fp64, st);
+    if (c->hbond && !count_only) launch_hb_list(P, c->hb_cap, c->zc.nt1, nb, q == 0, st);
+  }
   if (count_only) return;
-  if (c->hbond) launch_hb_list(P, c->hb_cap, c->zc.nt1, c->nblk, st);
-  c->launches_rebuild = nl + ncmm + (c->hbond ? 1 : 0);
+  c->launches_rebuild = nl + ncmm + (parts - 1) + (c->hbond ? parts : 0);
 }
 
 // ---- one MD step ------------------------------------------------------------------------
@@ -1521,6 +1527,35 @@ int jp_create(const jp_system *sys, int32_t nrep, const jp_params *prm, jp_ctx *
     blk_tile0[bb] = (long long)c->tile_cap_total;
     c->tile_cap_total += R.blk0 + R.nblk - bb;
   }
+  // What the list build keeps of a tile until its records are made (beyond those it holds in
+  // shared memory) has room for every possible tile of a launch.  One launch takes all i-blocks
+  // where the device has the memory for that: 1,484 bytes a possible tile with the two records.
+  // Else three launches of about as many possible tiles follow each other in a third of the
+  // room, 1,354 bytes, so that the largest system that fits is not smaller than it was with the
+  // list build in separate kernels (1,373).  Their tails cost: 147,000 atoms 628 us a build
+  // instead of 511, 270,000 atoms 1,177 instead of 1,035.
+  const size_t tile_bytes =
+      sizeof(BlkTile) + 32 * sizeof(unsigned) * (c->cmm ? 2 : 1) + (c->hbond ? sizeof(int2) + sizeof(long long) : 0);
+  const size_t rec_bytes = sizeof(int) + 32 * (sizeof(float4) + sizeof(unsigned short)) +
+                           kHalf * sizeof(unsigned) * (c->cmm ? 2 : 1);
+  constexpr size_t kAtomBytes = 2048;   // the other arrays, the copies of the state among them: well below this
+  size_t mem_free = 0, mem_total = 0;
+  if (cudaMemGetInfo(&mem_free, &mem_total) != cudaSuccess) mem_free = 0;
+  const bool fits = c->tile_cap_total * (tile_bytes + 2 * rec_bytes) + kAtomBytes * (size_t)c->natom <= mem_free;
+  const int parts = fits ? 1 : std::min(3, c->nblk);
+  size_t tile_scratch = 0;
+  c->list_part.assign(1, 0);
+  for (int q = 1; q <= parts; ++q) {
+    const int b0 = c->list_part.back();
+    const long long t0 = blk_tile0[b0];
+    const long long target = (long long)(c->tile_cap_total / parts * q);
+    int b1 = b0 + 1;
+    while (b1 < c->nblk && (q == parts || blk_tile0[b1] < target)) ++b1;
+    const long long t1 = b1 < c->nblk ? blk_tile0[b1] : (long long)c->tile_cap_total;
+    tile_scratch = std::max(tile_scratch, (size_t)(t1 - t0));
+    for (int bb = b0; bb < b1; ++bb) blk_tile0[bb] -= t0;
+    c->list_part.push_back(b1);
+  }
 
   // ---- device allocation ---------------------------------------------------------------
   DevPtrs &P = c->P;
@@ -1558,11 +1593,11 @@ int jp_create(const jp_system *sys, int32_t nrep, const jp_params *prm, jp_ctx *
   e |= dalloc(c, &P.blk_ref, 3 * (size_t)c->nblk);
   e |= dput(c, &P.blk_tile0, blk_tile0);
   e |= dalloc(c, &P.blk_kind, (size_t)c->nblk);
-  e |= dalloc(c, &P.blk_tiles, c->tile_cap_total);
-  e |= dalloc(c, &P.tmp_masks, c->tile_cap_total * 32);
+  e |= dalloc(c, &P.blk_tiles, tile_scratch);
+  e |= dalloc(c, &P.tmp_masks, tile_scratch * 32);
   if (c->hbond) {
-    e |= dalloc(c, &P.tiles, c->tile_cap_total);
-    e |= dalloc(c, &P.tile_src, c->tile_cap_total);
+    e |= dalloc(c, &P.tiles, tile_scratch);
+    e |= dalloc(c, &P.tile_src, tile_scratch);
   }
   // pair records: at most one per tile and half (a unit's records never outnumber the tiles
   // of its block), plus padding so that the kernels' record groups (up to four) stay inside
@@ -1579,7 +1614,7 @@ int jp_create(const jp_system *sys, int32_t nrep, const jp_params *prm, jp_ctx *
   if (c->cmm) {
     int ntot = 0;
     for (int l = 1; l <= 5; ++l) ntot += c->cmm_ncell[l];
-    e |= dalloc(c, &P.tmp_masks_el, c->tile_cap_total * 32);
+    e |= dalloc(c, &P.tmp_masks_el, tile_scratch * 32);
     e |= dalloc(c, &P.cmm_cell, (size_t)N);
     if (!hres_cmm.empty()) e |= dput(c, &P.cmm_res, hres_cmm);
     e |= dalloc(c, &P.gwk, 3 * (size_t)N);

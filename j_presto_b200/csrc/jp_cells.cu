@@ -452,14 +452,14 @@ __device__ __forceinline__ unsigned record_rows(const unsigned* rows, bool live,
 // mixed path): records with a cluster atom go to the top end of the record arrays, downwards,
 // as their pairs take class weights and class energies in a launch of their own
 template <bool CMM>
-__global__ void __launch_bounds__(32 * kListWarps, CMM ? 3 : 4) k_block_list(DevPtrs P, double rlim2, float rlimf,
+__global__ void __launch_bounds__(32 * kListWarps, CMM ? 3 : 4) k_block_list(DevPtrs P, int bi0, double rlim2, float rlimf,
                                                                              double rc2, int dummy_type, int count_only,
                                                                              int keep, int split_cls) {
   extern __shared__ __align__(16) unsigned char s_dyn[];
   ListShared& S = *reinterpret_cast<ListShared*>(s_dyn);
   unsigned* s_mask = reinterpret_cast<unsigned*>(s_dyn + sizeof(ListShared));   // [kTileCache][32], CMM: twice
   const unsigned full = 0xffffffffu;
-  const int bi = blockIdx.x, lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  const int bi = bi0 + blockIdx.x, lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
   const int ai = P.satom[bi * kTile + lane];
   // a block fills from its first slot: this one is not used by the present sort
   if (!__any_sync(full, ai >= 0)) {
@@ -767,15 +767,15 @@ void init_block_list() {
   cudaFuncSetAttribute(k_block_list<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)list_smem(true));
 }
 
-void launch_block_list(const DevPtrs& P, int nblk, int nsm, double rlim2, float rlimf, double rc2, bool cmm,
+void launch_block_list(const DevPtrs& P, int bi0, int nblk, int nsm, double rlim2, float rlimf, double rc2, bool cmm,
                        int dummy_type, bool count_only, bool keep, bool split_cls, cudaStream_t st) {
   // eight warps a block where the blocks alone do not fill the chip (each i-block's tiles in fewer
   // rounds), four where they do (64 replicas: 2,994 us a build with four, 3,287 with eight)
   const int nt = 32 * (nblk < 8 * nsm ? 8 : 4);
   if (cmm)
-    k_block_list<true><<<nblk, nt, list_smem(true), st>>>(P, rlim2, rlimf, rc2, dummy_type, count_only, keep, split_cls);
+    k_block_list<true><<<nblk, nt, list_smem(true), st>>>(P, bi0, rlim2, rlimf, rc2, dummy_type, count_only, keep, split_cls);
   else
-    k_block_list<false><<<nblk, nt, list_smem(false), st>>>(P, rlim2, rlimf, rc2, dummy_type, count_only, keep, split_cls);
+    k_block_list<false><<<nblk, nt, list_smem(false), st>>>(P, bi0, rlim2, rlimf, rc2, dummy_type, count_only, keep, split_cls);
 }
 
 // ---- deterministic exclusive scan (3 passes) --------------------------------------------

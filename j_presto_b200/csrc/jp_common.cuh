@@ -204,7 +204,7 @@ struct DevPtrs {
   float4 *blk_ctr, *blk_half;     // bbox (wrapped frame) centre / half extent
   double *blk_ref;                // [B][3]
   // pair list build: an i-block's tiles (its candidate j blocks that passed the bounding-box
-  // test) start at blk_tile0 in the arrays that hold one element per possible tile
+  // test) start at blk_tile0 in the arrays that hold one element per possible tile of a launch
   long long *blk_tile0;           // [nblk] (static)
   uint2 *blk_kind;                // the lanes of each block with an LJ term, with an ALSD cluster atom
   unsigned char *lj_free;         // types without an LJ term with any type

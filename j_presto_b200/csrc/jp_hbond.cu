@@ -113,8 +113,9 @@ static int hb_blocks(int cap) {
   return std::max(1, std::min((cap + kHbThreads - 1) / kHbThreads, 148 * 8));
 }
 
-void launch_hb_list(const DevPtrs& P, int cap, int nt1, int nblk, cudaStream_t st) {
-  cudaMemsetAsync(P.hb_n, 0, sizeof(int), st);
+// the marked pairs of the tiles listed last; first: of a list build's first part
+void launch_hb_list(const DevPtrs& P, int cap, int nt1, int nblk, bool first, cudaStream_t st) {
+  if (first) cudaMemsetAsync(P.hb_n, 0, sizeof(int), st);
   // eight warps a block, four blocks per block of atoms: about one warp per tile
   const int nb = std::max(1, std::min(nblk * 4, 148 * 8));
   k_hb_list<<<nb, kHbThreads, 0, st>>>(P, cap, nt1);

@@ -13,13 +13,13 @@ __global__ void k_scatter(DevPtrs P, int natom, int ncol);
 __global__ void k_fill_slots(DevPtrs P, int natom);
 constexpr int kSetupWarps = 8;   // warps of a thread block of k_block_setup
 __global__ void k_block_setup(DevPtrs P, int nblk, double qscale, int nsetup, int natom);
-// tiles and pair records of every i-block.  CMM: masks from the level-1 cells (neighbours:
+// tiles and pair records of i-blocks [bi0, bi0 + nblk).  CMM: masks from the level-1 cells (neighbours:
 // Coulomb + LJ into masks and masks_el; cells up to idelay apart and r^2 < rc2: LJ only) instead
 // of the list radius.  count_only: the records per unit alone; keep: masks left in global
 // memory and the tiles listed (for the H-bond list); split_cls: records with ALSD cluster atoms
 // apart (k_block_list).  init_block_list: once per context.
 void init_block_list();
-void launch_block_list(const DevPtrs& P, int nblk, int nsm, double rlim2, float rlimf, double rc2, bool cmm,
+void launch_block_list(const DevPtrs& P, int bi0, int nblk, int nsm, double rlim2, float rlimf, double rc2, bool cmm,
                        int dummy_type, bool count_only, bool keep, bool split_cls, cudaStream_t st);
 // deterministic exclusive scan of n ints (total: the sum, or null); returns the launches
 int scan_exclusive(const int* in, int* out, int n, int* scratch, int* total, cudaStream_t st);
@@ -58,7 +58,7 @@ void launch_update_pos(const DevPtrs& P, int natom, int nrep, bool fp64, double 
 
 // H-bond 10-12 pairs (jp_hbond.cu): their list at a rebuild (after the tile list), their
 // term at every force evaluation
-void launch_hb_list(const DevPtrs& P, int cap, int nt1, int nblk, cudaStream_t st);
+void launch_hb_list(const DevPtrs& P, int cap, int nt1, int nblk, bool first, cudaStream_t st);
 void launch_hbond(const DevPtrs& P, int cap, double rc2, int nt1, bool fp64, bool alsd, cudaStream_t st);
 
 // restraints and CAP boundary (jp_restraint.cu)
