@@ -198,8 +198,8 @@ __global__ void k_block_setup(DevPtrs P, int nblk, double qscale, int nsetup, in
 // without, and the same two, without first, of the entries that make a record take per-pair
 // images or ALSD classes.  The pair kernels leave the LJ term out over eight entries of a
 // warp's records that have none (in waters two thirds of the entries), and few records mix
-// the forms.  Pair kernel with entries in tile order and so: 64 replicas (883,000
-// atoms) 1,345 and 1,290 us, 99,200 atoms 181 and 166, 22,700 atoms 54 and 51.  With the LJ order alone
+// the forms.  Pair kernel (eight warps a block, an i atom's 32 terms in one sum) with entries
+// in tile order and so: 64 replicas (883,000 atoms) 1,345 and 1,290 us, 99,200 atoms 181 and 166, 22,700 atoms 54 and 51.  With the LJ order alone
 // the entries of image tiles, scattered over more records, cost 64 replicas more than it gave
 // (1,480 us).
 constexpr int kListWarps = 8;     // warps of a block, at most
@@ -769,9 +769,11 @@ void init_block_list() {
 
 void launch_block_list(const DevPtrs& P, int bi0, int nblk, int nsm, double rlim2, float rlimf, double rc2, bool cmm,
                        int dummy_type, bool count_only, bool keep, bool split_cls, cudaStream_t st) {
-  // eight warps a block where the blocks alone do not fill the chip (each i-block's tiles in fewer
-  // rounds), four where they do (64 replicas: 2,994 us a build with four, 3,287 with eight)
-  const int nt = 32 * (nblk < 8 * nsm ? 8 : 4);
+  // eight warps a block where the blocks fill the chip a few times at most (each i-block's tiles in
+  // fewer rounds), four where they fill it often and eight mostly wait for each other.  A build
+  // with eight and with four: 816 blocks 111 and 160 us, 1,482 blocks 162 and 184, 2,288 blocks
+  // 233 and 231, 3,383 blocks 343 and 330, 64 replicas (some 28,000 blocks) 2,447 and 2,310
+  const int nt = 32 * (nblk < 16 * nsm ? 8 : 4);
   if (cmm)
     k_block_list<true><<<nblk, nt, list_smem(true), st>>>(P, bi0, rlim2, rlimf, rc2, dummy_type, count_only, keep, split_cls);
   else

@@ -2453,8 +2453,8 @@ enum : int {
 };
 
 // blocks per SM the unit-lane launches are compiled for (their registers: 65,536 / (64 x this));
-// 64 chains take 264 us a step with 4, 262 with 6 and 265 with 8 (spills), 32 take 160, 160
-// and 170
+// 64 chains take 223 us a step with 4, 225 with 6 and 228 with 8 (spills), 32 take 118, 118
+// and 128
 constexpr int kPhaseBlocks = 4;
 
 // shared-memory state of the 4-atom group lanes of a launch (component 0-2)
