@@ -185,23 +185,22 @@ __global__ void k_block_setup(DevPtrs P, int nblk, double qscale, int nsetup, in
 // Pair record: a half block (16 i atoms: rows 0-15 or 16-31 of an i-block, unit u = 2 i-block +
 // half) with 32 j entries, the j atoms of that block's tiles that at least one of the 16 i
 // atoms lists, by kind (below) and in tile order (ascending j block, ascending slot).
-// A 32 x 32 tile of two
-// blocks holds ~26 % listed pairs at the md_run list radius; keeping only the j atoms a half
+// A 32 x 32 tile of two blocks holds ~26 % listed pairs at the md_run list radius; keeping only the j atoms a half
 // block lists raises that to ~55 %, because 16 atoms span a smaller volume than 32 (within the
 // cut-off: 32 % of the slots with whole blocks, 39 % with half blocks), and the pair kernels'
 // work per pair falls in proportion.  Each entry carries its tile's image shift (into the i
 // block's frame) and its atom, with the atom's type beside it; the mask of i atom l (0..15)
 // has bit k = entry (l + k) & 15 and bit 16 + k = entry 16 + ((l + k) & 15).
 
-// The four kinds of entries (0 .. 3), in their order in the first half of a block (in the second half the other
-// way round, so that a unit ends with the kind that the next one begins with): with an LJ term,
-// without, and the same two, without first, of the entries that make a record take per-pair
+// The four kinds of entries (0 .. 3), in their order in the first half of a block (in the second
+// half the other way round, so that a unit ends with the kind that the next one begins with): with
+// an LJ term, without, and the same two, without first, of the entries that make a record take per-pair
 // images or ALSD classes.  The pair kernels leave the LJ term out over eight entries of a
 // warp's records that have none (in waters two thirds of the entries), and few records mix
 // the forms.  Pair kernel (eight warps a block, an i atom's 32 terms in one sum) with entries
-// in tile order and so: 64 replicas (883,000 atoms) 1,345 and 1,290 us, 99,200 atoms 181 and 166, 22,700 atoms 54 and 51.  With the LJ order alone
-// the entries of image tiles, scattered over more records, cost 64 replicas more than it gave
-// (1,480 us).
+// in tile order and so: 64 replicas (883,000 atoms) 1,345 and 1,290 us, 99,200 atoms 181 and
+// 166, 22,700 atoms 54 and 51.  With the LJ order alone the entries of image tiles, scattered
+// over more records, cost 64 replicas more than it gave (1,480 us).
 constexpr int kListWarps = 8;     // warps of a block, at most
 constexpr int kTileListImg = 1 << 30, kTilePairImg = 1 << 29, kTileBlock = kTilePairImg - 1;   // BlkTile.j
 constexpr int kSegment = 512;     // candidate blocks tested at a time
@@ -415,15 +414,6 @@ __device__ __forceinline__ unsigned tile_row_f32(const Rep& R, float3 c, float4 
 // where tile c of i-block b keeps its mask rows and its record
 __device__ __forceinline__ BlkTile& blk_tile(const DevPtrs& P, ListShared& S, long long t0, int c) {
   return c < kTileCache ? S.tile[c] : P.blk_tiles[t0 + c];
-}
-
-// a record row (bit e: entry e) into the kernels' order for i atom l: each 16-bit half
-// rotated right by l
-__device__ __forceinline__ unsigned record_row(unsigned row, int l) {
-  const unsigned lo = row & 0xffffu, hi = row >> 16;
-  const unsigned rl = ((lo >> l) | (lo << (16 - l))) & 0xffffu;
-  const unsigned rh = ((hi >> l) | (hi << (16 - l))) & 0xffffu;
-  return rl | (rh << 16);
 }
 
 // 16 mask rows (64 bytes) of a half block's record slots: every slot contributes, per row, the

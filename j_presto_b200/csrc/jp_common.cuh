@@ -120,10 +120,40 @@ constexpr int kRegionShift = 28;
 
 // a type word in 16 bits, as the pair records carry it: type (below 4,096, far above the types
 // whose pair table fits shared memory), region code in bits 12-13, cluster in bit 14
-__device__ __forceinline__ unsigned short type_half(int t) {
+__host__ __device__ __forceinline__ unsigned short type_half(int t) {
   return (unsigned short)((t & 0xfff) | ((t >> 16) & 0x7000));
 }
-__device__ __forceinline__ int type_word(unsigned short h) { return (h & 0xfff) | ((h & 0x7000) << 16); }
+__host__ __device__ __forceinline__ int type_word(unsigned short h) { return (h & 0xfff) | ((h & 0x7000) << 16); }
+
+// ---- pair records: bit orders (jp_cells.cu, jp_pair.cu) ----
+// a record row (bit e: entry e) into the kernels' order for i atom l: each 16-bit half
+// rotated right by l
+__host__ __device__ __forceinline__ unsigned record_row(unsigned row, int l) {
+  const unsigned lo = row & 0xffffu, hi = row >> 16;
+  const unsigned rl = ((lo >> l) | (lo << (16 - l))) & 0xffffu;
+  const unsigned rh = ((hi >> l) | (hi << (16 - l))) & 0xffffu;
+  return rl | (rh << 16);
+}
+
+// a record's mask word of i atom r (entry halves rotated right by r, jp_cells.cu) in the
+// order of the kernels with two i atoms a lane: bit 8 g + k is entry 8 g + ((l + k) & 7), l = r & 7
+__host__ __device__ __forceinline__ unsigned byte_rotr(unsigned row, int l) {
+  const unsigned m = (0xffu >> l) * 0x01010101u;
+  return ((row >> l) & m) | ((row << (8 - l)) & ~m);
+}
+
+__host__ __device__ __forceinline__ unsigned step_mask(unsigned w, int r) {
+  const unsigned lo = (w & 0xffffu) | (w << 16), hi = (w >> 16) | (w & 0xffff0000u);
+  return byte_rotr(((lo << r) >> 16) | ((hi << r) & 0xffff0000u), r & 7);
+}
+
+// Householder's third-order step y + y e (1/2 + 3/8 e), e = 1 - x y^2, towards 1/sqrt(x): its error is
+// 5/16 e^3 and the roundings of e (half) and of the result, 1.52 x 2^-53 in all from a y within
+// 2^-20
+__host__ __device__ __forceinline__ double rsqrt_step(double x, double y) {
+  const double e = fma(-(x * y), y, 1.0);
+  return fma(y * e, fma(e, 0.375, 0.5), y);
+}
 
 // integration unit: a SHAKE group (2-4 atoms) or a lone atom (n = 1)
 struct Unit {
