@@ -68,7 +68,7 @@ struct jp_ctx {
   double qscale = 1.0;
   bool fp64 = false;
   bool minimg = true;
-  int pair_warps = 0;
+  int pair_blocks = 0;
   int nsm = 148;                    // the device's SM count
   bool alsd = false;                // some replica has ALSD classes (lambda)
   bool split = false;               // some replica keeps partial-McMD class-1 forces apart
@@ -227,8 +227,8 @@ void enqueue_zero(jp_ctx *c, bool count) {
 // the non-bonded forces: pair tiles, and with CMM the far field (recomputed every CMMUPD
 // steps by the step counter, or always with force_far: a single-point evaluation)
 void enqueue_pair(jp_ctx *c, bool count, bool force_far = false) {
-  if (c->fp64) launch_pair_fp64(c->P, c->zc, c->pair_warps, count, c->alsd, c->split, c->st);
-  else launch_pair_mixed(c->P, c->zc, c->pair_warps, count, c->alsd, c->every_cls, c->split, c->st);
+  if (c->fp64) launch_pair_fp64(c->P, c->zc, c->pair_blocks, count, c->alsd, c->split, c->st);
+  else launch_pair_mixed(c->P, c->zc, c->pair_blocks, count, c->alsd, c->every_cls, c->split, c->st);
   if (c->hbond) launch_hbond(c->P, c->hb_cap, c->zc.rc2, c->zc.nt1, c->fp64, c->classes, c->st);
   if (c->cmm) launch_cmm_far(c->P, c->natom, c->nrep, c->fp64, force_far, c->qscale * c->qscale, c->st);
 }
@@ -1788,7 +1788,7 @@ int jp_create(const jp_system *sys, int32_t nrep, const jp_params *prm, jp_ctx *
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, c->device);
   c->nsm = std::max(1, nsm);
   // one wave: every warp resident at once, each with an equal share of the tiles
-  c->pair_warps = std::max(1, nsm) * kPairWarps * pair_blocks_per_sm(c->fp64, !c->split && !c->cmm && !(c->fp64 && c->alsd), c->zc.nt1);
+  c->pair_blocks = c->nsm * pair_blocks_per_sm(c->fp64, !c->split && !c->cmm && !(c->fp64 && c->alsd), c->zc.nt1);
   c->cano_grid = cano_grid(c->fp64, c->device);
   CK(cudaStreamCreateWithFlags(&c->st, cudaStreamNonBlocking));
   CK(cudaStreamCreateWithFlags(&c->st2, cudaStreamNonBlocking));

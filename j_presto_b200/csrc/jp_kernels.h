@@ -40,13 +40,12 @@ void launch_cmm_far(const DevPtrs& P, int natom, int nrep, bool fp64, bool force
                     cudaStream_t st);
 
 // pair kernels (jp_pair.cu)
-constexpr int kPairWarps = 6;    // warps of a thread block
 // alsd: some replica has ALSD classes (every_cls: class weights that are not lambda's, so the
 // records without cluster atoms are weighted too); split: some replica keeps partial-McMD class-1 forces
 // apart (frc1 / grd1)
-void launch_pair_mixed(const DevPtrs& P, const ZdConst& z, int nwarps, bool count, bool alsd, bool every_cls,
+void launch_pair_mixed(const DevPtrs& P, const ZdConst& z, int nblocks, bool count, bool alsd, bool every_cls,
                        bool split, cudaStream_t st);
-void launch_pair_fp64(const DevPtrs& P, const ZdConst& z, int nwarps, bool count, bool alsd, bool split,
+void launch_pair_fp64(const DevPtrs& P, const ZdConst& z, int nblocks, bool count, bool alsd, bool split,
                       cudaStream_t st);
 // co-resident blocks per SM of the (non-counting) pair kernel: the grid is one full wave
 // (packed: the kernels with two i atoms a lane -- the mixed path without CMM and partial McMD, the

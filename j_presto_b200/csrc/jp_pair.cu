@@ -38,8 +38,10 @@ namespace jp {
 
 // Six warps a block, two blocks an SM: 168 registers a thread, which the packed kernel's sums
 // need.  With eight warps (128 registers) they spilled: 64 replicas (883,000 atoms) 1,390 us, so
-// 1,307, 99,200 atoms 174 and 163, 2,200 atoms 21 and 17.
-constexpr int kPairThreads = 32 * kPairWarps;
+// 1,307, 99,200 atoms 174 and 163, 2,200 atoms 21 and 17.  The FP64 kernels keep eight (ALSD
+// replicas of 36,500 atoms 255 us, with six 289; 270,000 atoms 673 and 696).
+constexpr int kPairWarps = 6, kPairThreads = 32 * kPairWarps;
+constexpr int kFp64Warps = 8, kFp64Threads = 32 * kFp64Warps;
 constexpr long long kCopyWaitCycles = 2000000000LL;
 
 // ---- bulk copies into shared memory (TMA engine, no tensor map) -------------------------
@@ -159,11 +161,11 @@ __device__ __forceinline__ float rint1(float v) {
 // same two addresses, and L2 takes atomics on one address one after the other: with one pair
 // of them per lane group (19,000 atomics) a launch on 24,000 atoms took 59.1 us, so 52.0.
 // Called by all threads of the block.
-template <int W>
+template <int W, int WARPS>
 __device__ __forceinline__ void flush_block(const DevPtrs& P, int rep, long long eel, long long elj, long long eaa,
                                             long long eab, long long npair, bool count, bool cls) {
-  __shared__ long long s_sum[kPairWarps][5];
-  __shared__ int s_rep[kPairWarps];
+  __shared__ long long s_sum[WARPS][5];
+  __shared__ int s_rep[WARPS];
   const unsigned full = 0xffffffffu;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   int r = __reduce_max_sync(full, rep);
@@ -190,11 +192,11 @@ __device__ __forceinline__ void flush_block(const DevPtrs& P, int rep, long long
   }
   __syncthreads();
   if (threadIdx.x == 0) {
-    for (int w = 0; w < kPairWarps; ++w) {
+    for (int w = 0; w < WARPS; ++w) {
       const int rw = s_rep[w];
       if (rw < 0) continue;
       long long a = 0, b = 0, n = 0, ca = 0, cb = 0;   // the warps of this replica, taken together
-      for (int v = w; v < kPairWarps; ++v)
+      for (int v = w; v < WARPS; ++v)
         if (s_rep[v] == rw) {
           a += s_sum[v][0];
           b += s_sum[v][1];
@@ -681,7 +683,7 @@ __global__ void __launch_bounds__(kPairThreads, CLS ? 1 : 2) k_pair_packed(DevPt
     b ^= 1;
   }
   flush_i();
-  flush_block<8>(P, cur_rep, eel, elj, eaa, eab, npair, COUNT, CLS || cls_sum);
+  flush_block<8, kPairWarps>(P, cur_rep, eel, elj, eaa, eab, npair, COUNT, CLS || cls_sum);
   // a copy still in flight (only after a timed-out wait) must land before the block exits
   for (int k = 0; k < 2; ++k)
     if ((pend >> k) & 1u) mbar_wait(&S.bar[k], (phase >> k) & 1u, wlim);
@@ -1150,11 +1152,11 @@ __device__ __forceinline__ void record_fp64(const DevPtrs& P, const QuadStageD& 
 }
 
 template <bool COUNT>
-__global__ void __launch_bounds__(kPairThreads, 2) k_pair_fp64q(DevPtrs P, ZdConst z) {
+__global__ void __launch_bounds__(kFp64Threads, 2) k_pair_fp64q(DevPtrs P, ZdConst z) {
   extern __shared__ __align__(16) unsigned char s_dynd[];
   const unsigned full = 0xffffffffu;
   QuadStageD& S = reinterpret_cast<QuadStageD*>(s_dynd)[threadIdx.x >> 5];
-  double2* s_lj = reinterpret_cast<double2*>(s_dynd + sizeof(QuadStageD) * kPairWarps);
+  double2* s_lj = reinterpret_cast<double2*>(s_dynd + sizeof(QuadStageD) * kFp64Warps);
   for (int i = threadIdx.x; i < z.nt1 * z.nt1; i += blockDim.x) {
     const double2 c = P.lj_d[i];
     s_lj[i] = make_double2(-6.0 * c.x, 12.0 * c.y);
@@ -1166,7 +1168,7 @@ __global__ void __launch_bounds__(kPairThreads, 2) k_pair_fp64q(DevPtrs P, ZdCon
   const int T = P.nctiles[0];
   const bool ext = *P.ext_pos != 0;
   const int TU = (T + 3) >> 2;
-  const int gw = blockIdx.x * kPairWarps + (threadIdx.x >> 5), nw = gridDim.x * kPairWarps;
+  const int gw = blockIdx.x * kFp64Warps + (threadIdx.x >> 5), nw = gridDim.x * kFp64Warps;
   int cur_unit = -2, cur_rep = -1, rep = -1, aia = -1, aib = -1, tia = z.nt1 - 1, tib = tia;
   double xa[4] = {0, 0, 0, 0}, xb[4] = {0, 0, 0, 0}, fa[3] = {0, 0, 0}, fb[3] = {0, 0, 0};
   double box[3] = {0, 0, 0}, inv[3] = {0, 0, 0}, ref[3] = {0, 0, 0};
@@ -1265,7 +1267,7 @@ __global__ void __launch_bounds__(kPairThreads, 2) k_pair_fp64q(DevPtrs P, ZdCon
     }
   }
   flush_i();
-  flush_block<8>(P, cur_rep, eel, elj, 0, 0, npair, COUNT, false);
+  flush_block<8, kFp64Warps>(P, cur_rep, eel, elj, 0, 0, npair, COUNT, false);
 }
 
 // Per-warp shared memory of k_pair_fp64 (classes, CMM): each half-warp's record, entries a and b
@@ -1276,10 +1278,10 @@ struct __align__(16) F64Stage {
 };
 
 template <bool COUNT, bool ALSD, bool CMM, bool SPLIT = false>
-__global__ void __launch_bounds__(kPairThreads)
+__global__ void __launch_bounds__(kFp64Threads)
 k_pair_fp64(DevPtrs P, ZdConst z) {
   extern __shared__ double2 s_ljd[];
-  __shared__ F64Stage s_stage[kPairWarps];
+  __shared__ F64Stage s_stage[kFp64Warps];
   const unsigned full = 0xffffffffu;
   const int nlj = z.nt1 * z.nt1;
   for (int i = threadIdx.x; i < nlj; i += blockDim.x) s_ljd[i] = P.lj_d[i];
@@ -1458,7 +1460,7 @@ k_pair_fp64(DevPtrs P, ZdConst z) {
 // fewer types created later lowered it below what an earlier context launches with.
 // Resident blocks of the kernel an SM, 0 if `bytes` do not fit.
 template <class Kernel>
-static int raise_smem_limit(Kernel kernel, int bytes) {
+static int raise_smem_limit(Kernel kernel, int threads, int bytes) {
   int dev = 0, optin = 0, per = 0;
   cudaFuncAttributes fa{};
   if (cudaGetDevice(&dev) != cudaSuccess ||
@@ -1468,17 +1470,17 @@ static int raise_smem_limit(Kernel kernel, int bytes) {
   const int limit = optin - (int)fa.sharedSizeBytes;
   if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, limit) != cudaSuccess) return 0;
   if (bytes > limit ||
-      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kernel, kPairThreads, bytes) != cudaSuccess)
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kernel, threads, bytes) != cudaSuccess)
     return 0;
   return per;
 }
 
 template <bool TRI>
 static int packed_blocks_per_sm(int bytes) {
-  const int per = raise_smem_limit(k_pair_packed<false, false, TRI>, bytes);
-  raise_smem_limit(k_pair_packed<true, false, TRI>, bytes);
-  raise_smem_limit(k_pair_packed<false, true, TRI>, bytes);
-  raise_smem_limit(k_pair_packed<true, true, TRI>, bytes);
+  const int per = raise_smem_limit(k_pair_packed<false, false, TRI>, kPairThreads, bytes);
+  raise_smem_limit(k_pair_packed<true, false, TRI>, kPairThreads, bytes);
+  raise_smem_limit(k_pair_packed<false, true, TRI>, kPairThreads, bytes);
+  raise_smem_limit(k_pair_packed<true, true, TRI>, kPairThreads, bytes);
   return per;
 }
 
@@ -1505,16 +1507,16 @@ void pack_lj_table(const float2* lj, int nt1, std::vector<float>& out) {
       }
 }
 
-static size_t fp64q_bytes(int nt1) { return sizeof(QuadStageD) * kPairWarps + sizeof(double2) * nt1 * nt1; }
+static size_t fp64q_bytes(int nt1) { return sizeof(QuadStageD) * kFp64Warps + sizeof(double2) * nt1 * nt1; }
 
 int pair_blocks_per_sm(bool fp64, bool packed, int nt1) {
   int per = 0;
   if (fp64 && packed) {
     const int bytes = (int)fp64q_bytes(nt1);
-    per = raise_smem_limit(k_pair_fp64q<false>, bytes);
-    raise_smem_limit(k_pair_fp64q<true>, bytes);
+    per = raise_smem_limit(k_pair_fp64q<false>, kFp64Threads, bytes);
+    raise_smem_limit(k_pair_fp64q<true>, kFp64Threads, bytes);
   } else if (fp64) {
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_pair_fp64<false, true, false>, kPairThreads,
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_pair_fp64<false, true, false>, kFp64Threads,
                                                   sizeof(double2) * nt1 * nt1);
   } else if (packed) {
     const int bytes = (int)(kPackedStageBytes + lj_bytes(nt1));
@@ -1544,29 +1546,27 @@ static void launch_mixed(const DevPtrs& P, const ZdConst& z, int nb, bool alsd, 
   }
 }
 
-void launch_pair_mixed(const DevPtrs& P, const ZdConst& z, int nwarps, bool count, bool alsd, bool every_cls,
+void launch_pair_mixed(const DevPtrs& P, const ZdConst& z, int nb, bool count, bool alsd, bool every_cls,
                        bool split, cudaStream_t st) {
-  const int nb = (nwarps + kPairWarps - 1) / kPairWarps;
   if (count) launch_mixed<true>(P, z, nb, alsd, every_cls, split, st);
   else launch_mixed<false>(P, z, nb, alsd, every_cls, split, st);
 }
 
-void launch_pair_fp64(const DevPtrs& P, const ZdConst& z, int nwarps, bool count, bool alsd, bool split,
+void launch_pair_fp64(const DevPtrs& P, const ZdConst& z, int nb, bool count, bool alsd, bool split,
                       cudaStream_t st) {
-  const int nb = (nwarps + kPairWarps - 1) / kPairWarps;
   const size_t sh = sizeof(double2) * z.nt1 * z.nt1;
   if (split) {
-    if (count) k_pair_fp64<true, true, false, true><<<nb, kPairThreads, sh, st>>>(P, z);
-    else k_pair_fp64<false, true, false, true><<<nb, kPairThreads, sh, st>>>(P, z);
+    if (count) k_pair_fp64<true, true, false, true><<<nb, kFp64Threads, sh, st>>>(P, z);
+    else k_pair_fp64<false, true, false, true><<<nb, kFp64Threads, sh, st>>>(P, z);
   } else if (z.cmm) {
-    if (count) k_pair_fp64<true, false, true><<<nb, kPairThreads, sh, st>>>(P, z);
-    else k_pair_fp64<false, false, true><<<nb, kPairThreads, sh, st>>>(P, z);
+    if (count) k_pair_fp64<true, false, true><<<nb, kFp64Threads, sh, st>>>(P, z);
+    else k_pair_fp64<false, false, true><<<nb, kFp64Threads, sh, st>>>(P, z);
   } else if (alsd) {
-    if (count) k_pair_fp64<true, true, false><<<nb, kPairThreads, sh, st>>>(P, z);
-    else k_pair_fp64<false, true, false><<<nb, kPairThreads, sh, st>>>(P, z);
+    if (count) k_pair_fp64<true, true, false><<<nb, kFp64Threads, sh, st>>>(P, z);
+    else k_pair_fp64<false, true, false><<<nb, kFp64Threads, sh, st>>>(P, z);
   } else {
-    if (count) k_pair_fp64q<true><<<nb, kPairThreads, fp64q_bytes(z.nt1), st>>>(P, z);
-    else k_pair_fp64q<false><<<nb, kPairThreads, fp64q_bytes(z.nt1), st>>>(P, z);
+    if (count) k_pair_fp64q<true><<<nb, kFp64Threads, fp64q_bytes(z.nt1), st>>>(P, z);
+    else k_pair_fp64q<false><<<nb, kFp64Threads, fp64q_bytes(z.nt1), st>>>(P, z);
   }
 }
 
