@@ -204,7 +204,7 @@ void enqueue_rebuild(jp_ctx *c, bool count_only = false) {
     const int b0 = c->list_part[q], nb = c->list_part[q + 1] - b0;
     if (q > 0 && c->hbond) cudaMemsetAsync(P.ntiles, 0, sizeof(int), st);
     launch_block_list(P, b0, nb, c->nsm, rlim * rlim, (float)rlim, rc * rc, c->cmm, c->zc.nt1 - 1, count_only,
-                      c->hbond, c->alsd && !c->fp64, st);
+                      c->hbond, c->fp64 || c->cmm || c->split ? kApartNone : c->alsd ? kApartCls : kApartImg, st);
     if (c->hbond && !count_only) launch_hb_list(P, c->hb_cap, c->zc.nt1, nb, q == 0, st);
   }
   if (count_only) return;

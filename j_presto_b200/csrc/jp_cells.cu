@@ -226,7 +226,7 @@ struct __align__(16) ListShared {
   unsigned excl[kSegment / 32];            // blocks that hold an exclusion partner
   int carry[8];                            // entries by half and kind
   int first[2][4];                         // a half's first entry of each kind
-  int base;
+  int base[2];                             // of the records at the start and at the end
   // ALSD: which of a window's records hold a class but BB, and each one's place
   unsigned char rcls[2 * kWindow];
   size_t rpos[2 * kWindow];
@@ -444,7 +444,7 @@ __device__ __forceinline__ unsigned record_rows(const unsigned* rows, bool live,
 template <bool CMM>
 __global__ void __launch_bounds__(32 * kListWarps, CMM ? 3 : 4) k_block_list(DevPtrs P, int bi0, double rlim2, float rlimf,
                                                                              double rc2, int dummy_type, int count_only,
-                                                                             int keep, int split_cls) {
+                                                                             int keep, int apart) {
   extern __shared__ __align__(16) unsigned char s_dyn[];
   ListShared& S = *reinterpret_cast<ListShared*>(s_dyn);
   unsigned* s_mask = reinterpret_cast<unsigned*>(s_dyn + sizeof(ListShared));   // [kTileCache][32], CMM: twice
@@ -649,9 +649,19 @@ __global__ void __launch_bounds__(32 * kListWarps, CMM ? 3 : 4) k_block_list(Dev
   if (threadIdx.x == 0) {
     P.ct_cnt[2 * bi] = nr0;
     P.ct_cnt[2 * bi + 1] = nr1;
-    if (!count_only && !split_cls) S.base = atomicAdd(P.nctiles, nr0 + nr1);
   }
   if (count_only) return;
+  const bool split_cls = apart == kApartCls;
+  // records of each half at the array's end (kApartImg)
+  int na0 = 0, na1 = 0;
+  if (apart == kApartImg) {
+    na0 = S.carry[2] + S.carry[3] > 0 ? nr0 - ((S.carry[0] + S.carry[1]) >> 5) : 0;
+    na1 = (S.carry[6] + S.carry[7] + 31) >> 5;
+  }
+  if (threadIdx.x < 2 && !split_cls) {
+    const int na = na0 + na1;
+    S.base[threadIdx.x] = atomicAdd(&P.nctiles[threadIdx.x], threadIdx.x ? na : nr0 + nr1 - na);
+  }
 
   const bool wide = nt > kNarrowTiles;
   const int win = wide ? kWindow / 2 : kWindow;
@@ -717,7 +727,14 @@ __global__ void __launch_bounds__(32 * kListWarps, CMM ? 3 : 4) k_block_list(Dev
     }
     for (int q = w; q < m0 + m1; q += nw) {
       const int h = q < m0 ? 0 : 1, r = q < m0 ? q : q - m0;   // record r of the window of half h
-      const size_t ct = split_cls ? S.rpos[q] : (size_t)S.base + (h ? nr0 : 0) + w0 + r;
+      size_t ct;
+      if (split_cls) ct = S.rpos[q];
+      else if (h == 0)
+        ct = w0 + r < nr0 - na0 ? (size_t)(S.base[0] + w0 + r)
+                                : P.rec_cap - 1 - (size_t)(S.base[1] + w0 + r - (nr0 - na0));
+      else
+        ct = w0 + r < na1 ? P.rec_cap - 1 - (size_t)(S.base[1] + na0 + w0 + r)
+                          : (size_t)(S.base[0] + nr0 - na0 + w0 + r - na1);
       const bool live = 32 * (w0 + r) + lane < E[h];
       const unsigned v = live ? entry(h, 32 * r + lane) : 0u;
       const int c = (int)(v >> 5), jl = (int)(v & 31u);
@@ -758,16 +775,16 @@ void init_block_list() {
 }
 
 void launch_block_list(const DevPtrs& P, int bi0, int nblk, int nsm, double rlim2, float rlimf, double rc2, bool cmm,
-                       int dummy_type, bool count_only, bool keep, bool split_cls, cudaStream_t st) {
+                       int dummy_type, bool count_only, bool keep, int apart, cudaStream_t st) {
   // eight warps a block where the blocks fill the chip a few times at most (each i-block's tiles in
   // fewer rounds), four where they fill it often and eight mostly wait for each other.  A build
   // with eight and with four: 816 blocks 111 and 160 us, 1,482 blocks 162 and 184, 2,288 blocks
   // 233 and 231, 3,383 blocks 343 and 330, 64 replicas (some 28,000 blocks) 2,447 and 2,310
   const int nt = 32 * (nblk < 16 * nsm ? 8 : 4);
   if (cmm)
-    k_block_list<true><<<nblk, nt, list_smem(true), st>>>(P, bi0, rlim2, rlimf, rc2, dummy_type, count_only, keep, split_cls);
+    k_block_list<true><<<nblk, nt, list_smem(true), st>>>(P, bi0, rlim2, rlimf, rc2, dummy_type, count_only, keep, apart);
   else
-    k_block_list<false><<<nblk, nt, list_smem(false), st>>>(P, bi0, rlim2, rlimf, rc2, dummy_type, count_only, keep, split_cls);
+    k_block_list<false><<<nblk, nt, list_smem(false), st>>>(P, bi0, rlim2, rlimf, rc2, dummy_type, count_only, keep, apart);
 }
 
 // ---- deterministic exclusive scan (3 passes) --------------------------------------------

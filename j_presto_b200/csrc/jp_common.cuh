@@ -252,7 +252,7 @@ struct DevPtrs {
   float4 *ct_j;                   // [CT][32] (image shift into the i frame, atom bits; -1 = empty)
   unsigned short *ct_ty;          // [CT][32] type word of each entry (type_half; empty: dummy type)
   unsigned *ct_mask, *ct_mask_el; // [CT][32] rotated masks (listed pairs; CMM Coulomb pairs)
-  int *nctiles;                   // records from the start of the arrays, and (ALSD, mixed) from their end
+  int *nctiles;                   // records from the start of the arrays, and (packed kernel) from their end
   size_t rec_cap;                 // length of the record arrays
   // cell sort
   unsigned *key;                  // per atom

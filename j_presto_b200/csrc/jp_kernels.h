@@ -16,11 +16,12 @@ __global__ void k_block_setup(DevPtrs P, int nblk, double qscale, int nsetup, in
 // tiles and pair records of i-blocks [bi0, bi0 + nblk).  CMM: masks from the level-1 cells (neighbours:
 // Coulomb + LJ into masks and masks_el; cells up to idelay apart and r^2 < rc2: LJ only) instead
 // of the list radius.  count_only: the records per unit alone; keep: masks left in global
-// memory and the tiles listed (for the H-bond list); split_cls: records with ALSD cluster atoms
-// apart (k_block_list).  init_block_list: once per context.
+// memory and the tiles listed (for the H-bond list); apart: which records go to the end of the
+// arrays (k_block_list).  init_block_list: once per context.
+enum : int { kApartNone = 0, kApartCls = 1, kApartImg = 2 };
 void init_block_list();
 void launch_block_list(const DevPtrs& P, int bi0, int nblk, int nsm, double rlim2, float rlimf, double rc2, bool cmm,
-                       int dummy_type, bool count_only, bool keep, bool split_cls, cudaStream_t st);
+                       int dummy_type, bool count_only, bool keep, int apart, cudaStream_t st);
 // deterministic exclusive scan of n ints (total: the sum, or null); returns the launches
 int scan_exclusive(const int* in, int* out, int n, int* scratch, int* total, cudaStream_t st);
 

@@ -459,10 +459,14 @@ __host__ __device__ constexpr size_t lj_bytes(int nt1) {
 }
 constexpr size_t kPackedStageBytes = sizeof(QuadStage) * kPairWarps;
 
-// CLS: every record with class weights and energies, from the sequence at the arrays' end
-// (seq = 1) or the one at their start; without it cls_sum adds the energies to class BB
+// CLS: every record with class weights and energies; without it cls_sum adds the energies to class
+// BB.  which: the records at the start of the arrays (1), at their end (2), or both (3), those at
+// the end first.  Without classes these are the records whose pairs take their own images: the
+// two image forms' code does not fit the instruction cache together, and with both kinds of
+// records in turn 200 replicas in boxes of 28 A took 1,134 us, 20 in boxes of 39 A 275; with one
+// kind after the other 697 and 210.
 template <bool COUNT, bool CLS, bool TRI>
-__global__ void __launch_bounds__(kPairThreads, CLS ? 1 : 2) k_pair_packed(DevPtrs P, ZdConst z, int seq, int cls_sum) {
+__global__ void __launch_bounds__(kPairThreads, CLS ? 1 : 2) k_pair_packed(DevPtrs P, ZdConst z, int which, int cls_sum) {
   extern __shared__ __align__(16) unsigned char s_dyn[];
   __shared__ unsigned long long s_tab_bar;
   const unsigned full = 0xffffffffu;
@@ -485,11 +489,13 @@ __global__ void __launch_bounds__(kPairThreads, CLS ? 1 : 2) k_pair_packed(DevPt
     bulk_load(s_dyn + kPackedStageBytes, P.lj_tab, (unsigned)lj_bytes(z.nt1), &s_tab_bar);
   }
   __syncthreads();
-  const int T = P.nctiles[seq];     // records
-  // record of lane group qd in group t, and the first record of the group's copies
-  auto rec0 = [&](int t) { return seq ? P.rec_cap - 4 * (size_t)(t + 1) : 4 * (size_t)t; };
+  // records at the arrays' start and end; the record groups at the end come first, downwards
+  const int T0 = which & 1 ? P.nctiles[0] : 0, T1 = which & 2 ? P.nctiles[1] : 0;
+  const int U1 = (T1 + 3) >> 2;
+  // the first record of group t's copies
+  auto rec0 = [&](int t) { return t < U1 ? P.rec_cap - 4 * (size_t)(t + 1) : 4 * (size_t)(t - U1); };
   const bool ext = (*P.ext_pos & kExtImg) != 0;
-  const int TU = (T + 3) >> 2;      // record groups: a warp's work units
+  const int TU = U1 + ((T0 + 3) >> 2);   // record groups: a warp's work units
   // a 2.5-KiB copy lands in microseconds; the bound (about a second of SM clock) only ends
   // the wait on a broken device, and it is not the integrator's adjustable barrier bound:
   // a block must never leave with one of its copies still in flight
@@ -508,7 +514,7 @@ __global__ void __launch_bounds__(kPairThreads, CLS ? 1 : 2) k_pair_packed(DevPt
     if (run_next >= run_end) {
       if (nw * run >= TU) return TU;
       int t = 0;
-      if (lane == 0) t = atomicAdd(&P.tile_ctr[seq], run);
+      if (lane == 0) t = atomicAdd(&P.tile_ctr[which == 2 ? 1 : 0], run);
       t = __shfl_sync(full, t, 0) + nw * run;
       run_next = t;
       run_end = min(t + run, TU);
@@ -537,7 +543,7 @@ __global__ void __launch_bounds__(kPairThreads, CLS ? 1 : 2) k_pair_packed(DevPt
     }
     phase ^= 1u << b;
     pend &= ~(1u << b);
-    const bool valid = 4 * t + (seq ? 3 - qd : qd) < T;   // the sequence at the end runs downwards
+    const bool valid = t < U1 ? 4 * t + 3 - qd < T1 : 4 * (t - U1) + qd < T0;
     G.unit = valid ? P.ct_blk[rec0(t) + qd] : -1;
 #pragma unroll
     for (int g = 0; g < 4; ++g) {
@@ -1541,8 +1547,8 @@ static void launch_mixed(const DevPtrs& P, const ZdConst& z, int nb, bool alsd, 
     // the records with cluster atoms, and under every_cls the others too, by class
     auto plain = tri ? k_pair_packed<COUNT, false, true> : k_pair_packed<COUNT, false, false>;
     auto cls = tri ? k_pair_packed<COUNT, true, true> : k_pair_packed<COUNT, true, false>;
-    if (alsd) cls<<<nb, kPairThreads, shp, st>>>(P, z, 1, 0);
-    (every_cls ? cls : plain)<<<nb, kPairThreads, shp, st>>>(P, z, 0, alsd ? 1 : 0);
+    if (alsd) cls<<<nb, kPairThreads, shp, st>>>(P, z, 2, 0);
+    (every_cls ? cls : plain)<<<nb, kPairThreads, shp, st>>>(P, z, alsd ? 1 : 3, alsd ? 1 : 0);
   }
 }
 
