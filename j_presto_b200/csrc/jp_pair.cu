@@ -570,6 +570,23 @@ __global__ void __launch_bounds__(kPairThreads, CLS ? 1 : 2) k_pair_packed(DevPt
       for (int k = 0; k < 3; ++k) atomic_add_ll(&P.frc[3 * aib + k], gib[k]);
     for (int k = 0; k < 3; ++k) gia[k] = gib[k] = 0;
   };
+  // Where a warp's runs are short, a unit's records go to many warps and all add to the same i
+  // atoms at once: the four lane groups' sums are then added first if they are of one unit
+  // (called by all lanes; mine: the lane's unit ends).  9,300 atoms inside their cut-off 137 us
+  // without and 97 with it, 48,000 atoms 97 and 90; with longer runs it costs (64 replicas 1,310
+  // and 1,323 us).
+  const bool merge = run <= 2;
+  auto merge_i = [&](bool mine) {
+    const int u0 = __shfl_sync(full, cur_unit, 0);   // by every lane, whatever its `mine`
+    if (!__all_sync(full, mine && cur_unit == u0)) return;
+    for (int o = 8; o < 32; o <<= 1)
+      for (int k = 0; k < 3; ++k) {
+        gia[k] += __shfl_xor_sync(full, gia[k], o);
+        gib[k] += __shfl_xor_sync(full, gib[k], o);
+      }
+    if (qd != 0)
+      for (int k = 0; k < 3; ++k) gia[k] = gib[k] = 0;
+  };
 
   int t = claim(), tn = TU;
   Gather4 G;
@@ -606,6 +623,7 @@ __global__ void __launch_bounds__(kPairThreads, CLS ? 1 : 2) k_pair_packed(DevPt
     A.ma = unit >= 0 ? step_mask(S.msk[b][16 * qd + lp], lp) : 0u;
     A.mb = unit >= 0 ? step_mask(S.msk[b][16 * qd + 8 + lp], lp + 8) : 0u;
     // the lane's i atoms: a new unit flushes the last one's forces and loads the new atoms
+    if (merge && __any_sync(full, unit != cur_unit)) merge_i(unit != cur_unit);
     if (unit != cur_unit) {
       flush_i();
       cur_unit = unit;
@@ -688,6 +706,7 @@ __global__ void __launch_bounds__(kPairThreads, CLS ? 1 : 2) k_pair_packed(DevPt
     tn = t2;
     b ^= 1;
   }
+  if (merge) merge_i(true);
   flush_i();
   flush_block<8, kPairWarps>(P, cur_rep, eel, elj, eaa, eab, npair, COUNT, CLS || cls_sum);
   // a copy still in flight (only after a timed-out wait) must land before the block exits
