@@ -306,7 +306,8 @@ struct PackedArgs {
 // forces' error against FP64 (RMS, relative, mean of 27 systems of 2,100 to 15,300 atoms) is
 // 1.016e-6; 1.018e-6 with one i atom a lane and 16 terms a sum, 1.023e-6 with eight terms in a
 // row, 1.043e-6 with those groups added in FP32 (64 replicas 1,365 us, 99,200 atoms 171, 22,700
-// atoms 52; in this form 1,307, 163 and 50).
+// atoms 52; in this form 1,307, 163 and 50).  58 % of the issue slots and 65 % of that pipe are
+// busy, the FMA pipe 42 %.
 // Half or quarter groups as work units of small lists measured slower (the per-record work).
 template <bool MINIMG, bool COUNT, bool TRI, bool CLS, bool LJ>
 __device__ __forceinline__ void group_packed(const DevPtrs& P, const QuadStage& S, const float2* __restrict__ s_lj,
