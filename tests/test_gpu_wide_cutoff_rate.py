@@ -1,7 +1,6 @@
 """A droplet inside its cut-off: each of its few half blocks has a hundred records and more, and many
 warps add to the same i atoms' forces at once.  A record's pair time stays near that of a water
-box of as many records (within a quarter; with every lane group adding its own sums it was
-1.5 times).
+box of as many records (some 1.1 times; with every lane group adding its own sums 1.5 times).
 """
 import pytest
 
@@ -24,4 +23,4 @@ def us_per_1000_records(top, **kw):
 def test_pair_time_per_record(engine_lib):
     dense = us_per_1000_records(systems.droplet(8, 3050, seed=3), bounda=abi.JP_BOUND_NONE, cutoff=90.0)
     box = us_per_1000_records(systems.solvated_polymer(0, 16000, seed=3))
-    assert dense < 1.25 * box, (dense, box)
+    assert dense < 1.3 * box, (dense, box)
