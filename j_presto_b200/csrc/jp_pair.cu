@@ -90,6 +90,12 @@ __device__ __forceinline__ bool mbar_wait(unsigned long long* bar, unsigned pari
   }
 }
 
+// the same for a whole warp, one answer: after a wait that ran out in some lanes alone these would
+// leave the loop, and the others would wait for them in its next warp collective without end
+__device__ __forceinline__ bool mbar_wait_warp(unsigned long long* bar, unsigned parity, long long limit) {
+  return __all_sync(0xffffffffu, mbar_wait(bar, parity, limit));
+}
+
 // each lane group's energies (ELE15, VDW15; ALSD class AA / AB, BB the rest) and pair count
 // into the slots of its replica: 64-bit fixed point, summed per record, so the totals do not
 // depend on which warp took which record (the kernels claim their records dynamically).  The
@@ -537,7 +543,7 @@ __global__ void __launch_bounds__(kPairThreads, CLS ? 1 : 2) k_pair_packed(DevPt
   };
   // group t's copy has landed in buffer b: start the gathers of this lane's four entries
   auto fetch = [&](int t, int b, Gather4& G) {
-    if (!mbar_wait(&S.bar[b], (phase >> b) & 1u, wlim)) {
+    if (!mbar_wait_warp(&S.bar[b], (phase >> b) & 1u, wlim)) {
       ok = false;
       atomicOr(P.status, ERR_TIMEOUT);
       return;
@@ -597,7 +603,7 @@ __global__ void __launch_bounds__(kPairThreads, CLS ? 1 : 2) k_pair_packed(DevPt
     if (tn < TU) issue(tn, 1);
     fetch(t, 0, G);
   }
-  if (!mbar_wait(&s_tab_bar, 0u, wlim)) {
+  if (!mbar_wait_warp(&s_tab_bar, 0u, wlim)) {
     ok = false;
     atomicOr(P.status, ERR_TIMEOUT);
   }
@@ -890,7 +896,7 @@ k_pair_mixed(DevPtrs P, ZdConst z) {
   };
   // pair t's copy has landed in buffer b: start the gathers of this lane's two entries
   auto fetch = [&](int t, int b, Gather& G) {
-    if (!mbar_wait(&S.bar[b], (phase >> b) & 1u, wlim)) {
+    if (!mbar_wait_warp(&S.bar[b], (phase >> b) & 1u, wlim)) {
       ok = false;
       atomicOr(P.status, ERR_TIMEOUT);
       return;
