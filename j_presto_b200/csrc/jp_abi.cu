@@ -1608,7 +1608,7 @@ int jp_create(const jp_system *sys, int32_t nrep, const jp_params *prm, jp_ctx *
   e |= dalloc(c, &P.ct_j, rec_cap * 32);
   e |= dalloc(c, &P.ct_ty, rec_cap * 32);
   e |= dalloc(c, &P.ct_mask, rec_cap * kHalf);
-  e |= dalloc(c, &P.nctiles, 2);
+  e |= dalloc(c, &P.nctiles, 3);
   e |= dalloc(c, &P.ext_pos, 1);
   if (c->cmm) e |= dalloc(c, &P.ct_mask_el, rec_cap * kHalf);
   if (c->cmm) {

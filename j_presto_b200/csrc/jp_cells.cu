@@ -61,7 +61,7 @@ __global__ void k_list_reset(DevPtrs P, int nkeys, int nslot, int nrep, int dumm
     P.styp[i] = dummy_type;
   }
   if (i < 3 * nrep) P.rep_hmax[i] = 0.f;
-  if (i < 2) P.nctiles[i] = 0;
+  if (i < 3) P.nctiles[i] = 0;
   if (i == 0) *P.ext_pos = 0;
   if (i == 0 && hbond) *P.ntiles = 0;
 }
@@ -227,6 +227,7 @@ struct __align__(16) ListShared {
   int carry[8];                            // entries by half and kind
   int first[2][4];                         // a half's first entry of each kind
   int base[2];                             // of the records at the start and at the end
+  int nimg;                                // ALSD: records at the start whose pairs take their own images
   // ALSD: which of a window's records hold a class but BB, and each one's place
   unsigned char rcls[2 * kWindow];
   size_t rpos[2 * kWindow];
@@ -658,6 +659,7 @@ __global__ void __launch_bounds__(32 * kListWarps, CMM ? 3 : 4) k_block_list(Dev
     na0 = S.carry[2] + S.carry[3] > 0 ? nr0 - ((S.carry[0] + S.carry[1]) >> 5) : 0;
     na1 = (S.carry[6] + S.carry[7] + 31) >> 5;
   }
+  if (threadIdx.x == 0) S.nimg = 0;
   if (threadIdx.x < 2 && !split_cls) {
     const int na = na0 + na1;
     S.base[threadIdx.x] = atomicAdd(&P.nctiles[threadIdx.x], threadIdx.x ? na : nr0 + nr1 - na);
@@ -763,7 +765,12 @@ __global__ void __launch_bounds__(32 * kListWarps, CMM ? 3 : 4) k_block_list(Dev
 #pragma unroll
       for (int g = 0; g < 4; ++g) fl |= ((lj >> (8 * g)) & 0xffu) ? 0 : 1 << (kRecFree + g);
       if (lane == 0) P.ct_blk[ct] = (2 * bi + h) | fl;
+      if (lane == 0 && split_cls && any_img && !S.rcls[q]) atomicAdd(&S.nimg, 1);
     }
+  }
+  if (split_cls) {
+    __syncthreads();
+    if (threadIdx.x == 0 && S.nimg > 0) atomicAdd(&P.nctiles[2], S.nimg);
   }
 }
 

@@ -252,7 +252,8 @@ struct DevPtrs {
   float4 *ct_j;                   // [CT][32] (image shift into the i frame, atom bits; -1 = empty)
   unsigned short *ct_ty;          // [CT][32] type word of each entry (type_half; empty: dummy type)
   unsigned *ct_mask, *ct_mask_el; // [CT][32] rotated masks (listed pairs; CMM Coulomb pairs)
-  int *nctiles;                   // records from the start of the arrays, and (packed kernel) from their end
+  int *nctiles;                   // records from the start of the arrays, and (packed kernel) from their end;
+                                  // ALSD: of the first those whose pairs take their own images
   size_t rec_cap;                 // length of the record arrays
   // cell sort
   unsigned *key;                  // per atom

@@ -501,7 +501,9 @@ __global__ void __launch_bounds__(kPairThreads, CLS ? 1 : 2) k_pair_packed(DevPt
   const int U1 = (T1 + 3) >> 2;
   // the first record of group t's copies
   auto rec0 = [&](int t) { return t < U1 ? P.rec_cap - 4 * (size_t)(t + 1) : 4 * (size_t)(t - U1); };
-  const bool ext = (*P.ext_pos & kExtImg) != 0;
+  // every pair takes its own image: after replaced coordinates (below), or where most records need
+  // it and the others cannot stand apart (the ALSD records without classes): one form's code
+  const bool all_img = (*P.ext_pos & kExtImg) != 0 || 2 * (long long)P.nctiles[2] > T0;
   const int TU = U1 + ((T0 + 3) >> 2);   // record groups: a warp's work units
   // a 2.5-KiB copy lands in microseconds; the bound (about a second of SM clock) only ends
   // the wait on a broken device, and it is not the integrator's adjustable barrier bound:
@@ -670,7 +672,7 @@ __global__ void __launch_bounds__(kPairThreads, CLS ? 1 : 2) k_pair_packed(DevPt
     // Coordinates replaced without a build since may have moved farther than its margin: then
     // every pair takes its own, unless no box of the context can need it (k_update_pos).  One
     // form for the whole warp.
-    const bool wmi = ext || __any_sync(full, G.unit >= 0 && (G.unit & kRecImg));
+    const bool wmi = all_img || __any_sync(full, G.unit >= 0 && (G.unit & kRecImg));
     // (a record past the last one, -1, has every flag set)
     const unsigned ljg = (~__reduce_and_sync(full, (unsigned)G.unit) >> kRecFree) & 0xfu;
     __syncwarp();
